@@ -18,6 +18,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "advstencil.cuh"
 
 namespace {
 
@@ -104,15 +105,14 @@ MPASG_D T wduz_at(const T* __restrict__ u, T rwe, int kk, int L, const T* fzm, c
 // pv_edge * u at every edge level, the neighbour factor of the float64 PV flux sum (below),
 // formed once per tendency stage instead of once per reading edge; stored in ke_edge (the
 // diagnostics' edge kinetic-energy scratch, free between two diagnostics stages)
-template <typename T>
-__global__ void k_pvu(mpasg_mesh m, mpasg_fields f, long long n) {
+__global__ void k_pvu(mpasg_fields f, long long n) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  fpw<T>(f.ke_edge, f.ke_edge_f32)[i] = fp<T>(f.pv_edge, f.pv_edge_f32)[i] * fp<T>(f.u, f.u_f32)[i];
+  if (i < n) f.ke_edge[i] = f.pv_edge[i] * f.u[i];
 }
 
-// RAY: Rayleigh damping of u compiled in (a run-time test would cost float64 work in
-// every thread of the hot kernel once the compiler predicates it)
+// The mixed form's u tendency (T = float; the float64 form's is k_tend_u_fx).
+// RAY: Rayleigh damping of u compiled in (a run-time test would cost work in every thread
+// of the hot kernel once the compiler predicates it)
 template <typename T, bool RAY = false>
 __global__ void __launch_bounds__(kBlock) k_tend_u(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
   __shared__ T s_wd[kBlock];
@@ -151,35 +151,19 @@ __global__ void __launch_bounds__(kBlock) k_tend_u(mpasg_mesh m, mpasg_fields f,
   }
   T tu = -G(rdzw)[k] * (wd_k1 - wd_k);
   // nonlinear Coriolis / PV flux over the TRiSK stencil, sum_j w_j u_j 0.5 (pv_self + pv_j)
-  // over the slots in order.  float64: as 0.5 (pv_self sum_j w_j u_j + sum_j w_j (pv u)_j),
-  // two multiply-adds per neighbour on the float64 pipe that bounds the kernel, (pv u)
-  // formed once per edge level by k_pvu; float32: as written, the exact power-of-two
-  // factor 0.5 applied once to the sum (the extra pass would cost more than it saves)
+  // over the slots in order, the exact power-of-two factor 0.5 applied once to the sum
   const int n2 = m.nEdgesOnEdge[e];
   const int me2 = m.maxEdges2;
   const T* pv = fp<T>(f.pv_edge, f.pv_edge_f32);
   const T* woe = G(weightsOnEdge);
   const T pv_self = pv[i];
-  T q;
-  if constexpr (sizeof(T) == sizeof(double)) {
-    const double* pvu = f.ke_edge;
-    T sa = T(0), sb = T(0);
-    for (int j = 0; j < n2; ++j) {
-      const size_t io = (size_t)m.edgesOnEdge[e * me2 + j] * L + k;
-      const T w = woe[e * me2 + j];
-      sa = (j == 0) ? w * u[io] : sa + w * u[io];
-      sb = (j == 0) ? w * pvu[io] : sb + w * pvu[io];
-    }
-    q = T(0.5) * (pv_self * sa + sb);
-  } else {
-    q = T(0);
-    for (int j = 0; j < n2; ++j) {
-      int eo = m.edgesOnEdge[e * me2 + j];
-      T t = (woe[e * me2 + j] * u[(size_t)eo * L + k]) * (pv_self + pv[(size_t)eo * L + k]);
-      q = (j == 0) ? t : q + t;
-    }
-    q = T(0.5) * q;
+  T q = T(0);
+  for (int j = 0; j < n2; ++j) {
+    int eo = m.edgesOnEdge[e * me2 + j];
+    T t = (woe[e * me2 + j] * u[(size_t)eo * L + k]) * (pv_self + pv[(size_t)eo * L + k]);
+    q = (j == 0) ? t : q + t;
   }
+  q = T(0.5) * q;
   const size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2 * L + k;
   const T inv_dc = G(invDcEdge)[e];
   const T rho_e = cv<T>(f.h_edge[i]);
@@ -210,7 +194,8 @@ __global__ void __launch_bounds__(kBlock) k_tend_u(mpasg_mesh m, mpasg_fields f,
 // are independent, and the interface fluxes at k0 .. k0+V are computed in-thread (the
 // top one again by the next chunk).  Per level, the same expressions in the same order as
 // k_tend_u; the compiler may fuse multiply-adds differently in the two kernels, so the
-// tiles agree to the rounding of one FMA (last bit).
+// tiles agree to the rounding of one FMA (last bit).  Mixed form only: k_tend_u_fx has one
+// tile.
 template <typename T, int V, bool RAY = false>
 __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fields f, FastDiv flc, int nchunk,
                                                          TendScalars p) {
@@ -238,15 +223,12 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
   const int n2 = m.nEdgesOnEdge[e];
   const int me2 = m.maxEdges2;
   const T* pv = fp<T>(f.pv_edge, f.pv_edge_f32);
-  const T* pvu = fp<T>(f.ke_edge, f.ke_edge_f32);  // float64 only (k_tend_u)
   const T* woe = G(weightsOnEdge);
-  constexpr bool kSplit = sizeof(T) == sizeof(double);
-  T pv_self[V], sa[V], sb[V];
+  T pv_self[V], sa[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     pv_self[v] = (k0 + v < L) ? pv[(size_t)e * L + k0 + v] : T(0);
     sa[v] = T(0);
-    sb[v] = T(0);
   }
   for (int j = 0; j < n2; ++j) {
     const int eo = m.edgesOnEdge[e * me2 + j];
@@ -255,13 +237,8 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
     for (int v = 0; v < V; ++v) {
       if (k0 + v < L) {
         const size_t oo = (size_t)eo * L + k0 + v;
-        if (kSplit) {
-          sa[v] = (j == 0) ? w * u[oo] : sa[v] + w * u[oo];
-          sb[v] = (j == 0) ? w * pvu[oo] : sb[v] + w * pvu[oo];
-        } else {
-          const T t = (w * u[oo]) * (pv_self[v] + pv[oo]);
-          sa[v] = (j == 0) ? t : sa[v] + t;
-        }
+        const T t = (w * u[oo]) * (pv_self[v] + pv[oo]);
+        sa[v] = (j == 0) ? t : sa[v] + t;
       }
     }
   }
@@ -272,7 +249,7 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
     if (k >= L) break;
     const size_t ie = (size_t)e * L + k;
     T tu = -G(rdzw)[k] * ((k + 1 >= L ? T(0) : wd[v + 1]) - wd[v]);
-    const T qv = kSplit ? T(0.5) * (pv_self[v] * sa[v] + sb[v]) : T(0.5) * sa[v];
+    const T qv = T(0.5) * sa[v];
     const size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2 * L + k;
     const T rho_e = cv<T>(f.h_edge[ie]);
     tu = tu + rho_e * (qv - dif<T>(f.ke[i2], f.ke[i1]) * inv_dc) -
@@ -296,6 +273,147 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
       f.tend_u[ie] = f64(tu + cv<T>(f.tend_u_euler[ie]));
     }
   }
+}
+
+// ---------------------------------------------------------------- u tendency, float64 form
+// The PV flux sums of k_tend_u on the integer pipes (fixdot.cuh): sum_j w_j u_j and
+// sum_j w_j (pv u)_j over the TRiSK stencil were 20 of the ~44 float64 operations an edge level
+// issued on the pipe that bounded the kernel (82 % active, 14 % of the issue slots used).
+// 40962 x 55, a later RK stage: 628 us in float64, 359 us here (both sums on the integer
+// side; one of them in float64: 382 us), the first stage 970 -> 489 us.  48 registers (5 blocks
+// an SM): 346 us in a tuning loop against 593 us at 80 registers, 362 at 64 and 361 at 40, the
+// latency of 22 warps an SM being what held the 80-register build.
+// The block converts the weights of the 5-7 edges it covers once, into shared memory
+// (with the neighbour rows), so a term costs its thread one 16-byte broadcast and one gather.
+// The upwind combination of flux3 with coefficient 1 is a three-point formula,
+//   12 flux = (rw1 + rw2) (2 a + 5 b - c),  a / b downwind / upwind of the interface, c behind b,
+// so the vertical flux takes 4 float64 operations instead of 11.
+// N: slots a thread sums (unused slots hold zero weights); an edge with more than N
+// neighbours, and a sum the fixed-point format refuses, are summed in float64.
+
+// 12 times the vertical flux of u at interface kk; rw2 = rw1 + rw2 of the edge's two cells
+MPASG_D double wduz12_at(const double* __restrict__ u, double rw2, int kk, int L, const double* fzm,
+                         const double* fzp) {
+  if (kk <= 0 || kk >= L) return 0.0;
+  if (kk == 1 || kk == L - 1) return rw2 * (6.0 * (fzm[kk] * u[kk] + fzp[kk] * u[kk - 1]));
+  const bool down = __double2hiint(rw2) < 0;
+  const double a = u[down ? kk - 1 : kk], b = u[down ? kk : kk - 1], c = u[down ? kk + 1 : kk - 2];
+  return rw2 * fma(2.0, a, fma(5.0, b, -c));
+}
+
+// Per-edge constants of the u tendency, formed once per block and edge
+struct EdgeConst {
+  double inv_dc, inv_dc2;  // 1 / dc and 2 / dc
+  double r_dv, half_ms2;   // rk 1: min(1 / dv, 4 / dc), meshScalingDel2 / 2
+};
+
+// entries of the edges [e0, e0 + n) in the block's weight table
+template <int N>
+MPASG_D void load_trisk(const mpasg_mesh& m, uint32_t e0, uint32_t n, fx::Weight* tab, EdgeConst* ec) {
+  const int me2 = m.maxEdges2;
+  for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
+    const double idc = m.invDcEdge[e0 + t];
+    ec[t] = EdgeConst{idc, idc + idc, fmin(m.invDvEdge[e0 + t], 4.0 * idc), 0.5 * m.meshScalingDel2[e0 + t]};
+  }
+  for (uint32_t t = threadIdx.x; t < n * N; t += blockDim.x) {
+    const uint32_t el = t / N, j = t - el * N, e = e0 + el;
+    const int n2 = m.nEdgesOnEdge[e];
+    if ((int)j < n2 && n2 <= N) {
+      tab[t] = fx::weight(m.weightsOnEdge[e * me2 + j], m.edgesOnEdge[e * me2 + j]);
+    } else {
+      fx::Weight z{0, 0, n2 > N ? fx::kBadWeight : 0u, n2 > 0 ? m.edgesOnEdge[e * me2] : (int)e};
+      tab[t] = z;
+    }
+  }
+}
+
+template <int N>
+MPASG_D double trisk_sum(const mpasg_mesh& m, const double* __restrict__ field, const fx::Weight* w, uint32_t e,
+                         uint32_t k, uint32_t L) {
+  double x[N], out;
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = field[(uint32_t)w[j].row * L + k];
+  if (!fx::dot<N>(x, w, &out)) {
+    out = 0.0;
+    const size_t o = (size_t)e * m.maxEdges2;
+    for (int j = 0; j < m.nEdgesOnEdge[e]; ++j)
+      out = fma(m.weightsOnEdge[o + j], field[(size_t)m.edgesOnEdge[o + j] * L + k], out);
+  }
+  return out;
+}
+
+template <int N, bool RAY = false>
+__global__ void __launch_bounds__(kBlock, 5) k_tend_u_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
+  extern __shared__ fx::Weight s_w[];
+  __shared__ double s_wd[kBlock];
+  const uint32_t L = (uint32_t)m.nVertLevels;
+  const uint32_t n_all = (uint32_t)m.nEdges * L;
+  const double* __restrict__ u = f.u;
+  const double* __restrict__ rw = f.rw;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t e0 = fl.div(i0), e1 = fl.div(min(i0 + kBlock, n_all) - 1u);
+  EdgeConst* s_e = reinterpret_cast<EdgeConst*>(s_w + (kBlock - 1 + 2 * L) / L * N);
+  load_trisk<N>(m, e0, e1 - e0 + 1, s_w, s_e);
+  const bool active = i < n_all;
+  uint32_t e = e0, k = 0;
+  int c1 = 0, c2 = 0;
+  const double* ue = u;
+  double wd_k = 0.0;
+  if (active) {
+    e = fl.div(i);
+    k = i - e * L;
+    c1 = m.cellsOnEdge[2 * e];
+    c2 = m.cellsOnEdge[2 * e + 1];
+    ue = u + (size_t)e * L;
+    wd_k = wduz12_at(ue, rw[(size_t)c1 * (L + 1) + k] + rw[(size_t)c2 * (L + 1) + k], k, L, m.fzm, m.fzp);
+  }
+  s_wd[threadIdx.x] = wd_k;  // vertical flux at the interface below level k
+  __syncthreads();
+  if (!active) return;
+  double wd_k1 = 0.0;
+  if (k + 1 < L)
+    wd_k1 = threadIdx.x + 1 < kBlock
+                ? s_wd[threadIdx.x + 1]  // same edge, next level
+                : wduz12_at(ue, rw[(size_t)c1 * (L + 1) + k + 1] + rw[(size_t)c2 * (L + 1) + k + 1], k + 1, L, m.fzm,
+                            m.fzp);
+  const fx::Weight* w = s_w + (e - e0) * N;
+  const EdgeConst ec = s_e[e - e0];
+  const double sa = trisk_sum<N>(m, u, w, e, k, L);
+  const double sb = trisk_sum<N>(m, f.ke_edge, w, e, k, L);  // pv u (k_pvu)
+  const size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2 * L + k;
+  const double rho_e = f.h_edge[i], u_k = ue[k];
+  const double pv = fma(f.pv_edge[i], sa, sb);  // twice the PV flux
+  // 0.5 (rho_e (pv - 2 dke / dc) - u (hdiv_1 + hdiv_2)), the exact factors of two outside
+  const double g = fma(f.ke[i1] - f.ke[i2], ec.inv_dc2, pv);
+  const double br = fma(rho_e, g, -(u_k * (f.h_divergence[i1] + f.h_divergence[i2])));
+  double tu = fma(0.5, br, (m.rdzw[k] * kInv12) * (wd_k - wd_k1));
+  if (RAY) tu = rayleigh_u<double>(tu, rho_e, u_k, (int)k, (int)L, p);
+  if (p.rk_step == 1) {
+    double grad = (f.pressure_p[i2] - f.pressure_p[i1]) * ec.inv_dc;
+    const double z2 = m.zz[i2] + m.zz[i1];
+    if (!fx::is_two(z2)) grad = grad / (0.5 * z2);
+    if (!m.flatTerrain) grad = fma(-0.5 * m.zxu[i], f.dpdz[i1] + f.dpdz[i2], grad);
+    const int v1 = m.verticesOnEdge[2 * e], v2 = m.verticesOnEdge[2 * e + 1];
+    const double u_diff = (f.divergence[i2] - f.divergence[i1]) * ec.inv_dc -
+                          (f.vorticity[(size_t)v2 * L + k] - f.vorticity[(size_t)v1 * L + k]) * ec.r_dv;
+    f.delsq_u[i] = u_diff;
+    const double mix = (rho_e * (f.kdiff[i1] + f.kdiff[i2])) * (u_diff * ec.half_ms2);
+    const double teu = fma(-f.cqu_e[i], grad, mix);
+    f.tend_u_euler[i] = teu;
+    f.tend_u[i] = p.defer ? tu : tu + teu;
+  } else {
+    f.tend_u[i] = tu + f.tend_u_euler[i];
+  }
+}
+
+template <bool RAY>
+void launch_tend_u_fx(const mpasg_mesh* m, const mpasg_fields* f, const TendScalars& p, cudaStream_t s) {
+  const int L = m->nVertLevels;
+  const int nb = nblocks((long long)m->nEdges * L), ne = (kBlock - 1) / L + 2;
+  if (m->maxEdges2 <= 10)
+    k_tend_u_fx<10, RAY><<<nb, kBlock, ne * (10 * sizeof(fx::Weight) + sizeof(EdgeConst)), s>>>(*m, *f, FastDiv(L), p);
+  else
+    k_tend_u_fx<14, RAY><<<nb, kBlock, ne * (14 * sizeof(fx::Weight) + sizeof(EdgeConst)), s>>>(*m, *f, FastDiv(L), p);
 }
 
 template <typename T>
@@ -568,6 +686,35 @@ __global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   }
 }
 
+// The float64 form: the theta sum on the integer pipes, the w sum on the float64 pipe, so
+// that both are busy (two sums of ~10 terms are all this kernel does; both in float64 bound it
+// at 82 % of that pipe).  40962 x 55: 374 us in float64 alone, 271 us with both sums
+// on the integer side, 216 us with one each.
+template <int N>
+__global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
+  extern __shared__ fx::Weight s_w[];
+  const uint32_t L = (uint32_t)m.nVertLevels;
+  const uint32_t n_all = (uint32_t)m.nEdges * L;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t e0 = fl.div(i0), e1 = fl.div(min(i0 + kBlock, n_all) - 1u);
+  adv::load<N>(m, e0, e1 - e0 + 1, s_w);
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t e = fl.div(i), k = i - e * L;
+  const double rue = f.ru[i];
+  const bool back = __double2hiint(rue) < 0;
+  const fx::Weight* w = s_w + (e - e0) * (2 * N) + (back ? N : 0);
+  double x[N], th;
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = f.theta_m[(uint32_t)w[j].row * L + k];
+  if (!fx::dot<N>(x, w, &th)) th = adv::sum(m, e, back, f.theta_m, L, k);
+  f.flux_th_e[i] = rue * th;
+  if (k >= 1) {
+    const double ru_w = fma(m.fzm[k], rue, m.fzp[k] * f.ru[i - 1]);
+    f.flux_w_e[i] = ru_w * adv::sum(m, e, __double2hiint(ru_w) < 0, f.w, L + 1, k);
+  }
+}
+
 // w and theta tendencies (float64 form); index space (C, L+1)
 __global__ void __launch_bounds__(kBlock) k_tend_w_theta(mpasg_mesh m, mpasg_fields f, FastDiv fl1, TendScalars p) {
   using T = double;
@@ -819,19 +966,20 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
   else
     k_tend_cells_a<T><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
   MPASG_LAUNCH_CHECK();
-  if (sizeof(T) == sizeof(double)) {  // the float64 PV flux reads pv_edge * u (k_tend_u)
-    k_pvu<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, nel);
-    MPASG_LAUNCH_CHECK();
-  }
-  const int vt = tile_levels(c_tile);  // levels per thread of k_tend_u (autotuner choice)
   const bool ray = p.ray_n > 0;
-  if (vt == 1) {
-    if (ray) k_tend_u<T, true><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
-    else k_tend_u<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    k_pvu<<<nblocks(nel), kBlock, 0, s>>>(*f, nel);
+    MPASG_LAUNCH_CHECK();
+    if (ray) launch_tend_u_fx<true>(m, f, p, s);
+    else launch_tend_u_fx<false>(m, f, p, s);
   } else {
+    const int vt = tile_levels(c_tile);  // levels per thread of k_tend_u (autotuner choice)
     const int nchunk = (L + vt - 1) / vt;
     const long long nth = (long long)m->nEdges * nchunk;
-    if (vt == 2) {
+    if (vt == 1) {
+      if (ray) k_tend_u<T, true><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
+      else k_tend_u<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
+    } else if (vt == 2) {
       if (ray) k_tend_u_chunk<T, 2, true><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
       else k_tend_u_chunk<T, 2><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
     } else {
@@ -860,7 +1008,13 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
       MPASG_LAUNCH_CHECK();
     }
   }
-  k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const size_t smem = (size_t)((kBlock - 1) / L + 2) * adv::kEntryBytes;
+    if (m->nAdvMax <= 10) k_adv_edges_fx<10><<<nblocks(nel), kBlock, smem * 10, s>>>(*m, *f, fl);
+    else k_adv_edges_fx<14><<<nblocks(nel), kBlock, smem * 14, s>>>(*m, *f, fl);
+  } else {
+    k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl);
+  }
   MPASG_LAUNCH_CHECK();
   if (sizeof(T) == sizeof(double))
     k_tend_w_theta<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1, p);
@@ -938,7 +1092,7 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
 
 // Autotuner: times the u-tendency kernel with 1, 2 and 4 levels per thread on the current
 // state (rk-2 form, 3 launches each after one warm-up) and keeps the fastest in
-// c->tile_tend_u.  Host-synchronising: call it outside stream capture.  The kernels only
+// c->tile_tend_u.  (The float64 form has one tile: its three candidates are the same kernel.)  Host-synchronising: call it outside stream capture.  The kernels only
 // write their outputs (tend_u, ...) and the ke_edge scratch, so the state is unchanged.
 extern "C" int mpasg_autotune(const mpasg_mesh* m, mpasg_config* c, mpasg_fields* f, float* times_ms,
                               void* stream) {
@@ -957,7 +1111,7 @@ extern "C" int mpasg_autotune(const mpasg_mesh* m, mpasg_config* c, mpasg_fields
   cudaEvent_t a, b;
   if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) return MPASG_E_CUDA;
   if (!mixed) {
-    k_pvu<double><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, nel);
+    k_pvu<<<nblocks(nel), kBlock, 0, s>>>(*f, nel);
     mpasg_count_launch();
     if (cudaGetLastError() != cudaSuccess) return MPASG_E_LAUNCH;
   }
@@ -972,16 +1126,10 @@ extern "C" int mpasg_autotune(const mpasg_mesh* m, mpasg_config* c, mpasg_fields
     float ms = 0.0f;
     for (int rep = 0; rep < 4; ++rep) {
       if (rep == 1) cudaEventRecord(a, s);
-      if (vt == 1) {
-        if (mixed) k_tend_u<float><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, FastDiv(L), p);
-        else k_tend_u<double><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, FastDiv(L), p);
-      } else if (vt == 2) {
-        if (mixed) k_tend_u_chunk<float, 2><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
-        else k_tend_u_chunk<double, 2><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
-      } else {
-        if (mixed) k_tend_u_chunk<float, 4><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
-        else k_tend_u_chunk<double, 4><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
-      }
+      if (!mixed) launch_tend_u_fx<false>(m, f, p, s);
+      else if (vt == 1) k_tend_u<float><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, FastDiv(L), p);
+      else if (vt == 2) k_tend_u_chunk<float, 2><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
+      else k_tend_u_chunk<float, 4><<<nblocks(nth), kBlock, 0, s>>>(*m, *f, FastDiv(nchunk), nchunk, p);
       mpasg_count_launch();
       if (cudaGetLastError() != cudaSuccess) rc = MPASG_E_LAUNCH;
     }

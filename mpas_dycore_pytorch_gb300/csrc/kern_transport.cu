@@ -4,7 +4,7 @@
 // bounds autodiff/soft_limiter.py:72).  Scalar fields are (C+1, L, S), edge fluxes (E+1, L, S).
 #include <mutex>
 
-#include "common.cuh"
+#include "advstencil.cuh"
 
 namespace {
 
@@ -36,6 +36,57 @@ __global__ void k_pattern_c(mpasg_mesh m, FastDiv fl, int S, const double* __res
     }
   }
   for (int s = 0; s < S; ++s) out[(size_t)i * S + s] = f64(times_uh ? u * acc[s] : acc[s]);
+}
+
+// The float64 form.  A row of an edge, its (level, scalar) values in memory order, is cut in
+// two halves and a thread takes the same place of both: the first half's sum on the integer
+// pipes (fixdot.cuh), the second's on the float64 pipe beside it, so both are busy, and
+// neighbouring threads read neighbouring values.  Weights are converted once per block and edge.
+// 40962 x 55 with 3 tracers: 392 -> 363 us; 2562 x 37 with 8: 73 -> 47 us (48 registers; with
+// the two sums of a thread interleaved instruction by instruction 481 and 62 us, the
+// registers costing more warps than the overlap inside a warp gives).
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_pattern_c_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t n_all,
+                                                            uint32_t half, const double* __restrict__ uh,
+                                                            const double* __restrict__ q, double* __restrict__ out,
+                                                            int times_uh) {
+  extern __shared__ fx::Weight s_w[];
+  const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t e0 = fh.div(i0), e1 = fh.div(min(i0 + kBlock, n_all) - 1u);
+  adv::load<N>(m, e0, e1 - e0 + 1, s_w);
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t e = fh.div(i), a = i - e * half, b = a + half;
+  const fx::Weight* w = s_w + (e - e0) * (2 * N);
+  double* o = out + (size_t)e * row;
+  double x[N], acc;
+  const double ua = uh[(size_t)e * L + fs.div(a)];
+  const bool back = __double2hiint(ua) < 0;
+  if (back) w += N;
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = q[(size_t)w[j].row * row + a];
+  if (b < row) {
+    const double ub = uh[(size_t)e * L + fs.div(b)];
+    const double t = adv::sum(m, e, __double2hiint(ub) < 0, q, row, b);
+    o[b] = times_uh ? ub * t : t;
+  }
+  if (!fx::dot<N>(x, w, &acc)) acc = adv::sum(m, e, back, q, row, a);
+  o[a] = times_uh ? ua * acc : acc;
+}
+
+int launch_pattern_c_fx(const mpasg_mesh* m, int S, const double* uh, const double* q, double* out, int times_uh,
+                        cudaStream_t s) {
+  const uint32_t half = ((uint32_t)m->nVertLevels * S + 1) / 2, n = (uint32_t)m->nEdges * half;
+  const size_t smem = (size_t)((kBlock - 1) / half + 2) * adv::kEntryBytes;
+  if (m->nAdvMax <= 10)
+    k_pattern_c_fx<10><<<nblocks(n), kBlock, smem * 10, s>>>(*m, FastDiv(half), FastDiv(S), n, half, uh, q, out,
+                                                             times_uh);
+  else
+    k_pattern_c_fx<14><<<nblocks(n), kBlock, smem * 14, s>>>(*m, FastDiv(half), FastDiv(S), n, half, uh, q, out,
+                                                             times_uh);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
 }
 
 template <typename T>
@@ -372,8 +423,13 @@ int launch_scalars(const mpasg_mesh* m, const mpasg_config* c, const mpasg_field
   FastDiv fl(L);
   mpasg_fields g = *f;
   g.hflux = hflux;
-  k_pattern_c<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, fl, S, g.ruAvg, g.scalars_a, hflux, 0);
-  MPASG_LAUNCH_CHECK();
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const int rc = launch_pattern_c_fx(m, S, g.ruAvg, g.scalars_a, hflux, 0, s);
+    if (rc != MPASG_OK) return rc;
+  } else {
+    k_pattern_c<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, fl, S, g.ruAvg, g.scalars_a, hflux, 0);
+    MPASG_LAUNCH_CHECK();
+  }
   // density weights: advanced with the stage in the split transport loop; the stage's
   // new density in the coupled mode (one dynamics substep, time_integration.py:7930-8200)
   double w_old, w_new;
@@ -390,8 +446,13 @@ int launch_scalars_mono(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields
   const int L = m->nVertLevels, S = c->num_scalars;
   FastDiv fl(L);
   const long long nel = (long long)m->nEdges * L, ncl = (long long)m->nCells * L;
-  k_pattern_c<T><<<nblocks(nel), kBlock, 0, s>>>(*m, fl, S, f->ruAvg, f->scalars_a, f->hflux, 1);
-  MPASG_LAUNCH_CHECK();
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const int rc = launch_pattern_c_fx(m, S, f->ruAvg, f->scalars_a, f->hflux, 1, s);
+    if (rc != MPASG_OK) return rc;
+  } else {
+    k_pattern_c<T><<<nblocks(nel), kBlock, 0, s>>>(*m, fl, S, f->ruAvg, f->scalars_a, f->hflux, 1);
+    MPASG_LAUNCH_CHECK();
+  }
   k_mono_cells_a<T><<<nblocks(ncl), kBlock, kBlock * 2 * S * sizeof(T), s>>>(*m, *f, fl, S, dt_stage,
                                                                           c->coef_3rd_order, f->scalars_init,
                                                                           f->scalars_a);
