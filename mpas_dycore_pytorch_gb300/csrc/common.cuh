@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fastdiv64.cuh"
 #include "mpasg.h"
 
 #define MPASG_HD __host__ __device__ __forceinline__
@@ -100,10 +101,16 @@ MPASG_D double rcp_nr1(double d) {
   double x = f2d_bits(1.0f / d2f_bits(d));
   return fma(x, fma(-d, x, 1.0), x);
 }
-// a / b of float64 operands: the division in the float64 form, a * rcp_nr(b) in the
-// mixed form (within 2 ulp)
+// a / b of float64 operands: the rounded quotient in the float64 form (fastdiv64.cuh),
+// a * rcp_nr(b) in the mixed form (within 2 ulp)
 template <typename T> MPASG_D double fdiv(double a, double b) { return a * rcp_nr(b); }
-template <> MPASG_D double fdiv<double>(double a, double b) { return a / b; }
+template <> MPASG_D double fdiv<double>(double a, double b) { return fx::quotient(a, b); }
+
+// 1 / b: the rounded reciprocal (fastdiv64.cuh), rcp_nr(b) in the mixed form
+template <typename T> MPASG_D double recip(double b) { return rcp_nr(b); }
+template <> MPASG_D double recip<double>(double b) { return fx::rcp(b); }
+MPASG_D bool is_two(double x) { return fx::is_two(x); }
+MPASG_D bool is_two(float x) { return x == 2.0f; }
 
 // unfused (separately rounded) products and differences for cancellation-prone terms
 MPASG_D double mul_rn(double a, double b) { return __dmul_rn(a, b); }

@@ -51,6 +51,7 @@ FX_HD double from_bits(uint64_t b) {
 #endif
 }
 // tests of exact values on the integer side (a float64 compare costs a float64 slot)
+FX_HD bool is_zero(double x) { return (bits_of(x) << 1) == 0u; }
 FX_HD bool is_one(double x) { return bits_of(x) == 0x3ff0000000000000ull; }
 FX_HD bool is_two(double x) { return bits_of(x) == 0x4000000000000000ull; }
 FX_HD int clz64(uint64_t x) {  // x != 0

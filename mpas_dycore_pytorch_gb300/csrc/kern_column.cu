@@ -52,36 +52,54 @@ struct VimpLevel {
   double cofwt, coftz;
 };
 
-// (float64 in both forms; T selects the division: exact in the float64 form, Newton
-// reciprocal in the mixed form)
+// Products of the stage's scalars, formed once on the host (a thread would spend float64
+// operations on each): the reference's leading factors in its own association.
+struct VimpScalars {
+  double dtseps;  // 0.5 dts (1 + epssm)
+  double cw;      // 0.5 dtseps R/cv
+  double cg;      // 0.5 dtseps g
+  double c2;      // dtseps cp R/cv
+  double cm;      // mixed form: dtseps (0.5 R/cv g)
+};
+inline VimpScalars vimp_scalars(double dts, double epssm) {
+  const double rcv = kRgas / (kCp - kRgas);
+  VimpScalars p;
+  p.dtseps = 0.5 * dts * (1.0 + epssm);
+  p.cw = 0.5 * p.dtseps * rcv;
+  p.cg = 0.5 * p.dtseps * kGravity;
+  p.c2 = p.dtseps * (kCp * rcv);
+  p.cm = p.dtseps * (0.5 * rcv * kGravity);
+  return p;
+}
+
+// (float64 in both forms; T selects the division: the rounded quotient in the float64 form,
+// Newton reciprocal in the mixed form)
 template <typename T>
-MPASG_D VimpLevel vimp_level(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, int k,
-                             double dtseps, double rcv) {
+MPASG_D VimpLevel vimp_level(const mpasg_mesh& m, const mpasg_fields& f, size_t o, int k, const VimpScalars& s) {
   VimpLevel v;
   double zz = m.zz[o + k], p = f.exner[o + k];
   double rb = m.rho_base[o + k], rtb = f.rtheta_base[o + k], pb = f.exner_base[o + k];
   double rt = f.rtheta_p[o + k], q = f.qtot[o + k];
+  const bool dry = fx::is_zero(q);  // x / (1 + q) is x itself: the division is skipped, not changed
   if (sizeof(T) == sizeof(double)) {
-    // x / (1 + q) is x itself when q == 0 (dry columns): the division is skipped, not changed
-    const double x = 0.5 * dtseps * rcv * zz * kGravity * rb;
-    v.cofwt = fdiv<T>((q == 0.0 ? x : fdiv<T>(x, 1.0 + q)) * p, (rtb + rt) * pb);
+    const double x = s.cw * zz * kGravity * rb;
+    v.cofwt = fdiv<T>((dry ? x : fdiv<T>(x, 1.0 + q)) * p, (rtb + rt) * pb);
+  } else {  // constants folded into one factor
+    const double x = s.cm * zz * rb;
+    v.cofwt = (dry ? x : fdiv<T>(x, 1.0 + q)) * p * rcp_nr((rtb + rt) * pb);
   }
-  else {  // mixed form: the dry case needs no 1 / (1 + q); constants folded into one factor
-    const double x = (dtseps * (0.5 * rcv * kGravity)) * zz * rb;
-    v.cofwt = (q == 0.0 ? x : fdiv<T>(x, 1.0 + q)) * p * rcp_nr((rtb + rt) * pb);
-  }
-  v.coftz = (k == 0) ? 0.0 : dtseps * (m.fzm[k] * f.theta_m[o + k] + m.fzp[k] * f.theta_m[o + k - 1]);
+  v.coftz = (k == 0) ? 0.0 : s.dtseps * (m.fzm[k] * f.theta_m[o + k] + m.fzp[k] * f.theta_m[o + k - 1]);
   return v;
 }
 
+// Bound by the float64 pipe: 63 operations a level with two divisions in the reference's
+// expressions, 40 with the scalars' products formed on the host, the quotient of
+// fastdiv64.cuh and the common factors taken out of the diagonals (fewer roundings each):
+// 263 -> 193 us at 40962 x 55.
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_fields f, FastDiv fl, double dts,
-                                                       double epssm) {
+__global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_fields f, FastDiv fl, VimpScalars s) {
   __shared__ double s_cw[kBlock], s_ct[kBlock];
   const int L = m.nVertLevels;
-  const double dtseps = 0.5 * dts * (1.0 + epssm);
-  const double rcv = kRgas / (kCp - kRgas);
-  const double c2 = kCp * rcv;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = i < (uint32_t)m.nCells * L;
   uint32_t c = 0, k = 0;
@@ -92,8 +110,8 @@ __global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_field
     k = i - c * L;
     o = (size_t)c * L;
     ow = (size_t)c * (L + 1);
-    me_ = vimp_level<T>(m, f, o, ow, k, dtseps, rcv);
-    if (c == 0) f.cofrz[k] = dtseps * m.rdzw[k];
+    me_ = vimp_level<T>(m, f, o, k, s);
+    if (c == 0) f.cofrz[k] = s.dtseps * m.rdzw[k];
   }
   s_cw[threadIdx.x] = me_.cofwt;
   s_ct[threadIdx.x] = me_.coftz;
@@ -112,35 +130,28 @@ __global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_field
   }
   const double zz = m.zz[o + k], zzm = m.zz[o + k - 1];
   const double fzm = m.fzm[k], fzp = m.fzp[k];
-  const double cofwr = 0.5 * dtseps * kGravity * (fzm * zz + fzp * zzm);
   const double z_i = fzm * zz + fzp * zzm;
+  const double cofwr = s.cg * z_i;
   const double p_i = fzm * f.exner[o + k] + fzp * f.exner[o + k - 1];
-  const double cofwz = dtseps * c2 * z_i * m.rdzu[k] * f.cqw[ow + k] * p_i;
+  const double cofwz = s.c2 * z_i * m.rdzu[k] * f.cqw[ow + k] * p_i;
   f.cofwr[o + k] = cofwr;
   f.cofwz[o + k] = cofwz;
   // neighbour levels (k-1 below, k+1 above) from shared memory or recomputed at block edges
   VimpLevel lo = (threadIdx.x >= 1) ? VimpLevel{s_cw[threadIdx.x - 1], s_ct[threadIdx.x - 1]}
-                                    : vimp_level<T>(m, f, o, ow, k - 1, dtseps, rcv);
+                                    : vimp_level<T>(m, f, o, k - 1, s);
   double ct_kp1 = 0.0;
   if (k + 1 < (uint32_t)L)
-    ct_kp1 = (threadIdx.x + 1 < blockDim.x) ? s_ct[threadIdx.x + 1]
-                                            : vimp_level<T>(m, f, o, ow, k + 1, dtseps, rcv).coftz;
+    ct_kp1 = (threadIdx.x + 1 < blockDim.x) ? s_ct[threadIdx.x + 1] : vimp_level<T>(m, f, o, k + 1, s).coftz;
   const double ct_km1 = lo.coftz, ct_k = me_.coftz;
   const double cw_k = me_.cofwt, cw_km1 = lo.cofwt;
   const double rdzw_k = m.rdzw[k], rdzw_km1 = m.rdzw[k - 1];
-  const double cofrz_k = dtseps * rdzw_k, cofrz_km1 = dtseps * rdzw_km1;
-  if (sizeof(T) == sizeof(double)) {  // the reference's expressions (vert_imp_coefs.py:388-428)
-    f.a_tri[o + k] = -cofwz * ct_km1 * rdzw_km1 * zzm + cofwr * cofrz_km1 - cw_km1 * ct_km1 * rdzw_km1;
-    f.b_tri[o + k] = 1.0 + cofwz * (ct_k * rdzw_k * zz + ct_k * rdzw_km1 * zzm) -
-                     ct_k * (cw_k * rdzw_k - cw_km1 * rdzw_km1) + cofwr * (cofrz_k - cofrz_km1);
-    f.c_tri[o + k] = -cofwz * ct_kp1 * rdzw_k * zz - cofwr * cofrz_k + cw_k * ct_kp1 * rdzw_k;
-  } else {  // mixed form: the same float64 coefficients with the common factors taken out
-    const double tm = ct_km1 * rdzw_km1, tp = ct_kp1 * rdzw_k;
-    f.a_tri[o + k] = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
-    f.b_tri[o + k] = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
-                     cofwr * (cofrz_k - cofrz_km1);
-    f.c_tri[o + k] = tp * (cw_k - cofwz * zz) - cofwr * cofrz_k;
-  }
+  const double cofrz_k = s.dtseps * rdzw_k, cofrz_km1 = s.dtseps * rdzw_km1;
+  // the reference's coefficients (vert_imp_coefs.py:388-428) with their common factors taken out
+  const double tm = ct_km1 * rdzw_km1, tp = ct_kp1 * rdzw_k;
+  f.a_tri[o + k] = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
+  f.b_tri[o + k] = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
+                   cofwr * (cofrz_k - cofrz_km1);
+  f.c_tri[o + k] = fma(cw_k, tp, -fma(cofwz * zz, tp, cofwr * cofrz_k));
 }
 
 template <typename T>
@@ -153,7 +164,7 @@ __global__ void k_vimp_factor(mpasg_mesh m, mpasg_fields f) {
   f.alpha_tri[o] = 0.0;
   f.gamma_tri[o] = 0.0;
   for (int k = 1; k < L; ++k) {
-    double alpha = fdiv<T>(1.0, f.b_tri[o + k] - f.a_tri[o + k] * gam);
+    double alpha = recip<T>(f.b_tri[o + k] - f.a_tri[o + k] * gam);
     gam = f.c_tri[o + k] * alpha;
     f.alpha_tri[o + k] = alpha;
     f.gamma_tri[o + k] = gam;
@@ -172,21 +183,26 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
   uint32_t e = fl.div(i), k = i - e * L;
+  constexpr bool kDouble = sizeof(T) == sizeof(double);
+  double rup;
   if (small_step != 1) {
     int c1 = m.cellsOnEdge[2 * e], c2i = m.cellsOnEdge[2 * e + 1];
     size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2i * L + k;
-    T pgrad = div_or_one<T>((cv<T>(f.rtheta_pp[i2]) - cv<T>(f.rtheta_pp[i1])) * cv<T>(m.invDcEdge[e]),
-                            T(0.5) * (cv<T>(m.zz[i2]) + cv<T>(m.zz[i1])));
-    pgrad = cv<T>(f.cqu_e[i]) * T(0.5) * cv<T>(c2) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
-    pgrad = pgrad + T(0.5) * cv<T>(m.zxu[i]) * T(kGravity) * (cv<T>(f.rho_pp[i1]) + cv<T>(f.rho_pp[i2]));
-    double rup = f.ru_p[i] + f64(cv<T>(dts) * (cv<T>(f.tend_u[i]) - pgrad));
-    f.ru_p[i] = rup;
+    T pgrad = (cv<T>(f.rtheta_pp[i2]) - cv<T>(f.rtheta_pp[i1])) * cv<T>(m.invDcEdge[e]);
+    const T z2 = cv<T>(m.zz[i2]) + cv<T>(m.zz[i1]);
+    if (!is_two(z2)) pgrad = pgrad / (T(0.5) * z2);
+    pgrad = cv<T>(f.cqu_e[i]) * (T(0.5) * cv<T>(c2)) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
+    if (!m.flatTerrain)  // no slope: adds exact zeros
+      pgrad = pgrad + T(0.5) * cv<T>(m.zxu[i]) * T(kGravity) * (cv<T>(f.rho_pp[i1]) + cv<T>(f.rho_pp[i2]));
+    rup = f.ru_p[i] + f64(cv<T>(dts) * (cv<T>(f.tend_u[i]) - pgrad));
     f.ruAvg[i] = f.ruAvg[i] + rup;
   } else {
-    double rup = f64(cv<T>(dts) * cv<T>(f.tend_u[i]));
-    f.ru_p[i] = rup;
+    rup = f64(cv<T>(dts) * cv<T>(f.tend_u[i]));
     f.ruAvg[i] = rup;
   }
+  f.ru_p[i] = rup;
+  // the theta flux of both adjacent cells' sums, once per edge (ke_edge: scratch here)
+  if (kDouble) f.ke_edge[i] = rup * f.theta_edge_save[i];
 }
 
 // ---------------------------------------------------------------- acoustic substep, columns
@@ -196,50 +212,6 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
 // parallel: flux sums, rs / ts, tridiagonal right-hand side), k_ac_thomas (one thread
 // per column: forward elimination and back substitution only) and k_ac_post (every
 // level in parallel: Rayleigh damping, ww accumulation, rho_pp / rtheta_pp update).
-
-// rs / ts of one level before the implicit solve (acoustic_step.py :456, :675 first half)
-struct AcLevel {
-  double rs, ts, rho_in, rt_in;
-};
-
-// The horizontal flux sums (and dts times the tendencies) are formed in the stencil
-// type T; the right-hand side combines them with the implicit coefficients in float64.
-template <typename T>
-MPASG_D AcLevel ac_level(const mpasg_mesh& m, const mpasg_fields& f, int c, int k, bool first, double dts,
-                         double resm) {
-  const int L = m.nVertLevels;
-  const int me = m.maxEdges;
-  const int n = m.nEdgesOnCell[c];
-  const T dts_t = cv<T>(dts);
-  // sign * dvEdge * invAreaCell per slot (mesh constant) and the edge mean of the
-  // time-level-1 theta_m (formed once per dynamics substep by k_theta_edge): four float64
-  // operations per edge instead of eight
-  const double* geo = m.cell_edge_geo + (size_t)c * me;
-  T rs = T(0), ts = T(0);
-  for (int j = 0; j < n; ++j) {
-    int e = m.edgesOnCell[c * me + j];
-    T flux = (dts_t * cv<T>(geo[j])) * cv<T>(f.ru_p[(size_t)e * L + k]);
-    T th_e = cv<T>(f.theta_edge_save[(size_t)e * L + k]);
-    if (j == 0) {
-      rs = -flux;
-      ts = -(flux * th_e);
-    } else {
-      rs = rs + (-flux);
-      ts = ts + (-(flux * th_e));
-    }
-  }
-  const size_t o = (size_t)c * L + k;
-  const size_t ow = (size_t)c * (L + 1) + k;
-  AcLevel a;
-  a.rho_in = first ? 0.0 : f.rho_pp[o];
-  a.rt_in = first ? 0.0 : f.rtheta_pp[o];
-  double rwp_k = first ? 0.0 : f.rw_p[ow];
-  double rwp_k1 = first ? 0.0 : f.rw_p[ow + 1];
-  a.rs = a.rho_in + f64(dts_t * cv<T>(f.tend_rho[o])) + f64(rs) - f.cofrz[k] * resm * (rwp_k1 - rwp_k);
-  a.ts = a.rt_in + f64(dts_t * cv<T>(f.tend_theta[o])) + f64(ts) -
-         resm * m.rdzw[k] * (f.coftz[ow + 1] * rwp_k1 - f.coftz[ow] * rwp_k);
-  return a;
-}
 
 // edge mean of theta_m_save, 0.5 (theta_2 + theta_1), the value the acoustic right-hand
 // side takes per edge, and the reciprocal of the sum that divergence damping divides by
@@ -256,49 +228,123 @@ __global__ void k_theta_edge(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const double sum = f.theta_m_save[(size_t)c2 * L + k] + f.theta_m_save[(size_t)c1 * L + k];
   f.theta_edge_save[i] = 0.5 * sum;
   // divergence damping multiplies instead of dividing
-  f.theta_edge_rsum[i] = MIXED ? f2d_bits(1.0f / d2f_bits(sum)) : 1.0 / sum;
+  f.theta_edge_rsum[i] = MIXED ? f2d_bits(1.0f / d2f_bits(sum)) : fx::rcp(sum);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kBlock) k_ac_prep(mpasg_mesh m, mpasg_fields f, FastDiv fl1, int small_step,
-                                                    double dts, double epssm, double resm) {
-  __shared__ AcLevel s_lv[kBlock];
-  const int L = m.nVertLevels;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i < (uint32_t)m.nCells * (L + 1);
-  const bool first = (small_step == 1);
-  uint32_t c = 0, k = 0;
+// Right-hand sides of the float64 form.  With S1 = sum_j geo_j ru_p_j, S2 = sum_j geo_j (ru_p
+// theta)_j over a cell's edges (geo = sign dvEdge / areaCell),
+//   rs = rho_pp + dts (tend_rho - S1) - resm cofrz d(rw_p),       R = rs + resm rho_pp
+//   ts = rtheta_pp + dts (tend_theta - S2) - resm rdzw d(coftz rw_p),  P = ts + resm rtheta_pp
+//   x  = rw_p + dts tend_rw - cofwz (zz_k P_k - zz_km1 P_km1) - cofwr (R_k + R_km1)
+//        + cofwt_k P_k + cofwt_km1 P_km1
+// Bound by the float64 pipe (63 operations a level, 268 us at 40962 x 55).  S1 is formed on
+// the integer pipes (fixdot.cuh), S2 over products formed once per edge, and the first
+// substep, whose perturbations are all zero, has its own instance: 28 operations a level (145
+// us), 17 in the first substep (105 us).
+struct AcLevel {
+  double rs, ts, R, P;
+};
+
+template <int N, bool FIRST>
+MPASG_D AcLevel ac_level(const mpasg_mesh& m, const mpasg_fields& f, const fx::Weight* w, uint32_t c, uint32_t k,
+                         double dts, double resm) {
+  const uint32_t L = (uint32_t)m.nVertLevels;
+  const size_t g = (size_t)c * m.maxEdges;
+  const int n = m.nEdgesOnCell[c];
+  double x[N], s1, s2 = 0.0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = f.ru_p[(uint32_t)w[j].row * L + k];
+  for (int j = 0; j < n; ++j)
+    s2 = fma(m.cell_edge_geo[g + j], f.ke_edge[(size_t)m.edgesOnCell[g + j] * L + k], s2);
+  if (!fx::dot<N>(x, w, &s1)) {
+    s1 = 0.0;
+    for (int j = 0; j < n; ++j) s1 = fma(m.cell_edge_geo[g + j], f.ru_p[(size_t)m.edgesOnCell[g + j] * L + k], s1);
+  }
+  const size_t o = (size_t)c * L + k, ow = (size_t)c * (L + 1) + k;
+  AcLevel a;
+  if (FIRST) {
+    a.R = a.rs = dts * (f.tend_rho[o] - s1);
+    a.P = a.ts = dts * (f.tend_theta[o] - s2);
+  } else {
+    const double rho_in = f.rho_pp[o], rt_in = f.rtheta_pp[o], w0 = f.rw_p[ow], w1 = f.rw_p[ow + 1];
+    a.rs = fma(-(resm * f.cofrz[k]), w1 - w0, fma(dts, f.tend_rho[o] - s1, rho_in));
+    a.ts = fma(-(resm * m.rdzw[k]), f.coftz[ow + 1] * w1 - f.coftz[ow] * w0, fma(dts, f.tend_theta[o] - s2, rt_in));
+    a.R = fma(resm, rho_in, a.rs);
+    a.P = fma(resm, rt_in, a.ts);
+  }
+  return a;
+}
+
+template <int N, bool FIRST>
+__global__ void __launch_bounds__(kBlock, 5) k_ac_prep(mpasg_mesh m, mpasg_fields f, FastDiv fl1, double dts,
+                                                    double ww_lo, double resm) {
+  extern __shared__ fx::Weight s_w[];
+  __shared__ double s_R[kBlock], s_P[kBlock];
+  const uint32_t L = (uint32_t)m.nVertLevels;
+  const uint32_t n_all = (uint32_t)m.nCells * (L + 1);
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fl1.div(i0), c1 = fl1.div(min(i0 + kBlock, n_all) - 1u);
+  for (uint32_t t = threadIdx.x; t < (c1 - c0 + 1) * N; t += kBlock) {
+    const uint32_t cl = t / N, j = t - cl * N, c = c0 + cl;
+    const size_t g = (size_t)c * m.maxEdges;
+    const int n = m.nEdgesOnCell[c];
+    s_w[t] = ((int)j < n && n <= N) ? fx::weight(m.cell_edge_geo[g + j], m.edgesOnCell[g + j])
+                                    : fx::Weight{0, 0, n > N ? fx::kBadWeight : 0u, n > 0 ? m.edgesOnCell[g] : 0};
+  }
+  __syncthreads();
+  const bool active = i < n_all;
+  uint32_t c = c0, k = 0;
   AcLevel lv{0.0, 0.0, 0.0, 0.0};
   if (active) {
     c = fl1.div(i);
     k = i - c * (L + 1);
-    if (k < (uint32_t)L) lv = ac_level<T>(m, f, c, k, first, dts, resm);
+    if (k < L) lv = ac_level<N, FIRST>(m, f, s_w + (c - c0) * N, c, k, dts, resm);
   }
-  s_lv[threadIdx.x] = lv;
+  s_R[threadIdx.x] = lv.R;
+  s_P[threadIdx.x] = lv.P;
   __syncthreads();
   if (!active) return;
-  const size_t o = (size_t)c * L;
-  const size_t ow = (size_t)c * (L + 1);
-  if (k < (uint32_t)L) {
+  const size_t o = (size_t)c * L, ow = (size_t)c * (L + 1);
+  if (k < L) {
     f.ac_rs[o + k] = lv.rs;
     f.ac_ts[o + k] = lv.ts;
-    f.rtheta_pp_old[o + k] = lv.rt_in;
+    f.rtheta_pp_old[o + k] = FIRST ? 0.0 : f.rtheta_pp[o + k];
   }
-  const double rwp_k = first ? 0.0 : f.rw_p[ow + k];
-  if (k == 0 || k == (uint32_t)L) {  // boundary values pass through the solve unchanged
+  const double rwp_k = FIRST ? 0.0 : f.rw_p[ow + k];
+  if (k == 0 || k == L) {  // boundary values pass through the solve unchanged
     f.ac_x[ow + k] = rwp_k;
-    if (first) f.wwAvg[ow + k] = 0.0;
+    if (FIRST) f.wwAvg[ow + k] = 0.0;
     return;
   }
-  AcLevel lo = (threadIdx.x >= 1) ? s_lv[threadIdx.x - 1] : ac_level<T>(m, f, c, k - 1, first, dts, resm);
-  const double ww_in = first ? 0.0 : f.wwAvg[ow + k];
-  f.wwAvg[ow + k] = ww_in + 0.5 * (1.0 - epssm) * rwp_k;
-  const double zz_k = m.zz[o + k], zz_km1 = m.zz[o + k - 1];
-  const double cw_k = f.cofwt[o + k], cw_km1 = f.cofwt[o + k - 1];
-  f.ac_x[ow + k] = rwp_k + dts * f.tend_rw[ow + k] -
-                   f.cofwz[o + k] * ((zz_k * lv.ts - zz_km1 * lo.ts) + resm * (zz_k * lv.rt_in - zz_km1 * lo.rt_in)) -
-                   f.cofwr[o + k] * ((lv.rs + lo.rs) + resm * (lv.rho_in + lo.rho_in)) +
-                   cw_k * (lv.ts + resm * lv.rt_in) + cw_km1 * (lo.ts + resm * lo.rt_in);
+  double R_lo, P_lo;
+  if (threadIdx.x >= 1) {
+    R_lo = s_R[threadIdx.x - 1];
+    P_lo = s_P[threadIdx.x - 1];
+  } else {
+    const AcLevel lo = ac_level<N, FIRST>(m, f, s_w + (c - c0) * N, c, k - 1, dts, resm);
+    R_lo = lo.R;
+    P_lo = lo.P;
+  }
+  f.wwAvg[ow + k] = FIRST ? 0.0 : fma(ww_lo, rwp_k, f.wwAvg[ow + k]);
+  double x = FIRST ? dts * f.tend_rw[ow + k] : fma(dts, f.tend_rw[ow + k], rwp_k);
+  x = fma(-f.cofwz[o + k], m.zz[o + k] * lv.P - m.zz[o + k - 1] * P_lo, x);
+  x = fma(-f.cofwr[o + k], lv.R + R_lo, x);
+  f.ac_x[ow + k] = fma(f.cofwt[o + k - 1], P_lo, fma(f.cofwt[o + k], lv.P, x));
+}
+
+int launch_ac_prep(const mpasg_mesh* m, const mpasg_fields* f, int small_step, double dts, double epssm, double resm,
+                   cudaStream_t s) {
+  const int L = m->nVertLevels, nb = nblocks((long long)m->nCells * (L + 1)), nc = (kBlock - 1) / (L + 1) + 2;
+  const double ww_lo = 0.5 * (1.0 - epssm);
+  const FastDiv fl1(L + 1);
+  const bool first = small_step == 1, narrow = m->maxEdges <= 6;
+  const size_t smem = nc * (narrow ? 6 : 10) * sizeof(fx::Weight);
+  if (narrow && first) k_ac_prep<6, true><<<nb, kBlock, smem, s>>>(*m, *f, fl1, dts, ww_lo, resm);
+  else if (narrow) k_ac_prep<6, false><<<nb, kBlock, smem, s>>>(*m, *f, fl1, dts, ww_lo, resm);
+  else if (first) k_ac_prep<10, true><<<nb, kBlock, smem, s>>>(*m, *f, fl1, dts, ww_lo, resm);
+  else k_ac_prep<10, false><<<nb, kBlock, smem, s>>>(*m, *f, fl1, dts, ww_lo, resm);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
 }
 
 __global__ void k_ac_thomas(mpasg_mesh m, mpasg_fields f) {
@@ -590,7 +636,7 @@ __global__ void __launch_bounds__(kThomasThreads) k_vimp_factor_staged(mpasg_mes
     sal[t] = 0.0;
     sg[t] = 0.0;
     for (int k = 1; k < L; ++k) {
-      const double alpha = fdiv<T>(1.0, sb[k * kThomasPitch + t] - sa[k * kThomasPitch + t] * gam);
+      const double alpha = recip<T>(sb[k * kThomasPitch + t] - sa[k * kThomasPitch + t] * gam);
       gam = sc[k * kThomasPitch + t] * alpha;
       sal[k * kThomasPitch + t] = alpha;
       sg[k * kThomasPitch + t] = gam;
@@ -617,21 +663,24 @@ __global__ void k_tri_m(long long n, const double* __restrict__ a, const double*
 
 size_t thomas_smem_bytes(int L) { return (size_t)(4 * L + 1) * kThomasPitch * sizeof(double); }
 
+// Rayleigh damping of the solution, (x + d - dts dss zz rho w) / (1 + dts dss) - d with d =
+// rw_save - rw; a level without damping keeps x ((x + d) - d without its two roundings)
 MPASG_D double ac_damped(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, int k, int L, double x,
                          double dts) {
   if (k == 0 || k == L) return x;
-  double fzm = m.fzm[k], fzp = m.fzp[k];
-  double zz_i = fzm * m.zz[o + k] + fzp * m.zz[o + k - 1];
-  double rho_i = fzm * f.rho_zz[o + k] + fzp * f.rho_zz[o + k - 1];
-  double dss = m.dss[o + k];
-  double rw_delta = f.rw_save[ow + k] - f.rw[ow + k];
-  double num = x + rw_delta - dts * dss * zz_i * rho_i * f.w[ow + k];
-  double den = 1.0 + dts * dss;
-  return (den == 1.0 ? num : num / den) - rw_delta;  // x / 1.0 == x below the damping layer
+  const double dss = m.dss[o + k];
+  if (fx::is_zero(dss)) return x;
+  const double fzm = m.fzm[k], fzp = m.fzp[k];
+  const double zz_i = fzm * m.zz[o + k] + fzp * m.zz[o + k - 1];
+  const double rho_i = fzm * f.rho_zz[o + k] + fzp * f.rho_zz[o + k - 1];
+  const double rw_delta = f.rw_save[ow + k] - f.rw[ow + k], damp = dts * dss;
+  const double num = x + rw_delta - damp * zz_i * rho_i * f.w[ow + k];
+  return fx::quotient(num, 1.0 + damp) - rw_delta;
 }
 
+// ww_hi: 0.5 (1 + epssm)
 __global__ void __launch_bounds__(kBlock) k_ac_post(mpasg_mesh m, mpasg_fields f, FastDiv fl1, double dts,
-                                                    double epssm) {
+                                                    double ww_hi) {
   __shared__ double s_xr[kBlock];
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -650,7 +699,7 @@ __global__ void __launch_bounds__(kBlock) k_ac_post(mpasg_mesh m, mpasg_fields f
   __syncthreads();
   if (!active) return;
   f.rw_p[ow + k] = xr;
-  if (k >= 1 && k < (uint32_t)L) f.wwAvg[ow + k] = f.wwAvg[ow + k] + 0.5 * (1.0 + epssm) * xr;
+  if (k >= 1 && k < (uint32_t)L) f.wwAvg[ow + k] = fma(ww_hi, xr, f.wwAvg[ow + k]);
   if (k == (uint32_t)L) return;
   double xr1 = (threadIdx.x + 1 < blockDim.x) ? s_xr[threadIdx.x + 1]
                                               : ac_damped(m, f, o, ow, k + 1, L, f.ac_x[ow + k + 1], dts);
@@ -772,7 +821,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
     f.rho_p[o] = rho_p;
     f.rho_zz[o] = rho_zz;
     f.rtheta_p[o] = rtheta_p;
-    f.theta_m[o] = sizeof(T) == sizeof(double) ? (rtheta_p + rtb) / rho_zz : (rtheta_p + rtb) * rcp_nr1(rho_zz);
+    f.theta_m[o] = sizeof(T) == sizeof(double) ? fx::quotient(rtheta_p + rtb, rho_zz) : (rtheta_p + rtb) * rcp_nr1(rho_zz);
     if (rk_step == 3) {
       const double rcv = kRgas / (kCp - kRgas);
       double zz = m.zz[o];
@@ -805,7 +854,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
     if (sizeof(T) != sizeof(double)) f.rw_f32[ow] = d2f_bits(rw);
     size_t oc = (size_t)c * L;
     const double den = m.fzm[k] * m.zz[oc + k] + m.fzp[k] * m.zz[oc + k - 1];
-    const double wo = den == 1.0 ? rw : fdiv<T>(rw, den);
+    const double wo = fx::is_one(den) ? rw : fdiv<T>(rw, den);
     if (!FLAT) {
       f.w[ow] = wo;
     } else {
@@ -835,7 +884,8 @@ __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double
   double ru = rus + f.ru_p[i];
   f.ru[i] = ru;
   const double rho2 = f.rho_zz[(size_t)c1 * L + k] + f.rho_zz[(size_t)c2 * L + k];
-  const double u = sizeof(T) == sizeof(double) ? 2.0 * ru / rho2 : 2.0 * ru * rcp_nr1(rho2);
+  // 2 ru / rho2 (the factor two is exact wherever it is applied)
+  const double u = sizeof(T) == sizeof(double) ? fx::quotient(ru + ru, rho2) : 2.0 * ru * rcp_nr1(rho2);
   f.u[i] = u;
   if (sizeof(T) != sizeof(double)) f.u_f32[i] = d2f_bits(u);
 }
@@ -938,13 +988,14 @@ extern "C" int mpasg_vert_imp_coefs(const mpasg_mesh* m, const mpasg_config* c, 
                                             200 * 1024) == cudaSuccess;
   const bool staged = smem_opt_in[dev] && smem <= 200 * 1024;
   const int nblk = nblocks(m->nCells, kThomasCols);
+  const VimpScalars vs = vimp_scalars(dts, c->epssm);
   if (c->precision == MPASG_PRECISION_MIXED) {
-    k_vimp_coefs<float><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), dts, c->epssm);
+    k_vimp_coefs<float><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), vs);
     MPASG_LAUNCH_CHECK();
     if (staged) k_vimp_factor_staged<float><<<nblk, kThomasThreads, smem, s>>>(*m, *f, FastDiv(L));
     else k_vimp_factor<float><<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f);
   } else {
-    k_vimp_coefs<double><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), dts, c->epssm);
+    k_vimp_coefs<double><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), vs);
     MPASG_LAUNCH_CHECK();
     if (staged) k_vimp_factor_staged<double><<<nblk, kThomasThreads, smem, s>>>(*m, *f, FastDiv(L));
     else k_vimp_factor<double><<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f);
@@ -1012,8 +1063,8 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
       k_acoustic_edges<double><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), small_step,
                                                                                    dts, c2);
       MPASG_LAUNCH_CHECK();
-      k_ac_prep<double><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), small_step, dts, c->epssm, resm);
-      MPASG_LAUNCH_CHECK();
+      const int rc = launch_ac_prep(m, f, small_step, dts, c->epssm, resm, s);
+      if (rc != MPASG_OK) return rc;
     }
     if (part == 0) return MPASG_OK;
   }
@@ -1043,7 +1094,7 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
   if (mixed)
     k_ac_post_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, (float)c->epssm);
   else
-    k_ac_post<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, c->epssm);
+    k_ac_post<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, 0.5 * (1.0 + c->epssm));
   MPASG_LAUNCH_CHECK();
   return MPASG_OK;
 }
