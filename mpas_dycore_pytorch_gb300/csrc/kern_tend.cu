@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "advstencil.cuh"
+#include "cellsum.cuh"
 
 namespace {
 
@@ -30,6 +31,7 @@ struct TendScalars {
   int ncam;   // CAM damping levels (0: off)
   int ray_n;  // Rayleigh-damped top levels of u (0: off)
   int mix_pert;  // vertical mixing of the perturbation from the initial profiles
+  double f3[4];  // flux3 with coef3 by upwind side: 7 + 3 c, 7 - 3 c, 1 + c, 1 - c
   int defer;  // k_tend_u leaves tend_u_euler to k_tend_u_finish (del4 and / or vertical mixing)
 };
 
@@ -526,7 +528,133 @@ MPASG_D double theta_vmix(const mpasg_mesh& m, const mpasg_fields& f, uint32_t c
   return v * 1.0 * f.rho_zz[(size_t)c * L + k] * diff / (0.5 * (zp - zm));
 }
 
-// w / theta del2 mixing and the del2 fields for del4 (rk 1); index space (C, L+1)
+// ---------------------------------------------------------------- w / theta mixing, float64 form
+// The fluxes are formed once per edge instead of once per adjacent cell, the cells only sum
+// them (cellsum.cuh):
+//   k_mix_edges_a  F_w = (rho_k + rho_km1) dw dv/dc,  F_t = rho dtheta dv/dc   (flux_w_e, flux_th_e)
+//   k_mix_cells    their divergences: 2 delsq_w, delsq_theta                  (del4 on only)
+//   k_mix_edges_b  the del2 fluxes with the eddy viscosity, minus the del4 fluxes, in place
+//   k_mix_cells    their divergences: tend_w_euler, tend_theta_euler
+// 11 + 8 float64 operations an edge level and 14 a cell level instead of 193 a cell level; the
+// four kernels take 1.16 ms a step at 40962 x 55, the two cell kernels before them 2.44 ms.
+struct MixEdge {
+  double dvdc;      // dvEdge / dcEdge
+  double k_w, k_t;  // meshScalingDel2 / 8 and / 2
+  double d4_w, d4_t;  // meshScalingDel4 times the del4 viscosity times dv / dc
+};
+
+MPASG_D void load_mix(const mpasg_mesh& m, const TendScalars& p, uint32_t e0, uint32_t n, MixEdge* tab) {
+  for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
+    const uint32_t e = e0 + t;
+    const double dvdc = m.dvEdge[e] * m.invDcEdge[e], ms2 = m.meshScalingDel2[e], ms4 = m.meshScalingDel4[e];
+    tab[t] = MixEdge{dvdc, 0.125 * ms2, 0.5 * ms2, ms4 * p.h_mom_visc4 * dvdc, ms4 * p.h_theta_visc4 * dvdc};
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) k_mix_edges_a(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
+  extern __shared__ MixEdge s_m[];
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nEdges * L;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t e0 = fl.div(i0), e1 = fl.div(min(i0 + kBlock, n_all) - 1u);
+  load_mix(m, p, e0, e1 - e0 + 1, s_m);
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t e = fl.div(i), k = i - e * L;
+  const size_t c1 = (size_t)m.cellsOnEdge[2 * e], c2 = (size_t)m.cellsOnEdge[2 * e + 1];
+  const double dvdc = s_m[e - e0].dvdc, h = f.h_edge[i];
+  f.flux_th_e[i] = (h * dvdc) * (f.theta_m[c2 * L + k] - f.theta_m[c1 * L + k]);
+  if (k >= 1)
+    f.flux_w_e[i] = ((h + f.h_edge[i - 1]) * dvdc) * (f.w[c2 * (L + 1) + k] - f.w[c1 * (L + 1) + k]);
+}
+
+template <bool DEL4>
+__global__ void __launch_bounds__(kBlock) k_mix_edges_b(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
+  extern __shared__ MixEdge s_m[];
+  __shared__ double s_k[kBlock];
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nEdges * L;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t e0 = fl.div(i0), e1 = fl.div(min(i0 + kBlock, n_all) - 1u);
+  load_mix(m, p, e0, e1 - e0 + 1, s_m);
+  uint32_t e = e0, k = 0;
+  size_t c1 = 0, c2 = 0;
+  double kd = 0.0;
+  if (i < n_all) {
+    e = fl.div(i);
+    k = i - e * L;
+    c1 = (size_t)m.cellsOnEdge[2 * e];
+    c2 = (size_t)m.cellsOnEdge[2 * e + 1];
+    kd = f.kdiff[c1 * L + k] + f.kdiff[c2 * L + k];
+  }
+  s_k[threadIdx.x] = kd;
+  __syncthreads();
+  if (i >= n_all) return;
+  const MixEdge me = s_m[e - e0];
+  double ft = f.flux_th_e[i] * (kd * me.k_t);
+  if (DEL4) ft = fma(-me.d4_t, f.delsq_theta[c2 * L + k] - f.delsq_theta[c1 * L + k], ft);
+  f.flux_th_e[i] = ft;
+  if (k >= 1) {
+    const double km = threadIdx.x >= 1 ? s_k[threadIdx.x - 1] : f.kdiff[c1 * L + k - 1] + f.kdiff[c2 * L + k - 1];
+    double fw = f.flux_w_e[i] * ((kd + km) * me.k_w);
+    // (delsq_w holds the del2 of w; at the ends of the column no w equation, the sums skip them)
+    if (DEL4) fw = fma(-me.d4_w, f.delsq_w[c2 * (L + 1) + k] - f.delsq_w[c1 * (L + 1) + k], fw);
+    f.flux_w_e[i] = fw;
+  }
+}
+
+// divergences of flux_w_e (w levels 1..L-1, zero at the ends) and flux_th_e; `half`: the del2
+// pass, whose F_w is twice the flux
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_mix_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl1, int half,
+                                                      double* __restrict__ div_w, double* __restrict__ div_t) {
+  extern __shared__ cellsum::Slot s_c[];
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nCells * (L + 1);
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fl1.div(i0), c1 = fl1.div(min(i0 + kBlock, n_all) - 1u);
+  cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t c = fl1.div(i), k = i - c * (L + 1);
+  const int n = m.nEdgesOnCell[c];
+  const cellsum::Slot* s = s_c + (c - c0) * N;
+  const double ia = m.invAreaCell[c];
+  if (k < L) div_t[(size_t)c * L + k] = ia * cellsum::f64<N>(m, c, n, s, f.flux_th_e, L, k);
+  double dw = 0.0;
+  if (k >= 1 && k < L) {
+    dw = ia * cellsum::fixed<N>(m, c, n, s, f.flux_w_e, L, k);
+    if (half) dw = 0.5 * dw;
+  }
+  div_w[i] = dw;
+}
+
+int launch_mix_fx(const mpasg_mesh* m, const mpasg_fields* f, const TendScalars& p, cudaStream_t s) {
+  const int L = m->nVertLevels;
+  const int ne = nblocks((long long)m->nEdges * L), nc = nblocks((long long)m->nCells * (L + 1));
+  const size_t se = cellsum::max_cells(L) * sizeof(MixEdge);
+  const bool narrow = m->maxEdges <= 6, del4 = p.h_mom_visc4 > 0.0 || p.h_theta_visc4 > 0.0;
+  const size_t sc = cellsum::max_cells(L + 1) * (narrow ? 6 : 8) * sizeof(cellsum::Slot);
+  TendScalars q = p;
+  if (!(p.h_mom_visc4 > 0.0)) q.h_mom_visc4 = 0.0;
+  if (!(p.h_theta_visc4 > 0.0)) q.h_theta_visc4 = 0.0;
+  auto cells = [&](int half, double* w, double* t) {
+    if (narrow) k_mix_cells<6><<<nc, kBlock, sc, s>>>(*m, *f, FastDiv(L + 1), half, w, t);
+    else k_mix_cells<8><<<nc, kBlock, sc, s>>>(*m, *f, FastDiv(L + 1), half, w, t);
+  };
+  k_mix_edges_a<<<ne, kBlock, se, s>>>(*m, *f, FastDiv(L), q);
+  MPASG_LAUNCH_CHECK();
+  if (del4) {
+    cells(1, f->delsq_w, f->delsq_theta);
+    MPASG_LAUNCH_CHECK();
+    k_mix_edges_b<true><<<ne, kBlock, se, s>>>(*m, *f, FastDiv(L), q);
+  } else {
+    k_mix_edges_b<false><<<ne, kBlock, se, s>>>(*m, *f, FastDiv(L), q);
+  }
+  MPASG_LAUNCH_CHECK();
+  cells(0, f->tend_w_euler, f->tend_theta_euler);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
+}
+
+// w / theta del2 mixing and the del2 fields for del4 (rk 1), mixed form; index space (C, L+1)
 template <typename T>
 __global__ void k_mix_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   const int L = m.nVertLevels;
@@ -546,8 +674,7 @@ __global__ void k_mix_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
     for (int j = 0; j < n; ++j) {
       int e = m.edgesOnCell[c * me + j];
       int ec1 = m.cellsOnEdge[2 * e], ec2 = m.cellsOnEdge[2 * e + 1];
-      T es = sizeof(T) == sizeof(double) ? cv<T>(m.cell_edge_es_w[c * me + j])  // same product, formed once
-                                         : T(0.5) * ia * sg[c * me + j] * dv[e] * idc[e];
+      T es = T(0.5) * ia * sg[c * me + j] * dv[e] * idc[e];
       T flux = es * (cv<T>(f.h_edge[(size_t)e * L + k]) + cv<T>(f.h_edge[(size_t)e * L + k - 1])) *
                (w[(size_t)ec2 * (L + 1) + k] - w[(size_t)ec1 * (L + 1) + k]);
       dw = dw + flux;
@@ -568,7 +695,7 @@ __global__ void k_mix_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
     for (int j = 0; j < n; ++j) {
       int e = m.edgesOnCell[c * me + j];
       int ec1 = m.cellsOnEdge[2 * e], ec2 = m.cellsOnEdge[2 * e + 1];
-      T es = sizeof(T) == sizeof(double) ? cv<T>(m.cell_edge_es_t[c * me + j]) : ia * sg[c * me + j] * dv[e] * idc[e];
+      T es = ia * sg[c * me + j] * dv[e] * idc[e];
       T pr = T(1) * msd2[e];
       T flux = es * dif<T>(f.theta_m[(size_t)ec2 * L + k], f.theta_m[(size_t)ec1 * L + k]) *
                cv<T>(f.h_edge[(size_t)e * L + k]);
@@ -581,7 +708,7 @@ __global__ void k_mix_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   }
 }
 
-// del4 parts of w / theta mixing (rk 1)
+// del4 parts of w / theta mixing (rk 1), mixed form
 template <typename T>
 __global__ void k_mix_cells_b(mpasg_mesh m, mpasg_fields f, FastDiv fl1, TendScalars p) {
   const int L = m.nVertLevels;
@@ -690,7 +817,7 @@ __global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
 // that both are busy (two sums of ~10 terms are all this kernel does; both in float64 bound it
 // at 82 % of that pipe).  40962 x 55: 374 us in float64 alone, 271 us with both sums
 // on the integer side, 216 us with one each.
-template <int N>
+template <int N, bool PERT>
 __global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   extern __shared__ fx::Weight s_w[];
   const uint32_t L = (uint32_t)m.nVertLevels;
@@ -708,64 +835,98 @@ __global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_
 #pragma unroll
   for (int j = 0; j < N; ++j) x[j] = f.theta_m[(uint32_t)w[j].row * L + k];
   if (!fx::dot<N>(x, w, &th)) th = adv::sum(m, e, back, f.theta_m, L, k);
-  f.flux_th_e[i] = rue * th;
+  double ft = rue * th;
+  // later RK stages: the mass flux already applied, dv (ru_save - ru) theta_save, once per edge
+  // (k_tend_w_theta summed it over every cell's slots: 18 operations a cell level, 9 here)
+  if (PERT) ft = fma(m.dvEdge[e] * (f.ru_save[i] - rue), f.theta_edge_save[i], ft);
+  f.flux_th_e[i] = ft;
   if (k >= 1) {
     const double ru_w = fma(m.fzm[k], rue, m.fzp[k] * f.ru[i - 1]);
     f.flux_w_e[i] = ru_w * adv::sum(m, e, __double2hiint(ru_w) < 0, f.w, L + 1, k);
   }
 }
 
-// w and theta tendencies (float64 form); index space (C, L+1)
-__global__ void __launch_bounds__(kBlock) k_tend_w_theta(mpasg_mesh m, mpasg_fields f, FastDiv fl1, TendScalars p) {
-  using T = double;
-  __shared__ T s_wd[kBlock], s_wt[kBlock];
-  const int L = m.nVertLevels;
+// Vertical fluxes of the float64 form at interface kk, the upwind combination of flux3 taken
+// out (as in wduz12_at): of w (coefficient 1, times 12) and of theta (coefficient c,
+//   12 flux = rw ((7 + 3c) a + (7 - 3c) b - (1 + c) a' - (1 - c) b'),  a upwind, a' behind it)
+MPASG_D double wdwz12_at(const double* __restrict__ w, const double* __restrict__ rw, int kk, int L) {
+  if (kk <= 0 || kk >= L) return 0.0;
+  const double rw2 = rw[kk] + rw[kk - 1];
+  if (kk == 1 || kk == L - 1) return rw2 * (3.0 * (w[kk] + w[kk - 1]));
+  const bool down = __double2hiint(rw2) < 0;
+  const double a = w[down ? kk - 1 : kk], b = w[down ? kk : kk - 1], c = w[down ? kk + 1 : kk - 2];
+  return rw2 * fma(2.0, a, fma(5.0, b, -c));
+}
+
+MPASG_D double wdtz_fx_at(const double* __restrict__ th, const double* __restrict__ ths,
+                          const double* __restrict__ rw, const double* __restrict__ rws, int kk, int L,
+                          const double* fzm, const double* fzp, const TendScalars& p) {
+  if (kk <= 0 || kk >= L) return 0.0;
+  const double fm = fzm[kk], fp = fzp[kk];
+  if (kk == L - 1 && kk != 1) return rws[kk] * (fm * th[kk] + fp * th[kk - 1]);
+  const double r = rw[kk];
+  double v;
+  if (kk == 1) {
+    v = r * (fm * th[kk] + fp * th[kk - 1]);
+  } else {
+    const bool down = __double2hiint(r) < 0;
+    const double a = th[down ? kk : kk - 1], b = th[down ? kk - 1 : kk];
+    const double a2 = th[down ? kk + 1 : kk - 2], b2 = th[down ? kk - 2 : kk + 1];
+    v = (r * kInv12) * fma(p.f3[0], a, fma(p.f3[1], b, -fma(p.f3[2], a2, p.f3[3] * b2)));
+  }
+  return fma(rws[kk] - r, fm * ths[kk] + fp * ths[kk - 1], v);
+}
+
+// w and theta tendencies (float64 form); index space (C, L+1).  Bound by the float64 pipe: 89
+// operations a level before (369 us at 40962 x 55), about 40 with the upwind vertical fluxes,
+// the perturbation flux on the edges (k_adv_edges_fx, 216 -> 243 us for it), the w divergence
+// on the integer pipes and the quotient of fastdiv64.cuh (220 us).
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_tend_w_theta(mpasg_mesh m, mpasg_fields f, FastDiv fl1, TendScalars p) {
+  extern __shared__ cellsum::Slot s_c[];
+  __shared__ double s_wd[kBlock], s_wt[kBlock];
+  const uint32_t L = (uint32_t)m.nVertLevels;
   const uint32_t n_all = (uint32_t)m.nCells * (L + 1);
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fl1.div(i0), c1 = fl1.div(min(i0 + kBlock, n_all) - 1u);
+  cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   const bool active = i < n_all;
-  uint32_t c = 0, k = 0;
-  T wd_k = T(0), wt_k = T(0);
-  const T coef3 = p.coef3;
+  uint32_t c = c0, k = 0;
+  double wd_k = 0.0, wt_k = 0.0;
+  auto wd_at = [&](uint32_t kk) {
+    const size_t ow = (size_t)c * (L + 1);
+    return wdwz12_at(f.w + ow, f.rw + ow, kk, L);
+  };
+  auto wt_at = [&](uint32_t kk) {
+    const size_t ow = (size_t)c * (L + 1), oc = (size_t)c * L;
+    return wdtz_fx_at(f.theta_m + oc, f.theta_m_save + oc, f.rw + ow, f.rw_save + ow, kk, L, m.fzm, m.fzp, p);
+  };
   if (active) {
     c = fl1.div(i);
     k = i - c * (L + 1);
-    const size_t ow0 = (size_t)c * (L + 1), oc0 = (size_t)c * L;
-    wd_k = wdwz_at<T>(f.w + ow0, f.rw + ow0, k, L);
-    wt_k = wdtz_at<T>(f.theta_m + oc0, f.theta_m_save + oc0, f.rw + ow0, f.rw + ow0, f.rw_save + ow0, k, L, m.fzm,
-                      m.fzp, coef3);
+    wd_k = wd_at(k);
+    wt_k = wt_at(k);
   }
   s_wd[threadIdx.x] = wd_k;  // interface fluxes owned by this level
   s_wt[threadIdx.x] = wt_k;
   __syncthreads();
   if (!active) return;
-  T wd_k1 = T(0), wt_k1 = T(0);
-  if (k < (uint32_t)L) {
-    if (threadIdx.x + 1 < blockDim.x) {
-      wd_k1 = s_wd[threadIdx.x + 1];
-      wt_k1 = s_wt[threadIdx.x + 1];
-    } else {
-      const size_t ow0 = (size_t)c * (L + 1), oc0 = (size_t)c * L;
-      wd_k1 = wdwz_at<T>(f.w + ow0, f.rw + ow0, k + 1, L);
-      wt_k1 = wdtz_at<T>(f.theta_m + oc0, f.theta_m_save + oc0, f.rw + ow0, f.rw + ow0, f.rw_save + ow0, k + 1, L,
-                         m.fzm, m.fzp, coef3);
-    }
+  double wd_k1 = 0.0, wt_k1 = 0.0;
+  if (k < L) {
+    wd_k1 = threadIdx.x + 1 < kBlock ? s_wd[threadIdx.x + 1] : wd_at(k + 1);
+    wt_k1 = threadIdx.x + 1 < kBlock ? s_wt[threadIdx.x + 1] : wt_at(k + 1);
   }
-  const int me = m.maxEdges;
   const int n = m.nEdgesOnCell[c];
-  const T ia = m.invAreaCell[c];
-  const size_t oc = (size_t)c * L;
-  const size_t ow = (size_t)c * (L + 1);
-  if (k >= 1 && k < (uint32_t)L) {
-    T tw = T(0);
-    for (int j = 0; j < n; ++j) {
-      int e = m.edgesOnCell[c * me + j];
-      tw = tw - m.edgesOnCell_sign[c * me + j] * f.flux_w_e[(size_t)e * L + k];
-    }
-    tw = tw * ia - m.rdzu[k] * (wd_k1 - wd_k);
-    T teu = f.tend_w_euler[i];
+  const cellsum::Slot* s = s_c + (c - c0) * N;
+  const double ia = m.invAreaCell[c];
+  const size_t oc = (size_t)c * L, ow = (size_t)c * (L + 1);
+  if (k >= 1 && k < L) {
+    const double rdzu = m.rdzu[k];
+    const double tw = fma(-ia, cellsum::fixed<N>(m, c, n, s, f.flux_w_e, L, k), (rdzu * kInv12) * (wd_k - wd_k1));
+    double teu = f.tend_w_euler[i];
     if (p.rk_step == 1) {
       // vertical pressure gradient minus buoyancy: a near-hydrostatic residual
-      const double res = m.rdzu[k] * (f.pressure_p[oc + k] - f.pressure_p[oc + k - 1]) -
+      const double res = rdzu * (f.pressure_p[oc + k] - f.pressure_p[oc + k - 1]) -
                          (m.fzm[k] * f.dpdz[oc + k] + m.fzp[k] * f.dpdz[oc + k - 1]);
       teu = teu - f.cqw[ow + k] * res;
       if (p.v_mom > 0.0) teu = teu + w_vmix(m, f, oc, ow, k, p.v_mom);
@@ -775,37 +936,19 @@ __global__ void __launch_bounds__(kBlock) k_tend_w_theta(mpasg_mesh m, mpasg_fie
   } else {
     f.tend_w[i] = 0.0;
   }
-  if (k < (uint32_t)L) {
+  if (k < L) {
     const size_t o = oc + k;
-    T tt = T(0);
-    for (int j = 0; j < n; ++j) {
-      int e = m.edgesOnCell[c * me + j];
-      T x = -(m.edgesOnCell_sign[c * me + j] * f.flux_th_e[(size_t)e * L + k]);
-      tt = (j == 0) ? x : tt + x;
-    }
-    if (p.rk_step > 1) {
-      for (int j = 0; j < n; ++j) {
-        int e = m.edgesOnCell[c * me + j];
-        // (sign dvEdge) (ru_save - ru) 0.5 (theta_2 + theta_1), with the slot product and the
-        // edge mean formed once (scaling by 0.5 is exact, so the rounding is unchanged)
-        T flux = m.cell_edge_sdv[c * me + j] * (f.ru_save[(size_t)e * L + k] - f.ru[(size_t)e * L + k]) *
-                 f.theta_edge_save[(size_t)e * L + k];
-        tt = tt - flux;
-      }
-    }
-    tt = tt * ia - m.rdzw[k] * (wt_k1 - wt_k);
-    const T rz = f.rho_zz[o];
-    const T rtd = f.rt_diabatic_tend[o];
+    double tt = fma(-ia, cellsum::f64<N>(m, c, n, s, f.flux_th_e, L, k), m.rdzw[k] * (wt_k - wt_k1));
+    const double rz = f.rho_zz[o];
     // unfused: the difference cancels strongly (as rounded by the reference)
-    f.rthdynten[o] = sub_rn(tt, mul_rn(f.tend_rho[o], f.theta_m[o])) / rz;
-    tt = tt + rz * rtd;
+    f.rthdynten[o] = fx::quotient(sub_rn(tt, mul_rn(f.tend_rho[o], f.theta_m[o])), rz);
+    tt = tt + rz * f.rt_diabatic_tend[o];
     double tte = f.tend_theta_euler[o];
-    if (p.rk_step == 1 && p.v_theta > 0.0 && k >= 1 && k + 1 < (uint32_t)L) {
+    if (p.rk_step == 1 && p.v_theta > 0.0 && k >= 1 && k + 1 < L) {
       tte = tte + theta_vmix(m, f, c, k, L, p.v_theta, p.mix_pert);
       f.tend_theta_euler[o] = tte;
     }
-    tt = tt + tte;
-    f.tend_theta[o] = tt;
+    f.tend_theta[o] = tt + tte;
   }
 }
 
@@ -999,26 +1142,37 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
       k_tend_u_finish<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
       MPASG_LAUNCH_CHECK();
     }
-    k_mix_cells_a<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1);
-    MPASG_LAUNCH_CHECK();
-    if (p.h_mom_visc4 > 0.0 || p.h_theta_visc4 > 0.0) {
-      TendScalars q = p;
-      if (!(p.h_mom_visc4 > 0.0)) q.h_mom_visc4 = 0.0;
-      k_mix_cells_b<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1, q);
+    if constexpr (sizeof(T) == sizeof(double)) {
+      const int rc = launch_mix_fx(m, f, p, s);
+      if (rc != MPASG_OK) return rc;
+    } else {
+      k_mix_cells_a<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1);
       MPASG_LAUNCH_CHECK();
+      if (p.h_mom_visc4 > 0.0 || p.h_theta_visc4 > 0.0) {
+        TendScalars q = p;
+        if (!(p.h_mom_visc4 > 0.0)) q.h_mom_visc4 = 0.0;
+        k_mix_cells_b<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1, q);
+        MPASG_LAUNCH_CHECK();
+      }
     }
   }
   if constexpr (sizeof(T) == sizeof(double)) {
     const size_t smem = (size_t)((kBlock - 1) / L + 2) * adv::kEntryBytes;
-    if (m->nAdvMax <= 10) k_adv_edges_fx<10><<<nblocks(nel), kBlock, smem * 10, s>>>(*m, *f, fl);
-    else k_adv_edges_fx<14><<<nblocks(nel), kBlock, smem * 14, s>>>(*m, *f, fl);
+    const int nb = nblocks(nel);
+    const bool narrow = m->nAdvMax <= 10, pert = rk_step > 1;
+    if (narrow && pert) k_adv_edges_fx<10, true><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl);
+    else if (narrow) k_adv_edges_fx<10, false><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl);
+    else if (pert) k_adv_edges_fx<14, true><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl);
+    else k_adv_edges_fx<14, false><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl);
   } else {
     k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl);
   }
   MPASG_LAUNCH_CHECK();
-  if (sizeof(T) == sizeof(double))
-    k_tend_w_theta<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1, p);
-  else
+  if (sizeof(T) == sizeof(double)) {
+    const size_t sc = cellsum::max_cells(L + 1) * sizeof(cellsum::Slot);
+    if (m->maxEdges <= 6) k_tend_w_theta<6><<<nblocks(ncw), kBlock, sc * 6, s>>>(*m, *f, fl1, p);
+    else k_tend_w_theta<8><<<nblocks(ncw), kBlock, sc * 8, s>>>(*m, *f, fl1, p);
+  } else
     k_tend_w_theta_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1, p);
   MPASG_LAUNCH_CHECK();
   return MPASG_OK;
@@ -1063,6 +1217,10 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
   p.visc2 = p.smag ? 0.0 : c->h_theta_eddy_visc2;
   p.del4u_div = c->del4u_div_factor;
   p.coef3 = c->coef_3rd_order;
+  p.f3[0] = 7.0 + 3.0 * p.coef3;
+  p.f3[1] = 7.0 - 3.0 * p.coef3;
+  p.f3[2] = 1.0 + p.coef3;
+  p.f3[3] = 1.0 - p.coef3;
   p.rk_step = rk_step;
   p.del4 = (p.h_mom_visc4 > 0.0) ? 1 : 0;
   if (c->number_cam_damping_levels > m->nVertLevels) return MPASG_E_ARG;
