@@ -165,6 +165,9 @@ int mpasgi_reconstruct(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields*
 // theta_m - ref_theta and theta_m_save - ref_theta (float32) for the mixed form
 int mpasgi_theta_dev(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s);
 int mpasgi_theta_edge(const mpasg_mesh* m, mpasg_fields* f, bool mixed, cudaStream_t s);
+// float64 form: pv_edge * u in ke_edge, which the u tendency reads and the diagnostics keep
+// current (a step driver calls it once at the step start)
+int mpasgi_pvu(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s);
 int mpasgi_divergence_damping(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, double dts,
                               cudaStream_t s, bool copies_current);
 int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,

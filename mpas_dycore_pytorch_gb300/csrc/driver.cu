@@ -334,6 +334,7 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
   if (S > 0) CHECK_RC(copy(f.scalars_init, f.scalars, ncs, s));
   if (advect && coupled) CHECK_RC(copy(f.scalars_a, f.scalars_init, ncs, s));
   if (c->precision == MPASG_PRECISION_MIXED) CHECK_RC(mpasgi_pack_f32(m, &f, s));
+  else CHECK_RC(mpasgi_pvu(m, &f, s));
   // edge mean of theta_m_save and its reciprocal sum
   CHECK_RC(mpasgi_theta_edge(m, &f, c->precision == MPASG_PRECISION_MIXED, s));
   MARK(MPASG_STAGE_SETUP);

@@ -358,7 +358,7 @@ int forward_taped(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, co
   const bool mixed = c->precision == MPASG_PRECISION_MIXED;
   const mpasg_fields own = f;
   CHECK_RC(make_saves(m, T, f, 0, mixed, s));
-  if (mixed) CHECK_RC(mpasgi_pack_f32(m, &f, s));
+  CHECK_RC(mixed ? mpasgi_pack_f32(m, &f, s) : mpasgi_pvu(m, &f, s));
   CHECK_RC(mpasg_moist_coefficients(m, c, &f, stream));
   int a = 0;
   for (int sub = 1; sub <= T.hi; ++sub) {

@@ -69,6 +69,7 @@ int step_jvp(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, mpasg_f
     nsub[0] = nsub[1] = ns / 2 > 1 ? ns / 2 : 1; nsub[2] = ns;
   }
   CHECK_RC(saves_both(m, &f, d, s));
+  CHECK_RC(mpasgi_pvu(m, &f, s));
   CHECK_RC(mpasg_moist_coefficients(m, c, &f, stream));  // dry: constants, no tangent
   for (int sub = 1; sub <= split; ++sub) {
     for (int rk = 1; rk <= 3; ++rk) {

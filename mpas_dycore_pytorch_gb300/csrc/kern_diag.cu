@@ -2,6 +2,7 @@
 // cell-centre wind reconstruction (dynamics/vector_reconstruction.py:311) and the
 // cold-start coupled diagnostics (dynamics/init_coupled_diagnostics.py:147).
 #include "common.cuh"
+#include "trisk.cuh"
 #include "pow_exner.cuh"
 
 namespace {
@@ -44,13 +45,16 @@ __global__ void k_diag_vertices(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const double iat = m.invAreaTriangle[v];
   vort = vort * iat;
   f.vorticity[i] = vort;
-  f.ke_vertex[i] = f64(T(0.25) * G(invAreaTriangle)[v] * kev);
+  // (float64 form: k_diag_cells_fx applies the factor 0.25)
+  f.ke_vertex[i] = sizeof(T) == sizeof(double) ? f64(G(invAreaTriangle)[v] * kev)
+                                               : f64(T(0.25) * G(invAreaTriangle)[v] * kev);
   const double pvv = m.fVertex[v] + vort;
   f.pv_vertex[i] = pvv;
   if (sizeof(T) != sizeof(double)) f.pv_vertex_f32[i] = d2f_bits(pvv);
 }
 
-// divergence, cell kinetic energy (with the vertex-kite blend) and cell PV for APVM
+// divergence, cell kinetic energy (with the vertex-kite blend) and cell PV for APVM (mixed
+// form; float64: k_diag_cells_fx)
 template <typename T>
 __global__ void k_diag_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm) {
   const int L = m.nVertLevels;
@@ -98,7 +102,8 @@ __global__ void k_diag_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm)
   if (apvm) f.pv_cell[i] = f64(pvc);
 }
 
-// pv_edge (with APVM upwinding) and, at rk 3 / preparation, the TRiSK tangential wind
+// pv_edge (with APVM upwinding) and, at rk 3 / preparation, the TRiSK tangential wind (mixed
+// form; float64: k_diag_edges_b_fx)
 template <typename T>
 __global__ void k_diag_edges_b(mpasg_mesh m, mpasg_fields f, FastDiv fl, int recompute_v, double apvm_dt,
                                int apvm) {
@@ -134,6 +139,161 @@ __global__ void k_diag_edges_b(mpasg_mesh m, mpasg_fields f, FastDiv fl, int rec
   }
   f.pv_edge[i] = f64(pve);
   if (sizeof(T) != sizeof(double)) f.pv_edge_f32[i] = pve;
+}
+
+// ---------------------------------------------------------------- float64 form
+// k_diag_cells in float64 took 52 operations a level (217 us at 40962 x 55), most of them the
+// per-slot products of the vertex blend.  The area factors are taken out of the sums, the
+// divergence and the PV sum run on the integer pipes (fixdot.cuh), the kinetic energies on
+// the float64 pipe: 17 operations a level.
+// Block tables: per cell N divergence weights sign dvEdge (row: edge), then N kite weights
+// (row: vertex), then the kite areas as float64.
+template <int N>
+MPASG_D void load_cell_tables(const mpasg_mesh& m, uint32_t c0, uint32_t n, fx::Weight* edge, fx::Weight* kite,
+                              double* area) {
+  for (uint32_t t = threadIdx.x; t < n * N; t += blockDim.x) {
+    const uint32_t cl = t / N, j = t - cl * N, c = c0 + cl;
+    const size_t o = (size_t)c * m.maxEdges;
+    const int nc = m.nEdgesOnCell[c];
+    const uint32_t none = nc > N ? fx::kBadWeight : 0u;
+    fx::Weight we{0, 0, none, nc > 0 ? m.edgesOnCell[o] : 0}, wk{0, 0, none, 0};
+    double a = 0.0;
+    if ((int)j < nc && nc <= N) {
+      we = fx::weight(m.cell_edge_sdv[o + j], m.edgesOnCell[o + j]);
+      const int v = m.verticesOnCell[o + j], kk = m.kiteForCell[o + j];
+      if (v < m.nVertices && kk >= 0) {
+        a = m.kiteAreasOnVertex[(size_t)v * m.vertexDegree + kk];
+        wk = fx::weight(a, v);
+      }
+    }
+    edge[t] = we;
+    kite[t] = wk;
+    area[t] = a;
+  }
+}
+
+// the same sums over any number of slots, in float64
+MPASG_D void wide_cell_sums(const mpasg_mesh& m, const mpasg_fields& f, uint32_t c, uint32_t k, double* div,
+                            double* kee, double* kev, double* pv) {
+  const uint32_t L = (uint32_t)m.nVertLevels;
+  const size_t o = (size_t)c * m.maxEdges;
+  *div = *kee = *kev = *pv = 0.0;
+  for (int j = 0; j < m.nEdgesOnCell[c]; ++j) {
+    const size_t ie = (size_t)m.edgesOnCell[o + j] * L + k;
+    *div = fma(m.cell_edge_sdv[o + j], f.u[ie], *div);
+    *kee = *kee + f.ke_edge[ie];
+    const int v = m.verticesOnCell[o + j], kk = m.kiteForCell[o + j];
+    if (v >= m.nVertices || kk < 0) continue;
+    const double a = m.kiteAreasOnVertex[(size_t)v * m.vertexDegree + kk];
+    *kev = fma(a, f.ke_vertex[(size_t)v * L + k], *kev);
+    *pv = fma(a, f.pv_vertex[(size_t)v * L + k], *pv);
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm) {
+  extern __shared__ fx::Weight s_w[];
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nCells * L;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fl.div(i0), nc = fl.div(min(i0 + kBlock, n_all) - 1u) - c0 + 1;
+  fx::Weight* s_k = s_w + nc * N;
+  double* s_a = reinterpret_cast<double*>(s_k + nc * N);
+  load_cell_tables<N>(m, c0, nc, s_w, s_k, s_a);
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t c = fl.div(i), k = i - c * L, t = (c - c0) * N;
+  const int n = m.nEdgesOnCell[c];
+  double div, kee = 0.0, kev = 0.0, pv = 0.0;
+  if (n > N) {
+    wide_cell_sums(m, f, c, k, &div, &kee, &kev, &pv);
+  } else {
+    double x[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = f.u[(uint32_t)s_w[t + j].row * L + k];
+    bool ok = fx::dot<N>(x, s_w + t, &div);
+    if (apvm) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) x[j] = f.pv_vertex[(uint32_t)s_k[t + j].row * L + k];
+      ok = fx::dot<N>(x, s_k + t, &pv) && ok;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (j < n) {
+        kee = j == 0 ? f.ke_edge[(uint32_t)s_w[t + j].row * L + k] : kee + f.ke_edge[(uint32_t)s_w[t + j].row * L + k];
+        kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
+      }
+    if (!ok) {
+      double a, b;
+      wide_cell_sums(m, f, c, k, &div, &a, &b, &pv);
+    }
+  }
+  const double ia = m.invAreaCell[c];
+  f.divergence[i] = div * ia;
+  // 0.25 (0.625 sum_j ke_edge + 0.375 sum_j kite ke_vertex) / area
+  f.ke[i] = ia * fma(0.625 * 0.25, kee, (0.375 * 0.25) * kev);
+  if (apvm) f.pv_cell[i] = pv * ia;
+}
+
+// k_diag_edges_b in float64 (165 us, mean of a step's launches): the APVM factors are formed
+// once per block and edge, the tangential wind (rk 3 and preparation) on the integer pipes;
+// pv_edge * u, which the next u tendency reads, is left in ke_edge.
+struct ApvmEdge {
+  double gt, gn;  // apvm_dt / dv, apvm_dt / dc
+};
+
+template <int N, bool V>
+__global__ void __launch_bounds__(kBlock, 5) k_diag_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, double apvm_dt,
+                                                         int apvm) {
+  extern __shared__ fx::Weight s_w[];
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nEdges * L;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t e0 = fl.div(i0), ne = fl.div(min(i0 + kBlock, n_all) - 1u) - e0 + 1;
+  ApvmEdge* s_a = reinterpret_cast<ApvmEdge*>(s_w + (V ? ne * N : 0));
+  if (V) trisk::load<N>(m, e0, ne, s_w);
+  for (uint32_t t = threadIdx.x; t < ne; t += kBlock)
+    s_a[t] = ApvmEdge{apvm_dt * m.invDvEdge[e0 + t], apvm_dt * m.invDcEdge[e0 + t]};
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t e = fl.div(i), k = i - e * L;
+  const size_t v1 = (size_t)m.verticesOnEdge[2 * e], v2 = (size_t)m.verticesOnEdge[2 * e + 1];
+  const double pv1 = f.pv_vertex[v1 * L + k], pv2 = f.pv_vertex[v2 * L + k], u = f.u[i];
+  double vv;
+  if (V) {
+    vv = trisk::sum<N>(m, f.u, s_w + (e - e0) * N, e, k, L);
+    f.v[i] = vv;
+  } else {
+    vv = f.v[i];
+  }
+  double pve = 0.5 * (pv1 + pv2);
+  if (apvm) {
+    const size_t c1 = (size_t)m.cellsOnEdge[2 * e], c2 = (size_t)m.cellsOnEdge[2 * e + 1];
+    const ApvmEdge a = s_a[e - e0];
+    const double delta = fma(u, (f.pv_cell[c2 * L + k] - f.pv_cell[c1 * L + k]) * a.gn, vv * ((pv2 - pv1) * a.gt));
+    pve = pve - delta;
+  }
+  f.pv_edge[i] = pve;
+  f.ke_edge[i] = pve * u;
+}
+
+int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, int rk_step, int apvm,
+                   cudaStream_t s) {
+  const int L = m->nVertLevels, rows = (kBlock - 1) / L + 2;
+  const int nc = nblocks((long long)m->nCells * L), ne = nblocks((long long)m->nEdges * L);
+  const FastDiv fl(L);
+  const size_t slot = 2 * sizeof(fx::Weight) + sizeof(double);
+  if (m->maxEdges <= 6) k_diag_cells_fx<6><<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm);
+  else k_diag_cells_fx<10><<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm);
+  MPASG_LAUNCH_CHECK();
+  const double adt = c->apvm_upwinding * c->dt;
+  const size_t se = rows * sizeof(ApvmEdge);
+  if (rk_step != 3)
+    k_diag_edges_b_fx<1, false><<<ne, kBlock, se, s>>>(*m, *f, fl, adt, apvm);
+  else if (m->maxEdges2 <= 10)
+    k_diag_edges_b_fx<10, true><<<ne, kBlock, se + rows * 10 * sizeof(fx::Weight), s>>>(*m, *f, fl, adt, apvm);
+  else
+    k_diag_edges_b_fx<14, true><<<ne, kBlock, se + rows * 14 * sizeof(fx::Weight), s>>>(*m, *f, fl, adt, apvm);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
 }
 
 // mpas_reconstruct_2d: RBF reconstruction of the cell-centre wind
@@ -374,6 +534,7 @@ int launch_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields*
   MPASG_LAUNCH_CHECK();
   k_diag_vertices<T><<<nblocks((long long)m->nVertices * L), kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
+  if constexpr (sizeof(T) == sizeof(double)) return launch_diag_fx(m, c, f, rk_step, apvm, s);
   k_diag_cells<T><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, fl, apvm);
   MPASG_LAUNCH_CHECK();
   k_diag_edges_b<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(

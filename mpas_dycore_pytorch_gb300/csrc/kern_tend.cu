@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "advstencil.cuh"
 #include "cellsum.cuh"
+#include "trisk.cuh"
 
 namespace {
 
@@ -105,8 +106,9 @@ MPASG_D T wduz_at(const T* __restrict__ u, T rwe, int kk, int L, const T* fzm, c
 }
 
 // pv_edge * u at every edge level, the neighbour factor of the float64 PV flux sum (below),
-// formed once per tendency stage instead of once per reading edge; stored in ke_edge (the
-// diagnostics' edge kinetic-energy scratch, free between two diagnostics stages)
+// stored in ke_edge (the diagnostics' edge kinetic-energy scratch).  Inside a step the
+// diagnostics form it (k_diag_edges_b); this kernel serves the first stage and the stage entry
+// point
 __global__ void k_pvu(mpasg_fields f, long long n) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) f.ke_edge[i] = f.pv_edge[i] * f.u[i];
@@ -309,39 +311,11 @@ struct EdgeConst {
   double r_dv, half_ms2;   // rk 1: min(1 / dv, 4 / dc), meshScalingDel2 / 2
 };
 
-// entries of the edges [e0, e0 + n) in the block's weight table
-template <int N>
-MPASG_D void load_trisk(const mpasg_mesh& m, uint32_t e0, uint32_t n, fx::Weight* tab, EdgeConst* ec) {
-  const int me2 = m.maxEdges2;
+MPASG_D void load_edge_const(const mpasg_mesh& m, uint32_t e0, uint32_t n, EdgeConst* ec) {
   for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) {
     const double idc = m.invDcEdge[e0 + t];
     ec[t] = EdgeConst{idc, idc + idc, fmin(m.invDvEdge[e0 + t], 4.0 * idc), 0.5 * m.meshScalingDel2[e0 + t]};
   }
-  for (uint32_t t = threadIdx.x; t < n * N; t += blockDim.x) {
-    const uint32_t el = t / N, j = t - el * N, e = e0 + el;
-    const int n2 = m.nEdgesOnEdge[e];
-    if ((int)j < n2 && n2 <= N) {
-      tab[t] = fx::weight(m.weightsOnEdge[e * me2 + j], m.edgesOnEdge[e * me2 + j]);
-    } else {
-      fx::Weight z{0, 0, n2 > N ? fx::kBadWeight : 0u, n2 > 0 ? m.edgesOnEdge[e * me2] : (int)e};
-      tab[t] = z;
-    }
-  }
-}
-
-template <int N>
-MPASG_D double trisk_sum(const mpasg_mesh& m, const double* __restrict__ field, const fx::Weight* w, uint32_t e,
-                         uint32_t k, uint32_t L) {
-  double x[N], out;
-#pragma unroll
-  for (int j = 0; j < N; ++j) x[j] = field[(uint32_t)w[j].row * L + k];
-  if (!fx::dot<N>(x, w, &out)) {
-    out = 0.0;
-    const size_t o = (size_t)e * m.maxEdges2;
-    for (int j = 0; j < m.nEdgesOnEdge[e]; ++j)
-      out = fma(m.weightsOnEdge[o + j], field[(size_t)m.edgesOnEdge[o + j] * L + k], out);
-  }
-  return out;
 }
 
 template <int N, bool RAY = false>
@@ -354,8 +328,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_tend_u_fx(mpasg_mesh m, mpasg_fie
   const double* __restrict__ rw = f.rw;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
   const uint32_t e0 = fl.div(i0), e1 = fl.div(min(i0 + kBlock, n_all) - 1u);
-  EdgeConst* s_e = reinterpret_cast<EdgeConst*>(s_w + (kBlock - 1 + 2 * L) / L * N);
-  load_trisk<N>(m, e0, e1 - e0 + 1, s_w, s_e);
+  EdgeConst* s_e = reinterpret_cast<EdgeConst*>(s_w + (e1 - e0 + 1) * N);
+  trisk::load<N>(m, e0, e1 - e0 + 1, s_w);
+  load_edge_const(m, e0, e1 - e0 + 1, s_e);
   const bool active = i < n_all;
   uint32_t e = e0, k = 0;
   int c1 = 0, c2 = 0;
@@ -380,8 +355,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_tend_u_fx(mpasg_mesh m, mpasg_fie
                             m.fzp);
   const fx::Weight* w = s_w + (e - e0) * N;
   const EdgeConst ec = s_e[e - e0];
-  const double sa = trisk_sum<N>(m, u, w, e, k, L);
-  const double sb = trisk_sum<N>(m, f.ke_edge, w, e, k, L);  // pv u (k_pvu)
+  const double sa = trisk::sum<N>(m, u, w, e, k, L);
+  const double sb = trisk::sum<N>(m, f.ke_edge, w, e, k, L);  // pv u
   const size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2 * L + k;
   const double rho_e = f.h_edge[i], u_k = ue[k];
   const double pv = fma(f.pv_edge[i], sa, sb);  // twice the PV flux
@@ -1111,8 +1086,6 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
   MPASG_LAUNCH_CHECK();
   const bool ray = p.ray_n > 0;
   if constexpr (sizeof(T) == sizeof(double)) {
-    k_pvu<<<nblocks(nel), kBlock, 0, s>>>(*f, nel);
-    MPASG_LAUNCH_CHECK();
     if (ray) launch_tend_u_fx<true>(m, f, p, s);
     else launch_tend_u_fx<false>(m, f, p, s);
   } else {
@@ -1187,6 +1160,13 @@ int mpasgi_theta_dev(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s) {
   return MPASG_OK;
 }
 
+int mpasgi_pvu(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s) {
+  const long long n = (long long)m->nEdges * m->nVertLevels;
+  k_pvu<<<nblocks(n), kBlock, 0, s>>>(*f, n);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
+}
+
 extern "C" int mpasg_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step,
                               void* stream) {
   return mpasgi_dyn_tend(m, c, f, rk_step, (cudaStream_t)stream, false);
@@ -1195,8 +1175,9 @@ extern "C" int mpasg_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_
 int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s,
                     bool copies_current) {
   if (!m || !c || !f || rk_step < 1 || rk_step > 3) return MPASG_E_ARG;
-  if (!copies_current && rk_step > 1 && c->precision != MPASG_PRECISION_MIXED) {
-    const int rc = mpasgi_theta_edge(m, f, false, s);  // the edge mean of theta_m_save read below
+  if (!copies_current && c->precision != MPASG_PRECISION_MIXED) {
+    int rc = mpasgi_pvu(m, f, s);
+    if (rc == MPASG_OK && rk_step > 1) rc = mpasgi_theta_edge(m, f, false, s);  // the edge mean of theta_m_save
     if (rc != MPASG_OK) return rc;
   }
   if (m->nVertLevels < 4) return MPASG_E_ARG;
