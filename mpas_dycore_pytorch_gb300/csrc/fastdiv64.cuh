@@ -9,8 +9,8 @@
 //   reciprocal  r + r (1 - b r)                         (3)
 // Both last steps round once a value known to 2^-88, so the result is the correctly rounded
 // one but for about one argument in 2^34 (Markstein's residual correction).  Divisors outside
-// [2^-60, 2^60), negative or not finite, and dividends below 2^-700 or not finite take the
-// compiler's division.
+// [2^-100, 2^70), negative or not finite, and nonzero dividends below 2^-600 or not finite take
+// the compiler's division.
 #pragma once
 
 #include <math.h>
@@ -53,8 +53,9 @@ FX_HD double widen(float f) {
   return from_bits((uint64_t)hi << 32 | (b << 29));
 }
 
-// exponent inside [2^-60, 2^60) and positive
-FX_HD bool plain_divisor(double b) { return (uint32_t)(bits_of(b) >> 32) - ((1023u - 60u) << 20) < (120u << 20); }
+// positive, exponent inside [2^-100, 2^70): the float32 parts of b and 1 / b stay normal, what
+// widen() adds to a zero correction (2^-127) is below 2^-57 of 1 / b
+FX_HD bool plain_divisor(double b) { return (uint32_t)(bits_of(b) >> 32) - ((1023u - 100u) << 20) < (170u << 20); }
 
 // 1 / b to about 2^-44 for a plain divisor; `r0` (tests) replaces the float32 seed
 FX_HD double rcp44(double b, float r0) {
@@ -85,12 +86,12 @@ FX_HD double quotient_from(double a, double b, double r) {
   const double q = a * r;
   return fma(fma(-b, q, a), r, q);
 }
-// whether a dividend keeps the residual a - b q exact: at least 2^-700 and finite
+// whether a dividend keeps the residual a - b q exact and the quotient finite
 FX_HD bool plain_dividend(double a) {
-  return (((uint32_t)(bits_of(a) >> 32) & 0x7fffffffu) - ((1023u - 700u) << 20)) < ((700u + 900u) << 20);
+  return (((uint32_t)(bits_of(a) >> 32) & 0x7fffffffu) - ((1023u - 600u) << 20)) < (1400u << 20);
 }
 FX_HD double quotient(double a, double b) {
-  if (!plain_divisor(b) || !plain_dividend(a)) return a / b;
+  if (!plain_divisor(b) || !plain_dividend(a)) return plain_divisor(b) && is_zero(a) ? a : a / b;
   return quotient_from(a, b, rcp44(b, seed_of(b)));
 }
 

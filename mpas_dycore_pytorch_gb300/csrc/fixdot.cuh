@@ -202,4 +202,47 @@ FX_HD bool sum(const double (&x)[N], const uint32_t (&sgn)[N], double* out) {
   return true;
 }
 
+// The positive and the negative part of the terms s_j x_j, *pos = sum of the positive ones and
+// *neg = minus the sum of the negative ones, from one alignment.  False as for dot().
+template <int N>
+FX_HD bool sum_parts(const double (&x)[N], const uint32_t (&sgn)[N], double* pos, double* neg) {
+  static_assert(N <= 8, "the 64-bit sum holds 8 terms");
+  uint32_t amax = 0u;
+#pragma unroll
+  for (int j = 0; j < N; ++j) amax = umax(amax, (uint32_t)(bits_of(x[j]) >> 32) & kExpMask);
+  if ((amax >> 20) - 128u > 1912u) {
+    *pos = *neg = 0.0;
+    return amax == 0u && all_zero(x);
+  }
+  uint64_t p = 0u, q = 0u;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint64_t b = bits_of(x[j]);
+    const uint32_t hi = (uint32_t)(b >> 32);
+    const uint64_t t = (uint64_t)aligned(hi, (uint32_t)b, (amax - (hi & kExpMask)) >> 20, 0u);
+    if ((int32_t)(hi ^ sgn[j]) < 0) q += t;
+    else p += t;
+  }
+  *pos = pack(p, 0u, (int)(amax >> 20) + 4, false);
+  *neg = pack(q, 0u, (int)(amax >> 20) + 4, false);
+  return true;
+}
+
+FX_HD bool is_finite(double x) { return ((uint32_t)(bits_of(x) >> 32) & kExpMask) != kExpMask; }
+// x where x > 0, else +0 (NaN gives 0)
+FX_HD double positive(double x) { return bits_of(x) - 1u < 0x7ff0000000000000ull ? x : 0.0; }
+// min(max(x, 0), 1), NaN gives 0
+FX_HD double clamp01(double x) {
+  const uint64_t b = bits_of(positive(x));
+  return from_bits(b < 0x3ff0000000000000ull ? b : 0x3ff0000000000000ull);
+}
+// the smaller of two values in [0, inf]
+FX_HD double min_nonneg(double a, double b) { return bits_of(a) < bits_of(b) ? a : b; }
+// float64 order as integer order (negative values mirrored)
+FX_HD int64_t order_key(double x) {
+  const int64_t b = (int64_t)bits_of(x);
+  return b ^ (int64_t)((uint64_t)(b >> 63) >> 1);
+}
+FX_HD double from_order_key(int64_t k) { return from_bits((uint64_t)(k ^ (int64_t)((uint64_t)(k >> 63) >> 1))); }
+
 }  // namespace fx

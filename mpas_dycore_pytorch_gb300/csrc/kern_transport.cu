@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "advstencil.cuh"
+#include "cellsum.cuh"
 
 namespace {
 
@@ -12,7 +13,10 @@ namespace {
 // In the mixed form the edge values, flux divergences, bounds and limiter factors are
 // float32; the density weighting and the stage update of each scalar are float64.
 
-// sum_m (adv_coefs + sign(uh) adv_coefs_3rd) q[advCell_m]  for every scalar
+template <typename T>
+MPASG_D T mz(T x) { return x > T(0) ? x : T(0); }
+
+// sum_m (adv_coefs + sign(uh) adv_coefs_3rd) q[advCell_m]  for every scalar (mixed form)
 template <typename T>
 __global__ void k_pattern_c(mpasg_mesh m, FastDiv fl, int S, const double* __restrict__ uh,
                             const double* __restrict__ q, double* __restrict__ out, int times_uh) {
@@ -38,18 +42,49 @@ __global__ void k_pattern_c(mpasg_mesh m, FastDiv fl, int S, const double* __res
   for (int s = 0; s < S; ++s) out[(size_t)i * S + s] = f64(times_uh ? u * acc[s] : acc[s]);
 }
 
-// The float64 form.  A row of an edge, its (level, scalar) values in memory order, is cut in
-// two halves and a thread takes the same place of both: the first half's sum on the integer
-// pipes (fixdot.cuh), the second's on the float64 pipe beside it, so both are busy, and
-// neighbouring threads read neighbouring values.  Weights are converted once per block and edge.
-// 40962 x 55 with 3 tracers: 392 -> 363 us; 2562 x 37 with 8: 73 -> 47 us (48 registers; with
-// the two sums of a thread interleaved instruction by instruction 481 and 62 us, the
-// registers costing more warps than the overlap inside a warp gives).
-template <int N>
-__global__ void __launch_bounds__(kBlock, 5) k_pattern_c_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t n_all,
-                                                            uint32_t half, const double* __restrict__ uh,
-                                                            const double* __restrict__ q, double* __restrict__ out,
-                                                            int times_uh) {
+// ---------------------------------------------------------------- float64 form
+// A thread takes one (level, scalar) value of a row, so neighbouring threads read neighbouring
+// values and a scalar costs no strided pass; the horizontal sums run on the integer pipes
+// (fixdot.cuh), comparisons, minima and clamps on the integer side too (each would take a
+// float64 slot).
+struct TransportScalars {
+  double dt, w_old, w_new, f3[4];  // f3: 7 + 3 c, 7 - 3 c, 1 + c, 1 - c of the upwind flux3
+};
+
+inline TransportScalars transport_scalars(double dt, double w_old, double w_new, double c) {
+  return TransportScalars{dt, w_old, w_new, {7.0 + 3.0 * c, 7.0 - 3.0 * c, 1.0 + c, 1.0 - c}};
+}
+
+// Horizontal edge fluxes.  A row of an edge is cut in two halves and a thread takes the same
+// place of both: the first half's sum on the integer pipes, the second's on the float64 pipe
+// beside it.  Weights are converted once per block and edge.
+// MONO: out = the upwind flux of s_old, out2 = dt times the high-order flux minus it;
+// else out = the high-order flux.
+// 40962 x 55 with 3 tracers, edge values only: 392 -> 363 us; 2562 x 37 with 8: 73 -> 47 us (48
+// registers; with the two sums of a thread interleaved instruction by instruction 481 and 62
+// us, the registers costing more warps than the overlap inside a warp gives).
+template <bool MONO>
+MPASG_D void store_edge_flux(const mpasg_mesh& m, uint32_t e, uint32_t row, uint32_t r, double u, double value,
+                             double dvdt, double dt, const double* __restrict__ s_old, double* __restrict__ out,
+                             double* __restrict__ out2) {
+  const size_t o = (size_t)e * row + r;
+  const double flux = u * value;
+  if (!MONO) {
+    out[o] = flux;
+    return;
+  }
+  const int up = m.cellsOnEdge[2 * e + (__double2hiint(u) < 0 ? 1 : 0)];
+  const double fup = dvdt * (u * s_old[(size_t)up * row + r]);
+  out[o] = fup;
+  out2[o] = fma(dt, flux, -fup);
+}
+
+template <int N, bool MONO>
+__global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t n_all,
+                                                         uint32_t half, double dt, const double* __restrict__ uh,
+                                                         const double* __restrict__ q,
+                                                         const double* __restrict__ s_old, double* __restrict__ out,
+                                                         double* __restrict__ out2) {
   extern __shared__ fx::Weight s_w[];
   const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
@@ -59,34 +94,285 @@ __global__ void __launch_bounds__(kBlock, 5) k_pattern_c_fx(mpasg_mesh m, FastDi
   if (i >= n_all) return;
   const uint32_t e = fh.div(i), a = i - e * half, b = a + half;
   const fx::Weight* w = s_w + (e - e0) * (2 * N);
-  double* o = out + (size_t)e * row;
   double x[N], acc;
-  const double ua = uh[(size_t)e * L + fs.div(a)];
+  const double ua = uh[(size_t)e * L + fs.div(a)], dvdt = MONO ? m.dvEdge[e] * dt : 0.0;
   const bool back = __double2hiint(ua) < 0;
   if (back) w += N;
 #pragma unroll
   for (int j = 0; j < N; ++j) x[j] = q[(size_t)w[j].row * row + a];
   if (b < row) {
     const double ub = uh[(size_t)e * L + fs.div(b)];
-    const double t = adv::sum(m, e, __double2hiint(ub) < 0, q, row, b);
-    o[b] = times_uh ? ub * t : t;
+    store_edge_flux<MONO>(m, e, row, b, ub, adv::sum(m, e, __double2hiint(ub) < 0, q, row, b), dvdt, dt, s_old, out,
+                          out2);
   }
   if (!fx::dot<N>(x, w, &acc)) acc = adv::sum(m, e, back, q, row, a);
-  o[a] = times_uh ? ua * acc : acc;
+  store_edge_flux<MONO>(m, e, row, a, ua, acc, dvdt, dt, s_old, out, out2);
 }
 
-int launch_pattern_c_fx(const mpasg_mesh* m, int S, const double* uh, const double* q, double* out, int times_uh,
-                        cudaStream_t s) {
+template <bool MONO>
+int launch_edge_flux_fx(const mpasg_mesh* m, int S, double dt, const double* uh, const double* q, const double* s_old,
+                        double* out, double* out2, cudaStream_t s) {
   const uint32_t half = ((uint32_t)m->nVertLevels * S + 1) / 2, n = (uint32_t)m->nEdges * half;
   const size_t smem = (size_t)((kBlock - 1) / half + 2) * adv::kEntryBytes;
   if (m->nAdvMax <= 10)
-    k_pattern_c_fx<10><<<nblocks(n), kBlock, smem * 10, s>>>(*m, FastDiv(half), FastDiv(S), n, half, uh, q, out,
-                                                             times_uh);
+    k_edge_flux_fx<10, MONO><<<nblocks(n), kBlock, smem * 10, s>>>(*m, FastDiv(half), FastDiv(S), n, half, dt, uh, q,
+                                                                   s_old, out, out2);
   else
-    k_pattern_c_fx<14><<<nblocks(n), kBlock, smem * 14, s>>>(*m, FastDiv(half), FastDiv(S), n, half, uh, q, out,
-                                                             times_uh);
+    k_edge_flux_fx<14, MONO><<<nblocks(n), kBlock, smem * 14, s>>>(*m, FastDiv(half), FastDiv(S), n, half, dt, uh, q,
+                                                                   s_old, out, out2);
   MPASG_LAUNCH_CHECK();
   return MPASG_OK;
+}
+
+// the thread's place in a (cell, level, scalar) row
+struct CellRow {
+  uint32_t c, r, k, s;
+};
+MPASG_D CellRow cell_row(uint32_t i, uint32_t row, const FastDiv& fr, const FastDiv& fs) {
+  CellRow t;
+  t.c = fr.div(i);
+  t.r = i - t.c * row;
+  t.k = fs.div(t.r);
+  t.s = t.r - t.k * fs.d;
+  return t;
+}
+
+// vertical flux at the interface below level k, a linear combination of the column's values
+// times the interface velocity: returns the combination (times 12 inside) in *comb and the
+// factor 1 or 1/12 that goes with it
+MPASG_D double interface_value(const double* __restrict__ q, uint32_t S, double ww, uint32_t k, uint32_t L,
+                               const double* fnm, const double* fnp, const double* f3, double* factor) {
+  if (k == 1 || k == L - 1) {
+    *factor = 1.0;
+    return fma(fnm[k], q[0], fnp[k] * q[-(int)S]);
+  }
+  *factor = kInv12;
+  const bool down = __double2hiint(ww) < 0;
+  const int s = (int)S;
+  const double a = q[down ? 0 : -s], b = q[down ? -s : 0], a2 = q[down ? s : -2 * s], b2 = q[down ? -2 * s : s];
+  return fma(f3[0], a, fma(f3[1], b, -fma(f3[2], a2, f3[3] * b2)));
+}
+
+// explicit stage update: 17 float64 operations a value and one integer sum, about 33 in the
+// per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage)
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
+                                                              TransportScalars p, const double* __restrict__ s_old,
+                                                              const double* __restrict__ s_new,
+                                                              double* __restrict__ s_out) {
+  extern __shared__ cellsum::Slot s_c[];
+  __shared__ double s_wd[kBlock];
+  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S, n_all = (uint32_t)m.nCells * row;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
+  cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
+  const bool active = i < n_all;
+  CellRow t{c0, 0, 0, 0};
+  auto flux_at = [&](uint32_t k) {  // at the interface below level k of this thread's column
+    if (k == 0 || k >= L) return 0.0;
+    const double ww = f.wwAvg[(size_t)t.c * (L + 1) + k];
+    double fac;
+    const double v = interface_value(s_new + (size_t)t.c * row + k * S + t.s, S, ww, k, L, m.fnm, m.fnp, p.f3, &fac);
+    return (ww * fac) * v;
+  };
+  double lo = 0.0;
+  if (active) {
+    t = cell_row(i, row, fr, fs);
+    lo = flux_at(t.k);
+  }
+  s_wd[threadIdx.x] = lo;
+  __syncthreads();
+  if (!active) return;
+  const double hi = t.k + 1 >= L ? 0.0 : threadIdx.x + S < kBlock ? s_wd[threadIdx.x + S] : flux_at(t.k + 1);
+  const double div = cellsum::fixed<N>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
+  const size_t ic = (size_t)t.c * L + t.k;
+  const double tend = fma(m.rdnw[t.k], lo - hi, -(div * m.invAreaCell[t.c]));
+  const double rho_old = f.rho_zz_old_split[ic];
+  double rho = f.rho_zz[ic];
+  if (p.w_old != 0.0) rho = p.w_old * rho_old + p.w_new * rho;
+  s_out[i] = fx::quotient(fma(p.dt, tend, s_old[i] * rho_old), rho);
+}
+
+// monotone stage: density at its end
+__global__ void k_mono_density_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, double dt) {
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nCells * L;
+  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= n_all) return;
+  const uint32_t c = fl.div(i), k = i - c * L;
+  const size_t o = (size_t)c * m.maxEdges, ow = (size_t)c * (L + 1) + k;
+  double h = 0.0;
+  for (int j = 0; j < m.nEdgesOnCell[c]; ++j)
+    h = fma(m.cell_edge_geo[o + j], f.ruAvg[(size_t)m.edgesOnCell[o + j] * L + k], h);
+  f.rho_int[i] = f.rho_zz_old_split[i] - dt * fma(m.rdnw[k], f.wwAvg[ow + 1] - f.wwAvg[ow], h);
+}
+
+// Monotone stage, per value: local and neighbour bounds, vertical upwind update, vertical parts
+// of the limiter scale sums; the high-minus-upwind vertical flux at the interface below the
+// level goes to wflux (k >= 1).  The 18 minima and maxima of the bounds are integer comparisons
+// (735 -> 273 us at 40962 x 55 x 3, and 40 us for the density).
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
+                                                            TransportScalars p, const double* __restrict__ so,
+                                                            const double* __restrict__ sn) {
+  __shared__ double s_wm[kBlock], s_fu[kBlock];
+  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S, n_all = (uint32_t)m.nCells * row;
+  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+  const bool active = i < n_all;
+  CellRow t{0, 0, 0, 0};
+  auto fluxes = [&](uint32_t k, double* wm, double* fu) {
+    *wm = *fu = 0.0;
+    if (k == 0 || k >= L) return;
+    const double ww = f.wwAvg[(size_t)t.c * (L + 1) + k], dtw = p.dt * ww;
+    const size_t o = (size_t)t.c * row + k * S + t.s;
+    double fac;
+    const double v = interface_value(sn + o, S, ww, k, L, m.fnm, m.fnp, p.f3, &fac);
+    *fu = dtw * so[__double2hiint(ww) < 0 ? o : o - S];
+    *wm = fma(dtw * fac, v, -*fu);
+  };
+  double wm_lo = 0.0, fu_lo = 0.0;
+  if (active) {
+    t = cell_row(i, row, fr, fs);
+    fluxes(t.k, &wm_lo, &fu_lo);
+  }
+  s_wm[threadIdx.x] = wm_lo;
+  s_fu[threadIdx.x] = fu_lo;
+  __syncthreads();
+  if (!active) return;
+  double wm_hi = 0.0, fu_hi = 0.0;
+  if (t.k + 1 < L) {
+    if (threadIdx.x + S < kBlock) {
+      wm_hi = s_wm[threadIdx.x + S];
+      fu_hi = s_fu[threadIdx.x + S];
+    } else {
+      fluxes(t.k + 1, &wm_hi, &fu_hi);
+    }
+  }
+  if (t.k >= 1) f.wflux[((size_t)t.c * (L + 1) + t.k) * S + t.s] = wm_lo;
+  // bounds over the column's neighbours and the adjacent cells
+  const double here = so[i];
+  int64_t kmax = fx::order_key(here), kmin = kmax;
+  auto bound = [&](double x) {
+    const int64_t q = fx::order_key(x);
+    kmax = q > kmax ? q : kmax;
+    kmin = q < kmin ? q : kmin;
+  };
+  if (t.k >= 1) bound(so[i - S]);
+  if (t.k + 1 < L) bound(so[i + S]);
+  const size_t oc = (size_t)t.c * m.maxEdges;
+  const int n = m.nEdgesOnCell[t.c];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (j < n) {
+      const int nb = m.cellsOnCell[oc + j];
+      if (nb < m.nCells) bound(so[(size_t)nb * row + t.r]);
+    }
+  }
+  for (int j = N; j < n; ++j) {
+    const int nb = m.cellsOnCell[oc + j];
+    if (nb < m.nCells) bound(so[(size_t)nb * row + t.r]);
+  }
+  double smax = fx::from_order_key(kmax), smin = fx::from_order_key(kmin);
+  if (!(fx::is_finite(smax) && fx::is_finite(smin))) {  // a NaN among them: left out, as fmax / fmin do
+    smax = smin = here;
+    auto wide = [&](double x) {
+      smax = fmax(smax, x);
+      smin = fmin(smin, x);
+    };
+    if (t.k >= 1) wide(so[i - S]);
+    if (t.k + 1 < L) wide(so[i + S]);
+    for (int j = 0; j < n; ++j) {
+      const int nb = m.cellsOnCell[oc + j];
+      if (nb < m.nCells) wide(so[(size_t)nb * row + t.r]);
+    }
+  }
+  const double rd = m.rdnw[t.k];
+  f.rows[i] = fma(rd, fu_lo - fu_hi, here * f.rho_zz_old_split[(size_t)t.c * L + t.k]);
+  // in and out fluxes of the correction through the level's two interfaces
+  f.scale_in[i] = rd * (fx::positive(wm_lo) + fx::positive(-wm_hi));
+  f.scale_out[i] = -rd * (fx::positive(wm_hi) + fx::positive(-wm_lo));
+  f.s_max[i] = smax;
+  f.s_min[i] = smin;
+}
+
+// per value: horizontal upwind update and scale sums, then the limiter factors.  Three integer
+// sums and 13 float64 operations a value, about 65 with the comparisons and divisions of the
+// per-cell loop (913 -> 256 us at 40962 x 55 x 3).
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs) {
+  extern __shared__ cellsum::Slot s_c[];
+  const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d, n_all = (uint32_t)m.nCells * row;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
+  cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
+  __syncthreads();
+  if (i >= n_all) return;
+  const CellRow t = cell_row(i, row, fr, fs);
+  const int n = m.nEdgesOnCell[t.c];
+  const cellsum::Slot* s = s_c + (t.c - c0) * N;
+  const double ia = m.invAreaCell[t.c], rint = f.rho_int[(size_t)t.c * L + t.k];
+  const double up = cellsum::fixed<N>(m, t.c, n, s, f.flux_up, row, t.r);
+  double out = 0.0, in = 0.0;
+  bool ok = n <= N;
+  if (ok) {
+    double x[N];
+    uint32_t sgn[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      x[j] = j < n ? f.flux_tmp[(size_t)s[j].row * row + t.r] : 0.0;
+      sgn[j] = s[j].sgn;
+    }
+    ok = fx::sum_parts<N>(x, sgn, &out, &in);
+  }
+  if (!ok) {
+    out = in = 0.0;
+    const size_t o = (size_t)t.c * m.maxEdges;
+    for (int j = 0; j < n; ++j) {
+      const double sf = m.edgesOnCell_sign[o + j] * f.flux_tmp[(size_t)m.edgesOnCell[o + j] * row + t.r];
+      out = out + mz(sf);
+      in = in + mz(-sf);
+    }
+  }
+  const double rows = fma(-ia, up, f.rows[i]), eps = 1.0e-20;
+  const double sin_ = fma(ia, in, f.scale_in[i]) + eps, sout = fma(ia, out, -f.scale_out[i]) + eps;
+  f.rows[i] = rows;
+  f.scale_in[i] = fx::clamp01(fx::quotient(fma(f.s_max[i], rint, -rows), sin_));
+  f.scale_out[i] = fx::clamp01(fx::quotient(fma(-f.s_min[i], rint, rows), sout));
+}
+
+// per (edge, value): limited horizontal flux (stored in hflux)
+__global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint32_t n_all) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_all) return;
+  const uint32_t e = fr.div(i), r = i - e * fr.d;
+  const double ft = f.flux_tmp[i];
+  const uint32_t back = __double2hiint(ft) < 0 ? 1u : 0u;
+  const size_t from = (size_t)m.cellsOnEdge[2 * e + back] * fr.d + r;
+  const size_t to = (size_t)m.cellsOnEdge[2 * e + 1 - back] * fr.d + r;
+  f.hflux[i] = ft * fx::min_nonneg(f.scale_out[from], f.scale_in[to]);
+}
+
+// per value: limited horizontal and vertical fluxes, positivity
+template <int N>
+__global__ void __launch_bounds__(kBlock, 5) k_mono_cells_c_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
+                                                            double* __restrict__ s_out) {
+  extern __shared__ cellsum::Slot s_c[];
+  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S, n_all = (uint32_t)m.nCells * row;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
+  cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
+  __syncthreads();
+  if (i >= n_all) return;
+  const CellRow t = cell_row(i, row, fr, fs);
+  const double* wf = f.wflux + ((size_t)t.c * (L + 1) + t.k) * S + t.s;
+  auto limited = [&](double wm, uint32_t below, uint32_t above) {  // an upward flux leaves `below`
+    const bool down = __double2hiint(wm) < 0;
+    return wm * fx::min_nonneg(f.scale_out[down ? above : below], f.scale_in[down ? below : above]);
+  };
+  const double lo = t.k >= 1 ? limited(wf[0], i - S, i) : 0.0;
+  const double hi = t.k + 1 < L ? limited(wf[S], i, i + S) : 0.0;
+  const double h = cellsum::fixed<N>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
+  const double rows = fma(m.rdnw[t.k], lo - hi, fma(-m.invAreaCell[t.c], h, f.rows[i]));
+  s_out[i] = fx::positive(fx::quotient(rows, f.rho_int[(size_t)t.c * L + t.k]));
 }
 
 template <typename T>
@@ -99,7 +385,7 @@ MPASG_D T wdtn_at(const double* sn, const double* ww, int kk, int L, int S, int 
                   cv<T>(sn[(kk + 1) * S + s]), cv<T>(ww[kk]), coef3);
 }
 
-// explicit stage update for all scalars at (cell, level)
+// explicit stage update for all scalars at (cell, level) (mixed form)
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_scalars_update(mpasg_mesh m, mpasg_fields f, FastDiv fl, int S,
                                                            double dt, double w_old, double w_new, double coef3,
@@ -155,9 +441,7 @@ __global__ void __launch_bounds__(kBlock) k_scalars_update(mpasg_mesh m, mpasg_f
   }
 }
 
-// ---------------------------------------------------------------- monotone stage
-template <typename T>
-MPASG_D T mz(T x) { return x > T(0) ? x : T(0); }
+// ---------------------------------------------------------------- monotone stage, mixed form
 
 // per (cell, level): rho_int, local+neighbour bounds, vertical upwind update,
 // vertical parts of the limiter scale sums; stores the high-minus-upwind vertical flux
@@ -319,15 +603,12 @@ __global__ void k_mono_cells_b(mpasg_mesh m, mpasg_fields f, FastDiv fl, int S) 
       T sgn_ = cv<T>(m.edgesOnCell_sign[c * me + j]);
       T sw = sgn_ * ia;
       size_t oe = ((size_t)e * L + k) * S + s;
-      if (sizeof(T) == sizeof(double))
-        rows = rows - f64(cv<T>(f.flux_up[oe]) * sw);  // float64: the reference's running sum
-      else
-        hsum = hsum - cv<T>(f.flux_up[oe]) * sw;
+      hsum = hsum - cv<T>(f.flux_up[oe]) * sw;
       T sf = sgn_ * cv<T>(f.flux_tmp[oe]);
       sout = sout - mz(sf) * ia;
       sin_ = sin_ - (-mz(-sf)) * ia;
     }
-    if (sizeof(T) != sizeof(double)) rows = rows + f64(hsum);
+    rows = rows + f64(hsum);
     const T rows_t = cv<T>(rows), rint_t = cv<T>(rint);
     T a = (cv<T>(f.s_max[o]) * rint_t - rows_t) / (sin_ + eps);
     T b = (cv<T>(f.s_min[o]) * rint_t - rows_t) / (sout - eps);
@@ -389,12 +670,9 @@ __global__ void k_mono_cells_c(mpasg_mesh m, mpasg_fields f, FastDiv fl, int S, 
     for (int j = 0; j < n; ++j) {
       int e = m.edgesOnCell[c * me + j];
       T sw = cv<T>(m.edgesOnCell_sign[c * me + j]) * ia;
-      if (sizeof(T) == sizeof(double))
-        rows = rows - f64(cv<T>(f.hflux[((size_t)e * L + k) * S + s]) * sw);
-      else
-        hsum = hsum - cv<T>(f.hflux[((size_t)e * L + k) * S + s]) * sw;
+      hsum = hsum - cv<T>(f.hflux[((size_t)e * L + k) * S + s]) * sw;
     }
-    if (sizeof(T) != sizeof(double)) rows = rows + f64(hsum);
+    rows = rows + f64(hsum);
     double st2 = (rows - f64(cv<T>(m.rdnw[k]) * (wl_hi - wl_lo))) * inv_rint;
     s_out[o] = st2 > 0.0 ? st2 : 0.0;
   }
@@ -414,45 +692,81 @@ static void time_weights(int advance_density, int rk_step, int order, double* w_
 
 namespace {
 
-// One explicit RK transport stage with the edge values in `hflux` (f->hflux or the
-// library-owned scratch): scalars_init, scalars_a -> scalars_b.
-template <typename T>
+// Launches of the float64 form for cells of at most 6 edges (N = 6) or 8; cells with more
+// take the sums' float64 loops.
+template <int N>
+int launch_scalars_fx(const mpasg_mesh* m, const mpasg_fields& g, const TransportScalars& p, int S, cudaStream_t s) {
+  const int L = m->nVertLevels, row = L * S;
+  const int rc = launch_edge_flux_fx<false>(m, S, 0.0, g.ruAvg, g.scalars_a, nullptr, g.hflux, nullptr, s);
+  if (rc != MPASG_OK) return rc;
+  const size_t smem = cellsum::max_cells(row) * N * sizeof(cellsum::Slot);
+  k_scalars_update_fx<N><<<nblocks((long long)m->nCells * row), kBlock, smem, s>>>(
+      *m, g, FastDiv(row), FastDiv(S), p, g.scalars_init, g.scalars_a, g.scalars_b);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
+}
+
+template <int N>
+int launch_scalars_mono_fx(const mpasg_mesh* m, const mpasg_fields* f, const TransportScalars& p, int S,
+                           cudaStream_t s) {
+  const int L = m->nVertLevels, row = L * S;
+  const int nb = nblocks((long long)m->nCells * row);
+  const uint32_t ne = (uint32_t)m->nEdges * row;
+  const FastDiv fr(row), fs(S);
+  const size_t smem = cellsum::max_cells(row) * N * sizeof(cellsum::Slot);
+  const int rc = launch_edge_flux_fx<true>(m, S, p.dt, f->ruAvg, f->scalars_a, f->scalars_init, f->flux_up,
+                                           f->flux_tmp, s);
+  if (rc != MPASG_OK) return rc;
+  k_mono_density_fx<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), p.dt);
+  MPASG_LAUNCH_CHECK();
+  k_mono_cells_a_fx<N><<<nb, kBlock, 0, s>>>(*m, *f, fr, fs, p, f->scalars_init, f->scalars_a);
+  MPASG_LAUNCH_CHECK();
+  k_mono_cells_b_fx<N><<<nb, kBlock, smem, s>>>(*m, *f, fr, fs);
+  MPASG_LAUNCH_CHECK();
+  k_mono_edges_b_fx<<<nblocks(ne), kBlock, 0, s>>>(*m, *f, fr, ne);
+  MPASG_LAUNCH_CHECK();
+  k_mono_cells_c_fx<N><<<nb, kBlock, smem, s>>>(*m, *f, fr, fs, f->scalars_b);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
+}
+
+// One explicit RK transport stage with the edge values (mixed form) or fluxes in `hflux` (f->hflux
+// or the library-owned scratch): scalars_init, scalars_a -> scalars_b.
 int launch_scalars(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, double* hflux, int rk_step,
                    double dt_stage, cudaStream_t s) {
   const int L = m->nVertLevels, S = c->num_scalars;
-  FastDiv fl(L);
   mpasg_fields g = *f;
   g.hflux = hflux;
-  if constexpr (sizeof(T) == sizeof(double)) {
-    const int rc = launch_pattern_c_fx(m, S, g.ruAvg, g.scalars_a, hflux, 0, s);
-    if (rc != MPASG_OK) return rc;
-  } else {
-    k_pattern_c<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, fl, S, g.ruAvg, g.scalars_a, hflux, 0);
-    MPASG_LAUNCH_CHECK();
-  }
   // density weights: advanced with the stage in the split transport loop; the stage's
   // new density in the coupled mode (one dynamics substep, time_integration.py:7930-8200)
   double w_old, w_new;
   time_weights(c->dynamics_split_steps > 1 ? 1 : 0, rk_step, c->time_integration_order, &w_old, &w_new);
+  if (c->precision != MPASG_PRECISION_MIXED) {
+    const TransportScalars p = transport_scalars(dt_stage, w_old, w_new, c->coef_3rd_order);
+    return m->maxEdges <= 6 ? launch_scalars_fx<6>(m, g, p, S, s) : launch_scalars_fx<8>(m, g, p, S, s);
+  }
+  using T = float;
+  FastDiv fl(L);
+  k_pattern_c<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, fl, S, g.ruAvg, g.scalars_a, hflux, 0);
+  MPASG_LAUNCH_CHECK();
   k_scalars_update<T><<<nblocks((long long)m->nCells * L), kBlock, kBlock * S * sizeof(T), s>>>(
       *m, g, fl, S, dt_stage, w_old, w_new, c->coef_3rd_order, g.scalars_init, g.scalars_a, g.scalars_b);
   MPASG_LAUNCH_CHECK();
   return MPASG_OK;
 }
 
-template <typename T>
 int launch_scalars_mono(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, double dt_stage,
                         cudaStream_t s) {
   const int L = m->nVertLevels, S = c->num_scalars;
+  if (c->precision != MPASG_PRECISION_MIXED) {
+    const TransportScalars p = transport_scalars(dt_stage, 0.0, 1.0, c->coef_3rd_order);
+    return m->maxEdges <= 6 ? launch_scalars_mono_fx<6>(m, f, p, S, s) : launch_scalars_mono_fx<8>(m, f, p, S, s);
+  }
+  using T = float;
   FastDiv fl(L);
   const long long nel = (long long)m->nEdges * L, ncl = (long long)m->nCells * L;
-  if constexpr (sizeof(T) == sizeof(double)) {
-    const int rc = launch_pattern_c_fx(m, S, f->ruAvg, f->scalars_a, f->hflux, 1, s);
-    if (rc != MPASG_OK) return rc;
-  } else {
-    k_pattern_c<T><<<nblocks(nel), kBlock, 0, s>>>(*m, fl, S, f->ruAvg, f->scalars_a, f->hflux, 1);
-    MPASG_LAUNCH_CHECK();
-  }
+  k_pattern_c<T><<<nblocks(nel), kBlock, 0, s>>>(*m, fl, S, f->ruAvg, f->scalars_a, f->hflux, 1);
+  MPASG_LAUNCH_CHECK();
   k_mono_cells_a<T><<<nblocks(ncl), kBlock, kBlock * 2 * S * sizeof(T), s>>>(*m, *f, fl, S, dt_stage,
                                                                           c->coef_3rd_order, f->scalars_init,
                                                                           f->scalars_a);
@@ -474,16 +788,14 @@ extern "C" int mpasg_advance_scalars(const mpasg_mesh* m, const mpasg_config* c,
                                      double dt_stage, void* stream) {
   if (!m || !c || !f || c->num_scalars < 1 || c->num_scalars > 8) return MPASG_E_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  if (c->precision == MPASG_PRECISION_MIXED) return launch_scalars<float>(m, c, f, f->hflux, rk_step, dt_stage, s);
-  return launch_scalars<double>(m, c, f, f->hflux, rk_step, dt_stage, s);
+  return launch_scalars(m, c, f, f->hflux, rk_step, dt_stage, s);
 }
 
 extern "C" int mpasg_advance_scalars_mono(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
                                           double dt_stage, void* stream) {
   if (!m || !c || !f || c->num_scalars < 1 || c->num_scalars > 8) return MPASG_E_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  if (c->precision == MPASG_PRECISION_MIXED) return launch_scalars_mono<float>(m, c, f, dt_stage, s);
-  return launch_scalars_mono<double>(m, c, f, dt_stage, s);
+  return launch_scalars_mono(m, c, f, dt_stage, s);
 }
 
 // ---------------------------------------------------------------- library-owned scratch
@@ -530,6 +842,5 @@ extern "C" int mpasg_advance_scalars_static(const mpasg_mesh* m, const mpasg_con
   const int rc = static_scratch(&scratch);
   if (rc != MPASG_OK) return rc;
   cudaStream_t s = (cudaStream_t)stream;  // the caller's struct is left as it is
-  if (c->precision == MPASG_PRECISION_MIXED) return launch_scalars<float>(m, c, f, scratch, rk_step, dt_stage, s);
-  return launch_scalars<double>(m, c, f, scratch, rk_step, dt_stage, s);
+  return launch_scalars(m, c, f, scratch, rk_step, dt_stage, s);
 }

@@ -39,10 +39,10 @@ def _divide(lib, a, b, ulps=0):
 
 
 @pytest.mark.parametrize("ulps", [-1, 0, 1])
-@pytest.mark.parametrize("spread", [0.5, 8.0, 59.0])
+@pytest.mark.parametrize("spread", [0.5, 8.0, 65.0])
 def test_quotient_is_the_rounded_one(lib, ulps, spread):
     rng = np.random.default_rng(int(spread) + 2 + ulps)
-    b = np.exp2(rng.uniform(-spread, spread, 300_000))
+    b = np.exp2(rng.uniform(-1.4 * spread, spread, 300_000))
     a = rng.standard_normal(b.size) * np.exp2(rng.uniform(-spread, spread, b.size))
     assert np.array_equal(_divide(lib, a, b, ulps), a / b)
 
@@ -50,9 +50,9 @@ def test_quotient_is_the_rounded_one(lib, ulps, spread):
 def test_edges(lib):
     one = np.nextafter(1.0, 2.0)
     b = np.array([1.0, one, np.nextafter(1.0, 0.0), 2.0, np.nextafter(2.0, 1.0), 3.0, 1.0 + 2.0 ** -24,
-                  2.0 ** -60, np.nextafter(2.0 ** -60, 0.0), 2.0 ** 60, np.nextafter(2.0 ** 60, 0.0), 0.0, -0.0, -3.0,
+                  2.0 ** -100, np.nextafter(2.0 ** -100, 0.0), 2.0 ** 70, np.nextafter(2.0 ** 70, 0.0), 1e-20, 0.0, -0.0, -3.0,
                   5e-324, 1e-310, np.inf, -np.inf, np.nan, 1e300])
-    a = np.array([0.0, -0.0, 1.0, -1.0, 3.0, one, 2.0 ** -700, np.nextafter(2.0 ** -700, 0.0), 2.0 ** 899, 2.0 ** 901,
+    a = np.array([0.0, -0.0, 1.0, -1.0, 3.0, one, 2.0 ** -600, np.nextafter(2.0 ** -600, 0.0), 2.0 ** 799, 2.0 ** 801,
                   5e-324, np.inf, np.nan, 1e308])
     aa, bb = (np.ascontiguousarray(x.ravel()) for x in np.meshgrid(a, b))
     with np.errstate(all="ignore"):
@@ -67,13 +67,13 @@ def test_edges(lib):
             assert off <= Fraction(np.spacing(abs(g))) * (Fraction(1, 2) + Fraction(1, 2 ** 30)), (x, y)
     out = np.empty_like(b)
     lib.reciprocals(_p(b), _p(out), ctypes.c_long(b.size))
-    same = np.isnan(inv) | np.isinf(inv) | (np.abs(b - 1.0) > 1e-15) & (np.abs(b - 2.0) > 1e-15) & (b < 2.0 ** 59)
+    same = np.isnan(inv) | np.isinf(inv) | (np.abs(b - 1.0) > 1e-15) & (np.abs(b - 2.0) > 1e-15) & (b < 2.0 ** 69)
     assert np.array_equal(out[same], inv[same], equal_nan=True)
     assert np.all(np.abs(out[~same] - inv[~same]) <= np.spacing(inv[~same]))
 
 
 def test_reciprocal(lib):
-    b = np.exp2(np.random.default_rng(1).uniform(-59, 59, 300_000))
+    b = np.exp2(np.random.default_rng(1).uniform(-99, 69, 300_000))
     out = np.empty_like(b)
     lib.reciprocals(_p(b), _p(out), ctypes.c_long(b.size))
     assert np.array_equal(out, 1.0 / b)

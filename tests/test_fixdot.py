@@ -35,7 +35,12 @@ def lib(tmp_path_factory):
         out = np.empty(x.shape[0])
         getattr(dll, name)(*(ctypes.c_void_p(a.ctypes.data) for a in (x, w, out)), ctypes.c_long(x.shape[0]))
         return out
+    call.dll = dll
     return call
+
+
+def _p(a):
+    return ctypes.c_void_p(a.ctypes.data)
 
 
 KINDS = {"fx_dot10": 10, "fx_dot14": 14, "fx_sum6": 6}
@@ -112,3 +117,38 @@ def test_refused_weights(lib):
     x, w = _sample(np.random.default_rng(6), "fx_dot10", 3, 0)
     w[0, 4], w[1, 4], w[2, 4] = np.inf, np.nan, 1e-310
     assert np.isnan(lib("fx_dot10", x, w)).all()
+
+
+def test_selections(lib):
+    """The integer-side selections: x > 0, clamp to [0, 1] (NaN gives 0), float64 order."""
+    x = np.array([0.0, -0.0, 5e-324, -5e-324, 1.0, np.nextafter(1.0, 0.0), np.nextafter(1.0, 2.0), -1.0, 0.3, 1e308,
+                  np.inf, -np.inf, np.nan, -np.nan])
+    pos, clamp, key, back = np.empty_like(x), np.empty_like(x), np.empty(x.size, np.int64), np.empty_like(x)
+    lib.dll.fx_select(_p(x), _p(pos), _p(clamp), _p(key), _p(back), ctypes.c_long(x.size))
+    assert np.array_equal(pos, np.where(x > 0.0, x, 0.0)) and not np.signbit(pos).any()
+    assert np.array_equal(clamp, np.fmin(np.fmax(x, 0.0), 1.0)) and not np.signbit(clamp).any()
+    assert np.array_equal(back.view(np.int64), x.view(np.int64))
+    num = ~np.isnan(x)
+    a, b = x[num][:, None], x[num][None, :]
+    ka, kb = key[num][:, None], key[num][None, :]
+    assert np.all((a < b) <= (ka < kb)) and np.all((a > b) <= (ka > kb))
+    assert key[x == np.inf][0] < key[np.isnan(x) & ~np.signbit(x)][0]
+    assert key[x == -np.inf][0] > key[np.isnan(x) & np.signbit(x)][0]
+
+
+def test_parts(lib):
+    """Positive and negative parts of alternating sums: within a rounding of the exact parts."""
+    x, _ = _sample(np.random.default_rng(9), "fx_sum6", 400, 20)
+    x[::4, 2] = 0.0
+    x[7] = 0.0
+    x[8, 0] = np.nan
+    x[9, 3] = np.inf
+    pos, neg, ok = np.empty(400), np.empty(400), np.empty(400, np.int32)
+    lib.dll.fx_parts6(_p(x), _p(pos), _p(neg), _p(ok), ctypes.c_long(400))
+    assert list(np.where(ok == 0)[0]) == [8, 9]
+    assert pos[7] == 0.0 and neg[7] == 0.0
+    for i in np.where(ok)[0]:
+        t = [Fraction(v) * (-1) ** j for j, v in enumerate(x[i])]
+        big = max(map(abs, t))
+        for got, want in ((pos[i], sum(max(v, 0) for v in t)), (neg[i], sum(max(-v, 0) for v in t))):
+            assert abs(Fraction(got) - want) <= 6 * Fraction(1, 2 ** 53) * big
