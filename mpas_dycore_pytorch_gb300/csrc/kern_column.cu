@@ -151,7 +151,10 @@ __global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_field
   f.a_tri[o + k] = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
   f.b_tri[o + k] = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
                    cofwr * (cofrz_k - cofrz_km1);
-  f.c_tri[o + k] = fma(cw_k, tp, -fma(cofwz * zz, tp, cofwr * cofrz_k));
+  if (sizeof(T) == sizeof(double))
+    f.c_tri[o + k] = fma(cw_k, tp, -fma(cofwz * zz, tp, cofwr * cofrz_k));
+  else
+    f.c_tri[o + k] = tp * (cw_k - cofwz * zz) - cofwr * cofrz_k;
 }
 
 template <typename T>

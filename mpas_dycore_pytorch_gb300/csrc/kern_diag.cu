@@ -24,8 +24,9 @@ __global__ void k_diag_edges_a(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   fpw<T>(f.ke_edge, f.ke_edge_f32)[i] = dcdv * (u * u);
 }
 
-// vorticity, vertex kinetic energy and potential vorticity
-template <typename T>
+// vorticity, vertex kinetic energy (without its factor 0.25 unless QUARTER: k_diag_cells_fx
+// applies it) and potential vorticity
+template <typename T, bool QUARTER>
 __global__ void k_diag_vertices(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -45,9 +46,7 @@ __global__ void k_diag_vertices(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const double iat = m.invAreaTriangle[v];
   vort = vort * iat;
   f.vorticity[i] = vort;
-  // (float64 form: k_diag_cells_fx applies the factor 0.25)
-  f.ke_vertex[i] = sizeof(T) == sizeof(double) ? f64(G(invAreaTriangle)[v] * kev)
-                                               : f64(T(0.25) * G(invAreaTriangle)[v] * kev);
+  f.ke_vertex[i] = QUARTER ? f64(T(0.25) * G(invAreaTriangle)[v] * kev) : f64(G(invAreaTriangle)[v] * kev);
   const double pvv = m.fVertex[v] + vort;
   f.pv_vertex[i] = pvv;
   if (sizeof(T) != sizeof(double)) f.pv_vertex_f32[i] = d2f_bits(pvv);
@@ -264,22 +263,28 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_edges_b_fx(mpasg_mesh m, mpa
   } else {
     vv = f.v[i];
   }
-  double pve = 0.5 * (pv1 + pv2);
+  double pve;
   if (apvm) {
     const size_t c1 = (size_t)m.cellsOnEdge[2 * e], c2 = (size_t)m.cellsOnEdge[2 * e + 1];
     const ApvmEdge a = s_a[e - e0];
     const double delta = fma(u, (f.pv_cell[c2 * L + k] - f.pv_cell[c1 * L + k]) * a.gn, vv * ((pv2 - pv1) * a.gt));
-    pve = pve - delta;
+    pve = fma(0.5, pv1 + pv2, -delta);
+  } else {
+    pve = 0.5 * (pv1 + pv2);
   }
   f.pv_edge[i] = pve;
   f.ke_edge[i] = pve * u;
 }
 
-int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, int rk_step, int apvm,
-                   cudaStream_t s) {
+int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, int rk_step, cudaStream_t s) {
+  const int apvm = c->apvm_upwinding > 0.0 ? 1 : 0;
   const int L = m->nVertLevels, rows = (kBlock - 1) / L + 2;
   const int nc = nblocks((long long)m->nCells * L), ne = nblocks((long long)m->nEdges * L);
   const FastDiv fl(L);
+  k_diag_edges_a<double><<<ne, kBlock, 0, s>>>(*m, *f, fl);
+  MPASG_LAUNCH_CHECK();
+  k_diag_vertices<double, false><<<nblocks((long long)m->nVertices * L), kBlock, 0, s>>>(*m, *f, fl);
+  MPASG_LAUNCH_CHECK();
   const size_t slot = 2 * sizeof(fx::Weight) + sizeof(double);
   if (m->maxEdges <= 6) k_diag_cells_fx<6><<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm);
   else k_diag_cells_fx<10><<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm);
@@ -525,6 +530,9 @@ __global__ void k_prepare_rw(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   f.rw[i] = rw;
 }
 
+// T = float: the mixed form.  T = double: the cold start of the mixed form, whose float32
+// stencils carry a last-bit change of their start to the seventh digit; the float64 form takes
+// launch_diag_fx.
 template <typename T>
 int launch_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s) {
   const int L = m->nVertLevels;
@@ -532,9 +540,8 @@ int launch_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields*
   const int apvm = c->apvm_upwinding > 0.0 ? 1 : 0;
   k_diag_edges_a<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
-  k_diag_vertices<T><<<nblocks((long long)m->nVertices * L), kBlock, 0, s>>>(*m, *f, fl);
+  k_diag_vertices<T, true><<<nblocks((long long)m->nVertices * L), kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
-  if constexpr (sizeof(T) == sizeof(double)) return launch_diag_fx(m, c, f, rk_step, apvm, s);
   k_diag_cells<T><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, fl, apvm);
   MPASG_LAUNCH_CHECK();
   k_diag_edges_b<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(
@@ -560,7 +567,7 @@ int mpasgi_solve_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_f
     }
     return launch_diagnostics<float>(m, c, f, rk_step, s);
   }
-  return launch_diagnostics<double>(m, c, f, rk_step, s);
+  return launch_diag_fx(m, c, f, rk_step, s);
 }
 
 extern "C" int mpasg_reconstruct_2d(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, void* stream) {
@@ -604,7 +611,8 @@ int prepare(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, const d
   MPASG_LAUNCH_CHECK();
   mpasg_config c64 = *c;  // the cold start is float64 in both precisions
   c64.precision = MPASG_PRECISION_FLOAT64;
-  int rc = mpasg_solve_diagnostics(m, &c64, f, 3, stream);
+  int rc = c->precision == MPASG_PRECISION_MIXED ? launch_diagnostics<double>(m, &c64, f, 3, s)
+                                                 : mpasg_solve_diagnostics(m, &c64, f, 3, stream);
   if (rc) return rc;
   return mpasg_reconstruct_2d(m, &c64, f, stream);
 }
