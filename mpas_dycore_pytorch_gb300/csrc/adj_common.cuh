@@ -105,8 +105,6 @@ MPASG_D Flux3Grad flux3_grad(double qm2, double qm1, double q0, double qp1, doub
 }
 
 // internal entry points shared by the stage VJPs and the step driver
-int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
-                          cudaStream_t s, int part);
 int mpasgi_recover_vjp_core(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, mpasg_fields* g,
                             int rk_step, double rk_dt, const AdjWork& w, cudaStream_t s);
 int mpasgi_diag_vjp_core(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, mpasg_fields* g,

@@ -156,10 +156,23 @@ inline int nblocks(long long n, int block = kBlock) {
 // it calls these variants with copies_current = true; the public per-stage entry points
 // refresh the copies first.
 int mpasgi_pack_f32(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s);
+
+// What the step driver has a stage's kernels do beside the stage (each saves a launch and a
+// pass over its fields; the public stage entry points and the derivative drivers run the
+// stages alone):
+struct TendFusion {
+  double first_dts = 0.0;     // > 0: the first acoustic substep's edge update with this dts
+  bool smlstep = false;       // the small-step w tendency (flat terrain only)
+  bool hdiv_current = false;  // h_divergence already holds ru's divergence (later RK stages)
+};
 int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s,
-                    bool copies_current);
+                    bool copies_current, const TendFusion& fuse = TendFusion());
+struct DiagFusion {
+  bool edges_done = false;  // h_edge and ke_edge already formed (by the recovery)
+  bool hdiv = false;        // also h_divergence, for the next stage's tendencies
+};
 int mpasgi_solve_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step,
-                             cudaStream_t s, bool copies_current);
+                             cudaStream_t s, bool copies_current, const DiagFusion& fuse = DiagFusion());
 int mpasgi_reconstruct(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, cudaStream_t s,
                        bool copies_current);
 // theta_m - ref_theta and theta_m_save - ref_theta (float32) for the mixed form
@@ -170,8 +183,19 @@ int mpasgi_theta_edge(const mpasg_mesh* m, mpasg_fields* f, bool mixed, cudaStre
 int mpasgi_pvu(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s);
 int mpasgi_divergence_damping(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, double dts,
                               cudaStream_t s, bool copies_current);
+struct AcousticFusion {
+  bool edges_done = false;   // first substep: ru_p and ruAvg already formed (by the tendencies)
+  bool damp_before = false;  // later substeps: the previous substep's divergence damping first
+};
 int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
-                         cudaStream_t s, bool copies_current);
+                         cudaStream_t s, bool copies_current, const AcousticFusion& fuse = AcousticFusion());
+// the acoustic substep in two parts (kern_column.cu; part -1: both)
+int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
+                          cudaStream_t s, int part, const AcousticFusion& fuse = AcousticFusion());
+// recovery with the last acoustic substep's divergence damping (step dts) before it and the
+// diagnostics' edge fields after it
+int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
+                          double rk_dt, double dts, cudaStream_t s);
 
 // Number of kernels this library has launched (for launch accounting by callers).
 extern "C" long long mpasg_launch_count(void);

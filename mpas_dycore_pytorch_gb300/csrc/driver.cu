@@ -11,19 +11,63 @@
 
 namespace {
 
-__global__ void k_fill_d(double* __restrict__ p, long long n, double v) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
+// Elementwise work on up to ten arrays in one launch (blockIdx.y selects the array): the saves
+// and the flux sums at a substep's ends.  One launch instead of ten copies: on the small meshes
+// each of them cost a graph node of 1.5 to 2 us.
+struct ArrayJob {
+  static constexpr int kMax = 10;
+  enum Op { kCopy, kAdd, kScale };
+  const double* src[kMax];
+  double* dst[kMax];
+  double* dst2[kMax];     // second destination of a copy, or null
+  long long n[kMax];
+  long long zero_from[kMax];  // kCopy: values from this index on are zero, in src too
+  int op[kMax];
+  double scale;
+  int count = 0;
+  long long longest = 0;
+  void push(Op o, double* d, const double* s, long long len, double* d2 = nullptr, long long zero = -1) {
+    src[count] = s;
+    dst[count] = d;
+    dst2[count] = d2;
+    n[count] = len;
+    zero_from[count] = zero < 0 ? len : zero;
+    op[count] = o;
+    ++count;
+    longest = len > longest ? len : longest;
+  }
+};
+
+__global__ void k_arrays(const __grid_constant__ ArrayJob job) {
+  const int a = blockIdx.y;
+  const long long n = job.n[a], step = (long long)gridDim.x * blockDim.x;
+  const double* src = job.src[a];
+  double* dst = job.dst[a];
+  double* dst2 = job.dst2[a];
+  const long long zero = job.zero_from[a];
+  const int op = job.op[a];
+  const double scale = job.scale;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+    double x = src[i];
+    if (op == ArrayJob::kAdd) {
+      x = dst[i] + x;
+    } else if (op == ArrayJob::kScale) {
+      x = x * scale;
+    } else if (i >= zero) {
+      x = 0.0;
+      const_cast<double*>(src)[i] = 0.0;
+    }
+    dst[i] = x;
+    if (dst2) dst2[i] = x;
+  }
 }
 
-__global__ void k_add_d(double* __restrict__ y, const double* __restrict__ x, long long n) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = y[i] + x[i];
-}
-
-__global__ void k_scale_d(double* __restrict__ y, const double* __restrict__ x, double a, long long n) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = x[i] * a;
+int run_arrays(const ArrayJob& job, cudaStream_t s) {
+  if (job.count == 0 || job.longest == 0) return MPASG_OK;
+  const int blocks = nblocks((job.longest + 3) / 4);  // four values a thread in the longest array
+  k_arrays<<<dim3(blocks, job.count), kBlock, 0, s>>>(job);
+  MPASG_LAUNCH_CHECK();
+  return MPASG_OK;
 }
 
 __global__ void k_count_nonfinite(const double* __restrict__ p, long long n, int32_t* __restrict__ count) {
@@ -67,12 +111,6 @@ __global__ void k_permute_rows(const double* __restrict__ src, double* __restric
   if (i >= n * row_len) return;
   const long long r = i / row_len, j = i - r * row_len;
   dst[i] = src[rows[r] * row_len + j];
-}
-
-int fill(double* p, long long n, double v, cudaStream_t s) {
-  k_fill_d<<<nblocks(n), kBlock, 0, s>>>(p, n, v);
-  MPASG_LAUNCH_CHECK();
-  return MPASG_OK;
 }
 
 int copy(double* dst, const double* src, long long n, cudaStream_t s) {
@@ -265,24 +303,22 @@ int transport_stage(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
 // (the coupled mode advanced the scalars inside the RK stages already) and the final
 // scalars.  Of the step boundary it writes only the scalars.
 int step_tail(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, cudaStream_t s, StageRecorder* rec) {
-  const long long L = m->nVertLevels, nc = m->nCells;
-  const long long S = c->num_scalars;
-  const bool advect = S > 0 && !c->scalar_advection_off;
+  const bool advect = c->num_scalars > 0 && !c->scalar_advection_off;
   const bool coupled = c->dynamics_split_steps == 1;
   const double dt = c->dt;
   if (advect && !coupled) {
-    CHECK_RC(copy(f.scalars_a, f.scalars_init, (nc + 1) * L * S, s));
     // transport stage dts; the first is dt/2 for RK2 (time_integration.py:3366-3370)
     const double dts_t[3] = {c->time_integration_order == 2 ? dt / 2.0 : dt / 3.0, dt / 2.0, dt};
-    MARK(MPASG_STAGE_SPLIT);
+    // the first stage advances scalars_init itself, the last one writes the step's scalars
+    // (active rows only: the padding row passes through the step unchanged, as in the
+    // reference); scalars_a and scalars_b hold the stages between
+    mpasg_fields g = f;
     for (int rk = 1; rk <= 3; ++rk) {
-      CHECK_RC(transport_stage(m, c, &f, rk, dts_t[rk - 1], s));
+      g.scalars_a = rk == 1 ? f.scalars_init : rk == 2 ? f.scalars_b : f.scalars_a;
+      g.scalars_b = rk == 1 ? f.scalars_b : rk == 2 ? f.scalars_a : f.scalars;
+      CHECK_RC(transport_stage(m, c, &g, rk, dts_t[rk - 1], s));
       MARK(rk == 3 && c->monotonic ? MPASG_STAGE_SCALARS_MONO : MPASG_STAGE_SCALARS);
     }
-    // active rows only: the padding row of the scalars passes through the step unchanged,
-    // as in the reference
-    CHECK_RC(copy(f.scalars, f.scalars_a, nc * L * S, s));
-    MARK(MPASG_STAGE_SPLIT);
   }
   return MPASG_OK;
 }
@@ -323,16 +359,21 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
 
   // ---- RK integration setup
   MARK(MPASG_STAGE_BEGIN);
-  CHECK_RC(fill(f.theta_m + nc * L, L, 0.0, s));
-  CHECK_RC(copy(f.ru_save, f.ru, nel, s));
-  CHECK_RC(copy(f.rw_save, f.rw, ncw, s));
-  CHECK_RC(copy(f.rtheta_p_save, f.rtheta_p, ncl, s));
-  CHECK_RC(copy(f.rho_p_save, f.rho_p, ncl, s));
-  CHECK_RC(copy(f.theta_m_save, f.theta_m, ncl, s));
-  CHECK_RC(copy(f.rr_save, f.rho_p, ncl, s));
-  CHECK_RC(copy(f.rho_zz_old_split, f.rho_zz, ncl, s));
-  if (S > 0) CHECK_RC(copy(f.scalars_init, f.scalars, ncs, s));
-  if (advect && coupled) CHECK_RC(copy(f.scalars_a, f.scalars_init, ncs, s));
+  // the time-level saves of a dynamics substep (theta_m's padding row is zeroed)
+  auto push_saves = [&](ArrayJob& job) {
+    job.push(ArrayJob::kCopy, f.ru_save, f.ru, nel);
+    job.push(ArrayJob::kCopy, f.rw_save, f.rw, ncw);
+    job.push(ArrayJob::kCopy, f.rtheta_p_save, f.rtheta_p, ncl);
+    job.push(ArrayJob::kCopy, f.rho_p_save, f.rho_p, ncl, f.rr_save);
+    job.push(ArrayJob::kCopy, f.theta_m_save, f.theta_m, ncl, nullptr, nc * L);
+  };
+  {
+    ArrayJob job;
+    push_saves(job);
+    job.push(ArrayJob::kCopy, f.rho_zz_old_split, f.rho_zz, ncl);
+    if (S > 0) job.push(ArrayJob::kCopy, f.scalars_init, f.scalars, ncs, advect && coupled ? f.scalars_a : nullptr);
+    CHECK_RC(run_arrays(job, s));
+  }
   if (c->precision == MPASG_PRECISION_MIXED) CHECK_RC(mpasgi_pack_f32(m, &f, s));
   else CHECK_RC(mpasgi_pvu(m, &f, s));
   // edge mean of theta_m_save and its reciprocal sum
@@ -349,17 +390,23 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
         CHECK_RC(mpasg_vert_imp_coefs(m, c, &f, dts, stream));
         MARK(MPASG_STAGE_VIMP);
       }
-      CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true));
+      TendFusion tf;
+      tf.first_dts = dts;
+      tf.smlstep = m->flatTerrain != 0;
+      tf.hdiv_current = rk > 1;
+      CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true, tf));
       MARK(rk == 1 ? MPASG_STAGE_DYN_TEND_RK1 : MPASG_STAGE_DYN_TEND);
-      CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));
+      if (!tf.smlstep) CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));
       MARK(MPASG_STAGE_SMLSTEP);
       for (int small = 1; small <= nsub[rk - 1]; ++small) {
-        CHECK_RC(mpasgi_acoustic_step(m, c, &f, small, dts, s, true));
+        AcousticFusion af;
+        af.edges_done = small == 1;
+        af.damp_before = small > 1;
+        CHECK_RC(mpasgi_acoustic_step(m, c, &f, small, dts, s, true, af));
         MARK(MPASG_STAGE_ACOUSTIC);
-        CHECK_RC(mpasgi_divergence_damping(m, c, &f, dts, s, true));
-        MARK(MPASG_STAGE_DIVDAMP);
       }
-      CHECK_RC(mpasg_recover_large_step(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], stream));
+      // with the last substep's divergence damping and the diagnostics' edge fields
+      CHECK_RC(mpasgi_recover_finish(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], dts, s));
       MARK(MPASG_STAGE_RECOVER);
       if (coupled && advect) {  // time_integration.py:7890-8200: stage dt, this stage's mass fluxes
         CHECK_RC(transport_stage(m, c, &f, rk, rk_ts[rk - 1], s));
@@ -371,36 +418,29 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
           CHECK_RC(copy(t + nel + ncw, f.rho_zz, ncl, s));
         }
       }
-      CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true));
+      DiagFusion df;
+      df.edges_done = true;
+      df.hdiv = rk < 3;  // the next stage's tendencies read it
+      CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true, df));
       MARK(MPASG_STAGE_DIAG);
     }
-    // split bookkeeping
-    if (sub == 1) {
-      CHECK_RC(copy(f.ruAvg_split, f.ruAvg, nel, s));
-      CHECK_RC(copy(f.wwAvg_split, f.wwAvg, ncw, s));
-    } else {
-      k_add_d<<<nblocks(nel), kBlock, 0, s>>>(f.ruAvg_split, f.ruAvg, nel);
-      MPASG_LAUNCH_CHECK();
-      k_add_d<<<nblocks(ncw), kBlock, 0, s>>>(f.wwAvg_split, f.wwAvg, ncw);
-      MPASG_LAUNCH_CHECK();
-    }
-    if (sub < split) {
-      CHECK_RC(fill(f.theta_m + nc * L, L, 0.0, s));
-      CHECK_RC(copy(f.ru_save, f.ru, nel, s));
-      CHECK_RC(copy(f.rw_save, f.rw, ncw, s));
-      CHECK_RC(copy(f.rtheta_p_save, f.rtheta_p, ncl, s));
-      CHECK_RC(copy(f.rho_p_save, f.rho_p, ncl, s));
-      CHECK_RC(copy(f.theta_m_save, f.theta_m, ncl, s));
-      CHECK_RC(copy(f.rr_save, f.rho_p, ncl, s));
-      CHECK_RC(mpasgi_theta_edge(m, &f, c->precision == MPASG_PRECISION_MIXED, s));
-    }
+    // split bookkeeping: the substeps' mass fluxes summed, the saves of the next substep
+    ArrayJob job;
+    const ArrayJob::Op op = sub == 1 ? ArrayJob::kCopy : ArrayJob::kAdd;
+    job.push(op, f.ruAvg_split, f.ruAvg, nel);
+    job.push(op, f.wwAvg_split, f.wwAvg, ncw);
+    if (sub < split) push_saves(job);
+    CHECK_RC(run_arrays(job, s));
+    if (sub < split) CHECK_RC(mpasgi_theta_edge(m, &f, c->precision == MPASG_PRECISION_MIXED, s));
   }
   MARK(MPASG_STAGE_SPLIT);
-  const double inv = 1.0 / (double)split;
-  k_scale_d<<<nblocks(nel), kBlock, 0, s>>>(f.ruAvg, f.ruAvg_split, inv, nel);
-  MPASG_LAUNCH_CHECK();
-  k_scale_d<<<nblocks(ncw), kBlock, 0, s>>>(f.wwAvg, f.wwAvg_split, inv, ncw);
-  MPASG_LAUNCH_CHECK();
+  {
+    ArrayJob job;
+    job.scale = 1.0 / (double)split;
+    job.push(ArrayJob::kScale, f.ruAvg, f.ruAvg_split, nel);
+    job.push(ArrayJob::kScale, f.wwAvg, f.wwAvg_split, ncw);
+    CHECK_RC(run_arrays(job, s));
+  }
   // coupled mode: the scalars of the last RK stage are the step's (active rows only)
   if (advect && coupled) CHECK_RC(copy(f.scalars, f.scalars_a, nc * L * S, s));
   MARK(MPASG_STAGE_SPLIT);

@@ -374,7 +374,9 @@ int forward_taped(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, co
         if (taped) coef_view(T, f, coef_slot(p, sub, rk));
         CHECK_RC(mpasg_vert_imp_coefs(m, c, &f, dts, stream));
       }
-      CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true));
+      TendFusion tf;  // h_divergence from the previous stage's diagnostics, as in the step
+      tf.hdiv_current = rk > 1;
+      CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true, tf));
       if (taped && T.n_sg > 0) CHECK_RC(mpasgi_nonneg_bytes(f.tend_u, T.sg(i), (m->nEdges + 1LL) * m->nVertLevels, s));
       CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));
       for (int small = 1; small <= p.nsub[rk - 1]; ++small) {
@@ -389,7 +391,9 @@ int forward_taped(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, co
         snap_view(T, f, T.snap(i + 1));
       }
       CHECK_RC(mpasg_recover_large_step(m, c, &f, rk, p.nsub[rk - 1], p.rk_ts[rk - 1], stream));
-      CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true));
+      DiagFusion df;
+      df.hdiv = rk < 3;
+      CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true, df));
     }
     if (sub < p.split && sub < T.hi) CHECK_RC(make_saves(m, T, f, sub, mixed, s));
   }

@@ -78,7 +78,9 @@ int step_jvp(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, mpasg_f
         CHECK_RC(mpasg_vert_imp_coefs(m, c, &f, dts, stream));
         CHECK_RC(mpasgi_vimp_jvp_core(m, c, &f, d, dts, s));
       }
-      CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true));
+      TendFusion tf;  // h_divergence from the previous stage's diagnostics, as in the step
+      tf.hdiv_current = rk > 1;
+      CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true, tf));
       CHECK_RC(mpasgi_dyn_tend_jvp_core(m, c, &f, d, rk, s));
       CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));
       CHECK_RC(mpasgi_smlstep_jvp_core(m, &f, d, s));
@@ -89,7 +91,9 @@ int step_jvp(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, mpasg_f
       }
       CHECK_RC(mpasgi_recover_jvp_core(m, &f, d, rk, nsub[rk - 1], rk_ts[rk - 1], s));
       CHECK_RC(mpasg_recover_large_step(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], stream));
-      CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true));
+      DiagFusion df;
+      df.hdiv = rk < 3;
+      CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true, df));
       CHECK_RC(mpasgi_diag_jvp_core(m, c, &f, d, rk, s));
     }
     if (sub < split) CHECK_RC(saves_both(m, &f, d, s));

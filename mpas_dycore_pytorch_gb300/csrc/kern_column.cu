@@ -179,9 +179,24 @@ __global__ void k_vimp_factor(mpasg_mesh m, mpasg_fields f) {
 // dynamics/acoustic_step.py:576 (_acoustic_step_horizontal_momentum_update)
 // The increment dts (tend_u - pgrad) is formed in the stencil type T; ru_p and ruAvg
 // accumulate in float64.
+// ru_p after the divergence damping of a substep (dynamics/divergence_damping.py:187-299; the
+// increment in the stencil type T, ru_p accumulated in float64).  The fused and the separate
+// kernels share this and the explicit multiply-adds below, so a taped step, which runs the
+// stages one by one, repeats a step to the bit.
 template <typename T>
+MPASG_D double damped_ru_p(const mpasg_fields& f, uint32_t i, size_t i1, size_t i2, double coef) {
+  T d1 = -dif<T>(f.rtheta_pp[i1], f.rtheta_pp_old[i1]);  // substep change: float64 difference
+  T d2 = -dif<T>(f.rtheta_pp[i2], f.rtheta_pp_old[i2]);
+  // / (theta_m_save_1 + theta_m_save_2) as a product with the reciprocal formed once per
+  // dynamics substep (k_theta_edge); within one rounding of the quotient
+  if constexpr (sizeof(T) == sizeof(double)) return fma(coef * (d2 - d1), f.theta_edge_rsum[i], f.ru_p[i]);
+  return f.ru_p[i] + f64(cv<T>(coef) * (d2 - d1) * cv<T>(f.theta_edge_rsum[i]));
+}
+
+// DAMP (small_step > 1): the previous substep's divergence damping first
+template <typename T, bool DAMP>
 __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int small_step,
-                                 double dts, double c2) {
+                                 double dts, double c2, double damp_coef) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
@@ -197,7 +212,9 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
     pgrad = cv<T>(f.cqu_e[i]) * (T(0.5) * cv<T>(c2)) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
     if (!m.flatTerrain)  // no slope: adds exact zeros
       pgrad = pgrad + T(0.5) * cv<T>(m.zxu[i]) * T(kGravity) * (cv<T>(f.rho_pp[i1]) + cv<T>(f.rho_pp[i2]));
-    rup = f.ru_p[i] + f64(cv<T>(dts) * (cv<T>(f.tend_u[i]) - pgrad));
+    const double before = DAMP ? damped_ru_p<T>(f, i, i1, i2, damp_coef) : f.ru_p[i];
+    if constexpr (kDouble) rup = fma(dts, f.tend_u[i] - pgrad, before);
+    else rup = before + f64(cv<T>(dts) * (cv<T>(f.tend_u[i]) - pgrad));
     f.ruAvg[i] = f.ruAvg[i] + rup;
   } else {
     rup = f64(cv<T>(dts) * cv<T>(f.tend_u[i]));
@@ -711,8 +728,6 @@ __global__ void __launch_bounds__(kBlock) k_ac_post(mpasg_mesh m, mpasg_fields f
 }
 
 // ---------------------------------------------------------------- divergence damping
-// dynamics/divergence_damping.py:187-299
-// (the increment in the stencil type T, ru_p accumulated in float64)
 template <typename T>
 __global__ void k_divergence_damping(mpasg_mesh m, mpasg_fields f, FastDiv fl, double coef) {
   const int L = m.nVertLevels;
@@ -720,12 +735,7 @@ __global__ void k_divergence_damping(mpasg_mesh m, mpasg_fields f, FastDiv fl, d
   if (i >= (uint32_t)m.nEdges * L) return;
   uint32_t e = fl.div(i), k = i - e * L;
   int c1 = m.cellsOnEdge[2 * e], c2 = m.cellsOnEdge[2 * e + 1];
-  size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2 * L + k;
-  T d1 = -dif<T>(f.rtheta_pp[i1], f.rtheta_pp_old[i1]);  // substep change: float64 difference
-  T d2 = -dif<T>(f.rtheta_pp[i2], f.rtheta_pp_old[i2]);
-  // / (theta_m_save_1 + theta_m_save_2) as a product with the reciprocal formed once per
-  // dynamics substep (k_theta_edge); within one rounding of the quotient
-  f.ru_p[i] = f.ru_p[i] + f64(cv<T>(coef) * (d2 - d1) * cv<T>(f.theta_edge_rsum[i]));
+  f.ru_p[i] = damped_ru_p<T>(f, i, (size_t)c1 * L + k, (size_t)c2 * L + k, coef);
 }
 
 // ---------------------------------------------------------------- small-step perturbation
@@ -754,7 +764,10 @@ __global__ void k_smlstep_pert(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
     acc = acc - coef * flux;
   }
   size_t o = (size_t)c * L;
-  f.tend_rw[i] = f64((fzm * cv<T>(m.zz[o + k]) + fzp * cv<T>(m.zz[o + k - 1])) * acc);
+  if constexpr (sizeof(T) == sizeof(double))  // (as k_tend_w_theta forms it over flat terrain)
+    f.tend_rw[i] = fma(fzm, m.zz[o + k], fzp * m.zz[o + k - 1]) * acc;
+  else
+    f.tend_rw[i] = f64((fzm * cv<T>(m.zz[o + k]) + fzp * cv<T>(m.zz[o + k - 1])) * acc);
 }
 
 // ---------------------------------------------------------------- large-step recovery
@@ -875,22 +888,39 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
   }
 }
 
-template <typename T>
-__global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns) {
+// FINISH: with the last acoustic substep's divergence damping before it and the diagnostics'
+// edge fields (k_diag_edges_a) after it: one pass over the edges instead of three
+template <typename T, bool FINISH>
+__global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns, double damp_coef) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
   uint32_t e = fl.div(i), k = i - e * L;
-  int c1 = m.cellsOnEdge[2 * e], c2 = m.cellsOnEdge[2 * e + 1];
+  constexpr bool kDouble = sizeof(T) == sizeof(double);
+  const size_t i1 = (size_t)m.cellsOnEdge[2 * e] * L + k, i2 = (size_t)m.cellsOnEdge[2 * e + 1] * L + k;
   double rus = f.ru_save[i];
   f.ruAvg[i] = rus + f.ruAvg[i] * inv_ns;
-  double ru = rus + f.ru_p[i];
+  double rup;
+  if (FINISH) {
+    rup = damped_ru_p<T>(f, i, i1, i2, damp_coef);
+    f.ru_p[i] = rup;
+  } else {
+    rup = f.ru_p[i];
+  }
+  double ru = rus + rup;
   f.ru[i] = ru;
-  const double rho2 = f.rho_zz[(size_t)c1 * L + k] + f.rho_zz[(size_t)c2 * L + k];
+  const double rho_1 = f.rho_zz[i1], rho_2 = f.rho_zz[i2];
+  const double rho2 = rho_1 + rho_2;
   // 2 ru / rho2 (the factor two is exact wherever it is applied)
-  const double u = sizeof(T) == sizeof(double) ? fx::quotient(ru + ru, rho2) : 2.0 * ru * rcp_nr1(rho2);
+  const double u = kDouble ? fx::quotient(ru + ru, rho2) : 2.0 * ru * rcp_nr1(rho2);
   f.u[i] = u;
-  if (sizeof(T) != sizeof(double)) f.u_f32[i] = d2f_bits(u);
+  if (!kDouble) f.u_f32[i] = d2f_bits(u);
+  if (FINISH) {
+    f.h_edge[i] = f64(T(0.5) * (cv<T>(rho_1) + cv<T>(rho_2)));
+    const T u_t = cv<T>(u);
+    const T dcdv = kDouble ? cv<T>(m.edge_dcdv[e]) : G(dcEdge)[e] * G(dvEdge)[e];
+    fpw<T>(f.ke_edge, f.ke_edge_f32)[i] = dcdv * (u_t * u_t);
+  }
 }
 
 template <typename T>
@@ -939,7 +969,8 @@ __global__ void k_recover_w(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
 }
 
 template <typename T>
-int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv_ns, double rk_dt, cudaStream_t s) {
+int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv_ns, double rk_dt, cudaStream_t s,
+                   bool finish, double damp_coef) {
   const int L = m->nVertLevels;
   const long long ncw = (long long)m->nCells * (L + 1);
   if (m->flatTerrain)
@@ -947,7 +978,9 @@ int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv
   else
     k_recover_cells<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), rk_step, inv_ns, rk_dt);
   MPASG_LAUNCH_CHECK();
-  k_recover_edges<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns);
+  const int ne = nblocks((long long)m->nEdges * L);
+  if (finish) k_recover_edges<T, true><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, damp_coef);
+  else k_recover_edges<T, false><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, 0.0);
   MPASG_LAUNCH_CHECK();
   if (!m->flatTerrain) {  // slope fluxes need the new ru of k_recover_edges
     k_recover_w<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1));
@@ -957,6 +990,10 @@ int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv
 }
 
 }  // namespace
+
+static double damping_coefficient(const mpasg_config* c, double dts) {
+  return 2.0 * c->smdiv * c->len_disp / dts;
+}
 
 // ================================================================= C ABI
 extern "C" int mpasg_moist_coefficients(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
@@ -1022,11 +1059,8 @@ int mpasgi_theta_edge(const mpasg_mesh* m, mpasg_fields* f, bool mixed, cudaStre
   return MPASG_OK;
 }
 
-int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
-                          cudaStream_t s, int part);
-
 int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
-                         cudaStream_t s, bool copies_current) {
+                         cudaStream_t s, bool copies_current, const AcousticFusion& fuse) {
   if (!m || !c || !f || small_step < 1) return MPASG_E_ARG;
   if (!copies_current) {
     // the edge theta the right-hand side reads
@@ -1040,14 +1074,14 @@ int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_field
     k_tri_m<<<nblocks(n), kBlock, 0, s>>>(n, f->a_tri, f->alpha_tri, f->tri_m);  // forward-sweep factor
     MPASG_LAUNCH_CHECK();
   }
-  return mpasgi_acoustic_parts(m, c, f, small_step, dts, s, -1);
+  return mpasgi_acoustic_parts(m, c, f, small_step, dts, s, -1, fuse);
 }
 
 // The acoustic substep in two parts (part -1: both): part 0 updates ru_p / ruAvg on the
 // edges and builds the columns' right-hand sides (ac_x holds the tridiagonal right-hand
 // side after it); part 1 solves and finishes the columns.
 int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
-                          cudaStream_t s, int part) {
+                          cudaStream_t s, int part, const AcousticFusion& fuse) {
   const int L = m->nVertLevels;
   const double rcv = kRgas / (kCp - kRgas);
   const double c2 = kCp * rcv;
@@ -1055,17 +1089,25 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
   const long long ncw = (long long)m->nCells * (L + 1);
   const bool mixed = c->precision == MPASG_PRECISION_MIXED;
   if (part != 1) {
-    if (mixed) {
-      k_acoustic_edges<float><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), small_step,
-                                                                                  dts, c2);
+    if (!(small_step == 1 && fuse.edges_done)) {
+      const int ne = nblocks((long long)m->nEdges * L);
+      const double coef = damping_coefficient(c, dts);
+      const FastDiv fl(L);
+      if (mixed && fuse.damp_before)
+        k_acoustic_edges<float, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+      else if (mixed)
+        k_acoustic_edges<float, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+      else if (fuse.damp_before)
+        k_acoustic_edges<double, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+      else
+        k_acoustic_edges<double, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
       MPASG_LAUNCH_CHECK();
+    }
+    if (mixed) {
       k_ac_prep_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), small_step, (float)dts,
                                                       (float)c->epssm, (float)resm);
       MPASG_LAUNCH_CHECK();
     } else {
-      k_acoustic_edges<double><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), small_step,
-                                                                                   dts, c2);
-      MPASG_LAUNCH_CHECK();
       const int rc = launch_ac_prep(m, f, small_step, dts, c->epssm, resm, s);
       if (rc != MPASG_OK) return rc;
     }
@@ -1116,7 +1158,7 @@ int mpasgi_divergence_damping(const mpasg_mesh* m, const mpasg_config* c, mpasg_
     const int rc = mpasgi_theta_edge(m, f, c->precision == MPASG_PRECISION_MIXED, stream);
     if (rc != MPASG_OK) return rc;
   }
-  double coef = 2.0 * c->smdiv * c->len_disp / dts;
+  const double coef = damping_coefficient(c, dts);
   if (c->precision == MPASG_PRECISION_MIXED)
     k_divergence_damping<float><<<nblocks((long long)m->nEdges * L), kBlock, 0, (cudaStream_t)stream>>>(
         *m, *f, FastDiv(L), coef);
@@ -1141,12 +1183,23 @@ extern "C" int mpasg_smlstep_pert(const mpasg_mesh* m, const mpasg_config* c, mp
   return MPASG_OK;
 }
 
-extern "C" int mpasg_recover_large_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
-                                        int rk_step, int ns, double rk_dt, void* stream) {
+namespace {
+int recover(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns, double rk_dt,
+            cudaStream_t s, bool finish, double damp_coef) {
   if (!m || !c || !f || ns < 1) return MPASG_E_ARG;
-  cudaStream_t s = (cudaStream_t)stream;
   const double inv_ns = 1.0 / (double)ns;
   if (c->precision == MPASG_PRECISION_MIXED)
-    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s);
-  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s);
+    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef);
+  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef);
+}
+}  // namespace
+
+extern "C" int mpasg_recover_large_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
+                                        int rk_step, int ns, double rk_dt, void* stream) {
+  return recover(m, c, f, rk_step, ns, rk_dt, (cudaStream_t)stream, false, 0.0);
+}
+
+int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
+                          double rk_dt, double dts, cudaStream_t s) {
+  return recover(m, c, f, rk_step, ns, rk_dt, s, true, c ? damping_coefficient(c, dts) : 0.0);
 }

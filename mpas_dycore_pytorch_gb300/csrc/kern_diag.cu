@@ -55,14 +55,23 @@ __global__ void k_diag_vertices(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
 // divergence, cell kinetic energy (with the vertex-kite blend) and cell PV for APVM (mixed
 // form; float64: k_diag_cells_fx)
 template <typename T>
-__global__ void k_diag_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm) {
+__global__ void k_diag_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm, int hdiv) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nCells * L) return;
   uint32_t c = fl.div(i), k = i - c * L;
   const int me = m.maxEdges;
   const int n = m.nEdgesOnCell[c];
-  // the divergence sum cancels strongly: float64 in both forms
+  // the divergence sums cancel strongly: float64 in both forms
+  if (hdiv) {  // of ru, for the next stage's tendencies (k_tend_cells_a's sum)
+    double hd = 0.0;
+    for (int j = 0; j < n; ++j) {
+      int e = m.edgesOnCell[c * me + j];
+      double t = m.cell_edge_sdv[c * me + j] * f.ru[(size_t)e * L + k];
+      hd = (j == 0) ? t : hd + t;
+    }
+    f.h_divergence[i] = hd * m.invAreaCell[c];
+  }
   double div = 0.0;
   T ke = T(0);
   for (int j = 0; j < n; ++j) {
@@ -189,8 +198,17 @@ MPASG_D void wide_cell_sums(const mpasg_mesh& m, const mpasg_fields& f, uint32_t
   }
 }
 
+MPASG_D double wide_divergence(const mpasg_mesh& m, const double* flux, uint32_t c, uint32_t k) {
+  const size_t o = (size_t)c * m.maxEdges;
+  double d = 0.0;
+  for (int j = 0; j < m.nEdgesOnCell[c]; ++j)
+    d = fma(m.cell_edge_sdv[o + j], flux[(size_t)m.edgesOnCell[o + j] * m.nVertLevels + k], d);
+  return d;
+}
+
 template <int N>
-__global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm) {
+__global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm,
+                                                          int hdiv) {
   extern __shared__ fx::Weight s_w[];
   const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nCells * L;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
@@ -227,6 +245,17 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg
     }
   }
   const double ia = m.invAreaCell[c];
+  if (hdiv) {  // divergence of ru, for the next stage's tendencies
+    double x[N], hd;
+    bool ok = n <= N;
+    if (ok) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) x[j] = f.ru[(uint32_t)s_w[t + j].row * L + k];
+      ok = fx::dot<N>(x, s_w + t, &hd);
+    }
+    if (!ok) hd = wide_divergence(m, f.ru, c, k);
+    f.h_divergence[i] = hd * ia;
+  }
   f.divergence[i] = div * ia;
   // 0.25 (0.625 sum_j ke_edge + 0.375 sum_j kite ke_vertex) / area
   f.ke[i] = ia * fma(0.625 * 0.25, kee, (0.375 * 0.25) * kev);
@@ -276,18 +305,21 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_edges_b_fx(mpasg_mesh m, mpa
   f.ke_edge[i] = pve * u;
 }
 
-int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, int rk_step, cudaStream_t s) {
+int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, int rk_step, cudaStream_t s,
+                   const DiagFusion& fuse) {
   const int apvm = c->apvm_upwinding > 0.0 ? 1 : 0;
   const int L = m->nVertLevels, rows = (kBlock - 1) / L + 2;
   const int nc = nblocks((long long)m->nCells * L), ne = nblocks((long long)m->nEdges * L);
   const FastDiv fl(L);
-  k_diag_edges_a<double><<<ne, kBlock, 0, s>>>(*m, *f, fl);
-  MPASG_LAUNCH_CHECK();
+  if (!fuse.edges_done) {
+    k_diag_edges_a<double><<<ne, kBlock, 0, s>>>(*m, *f, fl);
+    MPASG_LAUNCH_CHECK();
+  }
   k_diag_vertices<double, false><<<nblocks((long long)m->nVertices * L), kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
   const size_t slot = 2 * sizeof(fx::Weight) + sizeof(double);
-  if (m->maxEdges <= 6) k_diag_cells_fx<6><<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm);
-  else k_diag_cells_fx<10><<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm);
+  if (m->maxEdges <= 6) k_diag_cells_fx<6><<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
+  else k_diag_cells_fx<10><<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
   MPASG_LAUNCH_CHECK();
   const double adt = c->apvm_upwinding * c->dt;
   const size_t se = rows * sizeof(ApvmEdge);
@@ -534,15 +566,18 @@ __global__ void k_prepare_rw(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
 // stencils carry a last-bit change of their start to the seventh digit; the float64 form takes
 // launch_diag_fx.
 template <typename T>
-int launch_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s) {
+int launch_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s,
+                       const DiagFusion& fuse = DiagFusion()) {
   const int L = m->nVertLevels;
   FastDiv fl(L);
   const int apvm = c->apvm_upwinding > 0.0 ? 1 : 0;
-  k_diag_edges_a<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, fl);
-  MPASG_LAUNCH_CHECK();
+  if (!fuse.edges_done) {
+    k_diag_edges_a<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(*m, *f, fl);
+    MPASG_LAUNCH_CHECK();
+  }
   k_diag_vertices<T, true><<<nblocks((long long)m->nVertices * L), kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
-  k_diag_cells<T><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, fl, apvm);
+  k_diag_cells<T><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
   MPASG_LAUNCH_CHECK();
   k_diag_edges_b<T><<<nblocks((long long)m->nEdges * L), kBlock, 0, s>>>(
       *m, *f, fl, rk_step == 3 ? 1 : 0, c->apvm_upwinding * c->dt, apvm);
@@ -558,16 +593,16 @@ extern "C" int mpasg_solve_diagnostics(const mpasg_mesh* m, const mpasg_config* 
 }
 
 int mpasgi_solve_diagnostics(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step,
-                             cudaStream_t s, bool copies_current) {
+                             cudaStream_t s, bool copies_current, const DiagFusion& fuse) {
   if (!m || !c || !f) return MPASG_E_ARG;
   if (c->precision == MPASG_PRECISION_MIXED) {
     if (!copies_current) {
       const int rc = mpasgi_pack_f32(m, f, s);
       if (rc != MPASG_OK) return rc;
     }
-    return launch_diagnostics<float>(m, c, f, rk_step, s);
+    return launch_diagnostics<float>(m, c, f, rk_step, s, fuse);
   }
-  return launch_diag_fx(m, c, f, rk_step, s);
+  return launch_diag_fx(m, c, f, rk_step, s, fuse);
 }
 
 extern "C" int mpasg_reconstruct_2d(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, void* stream) {

@@ -33,6 +33,8 @@ struct TendScalars {
   int ray_n;  // Rayleigh-damped top levels of u (0: off)
   int mix_pert;  // vertical mixing of the perturbation from the initial profiles
   double f3[4];  // flux3 with coef3 by upwind side: 7 + 3 c, 7 - 3 c, 1 + c, 1 - c
+  double first_dts;  // > 0: k_adv_edges also starts the acoustic substeps (TendFusion)
+  int smlstep;       // k_tend_w_theta also forms tend_rw
   int defer;  // k_tend_u leaves tend_u_euler to k_tend_u_finish (del4 and / or vertical mixing)
 };
 
@@ -753,8 +755,17 @@ MPASG_D T wdtz_at(const T* th, const T* ths, const T* rw_t, const double* rw, co
 // the reference's per-slot (sign * ru) * flux products bit for bit.  The mixed form
 // advects the deviation theta_m - ref_theta (its reference part is added in float64 by
 // k_tend_w_theta_mixed) and stores float32 fluxes.
+// first acoustic substep's edge update (k_acoustic_edges with small_step 1)
 template <typename T>
-__global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
+MPASG_D void first_acoustic_edge(const mpasg_fields& f, uint32_t i, double dts) {
+  const double rup = f64(cv<T>(dts) * cv<T>(f.tend_u[i]));
+  f.ru_p[i] = rup;
+  f.ruAvg[i] = rup;
+  if (sizeof(T) == sizeof(double)) f.ke_edge[i] = rup * f.theta_edge_save[i];
+}
+
+template <typename T>
+__global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double first_dts) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
@@ -765,6 +776,7 @@ __global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const T* cfp = G(adv_coefs_p) + (size_t)e * na;
   const T* cfm = G(adv_coefs_m) + (size_t)e * na;
   const T rue = cv<T>(f.ru[i]);
+  if (first_dts > 0.0) first_acoustic_edge<T>(f, i, first_dts);
   {
     const T* th = fp<T>(f.theta_m, f.theta_dev);
     const T* cf = rue >= T(0) ? cfp : cfm;
@@ -793,7 +805,8 @@ __global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
 // at 82 % of that pipe).  40962 x 55: 374 us in float64 alone, 271 us with both sums
 // on the integer side, 216 us with one each.
 template <int N, bool PERT>
-__global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
+__global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl,
+                                                         double first_dts) {
   extern __shared__ fx::Weight s_w[];
   const uint32_t L = (uint32_t)m.nVertLevels;
   const uint32_t n_all = (uint32_t)m.nEdges * L;
@@ -803,6 +816,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_
   __syncthreads();
   if (i >= n_all) return;
   const uint32_t e = fl.div(i), k = i - e * L;
+  if (first_dts > 0.0) first_acoustic_edge<double>(f, i, first_dts);
   const double rue = f.ru[i];
   const bool back = __double2hiint(rue) < 0;
   const fx::Weight* w = s_w + (e - e0) * (2 * N) + (back ? N : 0);
@@ -908,8 +922,11 @@ __global__ void __launch_bounds__(kBlock, 5) k_tend_w_theta(mpasg_mesh m, mpasg_
       f.tend_w_euler[i] = teu;
     }
     f.tend_w[i] = tw + teu;
+    // flat terrain: the small-step w tendency has no slope fluxes
+    if (p.smlstep) f.tend_rw[i] = fma(m.fzm[k], m.zz[oc + k], m.fzp[k] * m.zz[oc + k - 1]) * (tw + teu);
   } else {
     f.tend_w[i] = 0.0;
+    if (p.smlstep) f.tend_rw[i] = 0.0;
   }
   if (k < L) {
     const size_t o = oc + k;
@@ -1020,9 +1037,15 @@ __global__ void __launch_bounds__(kBlock) k_tend_w_theta_mixed(mpasg_mesh m, mpa
       if (p.v_mom > 0.0) teu = teu + cv<T>(w_vmix(m, f, oc, ow, k, p.v_mom));
       f.tend_w_euler[i] = f64(teu);
     }
-    f.tend_w[i] = f64(tw + teu);
+    const double w_tend = f64(tw + teu);
+    f.tend_w[i] = w_tend;
+    if (p.smlstep) {  // as k_smlstep_pert over flat terrain
+      const T fzm_t = cv<T>(m.fzm[k]), fzp_t = cv<T>(m.fzp[k]);
+      f.tend_rw[i] = f64((fzm_t * cv<T>(m.zz[oc + k]) + fzp_t * cv<T>(m.zz[oc + k - 1])) * cv<T>(w_tend));
+    }
   } else {
     f.tend_w[i] = 0.0;
+    if (p.smlstep) f.tend_rw[i] = 0.0;
   }
   if (k < (uint32_t)L) {
     const size_t o = oc + k;
@@ -1070,7 +1093,7 @@ MPASG_HD int tile_levels(int code) { return code == 2 ? 2 : code == 4 ? 4 : 1; }
 
 template <typename T>
 int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, int rk_step, cudaStream_t s,
-                    int c_tile) {
+                    int c_tile, bool hdiv_current) {
   const int L = m->nVertLevels;
   const long long ncl = (long long)m->nCells * L, nel = (long long)m->nEdges * L;
   const long long ncw = (long long)m->nCells * (L + 1), nvl = (long long)m->nVertices * L;
@@ -1079,11 +1102,13 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
     k_theta_dev<<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl);
     MPASG_LAUNCH_CHECK();
   }
-  if (p.ncam > 0 && rk_step == 1)
-    k_tend_cells_a<T, true><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
-  else
-    k_tend_cells_a<T><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
-  MPASG_LAUNCH_CHECK();
+  if (rk_step == 1 || !hdiv_current) {
+    if (p.ncam > 0 && rk_step == 1)
+      k_tend_cells_a<T, true><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
+    else
+      k_tend_cells_a<T><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
+    MPASG_LAUNCH_CHECK();
+  }
   const bool ray = p.ray_n > 0;
   if constexpr (sizeof(T) == sizeof(double)) {
     if (ray) launch_tend_u_fx<true>(m, f, p, s);
@@ -1133,12 +1158,12 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
     const size_t smem = (size_t)((kBlock - 1) / L + 2) * adv::kEntryBytes;
     const int nb = nblocks(nel);
     const bool narrow = m->nAdvMax <= 10, pert = rk_step > 1;
-    if (narrow && pert) k_adv_edges_fx<10, true><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl);
-    else if (narrow) k_adv_edges_fx<10, false><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl);
-    else if (pert) k_adv_edges_fx<14, true><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl);
-    else k_adv_edges_fx<14, false><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl);
+    if (narrow && pert) k_adv_edges_fx<10, true><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl, p.first_dts);
+    else if (narrow) k_adv_edges_fx<10, false><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl, p.first_dts);
+    else if (pert) k_adv_edges_fx<14, true><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl, p.first_dts);
+    else k_adv_edges_fx<14, false><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl, p.first_dts);
   } else {
-    k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl);
+    k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p.first_dts);
   }
   MPASG_LAUNCH_CHECK();
   if (sizeof(T) == sizeof(double)) {
@@ -1173,7 +1198,7 @@ extern "C" int mpasg_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_
 }
 
 int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s,
-                    bool copies_current) {
+                    bool copies_current, const TendFusion& fuse) {
   if (!m || !c || !f || rk_step < 1 || rk_step > 3) return MPASG_E_ARG;
   if (!copies_current && c->precision != MPASG_PRECISION_MIXED) {
     int rc = mpasgi_pvu(m, f, s);
@@ -1203,6 +1228,8 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
   p.f3[2] = 1.0 + p.coef3;
   p.f3[3] = 1.0 - p.coef3;
   p.rk_step = rk_step;
+  p.first_dts = fuse.first_dts;
+  p.smlstep = fuse.smlstep ? 1 : 0;
   p.del4 = (p.h_mom_visc4 > 0.0) ? 1 : 0;
   if (c->number_cam_damping_levels > m->nVertLevels) return MPASG_E_ARG;
   p.ncam = (c->mpas_cam_coef > 0.0 && c->number_cam_damping_levels > 0) ? c->number_cam_damping_levels : 0;
@@ -1224,9 +1251,9 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
       const int rc = mpasgi_pack_f32(m, f, s);
       if (rc != MPASG_OK) return rc;
     }
-    return launch_dyn_tend<float>(m, f, p, rk_step, s, c->tile_tend_u);
+    return launch_dyn_tend<float>(m, f, p, rk_step, s, c->tile_tend_u, fuse.hdiv_current);
   }
-  return launch_dyn_tend<double>(m, f, p, rk_step, s, c->tile_tend_u);
+  return launch_dyn_tend<double>(m, f, p, rk_step, s, c->tile_tend_u, fuse.hdiv_current);
 }
 
 // Autotuner: times the u-tendency kernel with 1, 2 and 4 levels per thread on the current
