@@ -26,6 +26,18 @@ struct FastDiv {
 // Fortran sign(1.0, x) as the reference's fct_sign_pm: +1 for x >= 0 (and -0.0).
 MPASG_D double sgn(double x) { return x >= 0.0 ? 1.0 : -1.0; }
 
+// x with its sign flipped where s is negative (a product with +-1, or with sign(s), on the
+// integer side)
+MPASG_D double flip_by(double x, double s) {
+  return __hiloint2double(__double2hiint(x) ^ (__double2hiint(s) & (int)0x80000000), __double2loint(x));
+}
+
+// the same for s < 0 strictly: sign(s) is +1 for -0.0, which matters where x does not carry s
+MPASG_D double flip_below(double x, double s) {
+  const bool neg = (unsigned long long)__double_as_longlong(s) > 0x8000000000000000ull;
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+
 // ---------------------------------------------------------------- stencil arithmetic type
 // Stencil kernels are templates on the arithmetic type T: double (plain float64 form) or
 // float (mixed form: float64 fields in memory, float32 stencil arithmetic).  On this part
@@ -164,6 +176,7 @@ struct TendFusion {
   double first_dts = 0.0;     // > 0: the first acoustic substep's edge update with this dts
   bool smlstep = false;       // the small-step w tendency (flat terrain only)
   bool hdiv_current = false;  // h_divergence already holds ru's divergence (later RK stages)
+  bool v_current = false;     // v is the TRiSK sum of u (left by the last RK stage's diagnostics)
 };
 int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s,
                     bool copies_current, const TendFusion& fuse = TendFusion());

@@ -394,6 +394,7 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
       tf.first_dts = dts;
       tf.smlstep = m->flatTerrain != 0;
       tf.hdiv_current = rk > 1;
+      tf.v_current = rk == 1 && sub > 1;  // the previous substep's last diagnostics
       CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true, tf));
       MARK(rk == 1 ? MPASG_STAGE_DYN_TEND_RK1 : MPASG_STAGE_DYN_TEND);
       if (!tf.smlstep) CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));

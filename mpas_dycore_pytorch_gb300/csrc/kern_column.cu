@@ -183,10 +183,12 @@ __global__ void k_vimp_factor(mpasg_mesh m, mpasg_fields f) {
 // increment in the stencil type T, ru_p accumulated in float64).  The fused and the separate
 // kernels share this and the explicit multiply-adds below, so a taped step, which runs the
 // stages one by one, repeats a step to the bit.
-template <typename T>
+// FROM_ZERO: rtheta_pp_old is zero (the first substep's), so rtheta_pp is the change itself.
+template <typename T, bool FROM_ZERO = false>
 MPASG_D double damped_ru_p(const mpasg_fields& f, uint32_t i, size_t i1, size_t i2, double coef) {
-  T d1 = -dif<T>(f.rtheta_pp[i1], f.rtheta_pp_old[i1]);  // substep change: float64 difference
-  T d2 = -dif<T>(f.rtheta_pp[i2], f.rtheta_pp_old[i2]);
+  // substep change: float64 difference
+  T d1 = FROM_ZERO ? -cv<T>(f.rtheta_pp[i1]) : -dif<T>(f.rtheta_pp[i1], f.rtheta_pp_old[i1]);
+  T d2 = FROM_ZERO ? -cv<T>(f.rtheta_pp[i2]) : -dif<T>(f.rtheta_pp[i2], f.rtheta_pp_old[i2]);
   // / (theta_m_save_1 + theta_m_save_2) as a product with the reciprocal formed once per
   // dynamics substep (k_theta_edge); within one rounding of the quotient
   if constexpr (sizeof(T) == sizeof(double)) return fma(coef * (d2 - d1), f.theta_edge_rsum[i], f.ru_p[i]);
@@ -194,7 +196,8 @@ MPASG_D double damped_ru_p(const mpasg_fields& f, uint32_t i, size_t i1, size_t 
 }
 
 // DAMP (small_step > 1): the previous substep's divergence damping first
-template <typename T, bool DAMP>
+// (the second substep's: FROM_ZERO)
+template <typename T, bool DAMP, bool FROM_ZERO = false>
 __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int small_step,
                                  double dts, double c2, double damp_coef) {
   const int L = m.nVertLevels;
@@ -212,7 +215,7 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
     pgrad = cv<T>(f.cqu_e[i]) * (T(0.5) * cv<T>(c2)) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
     if (!m.flatTerrain)  // no slope: adds exact zeros
       pgrad = pgrad + T(0.5) * cv<T>(m.zxu[i]) * T(kGravity) * (cv<T>(f.rho_pp[i1]) + cv<T>(f.rho_pp[i2]));
-    const double before = DAMP ? damped_ru_p<T>(f, i, i1, i2, damp_coef) : f.ru_p[i];
+    const double before = DAMP ? damped_ru_p<T, FROM_ZERO>(f, i, i1, i2, damp_coef) : f.ru_p[i];
     if constexpr (kDouble) rup = fma(dts, f.tend_u[i] - pgrad, before);
     else rup = before + f64(cv<T>(dts) * (cv<T>(f.tend_u[i]) - pgrad));
     f.ruAvg[i] = f.ruAvg[i] + rup;
@@ -754,14 +757,23 @@ __global__ void k_smlstep_pert(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   const T fzm = cv<T>(m.fzm[k]), fzp = cv<T>(m.fzp[k]);
   T acc = cv<T>(f.tend_w[i]);
   const int n = m.flatTerrain ? 0 : m.nEdgesOnCell[c];  // zero-slope terms add exact zeros
-  for (int j = 0; j < n; ++j) {
-    int e = m.edgesOnCell[c * me + j];
-    T ut_k = cv<T>(f.tend_u[(size_t)e * L + k]);
-    T u_i = fzm * ut_k + fzp * cv<T>(f.tend_u[(size_t)e * L + k - 1]);
-    T flux = cv<T>(m.edgesOnCell_sign[c * me + j]) * u_i;
-    size_t zi = ((size_t)c * me + j) * (L + 1) + k;
-    T coef = cv<T>(m.zb_cell[zi]) + (ut_k >= T(0) ? T(1) : T(-1)) * cv<T>(m.zb3_cell[zi]);
-    acc = acc - coef * flux;
+  if constexpr (sizeof(T) == sizeof(double)) {
+    for (int j = 0; j < n; ++j) {
+      const size_t i = (size_t)m.edgesOnCell[c * me + j] * L + k, zi = ((size_t)c * me + j) * (L + 1) + k;
+      const double ut_k = f.tend_u[i];
+      acc = fma(-flip_by(fma(fzm, ut_k, fzp * f.tend_u[i - 1]), m.edgesOnCell_sign[c * me + j]),
+                m.zb_cell[zi] + flip_below(m.zb3_cell[zi], ut_k), acc);
+    }
+  } else {
+    for (int j = 0; j < n; ++j) {
+      int e = m.edgesOnCell[c * me + j];
+      T ut_k = cv<T>(f.tend_u[(size_t)e * L + k]);
+      T u_i = fzm * ut_k + fzp * cv<T>(f.tend_u[(size_t)e * L + k - 1]);
+      T flux = cv<T>(m.edgesOnCell_sign[c * me + j]) * u_i;
+      size_t zi = ((size_t)c * me + j) * (L + 1) + k;
+      T coef = cv<T>(m.zb_cell[zi]) + (ut_k >= T(0) ? T(1) : T(-1)) * cv<T>(m.zb3_cell[zi]);
+      acc = acc - coef * flux;
+    }
   }
   size_t o = (size_t)c * L;
   if constexpr (sizeof(T) == sizeof(double))  // (as k_tend_w_theta forms it over flat terrain)
@@ -890,7 +902,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
 
 // FINISH: with the last acoustic substep's divergence damping before it and the diagnostics'
 // edge fields (k_diag_edges_a) after it: one pass over the edges instead of three
-template <typename T, bool FINISH>
+template <typename T, bool FINISH, bool FROM_ZERO>
 __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns, double damp_coef) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -902,7 +914,7 @@ __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double
   f.ruAvg[i] = rus + f.ruAvg[i] * inv_ns;
   double rup;
   if (FINISH) {
-    rup = damped_ru_p<T>(f, i, i1, i2, damp_coef);
+    rup = damped_ru_p<T, FROM_ZERO>(f, i, i1, i2, damp_coef);
     f.ru_p[i] = rup;
   } else {
     rup = f.ru_p[i];
@@ -912,11 +924,11 @@ __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double
   const double rho_1 = f.rho_zz[i1], rho_2 = f.rho_zz[i2];
   const double rho2 = rho_1 + rho_2;
   // 2 ru / rho2 (the factor two is exact wherever it is applied)
-  const double u = kDouble ? fx::quotient(ru + ru, rho2) : 2.0 * ru * rcp_nr1(rho2);
+  const double u = kDouble ? fx::quotient(ru, 0.5 * rho2) : 2.0 * ru * rcp_nr1(rho2);
   f.u[i] = u;
   if (!kDouble) f.u_f32[i] = d2f_bits(u);
   if (FINISH) {
-    f.h_edge[i] = f64(T(0.5) * (cv<T>(rho_1) + cv<T>(rho_2)));
+    f.h_edge[i] = kDouble ? 0.5 * rho2 : f64(T(0.5) * (cv<T>(rho_1) + cv<T>(rho_2)));
     const T u_t = cv<T>(u);
     const T dcdv = kDouble ? cv<T>(m.edge_dcdv[e]) : G(dcEdge)[e] * G(dvEdge)[e];
     fpw<T>(f.ke_edge, f.ke_edge_f32)[i] = dcdv * (u_t * u_t);
@@ -958,10 +970,16 @@ __global__ void k_recover_w(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   double acc = f.w[i];  // omega-derived part from k_recover_cells
   for (int j = 0; j < n; ++j) {
     int e = m.edgesOnCell[c * me + j];
-    double fi = fzm * f.ru[(size_t)e * L + k] + fzp * f.ru[(size_t)e * L + k - 1];
     size_t zi = ((size_t)c * me + j) * (L + 1) + k;
-    double ci = m.zb_cell[zi] + sgn(fi) * m.zb3_cell[zi];
-    acc = acc + m.edgesOnCell_sign[c * me + j] * ci * fi;
+    if (kMixed) {
+      double fi = fzm * f.ru[(size_t)e * L + k] + fzp * f.ru[(size_t)e * L + k - 1];
+      double ci = m.zb_cell[zi] + sgn(fi) * m.zb3_cell[zi];
+      acc = acc + m.edgesOnCell_sign[c * me + j] * ci * fi;
+    } else {
+      const size_t i = (size_t)e * L + k;
+      const double fi = fma(fzm, f.ru[i], fzp * f.ru[i - 1]);
+      acc = fma(flip_by(fi, m.edgesOnCell_sign[c * me + j]), m.zb_cell[zi] + flip_by(m.zb3_cell[zi], fi), acc);
+    }
   }
   const double wk = fdiv<T>(acc, fzm * f.rho_zz[oc + k] + fzp * f.rho_zz[oc + k - 1]);
   f.w[i] = wk;
@@ -970,7 +988,7 @@ __global__ void k_recover_w(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
 
 template <typename T>
 int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv_ns, double rk_dt, cudaStream_t s,
-                   bool finish, double damp_coef) {
+                   bool finish, double damp_coef, bool one_substep) {
   const int L = m->nVertLevels;
   const long long ncw = (long long)m->nCells * (L + 1);
   if (m->flatTerrain)
@@ -979,8 +997,9 @@ int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv
     k_recover_cells<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), rk_step, inv_ns, rk_dt);
   MPASG_LAUNCH_CHECK();
   const int ne = nblocks((long long)m->nEdges * L);
-  if (finish) k_recover_edges<T, true><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, damp_coef);
-  else k_recover_edges<T, false><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, 0.0);
+  if (finish && one_substep) k_recover_edges<T, true, true><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, damp_coef);
+  else if (finish) k_recover_edges<T, true, false><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, damp_coef);
+  else k_recover_edges<T, false, false><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, 0.0);
   MPASG_LAUNCH_CHECK();
   if (!m->flatTerrain) {  // slope fluxes need the new ru of k_recover_edges
     k_recover_w<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1));
@@ -1093,7 +1112,11 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
       const int ne = nblocks((long long)m->nEdges * L);
       const double coef = damping_coefficient(c, dts);
       const FastDiv fl(L);
-      if (mixed && fuse.damp_before)
+      if (mixed && fuse.damp_before && small_step == 2)
+        k_acoustic_edges<float, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+      else if (fuse.damp_before && small_step == 2)
+        k_acoustic_edges<double, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+      else if (mixed && fuse.damp_before)
         k_acoustic_edges<float, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
       else if (mixed)
         k_acoustic_edges<float, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
@@ -1189,8 +1212,8 @@ int recover(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_
   if (!m || !c || !f || ns < 1) return MPASG_E_ARG;
   const double inv_ns = 1.0 / (double)ns;
   if (c->precision == MPASG_PRECISION_MIXED)
-    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef);
-  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef);
+    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1);
+  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1);
 }
 }  // namespace
 

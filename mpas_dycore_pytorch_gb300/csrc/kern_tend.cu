@@ -35,6 +35,7 @@ struct TendScalars {
   double f3[4];  // flux3 with coef3 by upwind side: 7 + 3 c, 7 - 3 c, 1 + c, 1 - c
   double first_dts;  // > 0: k_adv_edges also starts the acoustic substeps (TendFusion)
   int smlstep;       // k_tend_w_theta also forms tend_rw
+  int v_current;     // v already holds the TRiSK sum of u
   int defer;  // k_tend_u leaves tend_u_euler to k_tend_u_finish (del4 and / or vertical mixing)
 };
 
@@ -82,7 +83,11 @@ __global__ void k_tend_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendSca
       dd = ndd;
       dof = ndo;
     }
-    double kd = f64(vmin(cv<T>(p.c_s_len2) * vsqrt(dd * dd + dof * dof), cv<T>(p.kdiff_cap)));
+    double kd;
+    if constexpr (sizeof(T) == sizeof(double))
+      kd = fx::min_nonneg(p.c_s_len2 * sqrt(dd * dd + dof * dof), p.kdiff_cap);
+    else
+      kd = f64(vmin(cv<T>(p.c_s_len2) * vsqrt(dd * dd + dof * dof), cv<T>(p.kdiff_cap)));
     if (CAM && (int)k >= L - p.ncam) kd = cam_kdiff(kd, p, k, L);
     f.kdiff[i] = kd;
   } else {  // 2d_fixed: the theta del2 coefficient everywhere
@@ -357,7 +362,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_tend_u_fx(mpasg_mesh m, mpasg_fie
                             m.fzp);
   const fx::Weight* w = s_w + (e - e0) * N;
   const EdgeConst ec = s_e[e - e0];
-  const double sa = trisk::sum<N>(m, u, w, e, k, L);
+  const double sa = p.v_current ? f.v[i] : trisk::sum<N>(m, u, w, e, k, L);
   const double sb = trisk::sum<N>(m, f.ke_edge, w, e, k, L);  // pv u
   const size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2 * L + k;
   const double rho_e = f.h_edge[i], u_k = ue[k];
@@ -1230,6 +1235,7 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
   p.rk_step = rk_step;
   p.first_dts = fuse.first_dts;
   p.smlstep = fuse.smlstep ? 1 : 0;
+  p.v_current = fuse.v_current ? 1 : 0;
   p.del4 = (p.h_mom_visc4 > 0.0) ? 1 : 0;
   if (c->number_cam_damping_levels > m->nVertLevels) return MPASG_E_ARG;
   p.ncam = (c->mpas_cam_coef > 0.0 && c->number_cam_damping_levels > 0) ? c->number_cam_damping_levels : 0;
