@@ -199,6 +199,7 @@ int mpasgi_divergence_damping(const mpasg_mesh* m, const mpasg_config* c, mpasg_
 struct AcousticFusion {
   bool edges_done = false;   // first substep: ru_p and ruAvg already formed (by the tendencies)
   bool damp_before = false;  // later substeps: the previous substep's divergence damping first
+  bool scratch = false;      // ac_rs, ac_ts and ac_x need not be left behind
 };
 int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
                          cudaStream_t s, bool copies_current, const AcousticFusion& fuse = AcousticFusion());

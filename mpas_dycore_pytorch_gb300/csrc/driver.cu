@@ -403,6 +403,7 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
         AcousticFusion af;
         af.edges_done = small == 1;
         af.damp_before = small > 1;
+        af.scratch = true;
         CHECK_RC(mpasgi_acoustic_step(m, c, &f, small, dts, s, true, af));
         MARK(MPASG_STAGE_ACOUSTIC);
       }

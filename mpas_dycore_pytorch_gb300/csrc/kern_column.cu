@@ -8,6 +8,8 @@
 #include "common.cuh"
 #include "pow_exner.cuh"
 
+#include <algorithm>
+
 namespace {
 
 // ---------------------------------------------------------------- moist coefficients
@@ -43,11 +45,26 @@ __global__ void k_moist_edges(int ne, int L, FastDiv fl, int ms, int me, const i
   }
 }
 
+// Columns of a block in the kernels that keep whole columns in shared memory (`items`: the
+// levels or faces of one that the block's 256 threads share out).  Two full passes of the
+// threads over a block's items, so that no pass is nearly empty (33 levels, 10242 columns:
+// acoustic stage 276 us with 14 columns, 303 with 11, whose last pass fills 46 of 256 threads),
+// and at most 18: the serial sweeps take one lane a column, and more than that buys nothing.
+// A small mesh takes fewer, one pass, down to 4: float64 work is bound to its SM and the
+// sweeps of a block wait for all its levels (162 columns of 12 levels: step 666 us with 4, 674
+// with 16, 724 with 32; 642 of 55: 1013, 1159, 1319).
+inline int columns_per_block(int nCells, int items, int cells_per_column) {
+  const int least = std::max(2, std::min(4, kBlock / items));
+  return std::max(least, std::min({18, 2 * kBlock / items, nCells / cells_per_column}));
+}
+constexpr size_t kMaxSmem = 200 * 1024;
+
 // ---------------------------------------------------------------- vertical implicit coefficients
 // dynamics/vert_imp_coefs.py:188 (coefficients :343-446, Thomas factor :100-121).
-// k_vimp_coefs builds every level's coefficients and tridiagonal diagonals in parallel
-// (neighbour levels shared through shared memory); k_vimp_factor runs the sequential
-// Thomas factorisation, one thread per column.
+// k_vimp_columns builds every level's coefficients and tridiagonal diagonals in parallel
+// and runs the sequential Thomas factorisation, one thread per column, on columns held in
+// shared memory; k_vimp_coefs and k_vimp_factor do the same through memory for columns
+// too high for it.
 struct VimpLevel {
   double cofwt, coftz;
 };
@@ -92,10 +109,43 @@ MPASG_D VimpLevel vimp_level(const mpasg_mesh& m, const mpasg_fields& f, size_t 
   return v;
 }
 
+// An inner level's cofwr and cofwz and its row of the tridiagonal matrix, from the level
+// itself and its neighbours below (lo) and above (coftz only).
+struct VimpRow {
+  double a, b, c;
+};
+template <typename T>
+MPASG_D VimpRow vimp_row(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k,
+                         const VimpLevel& at, const VimpLevel& lo, double ct_kp1, const VimpScalars& s) {
+  const double zz = m.zz[o + k], zzm = m.zz[o + k - 1];
+  const double fzm = m.fzm[k], fzp = m.fzp[k];
+  const double z_i = fzm * zz + fzp * zzm;
+  const double cofwr = s.cg * z_i;
+  const double p_i = fzm * f.exner[o + k] + fzp * f.exner[o + k - 1];
+  const double cofwz = s.c2 * z_i * m.rdzu[k] * f.cqw[ow + k] * p_i;
+  f.cofwr[o + k] = cofwr;
+  f.cofwz[o + k] = cofwz;
+  const double ct_km1 = lo.coftz, ct_k = at.coftz;
+  const double cw_k = at.cofwt, cw_km1 = lo.cofwt;
+  const double rdzw_k = m.rdzw[k], rdzw_km1 = m.rdzw[k - 1];
+  const double cofrz_k = s.dtseps * rdzw_k, cofrz_km1 = s.dtseps * rdzw_km1;
+  // the reference's coefficients (vert_imp_coefs.py:388-428) with their common factors taken out
+  const double tm = ct_km1 * rdzw_km1, tp = ct_kp1 * rdzw_k;
+  VimpRow r;
+  r.a = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
+  r.b = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
+        cofwr * (cofrz_k - cofrz_km1);
+  if (sizeof(T) == sizeof(double))
+    r.c = fma(cw_k, tp, -fma(cofwz * zz, tp, cofwr * cofrz_k));
+  else
+    r.c = tp * (cw_k - cofwz * zz) - cofwr * cofrz_k;
+  return r;
+}
+
 // Bound by the float64 pipe: 63 operations a level with two divisions in the reference's
 // expressions, 40 with the scalars' products formed on the host, the quotient of
 // fastdiv64.cuh and the common factors taken out of the diagonals (fewer roundings each):
-// 263 -> 193 us at 40962 x 55.
+// 263 -> 193 us at 40962 x 55 before the factorisation joined it (k_vimp_columns).
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_fields f, FastDiv fl, VimpScalars s) {
   __shared__ double s_cw[kBlock], s_ct[kBlock];
@@ -128,34 +178,89 @@ __global__ void __launch_bounds__(kBlock) k_vimp_coefs(mpasg_mesh m, mpasg_field
     f.c_tri[o] = 0.0;
     return;
   }
-  const double zz = m.zz[o + k], zzm = m.zz[o + k - 1];
-  const double fzm = m.fzm[k], fzp = m.fzp[k];
-  const double z_i = fzm * zz + fzp * zzm;
-  const double cofwr = s.cg * z_i;
-  const double p_i = fzm * f.exner[o + k] + fzp * f.exner[o + k - 1];
-  const double cofwz = s.c2 * z_i * m.rdzu[k] * f.cqw[ow + k] * p_i;
-  f.cofwr[o + k] = cofwr;
-  f.cofwz[o + k] = cofwz;
   // neighbour levels (k-1 below, k+1 above) from shared memory or recomputed at block edges
   VimpLevel lo = (threadIdx.x >= 1) ? VimpLevel{s_cw[threadIdx.x - 1], s_ct[threadIdx.x - 1]}
                                     : vimp_level<T>(m, f, o, k - 1, s);
   double ct_kp1 = 0.0;
   if (k + 1 < (uint32_t)L)
     ct_kp1 = (threadIdx.x + 1 < blockDim.x) ? s_ct[threadIdx.x + 1] : vimp_level<T>(m, f, o, k + 1, s).coftz;
-  const double ct_km1 = lo.coftz, ct_k = me_.coftz;
-  const double cw_k = me_.cofwt, cw_km1 = lo.cofwt;
-  const double rdzw_k = m.rdzw[k], rdzw_km1 = m.rdzw[k - 1];
-  const double cofrz_k = s.dtseps * rdzw_k, cofrz_km1 = s.dtseps * rdzw_km1;
-  // the reference's coefficients (vert_imp_coefs.py:388-428) with their common factors taken out
-  const double tm = ct_km1 * rdzw_km1, tp = ct_kp1 * rdzw_k;
-  f.a_tri[o + k] = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
-  f.b_tri[o + k] = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
-                   cofwr * (cofrz_k - cofrz_km1);
-  if (sizeof(T) == sizeof(double))
-    f.c_tri[o + k] = fma(cw_k, tp, -fma(cofwz * zz, tp, cofwr * cofrz_k));
-  else
-    f.c_tri[o + k] = tp * (cw_k - cofwz * zz) - cofwr * cofrz_k;
+  const VimpRow r = vimp_row<T>(m, f, o, ow, k, me_, lo, ct_kp1, s);
+  f.a_tri[o + k] = r.a;
+  f.b_tri[o + k] = r.b;
+  f.c_tri[o + k] = r.c;
 }
+
+// One column's Thomas factors over rows `pitch` apart (al may be b, gm may be c)
+template <typename T>
+MPASG_D void factor_column(const double* a, const double* b, const double* c, double* al, double* gm, uint32_t L,
+                           uint32_t pitch) {
+  double gam = 0.0;
+  al[0] = 0.0;
+  gm[0] = 0.0;
+  for (uint32_t k = 1, q = pitch; k < L; ++k, q += pitch) {
+    const double alpha = recip<T>(b[q] - a[q] * gam);
+    gam = c[q] * alpha;
+    al[q] = alpha;
+    gm[q] = gam;
+  }
+}
+
+// Coefficients and factorisation of `cols` columns in one launch, what passes between them in
+// shared memory ([level][column], odd pitch).  In place of two launches, each a few waves of
+// latency on a small mesh: a step of 162 columns x 12 levels 664 -> 640 us, 2562 x 26 1359 ->
+// 1334, 40962 x 55 25.58 -> 25.52 ms (mixed form 17.61 -> 17.56).
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fields f, FastDiv fl, int cols,
+                                                         VimpScalars s) {
+  extern __shared__ double s_col[];
+  const uint32_t L = (uint32_t)m.nVertLevels, pitch = (uint32_t)cols | 1u, nlp = L * pitch;
+  double* s_cw = s_col;  // L x pitch each
+  double* s_ct = s_cw + nlp;
+  double* sa = s_ct + nlp;
+  double* sb = sa + nlp;
+  double* sc = sb + nlp;
+  const uint32_t c0 = blockIdx.x * (uint32_t)cols, ncol = min((uint32_t)cols, (uint32_t)m.nCells - c0), nl = ncol * L;
+  const size_t o0 = (size_t)c0 * L, ow0 = o0 + c0;
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    const VimpLevel v = vimp_level<T>(m, f, o0 + col * L, k, s);
+    if (c0 + col == 0) f.cofrz[k] = s.dtseps * m.rdzw[k];
+    s_cw[q] = v.cofwt;
+    s_ct[q] = v.coftz;
+    f.cofwt[o0 + i] = v.cofwt;
+    f.coftz[ow0 + i + col] = v.coftz;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    VimpRow r{0.0, 1.0, 0.0};
+    if (k == 0) {
+      f.cofwr[o0 + i] = 0.0;
+      f.cofwz[o0 + i] = 0.0;
+      f.coftz[ow0 + i + col + L] = 0.0;
+    } else {
+      r = vimp_row<T>(m, f, o0 + col * L, ow0 + col * (L + 1), k, VimpLevel{s_cw[q], s_ct[q]},
+                      VimpLevel{s_cw[q - pitch], s_ct[q - pitch]}, k + 1 < L ? s_ct[q + pitch] : 0.0, s);
+    }
+    f.a_tri[o0 + i] = sa[q] = r.a;
+    f.b_tri[o0 + i] = sb[q] = r.b;
+    f.c_tri[o0 + i] = sc[q] = r.c;
+  }
+  __syncthreads();
+  if (threadIdx.x < ncol) {
+    const uint32_t t = threadIdx.x;
+    factor_column<T>(sa + t, sb + t, sc + t, sb + t, sc + t, L, pitch);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    f.alpha_tri[o0 + i] = sb[q];
+    f.gamma_tri[o0 + i] = sc[q];
+    if (sizeof(T) != sizeof(double) && k > 0) f.tri_m[o0 + i] = -(sb[q] * sa[q]);
+  }
+}
+
+size_t vimp_columns_smem_bytes(int L, int cols) { return (size_t)5 * L * (cols | 1) * sizeof(double); }
 
 template <typename T>
 __global__ void k_vimp_factor(mpasg_mesh m, mpasg_fields f) {
@@ -163,16 +268,9 @@ __global__ void k_vimp_factor(mpasg_mesh m, mpasg_fields f) {
   if (c >= m.nCells) return;
   const int L = m.nVertLevels;
   const size_t o = (size_t)c * L;
-  double gam = 0.0;
-  f.alpha_tri[o] = 0.0;
-  f.gamma_tri[o] = 0.0;
-  for (int k = 1; k < L; ++k) {
-    double alpha = recip<T>(f.b_tri[o + k] - f.a_tri[o + k] * gam);
-    gam = f.c_tri[o + k] * alpha;
-    f.alpha_tri[o + k] = alpha;
-    f.gamma_tri[o + k] = gam;
-    if (sizeof(T) != sizeof(double)) f.tri_m[o + k] = -(alpha * f.a_tri[o + k]);
-  }
+  factor_column<T>(f.a_tri + o, f.b_tri + o, f.c_tri + o, f.alpha_tri + o, f.gamma_tri + o, L, 1);
+  if (sizeof(T) != sizeof(double))
+    for (int k = 1; k < L; ++k) f.tri_m[o + k] = -(f.alpha_tri[o + k] * f.a_tri[o + k]);
 }
 
 // ---------------------------------------------------------------- acoustic substep, edges
@@ -291,11 +389,29 @@ MPASG_D AcLevel ac_level(const mpasg_mesh& m, const mpasg_fields& f, const fx::W
   } else {
     const double rho_in = f.rho_pp[o], rt_in = f.rtheta_pp[o], w0 = f.rw_p[ow], w1 = f.rw_p[ow + 1];
     a.rs = fma(-(resm * f.cofrz[k]), w1 - w0, fma(dts, f.tend_rho[o] - s1, rho_in));
-    a.ts = fma(-(resm * m.rdzw[k]), f.coftz[ow + 1] * w1 - f.coftz[ow] * w0, fma(dts, f.tend_theta[o] - s2, rt_in));
+    a.ts = fma(-(resm * m.rdzw[k]), fma(f.coftz[ow + 1], w1, -(f.coftz[ow] * w0)),
+               fma(dts, f.tend_theta[o] - s2, rt_in));
     a.R = fma(resm, rho_in, a.rs);
     a.P = fma(resm, rt_in, a.ts);
   }
   return a;
+}
+
+// the tridiagonal right-hand side of an inner level
+template <bool FIRST>
+MPASG_D double ac_rhs(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, double rwp, double R, double P,
+                      double R_lo, double P_lo, double dts) {
+  double x = FIRST ? dts * f.tend_rw[ow] : fma(dts, f.tend_rw[ow], rwp);
+  x = fma(-f.cofwz[o], fma(m.zz[o], P, -(m.zz[o - 1] * P_lo)), x);
+  x = fma(-f.cofwr[o], R + R_lo, x);
+  return fma(f.cofwt[o - 1], P_lo, fma(f.cofwt[o], P, x));
+}
+
+// rho_pp and rtheta_pp from the solution above and below a level
+MPASG_D void ac_level_out(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k, double rs,
+                          double ts, double xr, double xr1) {
+  f.rho_pp[o] = fma(-f.cofrz[k], xr1 - xr, rs);
+  f.rtheta_pp[o] = fma(-m.rdzw[k], fma(f.coftz[ow + 1], xr1, -(f.coftz[ow] * xr)), ts);
 }
 
 template <int N, bool FIRST>
@@ -349,10 +465,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_ac_prep(mpasg_mesh m, mpasg_field
     P_lo = lo.P;
   }
   f.wwAvg[ow + k] = FIRST ? 0.0 : fma(ww_lo, rwp_k, f.wwAvg[ow + k]);
-  double x = FIRST ? dts * f.tend_rw[ow + k] : fma(dts, f.tend_rw[ow + k], rwp_k);
-  x = fma(-f.cofwz[o + k], m.zz[o + k] * lv.P - m.zz[o + k - 1] * P_lo, x);
-  x = fma(-f.cofwr[o + k], lv.R + R_lo, x);
-  f.ac_x[ow + k] = fma(f.cofwt[o + k - 1], P_lo, fma(f.cofwt[o + k], lv.P, x));
+  f.ac_x[ow + k] = ac_rhs<FIRST>(m, f, o + k, ow + k, rwp_k, lv.R, lv.P, R_lo, P_lo, dts);
 }
 
 int launch_ac_prep(const mpasg_mesh* m, const mpasg_fields* f, int small_step, double dts, double epssm, double resm,
@@ -370,23 +483,43 @@ int launch_ac_prep(const mpasg_mesh* m, const mpasg_fields* f, int small_step, d
   return MPASG_OK;
 }
 
+// One column's sweeps over rows `pitch` apart; the next level's operands are read ahead of
+// the serial chain.  MIXED: `a` holds -alpha a, one multiply-add a level in the chain
+// (alpha x does not depend on it and issues ahead).
+template <bool MIXED = false>
+MPASG_D void thomas_column(double* x, const double* a, const double* al, const double* g, uint32_t L, uint32_t pitch) {
+  const uint32_t q1 = L > 1 ? pitch : 0;
+  double xp = x[0], xk = x[q1], ak = a[q1], alk = al[q1];
+  for (uint32_t k = 1, q = pitch; k < L; ++k, q += pitch) {
+    const uint32_t qn = k + 1 < L ? q + pitch : q;
+    const double xn = x[qn], an = a[qn], aln = al[qn];
+    xp = MIXED ? fma(ak, xp, alk * xk) : fma(-ak, xp, xk) * alk;
+    x[q] = xp;
+    xk = xn;
+    ak = an;
+    alk = aln;
+  }
+  uint32_t q = (L - 1) * pitch;
+  double xn = x[q + pitch], gk = g[q];
+  xk = x[q];
+  for (uint32_t k = L; k-- > 0;) {
+    const uint32_t qn = k > 0 ? q - pitch : q;
+    const double xl = x[qn], gl = g[qn];
+    xn = fma(-gk, xn, xk);
+    x[q] = xn;
+    xk = xl;
+    gk = gl;
+    q = qn;
+  }
+}
+
 __global__ void k_ac_thomas(mpasg_mesh m, mpasg_fields f) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nCells) return;
   const int L = m.nVertLevels;
   const size_t o = (size_t)c * L;
   const size_t ow = (size_t)c * (L + 1);
-  double* x = f.ac_x + ow;
-  double xp = x[0];
-  for (int k = 1; k < L; ++k) {
-    xp = (x[k] - f.a_tri[o + k] * xp) * f.alpha_tri[o + k];
-    x[k] = xp;
-  }
-  double xn = x[L];
-  for (int k = L - 1; k >= 0; --k) {
-    xn = x[k] - f.gamma_tri[o + k] * xn;
-    x[k] = xn;
-  }
+  thomas_column(f.ac_x + ow, f.a_tri + o, f.alpha_tri + o, f.gamma_tri + o, L, 1);
 }
 
 // ---------------------------------------------------------------- acoustic columns, mixed form
@@ -395,7 +528,7 @@ __global__ void k_ac_thomas(mpasg_mesh m, mpasg_fields f) {
 // increments in float32 and accumulates them in float64 (ac_rs, ac_ts, ac_x, rho_pp,
 // rtheta_pp, wwAvg); the tridiagonal solve stays float64.  theta at the edges is split
 // into the reference profile and the float32 deviation (theta_save_dev).
-struct AcLevelF {
+struct alignas(16) AcLevelF {
   float drs, dts, rho_in, rt_in;  // float32 increments of rs / ts, and the inputs
 };
 
@@ -433,6 +566,20 @@ MPASG_D AcLevelF ac_level_mixed(const mpasg_mesh& m, const mpasg_fields& f, int 
   return a;
 }
 
+// the tridiagonal right-hand side's float32 increment at an inner level
+MPASG_D float ac_rhs_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k,
+                           const AcLevelF& lv, const AcLevelF& lo, float dts, float resm) {
+  const float zz_k = m.zz_f32[o + k], zz_km1 = m.zz_f32[o + k - 1];
+  const float cw_k = cv<float>(f.cofwt[o + k]), cw_km1 = cv<float>(f.cofwt[o + k - 1]);
+  const float ts_k = lv.rt_in + lv.dts, ts_km1 = lo.rt_in + lo.dts;
+  const float rs_k = lv.rho_in + lv.drs, rs_km1 = lo.rho_in + lo.drs;
+  return dts * cv<float>(f.tend_rw[ow + k]) -
+         cv<float>(f.cofwz[o + k]) *
+             ((zz_k * ts_k - zz_km1 * ts_km1) + resm * (zz_k * lv.rt_in - zz_km1 * lo.rt_in)) -
+         cv<float>(f.cofwr[o + k]) * ((rs_k + rs_km1) + resm * (lv.rho_in + lo.rho_in)) +
+         cw_k * (ts_k + resm * lv.rt_in) + cw_km1 * (ts_km1 + resm * lo.rt_in);
+}
+
 __global__ void __launch_bounds__(kBlock) k_ac_prep_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl1,
                                                           int small_step, float dts, float epssm, float resm) {
   __shared__ AcLevelF s_lv[kBlock];
@@ -467,17 +614,8 @@ __global__ void __launch_bounds__(kBlock) k_ac_prep_mixed(mpasg_mesh m, mpasg_fi
   const AcLevelF lo = (threadIdx.x >= 1) ? s_lv[threadIdx.x - 1]
                                          : ac_level_mixed(m, f, c, k - 1, first, dts, resm, nullptr, nullptr);
   const double ww_in = first ? 0.0 : f.wwAvg[ow + k];
-  const float rwp = cv<float>(rwp_k);
-  f.wwAvg[ow + k] = ww_in + f64(0.5f * (1.0f - epssm) * rwp);
-  const float zz_k = m.zz_f32[o + k], zz_km1 = m.zz_f32[o + k - 1];
-  const float cw_k = cv<float>(f.cofwt[o + k]), cw_km1 = cv<float>(f.cofwt[o + k - 1]);
-  const float ts_k = lv.rt_in + lv.dts, ts_km1 = lo.rt_in + lo.dts;
-  const float rs_k = lv.rho_in + lv.drs, rs_km1 = lo.rho_in + lo.drs;
-  const float inc = dts * cv<float>(f.tend_rw[ow + k]) -
-                    cv<float>(f.cofwz[o + k]) *
-                        ((zz_k * ts_k - zz_km1 * ts_km1) + resm * (zz_k * lv.rt_in - zz_km1 * lo.rt_in)) -
-                    cv<float>(f.cofwr[o + k]) * ((rs_k + rs_km1) + resm * (lv.rho_in + lo.rho_in)) +
-                    cw_k * (ts_k + resm * lv.rt_in) + cw_km1 * (ts_km1 + resm * lo.rt_in);
+  f.wwAvg[ow + k] = ww_in + f64(0.5f * (1.0f - epssm) * cv<float>(rwp_k));
+  const float inc = ac_rhs_mixed(m, f, o, ow, k, lv, lo, dts, resm);
   f.ac_x[ow + k] = rwp_k + f64(inc);
 }
 
@@ -493,6 +631,14 @@ MPASG_D double ac_damped_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_
   double rw_delta = f.rw_save[ow + k] - f.rw[ow + k];
   double num = x + rw_delta - dts * dss * zz_i * rho_i * f.w[ow + k];
   return fdiv<float>(num, 1.0 + dts * dss) - rw_delta;
+}
+
+// rho_pp and rtheta_pp from the solution above and below a level
+MPASG_D void ac_level_out_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k, double rs,
+                                double ts, double xr, double xr1) {
+  const float x0 = cv<float>(xr), x1 = cv<float>(xr1);
+  f.rho_pp[o] = rs - f64(cv<float>(f.cofrz[k]) * dif<float>(xr1, xr));
+  f.rtheta_pp[o] = ts - f64(m.rdzw_f32[k] * (cv<float>(f.coftz[ow + 1]) * x1 - cv<float>(f.coftz[ow]) * x0));
 }
 
 __global__ void __launch_bounds__(kBlock) k_ac_post_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl1, double dts,
@@ -519,10 +665,7 @@ __global__ void __launch_bounds__(kBlock) k_ac_post_mixed(mpasg_mesh m, mpasg_fi
   if (k == (uint32_t)L) return;
   const double xr1 = (threadIdx.x + 1 < blockDim.x) ? s_xr[threadIdx.x + 1]
                                                     : ac_damped_mixed(m, f, o, ow, k + 1, L, f.ac_x[ow + k + 1], dts);
-  const float x0 = cv<float>(xr), x1 = cv<float>(xr1);
-  f.rho_pp[o + k] = f.ac_rs[o + k] - f64(cv<float>(f.cofrz[k]) * dif<float>(xr1, xr));
-  f.rtheta_pp[o + k] = f.ac_ts[o + k] - f64(m.rdzw_f32[k] * (cv<float>(f.coftz[ow + k + 1]) * x1 -
-                                                             cv<float>(f.coftz[ow + k]) * x0));
+  ac_level_out_mixed(m, f, o + k, ow + k, k, f.ac_rs[o + k], f.ac_ts[o + k], xr, xr1);
 }
 
 // The same sweeps with the columns staged through shared memory: one warp solves 32
@@ -561,18 +704,7 @@ __global__ void __launch_bounds__(kThomasThreads) k_ac_thomas_staged(mpasg_mesh 
     sg[k * kThomasPitch + col] = f.gamma_tri[o0 + idx];
   }
   __syncthreads();
-  if (t < ncol) {
-    double xp = sx[t];
-    for (int k = 1; k < L; ++k) {
-      xp = (sx[k * kThomasPitch + t] - sa[k * kThomasPitch + t] * xp) * sal[k * kThomasPitch + t];
-      sx[k * kThomasPitch + t] = xp;
-    }
-    double xn = sx[L * kThomasPitch + t];
-    for (int k = L - 1; k >= 0; --k) {
-      xn = sx[k * kThomasPitch + t] - sg[k * kThomasPitch + t] * xn;
-      sx[k * kThomasPitch + t] = xn;
-    }
-  }
+  if (t < ncol) thomas_column(sx + t, sa + t, sal + t, sg + t, L, kThomasPitch);
   __syncthreads();
   double* gxo = f.ac_x + (size_t)c0 * (L + 1);
   for (uint32_t idx = t; idx < nw; idx += kThomasThreads) {
@@ -609,18 +741,7 @@ __global__ void __launch_bounds__(kThomasThreads) k_ac_thomas_staged_mixed(mpasg
     sg[k * kThomasPitch + col] = f.gamma_tri[o0 + idx];
   }
   __syncthreads();
-  if (t < ncol) {
-    double xp = sx[t];
-    for (int k = 1; k < L; ++k) {
-      xp = fma(sm[k * kThomasPitch + t], xp, sal[k * kThomasPitch + t] * sx[k * kThomasPitch + t]);
-      sx[k * kThomasPitch + t] = xp;
-    }
-    double xn = sx[L * kThomasPitch + t];
-    for (int k = L - 1; k >= 0; --k) {
-      xn = fma(-sg[k * kThomasPitch + t], xn, sx[k * kThomasPitch + t]);
-      sx[k * kThomasPitch + t] = xn;
-    }
-  }
+  if (t < ncol) thomas_column<true>(sx + t, sm + t, sal + t, sg + t, L, kThomasPitch);
   __syncthreads();
   double* gxo = f.ac_x + (size_t)c0 * (L + 1);
   for (uint32_t idx = t; idx < nw; idx += kThomasThreads) {
@@ -628,54 +749,6 @@ __global__ void __launch_bounds__(kThomasThreads) k_ac_thomas_staged_mixed(mpasg
     gxo[idx] = sx[k * kThomasPitch + col];
   }
 }
-
-// Thomas factorisation (k_vimp_factor) with the columns staged the same way: a, b, c in
-// and alpha, gamma (and the mixed form's tri_m) out through a [level][33] layout with
-// coalesced copies by 4 warps; the division chain of each column runs on the first warp
-// from shared memory.  Same arithmetic as k_vimp_factor.
-template <typename T>
-__global__ void __launch_bounds__(kThomasThreads) k_vimp_factor_staged(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
-  extern __shared__ double s_col[];
-  const int L = m.nVertLevels;
-  double* sa = s_col;  // L x pitch each
-  double* sb = sa + (size_t)L * kThomasPitch;
-  double* sc = sb + (size_t)L * kThomasPitch;
-  double* sal = sc + (size_t)L * kThomasPitch;
-  double* sg = sal + (size_t)L * kThomasPitch;
-  const int c0 = blockIdx.x * kThomasCols;
-  const int ncol = min(kThomasCols, m.nCells - c0);
-  const int t = threadIdx.x;
-  const uint32_t nl = (uint32_t)ncol * L;
-  const size_t o0 = (size_t)c0 * L;
-  for (uint32_t idx = t; idx < nl; idx += kThomasThreads) {
-    uint32_t col = fl.div(idx), k = idx - col * L;
-    sa[k * kThomasPitch + col] = f.a_tri[o0 + idx];
-    sb[k * kThomasPitch + col] = f.b_tri[o0 + idx];
-    sc[k * kThomasPitch + col] = f.c_tri[o0 + idx];
-  }
-  __syncthreads();
-  if (t < ncol) {
-    double gam = 0.0;
-    sal[t] = 0.0;
-    sg[t] = 0.0;
-    for (int k = 1; k < L; ++k) {
-      const double alpha = recip<T>(sb[k * kThomasPitch + t] - sa[k * kThomasPitch + t] * gam);
-      gam = sc[k * kThomasPitch + t] * alpha;
-      sal[k * kThomasPitch + t] = alpha;
-      sg[k * kThomasPitch + t] = gam;
-    }
-  }
-  __syncthreads();
-  for (uint32_t idx = t; idx < nl; idx += kThomasThreads) {
-    uint32_t col = fl.div(idx), k = idx - col * L;
-    const double alpha = sal[k * kThomasPitch + col];
-    f.alpha_tri[o0 + idx] = alpha;
-    f.gamma_tri[o0 + idx] = sg[k * kThomasPitch + col];
-    if (sizeof(T) != sizeof(double) && k > 0) f.tri_m[o0 + idx] = -(alpha * sa[k * kThomasPitch + col]);
-  }
-}
-
-size_t vimp_factor_smem_bytes(int L) { return (size_t)5 * L * kThomasPitch * sizeof(double); }
 
 // tri_m = -alpha_tri * a_tri (the mixed forward-sweep factor) from the stored factors
 __global__ void k_tri_m(long long n, const double* __restrict__ a, const double* __restrict__ al,
@@ -726,8 +799,174 @@ __global__ void __launch_bounds__(kBlock) k_ac_post(mpasg_mesh m, mpasg_fields f
   if (k == (uint32_t)L) return;
   double xr1 = (threadIdx.x + 1 < blockDim.x) ? s_xr[threadIdx.x + 1]
                                               : ac_damped(m, f, o, ow, k + 1, L, f.ac_x[ow + k + 1], dts);
-  f.rho_pp[o + k] = f.ac_rs[o + k] - f.cofrz[k] * (xr1 - xr);
-  f.rtheta_pp[o + k] = f.ac_ts[o + k] - m.rdzw[k] * (f.coftz[ow + k + 1] * xr1 - f.coftz[ow + k] * xr);
+  ac_level_out(m, f, o + k, ow + k, k, f.ac_rs[o + k], f.ac_ts[o + k], xr, xr1);
+}
+
+// The float64 substep's columns in one launch: right-hand sides, solve and update of `cols`
+// columns a block, with what passes between them in shared memory in a [level][column]
+// layout (pitch odd: no bank conflicts).  The three kernels, which the forward mode still
+// runs apart, write and read five arrays of a level between them, wait for memory at each
+// start and leave the chip idle in the sweeps (one lane a column, ~190 clocks a level); here
+// the sweeps run beside other blocks' level work.  Step of 162 columns x 12 levels 744 -> 666
+// us, 2562 x 26 1443 -> 1353, 10242 x 33 4530 -> 4314, 40962 x 55 25.81 -> 25.49 ms; acoustic
+// stage at 40962 x 55 1505 -> 1440 us.  Bound by the float64 pipe on a large mesh, by the
+// chain of its phases on a small one.
+// keep: leave rs, ts and the undamped solution in ac_rs, ac_ts, ac_x (the reverse mode).
+template <int N, bool FIRST>
+__global__ void __launch_bounds__(kBlock, 5) k_ac_columns(mpasg_mesh m, mpasg_fields f, FastDiv fl, FastDiv fl1,
+                                                          int cols, bool keep, double dts, double ww_lo, double ww_hi,
+                                                          double resm) {
+  extern __shared__ fx::Weight s_w[];  // first: its alignment is the wider one
+  const uint32_t L = (uint32_t)m.nVertLevels, pitch = (uint32_t)cols | 1u, nlp = L * pitch;
+  double* sx = (double*)(s_w + cols * N);  // (L + 1) x pitch, the others L x pitch
+  double* sa = sx + nlp + pitch;
+  double* sal = sa + nlp;
+  double* sg = sal + nlp;
+  double* srs = sg + nlp;
+  double* sts = srs + nlp;
+  double* sR = FIRST ? srs : sts + nlp;  // R = rs, P = ts in the first substep
+  double* sP = FIRST ? sts : sR + nlp;
+  const uint32_t c0 = blockIdx.x * (uint32_t)cols, ncol = min((uint32_t)cols, (uint32_t)m.nCells - c0);
+  const uint32_t nl = ncol * L, nw = nl + ncol;
+  const size_t o0 = (size_t)c0 * L, ow0 = o0 + c0;
+  for (uint32_t t = threadIdx.x; t < ncol * N; t += kBlock) {
+    const uint32_t cl = t / N, j = t - cl * N, c = c0 + cl;
+    const size_t g = (size_t)c * m.maxEdges;
+    const int n = m.nEdgesOnCell[c];
+    s_w[t] = ((int)j < n && n <= N) ? fx::weight(m.cell_edge_geo[g + j], m.edgesOnCell[g + j])
+                                    : fx::Weight{0, 0, n > N ? fx::kBadWeight : 0u, n > 0 ? m.edgesOnCell[g] : 0};
+  }
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), q = (i - col * L) * pitch + col;
+    sa[q] = f.a_tri[o0 + i];
+    sal[q] = f.alpha_tri[o0 + i];
+    sg[q] = f.gamma_tri[o0 + i];
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    const AcLevel lv = ac_level<N, FIRST>(m, f, s_w + col * N, c0 + col, k, dts, resm);
+    srs[q] = lv.rs;
+    sts[q] = lv.ts;
+    if (!FIRST) {
+      sR[q] = lv.R;
+      sP[q] = lv.P;
+    }
+    if (keep) {
+      f.ac_rs[o0 + i] = lv.rs;
+      f.ac_ts[o0 + i] = lv.ts;
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nw; i += kBlock) {
+    const uint32_t col = fl1.div(i), k = i - col * (L + 1), q = k * pitch + col;
+    const double rwp = FIRST ? 0.0 : f.rw_p[ow0 + i];
+    sx[q] = (k == 0 || k == L) ? rwp  // boundary values pass through the solve unchanged
+                               : ac_rhs<FIRST>(m, f, o0 + col * L + k, ow0 + i, rwp, sR[q], sP[q], sR[q - pitch],
+                                               sP[q - pitch], dts);
+  }
+  __syncthreads();
+  if (threadIdx.x < ncol) {
+    const uint32_t t = threadIdx.x;
+    thomas_column(sx + t, sa + t, sal + t, sg + t, L, pitch);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nw; i += kBlock) {
+    const uint32_t col = fl1.div(i), k = i - col * (L + 1), q = k * pitch + col;
+    const double x = sx[q];
+    if (keep) f.ac_x[ow0 + i] = x;
+    const double xr = ac_damped(m, f, o0 + col * L, ow0 + col * (L + 1), k, L, x, dts);
+    sx[q] = xr;
+    if (k == 0 || k == L) {
+      if (FIRST) f.wwAvg[ow0 + i] = 0.0;
+    } else {
+      f.wwAvg[ow0 + i] = fma(ww_hi, xr, FIRST ? 0.0 : fma(ww_lo, f.rw_p[ow0 + i], f.wwAvg[ow0 + i]));
+    }
+    f.rw_p[ow0 + i] = xr;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    f.rtheta_pp_old[o0 + i] = FIRST ? 0.0 : f.rtheta_pp[o0 + i];
+    ac_level_out(m, f, o0 + i, ow0 + col * (L + 1) + k, k, srs[q], sts[q], sx[q], sx[q + pitch]);
+  }
+}
+
+size_t ac_columns_smem_bytes(int L, int cols, int N, bool first) {
+  return ((size_t)(first ? 6 : 8) * L + 1) * (cols | 1) * sizeof(double) + (size_t)cols * N * sizeof(fx::Weight);
+}
+
+// The mixed form's substep columns in one launch, as k_ac_columns; the float32 increments
+// and inputs of a level wait in shared memory as one 16-byte entry.
+__global__ void __launch_bounds__(kBlock, 5) k_ac_columns_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl, FastDiv fl1,
+                                                                int cols, bool keep, int small_step, double dts,
+                                                                float epssm, float resm) {
+  extern __shared__ AcLevelF s_lv[];  // L x pitch
+  const bool first = small_step == 1;
+  const float dtsf = (float)dts;
+  const uint32_t L = (uint32_t)m.nVertLevels, pitch = (uint32_t)cols | 1u, nlp = L * pitch;
+  double* sx = (double*)(s_lv + nlp);  // (L + 1) x pitch, the others L x pitch
+  double* sm = sx + nlp + pitch;
+  double* sal = sm + nlp;
+  double* sg = sal + nlp;
+  double* srs = sg + nlp;
+  double* sts = srs + nlp;
+  const uint32_t c0 = blockIdx.x * (uint32_t)cols, ncol = min((uint32_t)cols, (uint32_t)m.nCells - c0);
+  const uint32_t nl = ncol * L, nw = nl + ncol;
+  const size_t o0 = (size_t)c0 * L, ow0 = o0 + c0;
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    sm[q] = f.tri_m[o0 + i];
+    sal[q] = f.alpha_tri[o0 + i];
+    sg[q] = f.gamma_tri[o0 + i];
+    double rs, ts;
+    s_lv[q] = ac_level_mixed(m, f, c0 + col, k, first, dtsf, resm, &rs, &ts);
+    srs[q] = rs;
+    sts[q] = ts;
+    if (keep) {
+      f.ac_rs[o0 + i] = rs;
+      f.ac_ts[o0 + i] = ts;
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nw; i += kBlock) {
+    const uint32_t col = fl1.div(i), k = i - col * (L + 1), q = k * pitch + col;
+    const double rwp = first ? 0.0 : f.rw_p[ow0 + i];
+    sx[q] = (k == 0 || k == L) ? rwp  // boundary values pass through the solve unchanged
+                               : rwp + f64(ac_rhs_mixed(m, f, o0 + col * L, ow0 + col * (L + 1), k, s_lv[q],
+                                                        s_lv[q - pitch], dtsf, resm));
+  }
+  __syncthreads();
+  if (threadIdx.x < ncol) {
+    const uint32_t t = threadIdx.x;
+    thomas_column<true>(sx + t, sm + t, sal + t, sg + t, L, pitch);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nw; i += kBlock) {
+    const uint32_t col = fl1.div(i), k = i - col * (L + 1), q = k * pitch + col;
+    const double x = sx[q];
+    if (keep) f.ac_x[ow0 + i] = x;
+    const double xr = ac_damped_mixed(m, f, o0 + col * L, ow0 + col * (L + 1), k, L, x, dts);
+    sx[q] = xr;
+    if (k == 0 || k == L) {
+      if (first) f.wwAvg[ow0 + i] = 0.0;
+    } else {
+      const double ww = (first ? 0.0 : f.wwAvg[ow0 + i]) +
+                        f64(0.5f * (1.0f - epssm) * (first ? 0.0f : cv<float>(f.rw_p[ow0 + i])));
+      f.wwAvg[ow0 + i] = ww + f64(0.5f * (1.0f + epssm) * cv<float>(xr));
+    }
+    f.rw_p[ow0 + i] = xr;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
+    const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
+    f.rtheta_pp_old[o0 + i] = first ? 0.0 : f.rtheta_pp[o0 + i];
+    ac_level_out_mixed(m, f, o0 + i, ow0 + col * (L + 1) + k, k, srs[q], sts[q], sx[q], sx[q + pitch]);
+  }
+}
+
+size_t ac_columns_mixed_smem_bytes(int L, int cols) {
+  return (size_t)(cols | 1) * (L * sizeof(AcLevelF) + (size_t)(6 * L + 1) * sizeof(double));
 }
 
 // ---------------------------------------------------------------- divergence damping
@@ -1010,6 +1249,33 @@ int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv
 
 }  // namespace
 
+// The columns of a substep in one launch; *done is false where their arrays do not fit in
+// shared memory.
+static int launch_ac_columns(const mpasg_mesh* m, const mpasg_fields* f, bool mixed, int small_step, double dts,
+                             double epssm, double resm, bool keep, cudaStream_t s, bool* done) {
+  const int L = m->nVertLevels, N = m->maxEdges <= 6 ? 6 : 10;
+  const bool first = small_step == 1;
+  const int cols = columns_per_block(m->nCells, L + 1, 600), nb = nblocks(m->nCells, cols);
+  const size_t smem = mixed ? ac_columns_mixed_smem_bytes(L, cols) : ac_columns_smem_bytes(L, cols, N, first);
+  // the mixed form refuses the columns its staged solve cannot hold, on either path
+  *done = smem <= kMaxSmem && !(mixed && thomas_smem_bytes(L) > kMaxSmem);
+  if (!*done) return MPASG_OK;
+  const auto run = [&](auto kernel, auto... args) -> int {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess)
+      return MPASG_E_CUDA;
+    kernel<<<nb, kBlock, smem, s>>>(*m, *f, FastDiv(L), FastDiv(L + 1), cols, keep, args...);
+    MPASG_LAUNCH_CHECK();
+    return MPASG_OK;
+  };
+  if (mixed) return run(k_ac_columns_mixed, small_step, dts, (float)epssm, (float)resm);
+  const double ww_lo = 0.5 * (1.0 - epssm), ww_hi = 0.5 * (1.0 + epssm);
+  if (N == 6 && first) return run(k_ac_columns<6, true>, dts, ww_lo, ww_hi, resm);
+  if (N == 6) return run(k_ac_columns<6, false>, dts, ww_lo, ww_hi, resm);
+  if (first) return run(k_ac_columns<10, true>, dts, ww_lo, ww_hi, resm);
+  return run(k_ac_columns<10, false>, dts, ww_lo, ww_hi, resm);
+}
+
 static double damping_coefficient(const mpasg_config* c, double dts) {
   return 2.0 * c->smdiv * c->len_disp / dts;
 }
@@ -1034,31 +1300,31 @@ extern "C" int mpasg_vert_imp_coefs(const mpasg_mesh* m, const mpasg_config* c, 
   if (!m || !c || !f) return MPASG_E_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const int L = m->nVertLevels;
-  // the staged factorisation needs more than 48 KB of dynamic shared memory: opt in once
-  // per device (the first call on a device should come before any stream capture)
-  const size_t smem = vimp_factor_smem_bytes(L);
-  static bool smem_opt_in[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MPASG_E_CUDA;
-  if (!smem_opt_in[dev])
-    smem_opt_in[dev] = cudaFuncSetAttribute(k_vimp_factor_staged<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            200 * 1024) == cudaSuccess &&
-                       cudaFuncSetAttribute(k_vimp_factor_staged<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            200 * 1024) == cudaSuccess;
-  const bool staged = smem_opt_in[dev] && smem <= 200 * 1024;
-  const int nblk = nblocks(m->nCells, kThomasCols);
   const VimpScalars vs = vimp_scalars(dts, c->epssm);
-  if (c->precision == MPASG_PRECISION_MIXED) {
-    k_vimp_coefs<float><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), vs);
+  const FastDiv fl(L);
+  const int cols = columns_per_block(m->nCells, L, 400);
+  const size_t smem = vimp_columns_smem_bytes(L, cols);
+  const bool mixed = c->precision == MPASG_PRECISION_MIXED;
+  if (smem <= kMaxSmem) {
+    if (smem > 48 * 1024) {
+      const int b = (int)kMaxSmem;
+      const cudaError_t rc =
+          mixed ? cudaFuncSetAttribute(k_vimp_columns<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b)
+                : cudaFuncSetAttribute(k_vimp_columns<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+      if (rc != cudaSuccess) return MPASG_E_CUDA;
+    }
+    const int nb = nblocks(m->nCells, cols);
+    if (mixed) k_vimp_columns<float><<<nb, kBlock, smem, s>>>(*m, *f, fl, cols, vs);
+    else k_vimp_columns<double><<<nb, kBlock, smem, s>>>(*m, *f, fl, cols, vs);
     MPASG_LAUNCH_CHECK();
-    if (staged) k_vimp_factor_staged<float><<<nblk, kThomasThreads, smem, s>>>(*m, *f, FastDiv(L));
-    else k_vimp_factor<float><<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f);
-  } else {
-    k_vimp_coefs<double><<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), vs);
-    MPASG_LAUNCH_CHECK();
-    if (staged) k_vimp_factor_staged<double><<<nblk, kThomasThreads, smem, s>>>(*m, *f, FastDiv(L));
-    else k_vimp_factor<double><<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f);
+    return MPASG_OK;
   }
+  const int nb = nblocks((long long)m->nCells * L), nf = nblocks(m->nCells, 64);
+  if (mixed) k_vimp_coefs<float><<<nb, kBlock, 0, s>>>(*m, *f, fl, vs);
+  else k_vimp_coefs<double><<<nb, kBlock, 0, s>>>(*m, *f, fl, vs);
+  MPASG_LAUNCH_CHECK();
+  if (mixed) k_vimp_factor<float><<<nf, 64, 0, s>>>(*m, *f);
+  else k_vimp_factor<double><<<nf, 64, 0, s>>>(*m, *f);
   MPASG_LAUNCH_CHECK();
   return MPASG_OK;
 }
@@ -1125,6 +1391,11 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
       else
         k_acoustic_edges<double, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
       MPASG_LAUNCH_CHECK();
+    }
+    if (part == -1) {
+      bool done = false;
+      const int rc = launch_ac_columns(m, f, mixed, small_step, dts, c->epssm, resm, !fuse.scratch, s, &done);
+      if (rc != MPASG_OK || done) return rc;
     }
     if (mixed) {
       k_ac_prep_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), small_step, (float)dts,
