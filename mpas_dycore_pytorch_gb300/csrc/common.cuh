@@ -174,6 +174,7 @@ int mpasgi_pack_f32(const mpasg_mesh* m, mpasg_fields* f, cudaStream_t s);
 // stages alone):
 struct TendFusion {
   double first_dts = 0.0;     // > 0: the first acoustic substep's edge update with this dts
+  double* first_flux = nullptr;  // float64 form: where its ru_p theta goes (the acoustic ke_edge)
   bool smlstep = false;       // the small-step w tendency (flat terrain only)
   bool hdiv_current = false;  // h_divergence already holds ru's divergence (later RK stages)
   bool v_current = false;     // v is the TRiSK sum of u (left by the last RK stage's diagnostics)
@@ -200,6 +201,7 @@ struct AcousticFusion {
   bool edges_done = false;   // first substep: ru_p and ruAvg already formed (by the tendencies)
   bool damp_before = false;  // later substeps: the previous substep's divergence damping first
   bool scratch = false;      // ac_rs, ac_ts and ac_x need not be left behind
+  bool last = false;         // the stage's last substep: rho_p and rho_zz recovered with it
 };
 int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
                          cudaStream_t s, bool copies_current, const AcousticFusion& fuse = AcousticFusion());
@@ -207,9 +209,9 @@ int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_field
 int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
                           cudaStream_t s, int part, const AcousticFusion& fuse = AcousticFusion());
 // recovery with the last acoustic substep's divergence damping (step dts) before it and the
-// diagnostics' edge fields after it
+// diagnostics' edge fields after it; part 0: cells, 1: edges, 2: w over terrain (after both)
 int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
-                          double rk_dt, double dts, cudaStream_t s);
+                          double rk_dt, double dts, cudaStream_t s, int part);
 
 // Number of kernels this library has launched (for launch accounting by callers).
 extern "C" long long mpasg_launch_count(void);

@@ -8,6 +8,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "branches.cuh"
 
 namespace {
 
@@ -357,6 +358,11 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
     nsub[0] = nsub[1] = ns / 2 > 1 ? ns / 2 : 1; nsub[2] = ns;
   }
 
+  // the acoustic substeps' theta flux is formed while the tendencies still read ke_edge (pv u);
+  // delsq_u is free once tend_u is complete
+  mpasg_fields fa = f;
+  fa.ke_edge = f.delsq_u;
+
   // ---- RK integration setup
   MARK(MPASG_STAGE_BEGIN);
   // the time-level saves of a dynamics substep (theta_m's padding row is zeroed)
@@ -374,28 +380,34 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
     if (S > 0) job.push(ArrayJob::kCopy, f.scalars_init, f.scalars, ncs, advect && coupled ? f.scalars_a : nullptr);
     CHECK_RC(run_arrays(job, s));
   }
+  GraphBranches setup(s);
   if (c->precision == MPASG_PRECISION_MIXED) CHECK_RC(mpasgi_pack_f32(m, &f, s));
   else CHECK_RC(mpasgi_pvu(m, &f, s));
   // edge mean of theta_m_save and its reciprocal sum
   CHECK_RC(mpasgi_theta_edge(m, &f, c->precision == MPASG_PRECISION_MIXED, s));
   MARK(MPASG_STAGE_SETUP);
+  CHECK_RC(setup.next());
   CHECK_RC(mpasg_moist_coefficients(m, c, &f, stream));
+  CHECK_RC(setup.join());
   MARK(MPASG_STAGE_MOIST);
 
   for (int sub = 1; sub <= split; ++sub) {
     for (int rk = 1; rk <= 3; ++rk) {
       const double dts = rk_sub[rk - 1];
-      if (rk == 1 || (rk == 2 && c->time_integration_order == 3))
-      {
+      GraphBranches branches(s);  // the implicit coefficients beside the tendencies
+      if (rk == 1 || (rk == 2 && c->time_integration_order == 3)) {
         CHECK_RC(mpasg_vert_imp_coefs(m, c, &f, dts, stream));
         MARK(MPASG_STAGE_VIMP);
+        CHECK_RC(branches.next());
       }
       TendFusion tf;
       tf.first_dts = dts;
+      tf.first_flux = fa.ke_edge;
       tf.smlstep = m->flatTerrain != 0;
       tf.hdiv_current = rk > 1;
       tf.v_current = rk == 1 && sub > 1;  // the previous substep's last diagnostics
       CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true, tf));
+      CHECK_RC(branches.join());
       MARK(rk == 1 ? MPASG_STAGE_DYN_TEND_RK1 : MPASG_STAGE_DYN_TEND);
       if (!tf.smlstep) CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));
       MARK(MPASG_STAGE_SMLSTEP);
@@ -404,12 +416,25 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
         af.edges_done = small == 1;
         af.damp_before = small > 1;
         af.scratch = true;
-        CHECK_RC(mpasgi_acoustic_step(m, c, &f, small, dts, s, true, af));
+        af.last = small == nsub[rk - 1];
+        CHECK_RC(mpasgi_acoustic_step(m, c, &fa, small, dts, s, true, af));
         MARK(MPASG_STAGE_ACOUSTIC);
       }
       // with the last substep's divergence damping and the diagnostics' edge fields
-      CHECK_RC(mpasgi_recover_finish(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], dts, s));
+      auto recover = [&](int part) {
+        return mpasgi_recover_finish(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], dts, s, part);
+      };
+      // the cells' recovery beside the edges' and the diagnostics, which read only the edges;
+      // over terrain w needs both, and so does the coupled transport
+      GraphBranches cells(s);
+      CHECK_RC(recover(0));
+      CHECK_RC(cells.next());
+      CHECK_RC(recover(1));
+      if (!m->flatTerrain || (coupled && advect)) CHECK_RC(cells.join());
+      GraphBranches terrain(s);
+      CHECK_RC(recover(2));
       MARK(MPASG_STAGE_RECOVER);
+      if (!(coupled && advect)) CHECK_RC(terrain.next());
       if (coupled && advect) {  // time_integration.py:7890-8200: stage dt, this stage's mass fluxes
         CHECK_RC(transport_stage(m, c, &f, rk, rk_ts[rk - 1], s));
         MARK(rk == 3 && c->monotonic ? MPASG_STAGE_SCALARS_MONO : MPASG_STAGE_SCALARS);
@@ -424,6 +449,8 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
       df.edges_done = true;
       df.hdiv = rk < 3;  // the next stage's tendencies read it
       CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true, df));
+      CHECK_RC(terrain.join());
+      CHECK_RC(cells.join());
       MARK(MPASG_STAGE_DIAG);
     }
     // split bookkeeping: the substeps' mass fluxes summed, the saves of the next substep
@@ -446,10 +473,13 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
   // coupled mode: the scalars of the last RK stage are the step's (active rows only)
   if (advect && coupled) CHECK_RC(copy(f.scalars, f.scalars_a, nc * L * S, s));
   MARK(MPASG_STAGE_SPLIT);
+  GraphBranches last(s);  // the reconstructed wind beside the transport
   CHECK_RC(mpasgi_reconstruct(m, c, &f, s, true));
   MARK(MPASG_STAGE_RECONSTRUCT);
   if (part == 0) return MPASG_OK;
-  return step_tail(m, c, *fin, s, rec);
+  CHECK_RC(last.next());
+  CHECK_RC(step_tail(m, c, *fin, s, rec));
+  return last.join();
 }
 #undef MARK
 }  // namespace

@@ -407,11 +407,22 @@ MPASG_D double ac_rhs(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size
   return fma(f.cofwt[o - 1], P_lo, fma(f.cofwt[o], P, x));
 }
 
-// rho_pp and rtheta_pp from the solution above and below a level
-MPASG_D void ac_level_out(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k, double rs,
-                          double ts, double xr, double xr1) {
-  f.rho_pp[o] = fma(-f.cofrz[k], xr1 - xr, rs);
+// rho_pp and rtheta_pp from the solution above and below a level; returns rho_pp
+MPASG_D double ac_level_out(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k, double rs,
+                            double ts, double xr, double xr1) {
+  const double rho = fma(-f.cofrz[k], xr1 - xr, rs);
+  f.rho_pp[o] = rho;
   f.rtheta_pp[o] = fma(-m.rdzw[k], fma(f.coftz[ow + 1], xr1, -(f.coftz[ow] * xr)), ts);
+  return rho;
+}
+
+// rho_p and rho_zz after a stage's last substep; returns rho_zz
+MPASG_D double recover_rho(const mpasg_mesh& m, const mpasg_fields& f, size_t o, double rho_pp) {
+  const double rho_p = f.rho_p_save[o] + rho_pp;
+  const double rho_zz = rho_p + m.rho_base[o];
+  f.rho_p[o] = rho_p;
+  f.rho_zz[o] = rho_zz;
+  return rho_zz;
 }
 
 template <int N, bool FIRST>
@@ -633,12 +644,14 @@ MPASG_D double ac_damped_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_
   return fdiv<float>(num, 1.0 + dts * dss) - rw_delta;
 }
 
-// rho_pp and rtheta_pp from the solution above and below a level
-MPASG_D void ac_level_out_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k, double rs,
-                                double ts, double xr, double xr1) {
+// rho_pp and rtheta_pp from the solution above and below a level; returns rho_pp
+MPASG_D double ac_level_out_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k,
+                                  double rs, double ts, double xr, double xr1) {
   const float x0 = cv<float>(xr), x1 = cv<float>(xr1);
-  f.rho_pp[o] = rs - f64(cv<float>(f.cofrz[k]) * dif<float>(xr1, xr));
+  const double rho = rs - f64(cv<float>(f.cofrz[k]) * dif<float>(xr1, xr));
+  f.rho_pp[o] = rho;
   f.rtheta_pp[o] = ts - f64(m.rdzw_f32[k] * (cv<float>(f.coftz[ow + 1]) * x1 - cv<float>(f.coftz[ow]) * x0));
+  return rho;
 }
 
 __global__ void __launch_bounds__(kBlock) k_ac_post_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl1, double dts,
@@ -812,10 +825,11 @@ __global__ void __launch_bounds__(kBlock) k_ac_post(mpasg_mesh m, mpasg_fields f
 // stage at 40962 x 55 1505 -> 1440 us.  Bound by the float64 pipe on a large mesh, by the
 // chain of its phases on a small one.
 // keep: leave rs, ts and the undamped solution in ac_rs, ac_ts, ac_x (the reverse mode).
+// last: rho_p and rho_zz too, so that the recovery of u need not wait for that of the cells.
 template <int N, bool FIRST>
 __global__ void __launch_bounds__(kBlock, 5) k_ac_columns(mpasg_mesh m, mpasg_fields f, FastDiv fl, FastDiv fl1,
-                                                          int cols, bool keep, double dts, double ww_lo, double ww_hi,
-                                                          double resm) {
+                                                          int cols, bool keep, bool last, double dts, double ww_lo,
+                                                          double ww_hi, double resm) {
   extern __shared__ fx::Weight s_w[];  // first: its alignment is the wider one
   const uint32_t L = (uint32_t)m.nVertLevels, pitch = (uint32_t)cols | 1u, nlp = L * pitch;
   double* sx = (double*)(s_w + cols * N);  // (L + 1) x pitch, the others L x pitch
@@ -888,7 +902,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_ac_columns(mpasg_mesh m, mpasg_fi
   for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
     const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
     f.rtheta_pp_old[o0 + i] = FIRST ? 0.0 : f.rtheta_pp[o0 + i];
-    ac_level_out(m, f, o0 + i, ow0 + col * (L + 1) + k, k, srs[q], sts[q], sx[q], sx[q + pitch]);
+    const double rho = ac_level_out(m, f, o0 + i, ow0 + col * (L + 1) + k, k, srs[q], sts[q], sx[q], sx[q + pitch]);
+    if (last) recover_rho(m, f, o0 + i, rho);
   }
 }
 
@@ -899,8 +914,8 @@ size_t ac_columns_smem_bytes(int L, int cols, int N, bool first) {
 // The mixed form's substep columns in one launch, as k_ac_columns; the float32 increments
 // and inputs of a level wait in shared memory as one 16-byte entry.
 __global__ void __launch_bounds__(kBlock, 5) k_ac_columns_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl, FastDiv fl1,
-                                                                int cols, bool keep, int small_step, double dts,
-                                                                float epssm, float resm) {
+                                                                int cols, bool keep, bool last, int small_step,
+                                                                double dts, float epssm, float resm) {
   extern __shared__ AcLevelF s_lv[];  // L x pitch
   const bool first = small_step == 1;
   const float dtsf = (float)dts;
@@ -961,12 +976,19 @@ __global__ void __launch_bounds__(kBlock, 5) k_ac_columns_mixed(mpasg_mesh m, mp
   for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
     const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
     f.rtheta_pp_old[o0 + i] = first ? 0.0 : f.rtheta_pp[o0 + i];
-    ac_level_out_mixed(m, f, o0 + i, ow0 + col * (L + 1) + k, k, srs[q], sts[q], sx[q], sx[q + pitch]);
+    const double rho =
+        ac_level_out_mixed(m, f, o0 + i, ow0 + col * (L + 1) + k, k, srs[q], sts[q], sx[q], sx[q + pitch]);
+    if (last) recover_rho(m, f, o0 + i, rho);
   }
 }
 
 size_t ac_columns_mixed_smem_bytes(int L, int cols) {
   return (size_t)(cols | 1) * (L * sizeof(AcLevelF) + (size_t)(6 * L + 1) * sizeof(double));
+}
+
+__global__ void k_recover_rho(mpasg_mesh m, mpasg_fields f, uint32_t n) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) recover_rho(m, f, i, f.rho_pp[i]);
 }
 
 // ---------------------------------------------------------------- divergence damping
@@ -1059,7 +1081,7 @@ MPASG_D double pow1p_rcv_m1(double x) {
 // thread (shared memory) -- the same expressions k_recover_w evaluates, one launch fewer.
 template <typename T, bool FLAT = false>
 __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl1, int rk_step,
-                                                          double inv_ns, double rk_dt) {
+                                                          double inv_ns, double rk_dt, bool rho_done) {
   __shared__ double s_rho[FLAT ? kBlock : 1];
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1072,21 +1094,20 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
   }
   const size_t o = (size_t)c * L + k;
   if (FLAT) {
-    s_rho[threadIdx.x] = (active && k < (uint32_t)L) ? f.rho_p_save[o] + f.rho_pp[o] + m.rho_base[o] : 0.0;
+    double rho = 0.0;
+    if (active && k < (uint32_t)L) rho = rho_done ? f.rho_zz[o] : f.rho_p_save[o] + f.rho_pp[o] + m.rho_base[o];
+    s_rho[threadIdx.x] = rho;
     __syncthreads();
     if (!active) return;
   }
   if (k < (uint32_t)L) {
-    double rho_p = f.rho_p_save[o] + f.rho_pp[o];
-    double rho_zz = rho_p + m.rho_base[o];
+    const double rho_zz = rho_done ? f.rho_zz[o] : recover_rho(m, f, o, f.rho_pp[o]);
     double rtheta_p;
     if (rk_step == 3)
       rtheta_p = f.rtheta_p_save[o] + f.rtheta_pp[o] - rk_dt * rho_zz * f.rt_diabatic_tend[o];
     else
       rtheta_p = f.rtheta_p_save[o] + f.rtheta_pp[o];
     double rtb = f.rtheta_base[o];
-    f.rho_p[o] = rho_p;
-    f.rho_zz[o] = rho_zz;
     f.rtheta_p[o] = rtheta_p;
     f.theta_m[o] = sizeof(T) == sizeof(double) ? fx::quotient(rtheta_p + rtb, rho_zz) : (rtheta_p + rtb) * rcp_nr1(rho_zz);
     if (rk_step == 3) {
@@ -1127,6 +1148,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
     } else {
       const double rho_k = s_rho[threadIdx.x];
       const double rho_km1 = threadIdx.x >= 1 ? s_rho[threadIdx.x - 1]
+                             : rho_done       ? f.rho_zz[oc + k - 1]
                                               : f.rho_p_save[oc + k - 1] + f.rho_pp[oc + k - 1] + m.rho_base[oc + k - 1];
       const double wk = fdiv<T>(wo, m.fzm[k] * rho_k + m.fzp[k] * rho_km1);
       f.w[ow] = wk;
@@ -1225,25 +1247,24 @@ __global__ void k_recover_w(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   if (kMixed) f.w_f32[i] = d2f_bits(wk);
 }
 
+// part 0: cells, 1: edges, 2: w over terrain
 template <typename T>
 int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv_ns, double rk_dt, cudaStream_t s,
-                   bool finish, double damp_coef, bool one_substep) {
+                   bool finish, double damp_coef, bool one_substep, int part) {
   const int L = m->nVertLevels;
-  const long long ncw = (long long)m->nCells * (L + 1);
-  if (m->flatTerrain)
-    k_recover_cells<T, true><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), rk_step, inv_ns, rk_dt);
-  else
-    k_recover_cells<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), rk_step, inv_ns, rk_dt);
-  MPASG_LAUNCH_CHECK();
-  const int ne = nblocks((long long)m->nEdges * L);
-  if (finish && one_substep) k_recover_edges<T, true, true><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, damp_coef);
-  else if (finish) k_recover_edges<T, true, false><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, damp_coef);
-  else k_recover_edges<T, false, false><<<ne, kBlock, 0, s>>>(*m, *f, FastDiv(L), inv_ns, 0.0);
-  MPASG_LAUNCH_CHECK();
-  if (!m->flatTerrain) {  // slope fluxes need the new ru of k_recover_edges
-    k_recover_w<T><<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1));
-    MPASG_LAUNCH_CHECK();
+  const int nw = nblocks((long long)m->nCells * (L + 1)), ne = nblocks((long long)m->nEdges * L);
+  const FastDiv fl(L), fl1(L + 1);
+  if (part == 0) {
+    if (m->flatTerrain) k_recover_cells<T, true><<<nw, kBlock, 0, s>>>(*m, *f, fl1, rk_step, inv_ns, rk_dt, finish);
+    else k_recover_cells<T><<<nw, kBlock, 0, s>>>(*m, *f, fl1, rk_step, inv_ns, rk_dt, finish);
+  } else if (part == 1) {
+    if (finish && one_substep) k_recover_edges<T, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef);
+    else if (finish) k_recover_edges<T, true, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef);
+    else k_recover_edges<T, false, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, 0.0);
+  } else if (!m->flatTerrain) {  // slope fluxes need the new ru of k_recover_edges
+    k_recover_w<T><<<nw, kBlock, 0, s>>>(*m, *f, fl1);
   }
+  MPASG_LAUNCH_CHECK();
   return MPASG_OK;
 }
 
@@ -1252,7 +1273,7 @@ int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv
 // The columns of a substep in one launch; *done is false where their arrays do not fit in
 // shared memory.
 static int launch_ac_columns(const mpasg_mesh* m, const mpasg_fields* f, bool mixed, int small_step, double dts,
-                             double epssm, double resm, bool keep, cudaStream_t s, bool* done) {
+                             double epssm, double resm, bool keep, bool last, cudaStream_t s, bool* done) {
   const int L = m->nVertLevels, N = m->maxEdges <= 6 ? 6 : 10;
   const bool first = small_step == 1;
   const int cols = columns_per_block(m->nCells, L + 1, 600), nb = nblocks(m->nCells, cols);
@@ -1264,7 +1285,7 @@ static int launch_ac_columns(const mpasg_mesh* m, const mpasg_fields* f, bool mi
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess)
       return MPASG_E_CUDA;
-    kernel<<<nb, kBlock, smem, s>>>(*m, *f, FastDiv(L), FastDiv(L + 1), cols, keep, args...);
+    kernel<<<nb, kBlock, smem, s>>>(*m, *f, FastDiv(L), FastDiv(L + 1), cols, keep, last, args...);
     MPASG_LAUNCH_CHECK();
     return MPASG_OK;
   };
@@ -1394,7 +1415,7 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
     }
     if (part == -1) {
       bool done = false;
-      const int rc = launch_ac_columns(m, f, mixed, small_step, dts, c->epssm, resm, !fuse.scratch, s, &done);
+      const int rc = launch_ac_columns(m, f, mixed, small_step, dts, c->epssm, resm, !fuse.scratch, fuse.last, s, &done);
       if (rc != MPASG_OK || done) return rc;
     }
     if (mixed) {
@@ -1435,6 +1456,10 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
   else
     k_ac_post<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, 0.5 * (1.0 + c->epssm));
   MPASG_LAUNCH_CHECK();
+  if (fuse.last) {
+    k_recover_rho<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, (uint32_t)m->nCells * L);
+    MPASG_LAUNCH_CHECK();
+  }
   return MPASG_OK;
 }
 
@@ -1479,21 +1504,24 @@ extern "C" int mpasg_smlstep_pert(const mpasg_mesh* m, const mpasg_config* c, mp
 
 namespace {
 int recover(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns, double rk_dt,
-            cudaStream_t s, bool finish, double damp_coef) {
+            cudaStream_t s, bool finish, double damp_coef, int part) {
   if (!m || !c || !f || ns < 1) return MPASG_E_ARG;
   const double inv_ns = 1.0 / (double)ns;
   if (c->precision == MPASG_PRECISION_MIXED)
-    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1);
-  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1);
+    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1, part);
+  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1, part);
 }
 }  // namespace
 
 extern "C" int mpasg_recover_large_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
                                         int rk_step, int ns, double rk_dt, void* stream) {
-  return recover(m, c, f, rk_step, ns, rk_dt, (cudaStream_t)stream, false, 0.0);
+  int rc = MPASG_OK;
+  for (int part = 0; part < 3 && rc == MPASG_OK; ++part)
+    rc = recover(m, c, f, rk_step, ns, rk_dt, (cudaStream_t)stream, false, 0.0, part);
+  return rc;
 }
 
 int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
-                          double rk_dt, double dts, cudaStream_t s) {
-  return recover(m, c, f, rk_step, ns, rk_dt, s, true, c ? damping_coefficient(c, dts) : 0.0);
+                          double rk_dt, double dts, cudaStream_t s, int part) {
+  return recover(m, c, f, rk_step, ns, rk_dt, s, true, c ? damping_coefficient(c, dts) : 0.0, part);
 }

@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "advstencil.cuh"
+#include "branches.cuh"
 #include "cellsum.cuh"
 #include "trisk.cuh"
 
@@ -33,7 +34,8 @@ struct TendScalars {
   int ray_n;  // Rayleigh-damped top levels of u (0: off)
   int mix_pert;  // vertical mixing of the perturbation from the initial profiles
   double f3[4];  // flux3 with coef3 by upwind side: 7 + 3 c, 7 - 3 c, 1 + c, 1 - c
-  double first_dts;  // > 0: k_adv_edges also starts the acoustic substeps (TendFusion)
+  double first_dts;    // > 0: the kernel that completes tend_u also starts the acoustic substeps
+  double* first_flux;  // ru_p theta of their first edge update (TendFusion)
   int smlstep;       // k_tend_w_theta also forms tend_rw
   int v_current;     // v already holds the TRiSK sum of u
   int defer;  // k_tend_u leaves tend_u_euler to k_tend_u_finish (del4 and / or vertical mixing)
@@ -44,6 +46,19 @@ struct TendScalars {
 MPASG_D double cam_kdiff(double kd, const TendScalars& p, uint32_t k, int L) {
   const double factor = 1.0 - (double)(L - (int)(k + 1)) / (double)p.ncam;
   return fmax(kd, p.cam_base * factor);
+}
+
+// tend_u is complete: stored, and the first acoustic substep's edge update made from it
+// (k_acoustic_edges with small_step 1)
+template <typename T>
+MPASG_D void complete_tend_u(const mpasg_fields& f, size_t i, T tu, const TendScalars& p) {
+  f.tend_u[i] = f64(tu);
+  if (p.first_dts > 0.0) {
+    const double rup = f64(cv<T>(p.first_dts) * tu);
+    f.ru_p[i] = rup;
+    f.ruAvg[i] = rup;
+    if (sizeof(T) == sizeof(double)) p.first_flux[i] = rup * f.theta_edge_save[i];
+  }
 }
 
 template <typename T, bool CAM = false>
@@ -194,9 +209,10 @@ __global__ void __launch_bounds__(kBlock) k_tend_u(mpasg_mesh m, mpasg_fields f,
     T kdiffu = T(0.5) * (cv<T>(f.kdiff[i1]) + cv<T>(f.kdiff[i2]));
     teu = teu + rho_e * kdiffu * u_diff * G(meshScalingDel2)[e];
     f.tend_u_euler[i] = f64(teu);
-    f.tend_u[i] = f64(p.defer ? tu : tu + teu);
+    if (p.defer) f.tend_u[i] = f64(tu);
+    else complete_tend_u(f, i, tu + teu, p);
   } else {
-    f.tend_u[i] = f64(tu + cv<T>(f.tend_u_euler[i]));
+    complete_tend_u(f, i, tu + cv<T>(f.tend_u_euler[i]), p);
   }
 }
 
@@ -279,9 +295,10 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
       T kdiffu = T(0.5) * (cv<T>(f.kdiff[i1]) + cv<T>(f.kdiff[i2]));
       teu = teu + rho_e * kdiffu * u_diff * G(meshScalingDel2)[e];
       f.tend_u_euler[ie] = f64(teu);
-      f.tend_u[ie] = f64(p.defer ? tu : tu + teu);
+      if (p.defer) f.tend_u[ie] = f64(tu);
+      else complete_tend_u(f, ie, tu + teu, p);
     } else {
-      f.tend_u[ie] = f64(tu + cv<T>(f.tend_u_euler[ie]));
+      complete_tend_u(f, ie, tu + cv<T>(f.tend_u_euler[ie]), p);
     }
   }
 }
@@ -384,9 +401,10 @@ __global__ void __launch_bounds__(kBlock, 5) k_tend_u_fx(mpasg_mesh m, mpasg_fie
     const double mix = (rho_e * (f.kdiff[i1] + f.kdiff[i2])) * (u_diff * ec.half_ms2);
     const double teu = fma(-f.cqu_e[i], grad, mix);
     f.tend_u_euler[i] = teu;
-    f.tend_u[i] = p.defer ? tu : tu + teu;
+    if (p.defer) f.tend_u[i] = tu;
+    else complete_tend_u(f, i, tu + teu, p);
   } else {
-    f.tend_u[i] = tu + f.tend_u_euler[i];
+    complete_tend_u(f, i, tu + f.tend_u_euler[i], p);
   }
 }
 
@@ -481,7 +499,7 @@ __global__ void k_tend_u_finish(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendSc
     teu = teu + cv<T>(f.h_edge[i]) * cv<T>(p.v_mom) * (d_up - d_dn) / cv<T>(0.5 * (zp - zm));
   }
   f.tend_u_euler[i] = f64(teu);
-  f.tend_u[i] = f64(cv<T>(f.tend_u[i]) + teu);
+  complete_tend_u(f, i, cv<T>(f.tend_u[i]) + teu, p);
 }
 
 // vertical mixing of w at interface k, 1 <= k <= L-1 (dyn_tend.py:4636-4648, rk 1)
@@ -760,17 +778,8 @@ MPASG_D T wdtz_at(const T* th, const T* ths, const T* rw_t, const double* rw, co
 // the reference's per-slot (sign * ru) * flux products bit for bit.  The mixed form
 // advects the deviation theta_m - ref_theta (its reference part is added in float64 by
 // k_tend_w_theta_mixed) and stores float32 fluxes.
-// first acoustic substep's edge update (k_acoustic_edges with small_step 1)
 template <typename T>
-MPASG_D void first_acoustic_edge(const mpasg_fields& f, uint32_t i, double dts) {
-  const double rup = f64(cv<T>(dts) * cv<T>(f.tend_u[i]));
-  f.ru_p[i] = rup;
-  f.ruAvg[i] = rup;
-  if (sizeof(T) == sizeof(double)) f.ke_edge[i] = rup * f.theta_edge_save[i];
-}
-
-template <typename T>
-__global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double first_dts) {
+__global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
@@ -781,7 +790,6 @@ __global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double fir
   const T* cfp = G(adv_coefs_p) + (size_t)e * na;
   const T* cfm = G(adv_coefs_m) + (size_t)e * na;
   const T rue = cv<T>(f.ru[i]);
-  if (first_dts > 0.0) first_acoustic_edge<T>(f, i, first_dts);
   {
     const T* th = fp<T>(f.theta_m, f.theta_dev);
     const T* cf = rue >= T(0) ? cfp : cfm;
@@ -810,8 +818,7 @@ __global__ void k_adv_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double fir
 // at 82 % of that pipe).  40962 x 55: 374 us in float64 alone, 271 us with both sums
 // on the integer side, 216 us with one each.
 template <int N, bool PERT>
-__global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl,
-                                                         double first_dts) {
+__global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   extern __shared__ fx::Weight s_w[];
   const uint32_t L = (uint32_t)m.nVertLevels;
   const uint32_t n_all = (uint32_t)m.nEdges * L;
@@ -821,7 +828,6 @@ __global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_
   __syncthreads();
   if (i >= n_all) return;
   const uint32_t e = fl.div(i), k = i - e * L;
-  if (first_dts > 0.0) first_acoustic_edge<double>(f, i, first_dts);
   const double rue = f.ru[i];
   const bool back = __double2hiint(rue) < 0;
   const fx::Weight* w = s_w + (e - e0) * (2 * N) + (back ? N : 0);
@@ -1103,10 +1109,6 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
   const long long ncl = (long long)m->nCells * L, nel = (long long)m->nEdges * L;
   const long long ncw = (long long)m->nCells * (L + 1), nvl = (long long)m->nVertices * L;
   FastDiv fl(L), fl1(L + 1);
-  if (sizeof(T) != sizeof(double)) {
-    k_theta_dev<<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl);
-    MPASG_LAUNCH_CHECK();
-  }
   if (rk_step == 1 || !hdiv_current) {
     if (p.ncam > 0 && rk_step == 1)
       k_tend_cells_a<T, true><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
@@ -1114,6 +1116,7 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
       k_tend_cells_a<T><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
     MPASG_LAUNCH_CHECK();
   }
+  GraphBranches branches(s);  // u beside w and theta
   const bool ray = p.ray_n > 0;
   if constexpr (sizeof(T) == sizeof(double)) {
     if (ray) launch_tend_u_fx<true>(m, f, p, s);
@@ -1145,6 +1148,13 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
       k_tend_u_finish<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
       MPASG_LAUNCH_CHECK();
     }
+  }
+  if (const int rc = branches.next(); rc != MPASG_OK) return rc;
+  if (sizeof(T) != sizeof(double)) {
+    k_theta_dev<<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl);
+    MPASG_LAUNCH_CHECK();
+  }
+  if (rk_step == 1) {
     if constexpr (sizeof(T) == sizeof(double)) {
       const int rc = launch_mix_fx(m, f, p, s);
       if (rc != MPASG_OK) return rc;
@@ -1163,12 +1173,12 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
     const size_t smem = (size_t)((kBlock - 1) / L + 2) * adv::kEntryBytes;
     const int nb = nblocks(nel);
     const bool narrow = m->nAdvMax <= 10, pert = rk_step > 1;
-    if (narrow && pert) k_adv_edges_fx<10, true><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl, p.first_dts);
-    else if (narrow) k_adv_edges_fx<10, false><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl, p.first_dts);
-    else if (pert) k_adv_edges_fx<14, true><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl, p.first_dts);
-    else k_adv_edges_fx<14, false><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl, p.first_dts);
+    if (narrow && pert) k_adv_edges_fx<10, true><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl);
+    else if (narrow) k_adv_edges_fx<10, false><<<nb, kBlock, smem * 10, s>>>(*m, *f, fl);
+    else if (pert) k_adv_edges_fx<14, true><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl);
+    else k_adv_edges_fx<14, false><<<nb, kBlock, smem * 14, s>>>(*m, *f, fl);
   } else {
-    k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p.first_dts);
+    k_adv_edges<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl);
   }
   MPASG_LAUNCH_CHECK();
   if (sizeof(T) == sizeof(double)) {
@@ -1178,7 +1188,7 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
   } else
     k_tend_w_theta_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, fl1, p);
   MPASG_LAUNCH_CHECK();
-  return MPASG_OK;
+  return branches.join();
 }
 
 }  // namespace
@@ -1234,6 +1244,7 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
   p.f3[3] = 1.0 - p.coef3;
   p.rk_step = rk_step;
   p.first_dts = fuse.first_dts;
+  p.first_flux = fuse.first_flux;
   p.smlstep = fuse.smlstep ? 1 : 0;
   p.v_current = fuse.v_current ? 1 : 0;
   p.del4 = (p.h_mom_visc4 > 0.0) ? 1 : 0;
