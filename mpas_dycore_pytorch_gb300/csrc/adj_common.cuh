@@ -92,15 +92,15 @@ MPASG_D int vertex_side(const mpasg_mesh& m, int e, int v) { return m.verticesOn
 struct Flux3Grad {
   double qm2, qm1, q0, qp1, ua;
 };
-MPASG_D Flux3Grad flux3_grad(double qm2, double qm1, double q0, double qp1, double ua, double c3) {
-  const double au = fabs(ua);
-  const double s = ua > 0.0 ? 1.0 : (ua < 0.0 ? -1.0 : 0.0);
+// (times b; the upwind sign on the integer side, zero at ua = 0)
+MPASG_D Flux3Grad flux3_grad(double qm2, double qm1, double q0, double qp1, double ua, double c3, double b = 1.0) {
+  const double r = b * (ua * kInv12), cs = fx::is_zero(ua) ? 0.0 : flip_by(c3, ua), t = cs * r, r7 = 7.0 * r;
   Flux3Grad d;
-  d.qm2 = (-ua - c3 * au) * kInv12;
-  d.qm1 = (7.0 * ua + 3.0 * c3 * au) * kInv12;
-  d.q0 = (7.0 * ua - 3.0 * c3 * au) * kInv12;
-  d.qp1 = (-ua + c3 * au) * kInv12;
-  d.ua = ((7.0 * (q0 + qm1) - (qp1 + qm2)) + c3 * s * ((qp1 - qm2) - 3.0 * (q0 - qm1))) * kInv12;
+  d.qm2 = -r - t;
+  d.qm1 = fma(3.0, t, r7);
+  d.q0 = fma(-3.0, t, r7);
+  d.qp1 = t - r;
+  d.ua = (b * kInv12) * fma(cs, fma(-3.0, q0 - qm1, qp1 - qm2), fma(7.0, q0 + qm1, -(qp1 + qm2)));
   return d;
 }
 

@@ -209,7 +209,8 @@ int mpasgi_acoustic_step(const mpasg_mesh* m, const mpasg_config* c, mpasg_field
 int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int small_step, double dts,
                           cudaStream_t s, int part, const AcousticFusion& fuse = AcousticFusion());
 // recovery with the last acoustic substep's divergence damping (step dts) before it and the
-// diagnostics' edge fields after it; part 0: cells, 1: edges, 2: w over terrain (after both)
+// diagnostics' edge fields after it; part 0: cells, 1: edges, 2: w over terrain (after both);
+// rho_p and rho_zz before them, by the last substep (AcousticFusion::last) or as part 3
 int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
                           double rk_dt, double dts, cudaStream_t s, int part);
 

@@ -13,6 +13,7 @@
 #include <cmath>
 
 #include "adj_common.cuh"
+#include "branches.cuh"
 
 namespace {
 
@@ -256,10 +257,13 @@ int aco_store(const mpasg_mesh* m, const Tape& T, const mpasg_fields& f, int a, 
   const long long L = m->nVertLevels;
   const long long nel = (m->nEdges + 1LL) * L, ncw = (m->nCells + 1LL) * (L + 1), ncl = (m->nCells + 1LL) * L;
   double* b = T.aco(a);
+  GraphBranches copies(s);
   CHECK_RC(dcopy(b, f.ru_p, nel, s));
+  CHECK_RC(copies.next());
   CHECK_RC(dcopy(b + T.E + T.W, f.rw_p, ncw, s));
+  CHECK_RC(copies.next());
   CHECK_RC(dcopy(b + T.E + 2 * T.W + T.C, f.rtheta_pp, ncl, s));
-  return MPASG_OK;
+  return copies.join();
 }
 
 // a view whose acoustic fields are substep a's taped outputs
@@ -313,13 +317,18 @@ __global__ void k_theta_edge_vjp(mpasg_mesh m, mpasg_fields g, FastDiv fl) {
 int fold_saves(const mpasg_mesh* m, mpasg_fields* g, cudaStream_t s) {
   const long long L = m->nVertLevels;
   const long long nel = (m->nEdges + 1LL) * L, ncw = (m->nCells + 1LL) * (L + 1), ncl = (m->nCells + 1LL) * L;
+  GraphBranches folds(s);
   CHECK_RC(fold(g->ru, g->ru_save, nel, s));
+  CHECK_RC(folds.next());
   CHECK_RC(fold(g->rw, g->rw_save, ncw, s));
+  CHECK_RC(folds.next());
   CHECK_RC(fold(g->rtheta_p, g->rtheta_p_save, ncl, s));
+  CHECK_RC(folds.next());
   CHECK_RC(fold(g->rho_p, g->rho_p_save, ncl, s));
   CHECK_RC(fold(g->rho_p, g->rr_save, ncl, s));
+  CHECK_RC(folds.next());
   CHECK_RC(fold(g->theta_m, g->theta_m_save, ncl, s));
-  return MPASG_OK;
+  return folds.join();
 }
 
 // refresh the saves of the coming dynamics substep (writes go to the tape's save block);
@@ -330,13 +339,20 @@ int make_saves(const mpasg_mesh* m, const Tape& T, mpasg_fields& f, int sub, boo
   k_fill_row<<<1, 128, 0, s>>>(f.theta_m + nc * L, (int)L, 0.0);
   MPASG_LAUNCH_CHECK();
   if (T.in(sub + 1)) sv_view(T, f, sub);
+  GraphBranches copies(s);
   CHECK_RC(dcopy(f.ru_save, f.ru, nel, s));
+  CHECK_RC(copies.next());
   CHECK_RC(dcopy(f.rw_save, f.rw, ncw, s));
+  CHECK_RC(copies.next());
   CHECK_RC(dcopy(f.rtheta_p_save, f.rtheta_p, ncl, s));
+  CHECK_RC(copies.next());
   CHECK_RC(dcopy(f.rho_p_save, f.rho_p, ncl, s));
-  CHECK_RC(dcopy(f.theta_m_save, f.theta_m, ncl, s));
+  CHECK_RC(copies.next());
   CHECK_RC(dcopy(f.rr_save, f.rho_p, ncl, s));
-  return mpasgi_theta_edge(m, &f, mixed, s);
+  CHECK_RC(copies.next());
+  CHECK_RC(dcopy(f.theta_m_save, f.theta_m, ncl, s));
+  CHECK_RC(mpasgi_theta_edge(m, &f, mixed, s));
+  return copies.join();
 }
 
 int coef_slot(const StepPlan& p, int sub, int rk) {  // sub 1-based
@@ -370,30 +386,54 @@ int forward_taped(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields f, co
     for (int rk = 1; rk <= 3; ++rk) {
       const int i = (sub - 1) * 3 + rk - 1;
       const double dts = p.rk_sub[rk - 1];
+      GraphBranches branches(s);  // the step's branches and fused passes (step_impl)
       if (rk == 1 || (rk == 2 && p.order == 3)) {
         if (taped) coef_view(T, f, coef_slot(p, sub, rk));
         CHECK_RC(mpasg_vert_imp_coefs(m, c, &f, dts, stream));
+        CHECK_RC(branches.next());
       }
-      TendFusion tf;  // h_divergence from the previous stage's diagnostics, as in the step
+      TendFusion tf;  // h_divergence and v from the previous stage's diagnostics, as in the step
+      tf.first_dts = dts;
+      tf.first_flux = f.delsq_u;
       tf.hdiv_current = rk > 1;
+      tf.v_current = rk == 1 && sub > 1;
       CHECK_RC(mpasgi_dyn_tend(m, c, &f, rk, s, true, tf));
       if (taped && T.n_sg > 0) CHECK_RC(mpasgi_nonneg_bytes(f.tend_u, T.sg(i), (m->nEdges + 1LL) * m->nVertLevels, s));
       CHECK_RC(mpasg_smlstep_pert(m, c, &f, stream));
+      CHECK_RC(branches.join());
       for (int small = 1; small <= p.nsub[rk - 1]; ++small) {
         if (taped) aco_redirect(T, f, a);
-        CHECK_RC(mpasgi_acoustic_step(m, c, &f, small, dts, s, true));
+        mpasg_fields fa = f;
+        fa.ke_edge = f.delsq_u;
+        AcousticFusion af;
+        af.edges_done = small == 1;
+        CHECK_RC(mpasgi_acoustic_step(m, c, &fa, small, dts, s, true, af));
         if (taped) CHECK_RC(aco_store(m, T, f, a, s));
         ++a;
-        CHECK_RC(mpasgi_divergence_damping(m, c, &f, dts, s, true));
+        if (small < p.nsub[rk - 1]) CHECK_RC(mpasgi_divergence_damping(m, c, &f, dts, s, true));
       }
       if (taped) {
         CHECK_RC(carry_block(m, T, T.snap(i), T.snap(i + 1), rk, s));
         snap_view(T, f, T.snap(i + 1));
       }
-      CHECK_RC(mpasg_recover_large_step(m, c, &f, rk, p.nsub[rk - 1], p.rk_ts[rk - 1], stream));
+      auto recover = [&](int part) {
+        return mpasgi_recover_finish(m, c, &f, rk, p.nsub[rk - 1], p.rk_ts[rk - 1], dts, s, part);
+      };
+      CHECK_RC(recover(3));
+      GraphBranches cells(s);
+      CHECK_RC(recover(0));
+      CHECK_RC(cells.next());
+      CHECK_RC(recover(1));
+      if (!m->flatTerrain) CHECK_RC(cells.join());
+      GraphBranches terrain(s);
+      CHECK_RC(recover(2));
+      CHECK_RC(terrain.next());
       DiagFusion df;
+      df.edges_done = true;
       df.hdiv = rk < 3;
       CHECK_RC(mpasgi_solve_diagnostics(m, c, &f, rk, s, true, df));
+      CHECK_RC(terrain.join());
+      CHECK_RC(cells.join());
     }
     if (sub < p.split && sub < T.hi) CHECK_RC(make_saves(m, T, f, sub, mixed, s));
   }
@@ -464,11 +504,14 @@ int step_reverse(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields*
         CHECK_RC(mpasgi_acoustic_vjp_rev(m, c, &ac, g, t, small, dts, prev + T.E + 2 * T.W + T.C, prev + T.E + T.W,
                                          w, s));
       }
+      // every RK stage starts its acoustic perturbations from zero
+      GraphBranches zero(s);
+      CHECK_RC(zero_work_cotangents(m, g, s));
+      CHECK_RC(zero.next());
       CHECK_RC(mpasgi_smlstep_vjp_core(m, nullptr, T.n_sg > 0 ? T.sg(i) : nullptr, g, s));
       CHECK_RC(mpasgi_dyn_tend_vjp_core(m, c, &pre, g, t, rk, w, s));
       if (rk == 1 || (rk == 2 && p.order == 3)) CHECK_RC(mpasgi_vimp_vjp_core(m, c, &pre, g, dts, w, s));
-      // every RK stage starts its acoustic perturbations from zero
-      CHECK_RC(zero_work_cotangents(m, g, s));
+      CHECK_RC(zero.join());
     }
     // the edge-sum cotangent of this substep's theta_m_save, gathered on the cells
     k_theta_edge_vjp<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *g, FastDiv(L));

@@ -8,6 +8,7 @@
 // deterministic sum.  Cotangents live in `g` under the forward field names; work holds the
 // per-edge partial products a later cell gather reads.
 #include "adj_common.cuh"
+#include "columns.cuh"
 
 namespace {
 
@@ -45,18 +46,15 @@ __global__ void k_vimp_factor_vjp(mpasg_mesh m, mpasg_fields f, mpasg_fields g, 
   gc[o] = 0.0;
 }
 
-// The same with 32 columns staged through shared memory ([level][33] layout, coalesced
-// copies by 4 warps, the sweeps on the first warp), as the forward factorisation does.
-constexpr int kFacCols = 32;
-constexpr int kFacPitch = kFacCols + 1;
-constexpr int kFacThreads = 128;
-
-__global__ void __launch_bounds__(kFacThreads) k_vimp_factor_vjp_staged(mpasg_mesh m, mpasg_fields f, mpasg_fields g,
-                                                                        FastDiv fl, double* __restrict__ gb,
-                                                                        double* __restrict__ gc) {
+// The same with `cols` columns staged through shared memory ([level][column] layout, odd pitch,
+// coalesced copies, the sweeps on the first warp), as the forward factorisation does.
+// 2562 x 26: 20 us with 32 columns a block, 11 with 6.
+__global__ void __launch_bounds__(kBlock) k_vimp_factor_vjp_staged(mpasg_mesh m, mpasg_fields f, mpasg_fields g,
+                                                                   FastDiv fl, int cols, double* __restrict__ gb,
+                                                                   double* __restrict__ gc) {
   extern __shared__ double sm[];
-  const int L = m.nVertLevels;
-  const size_t plane = (size_t)L * kFacPitch;
+  const int L = m.nVertLevels, pitch = cols | 1;
+  const size_t plane = (size_t)L * pitch;
   double* s_gg = sm;              // gamma's cotangent in, c's out
   double* s_gal = sm + plane;     // alpha's cotangent in, b's out
   double* s_al = sm + 2 * plane;
@@ -64,14 +62,14 @@ __global__ void __launch_bounds__(kFacThreads) k_vimp_factor_vjp_staged(mpasg_me
   double* s_gam = sm + 4 * plane;
   double* s_a = sm + 5 * plane;
   double* s_ga = sm + 6 * plane;
-  const int c0 = blockIdx.x * kFacCols;
-  const int ncol = min(kFacCols, m.nCells - c0);
+  const int c0 = blockIdx.x * cols;
+  const int ncol = min(cols, m.nCells - c0);
   const int t = threadIdx.x;
   const uint32_t nl = (uint32_t)ncol * L;
   const size_t o0 = (size_t)c0 * L;
-  for (uint32_t idx = t; idx < nl; idx += kFacThreads) {
+  for (uint32_t idx = t; idx < nl; idx += kBlock) {
     const uint32_t col = fl.div(idx), k = idx - col * L;
-    const size_t q = k * kFacPitch + col;
+    const size_t q = k * pitch + col;
     s_gg[q] = g.gamma_tri[o0 + idx];
     s_gal[q] = g.alpha_tri[o0 + idx];
     s_al[q] = f.alpha_tri[o0 + idx];
@@ -84,29 +82,29 @@ __global__ void __launch_bounds__(kFacThreads) k_vimp_factor_vjp_staged(mpasg_me
   if (t < ncol) {
     double carry = 0.0;
     for (int k = L - 1; k >= 1; --k) {
-      const size_t q = k * kFacPitch + t;
+      const size_t q = k * pitch + t;
       const double ag = s_gg[q] + carry;
       const double al = s_al[q];
       s_gg[q] = ag * al;
       const double d = -(s_gal[q] + ag * s_c[q]) * al * al;
       s_gal[q] = d;
-      s_ga[q] = -d * s_gam[q - kFacPitch];
+      s_ga[q] = -d * s_gam[q - pitch];
       carry = -d * s_a[q];
     }
     s_gg[t] = 0.0;
     s_gal[t] = 0.0;
   }
   __syncthreads();
-  for (uint32_t idx = t; idx < nl; idx += kFacThreads) {
+  for (uint32_t idx = t; idx < nl; idx += kBlock) {
     const uint32_t col = fl.div(idx), k = idx - col * L;
-    const size_t q = k * kFacPitch + col;
+    const size_t q = k * pitch + col;
     gc[o0 + idx] = s_gg[q];
     gb[o0 + idx] = s_gal[q];
     g.a_tri[o0 + idx] += s_ga[q];
   }
 }
 
-size_t vimp_factor_vjp_smem_bytes(int L) { return (size_t)7 * L * kFacPitch * sizeof(double); }
+size_t vimp_factor_vjp_smem_bytes(int L, int cols) { return (size_t)7 * L * (cols | 1) * sizeof(double); }
 
 // a / b / c diagonals (vert_imp_coefs.py:388-428) read backwards: total cotangents of
 // cofwz (levels 1..L-1), coftz (0..L) and cofwt (0..L-1), written to wz / tz / wt.
@@ -326,38 +324,35 @@ __global__ void k_ac_vjp_solve(mpasg_mesh m, mpasg_fields f, mpasg_fields g) {
                    g.a_tri + o, g.alpha_tri + o, g.gamma_tri + o);
 }
 
-// The same with 32 columns staged through shared memory ([level][33] layout, coalesced
-// copies by 4 warps, the sweeps on the first warp), as the forward Thomas kernels do.
-constexpr int kSolveCols = 32;
-constexpr int kSolvePitch = kSolveCols + 1;
-constexpr int kSolveThreads = 128;
-
-__global__ void __launch_bounds__(kSolveThreads) k_ac_vjp_solve_staged(mpasg_mesh m, mpasg_fields f, mpasg_fields g,
-                                                                       FastDiv fl, FastDiv fl1) {
+// The same with `cols` columns staged through shared memory ([level][column] layout, odd pitch,
+// coalesced copies, the sweeps on the first warp).  2562 x 26: 25 us with 32 columns a block,
+// 11.6 with 6.
+__global__ void __launch_bounds__(kBlock) k_ac_vjp_solve_staged(mpasg_mesh m, mpasg_fields f, mpasg_fields g,
+                                                                FastDiv fl, FastDiv fl1, int cols) {
   extern __shared__ double sm[];
-  const int L = m.nVertLevels;
+  const int L = m.nVertLevels, pitch = cols | 1;
   double* sx = sm;                                   // (L+1) x pitch: the solution x
-  double* sb = sx + (size_t)(L + 1) * kSolvePitch;   // (L+1) x pitch: xb in, the rhs cotangent out
-  double* s1 = sb + (size_t)(L + 1) * kSolvePitch;   // (L+1) x pitch: first sweep's values
-  double* sa = s1 + (size_t)(L + 1) * kSolvePitch;   // L x pitch each below
-  double* sal = sa + (size_t)L * kSolvePitch;
-  double* sg = sal + (size_t)L * kSolvePitch;
-  double* s2 = sg + (size_t)L * kSolvePitch;         // second sweep's values before the alpha scaling
-  const int c0 = blockIdx.x * kSolveCols;
-  const int ncol = min(kSolveCols, m.nCells - c0);
+  double* sb = sx + (size_t)(L + 1) * pitch;   // (L+1) x pitch: xb in, the rhs cotangent out
+  double* s1 = sb + (size_t)(L + 1) * pitch;   // (L+1) x pitch: first sweep's values
+  double* sa = s1 + (size_t)(L + 1) * pitch;   // L x pitch each below
+  double* sal = sa + (size_t)L * pitch;
+  double* sg = sal + (size_t)L * pitch;
+  double* s2 = sg + (size_t)L * pitch;         // second sweep's values before the alpha scaling
+  const int c0 = blockIdx.x * cols;
+  const int ncol = min(cols, m.nCells - c0);
   const int t = threadIdx.x;
   const uint32_t nw = (uint32_t)ncol * (L + 1), nl = (uint32_t)ncol * L;
   const size_t ow0 = (size_t)c0 * (L + 1), o0 = (size_t)c0 * L;
-  for (uint32_t idx = t; idx < nw; idx += kSolveThreads) {
+  for (uint32_t idx = t; idx < nw; idx += kBlock) {
     const uint32_t col = fl1.div(idx), k = idx - col * (L + 1);
-    sx[k * kSolvePitch + col] = f.ac_x[ow0 + idx];
-    sb[k * kSolvePitch + col] = g.ac_x[ow0 + idx];
+    sx[k * pitch + col] = f.ac_x[ow0 + idx];
+    sb[k * pitch + col] = g.ac_x[ow0 + idx];
   }
-  for (uint32_t idx = t; idx < nl; idx += kSolveThreads) {
+  for (uint32_t idx = t; idx < nl; idx += kBlock) {
     const uint32_t col = fl.div(idx), k = idx - col * L;
-    sa[k * kSolvePitch + col] = f.a_tri[o0 + idx];
-    sal[k * kSolvePitch + col] = f.alpha_tri[o0 + idx];
-    sg[k * kSolvePitch + col] = f.gamma_tri[o0 + idx];
+    sa[k * pitch + col] = f.a_tri[o0 + idx];
+    sal[k * pitch + col] = f.alpha_tri[o0 + idx];
+    sg[k * pitch + col] = f.gamma_tri[o0 + idx];
   }
   __syncthreads();
   // the two sweeps keep only their recurrences (solve_vjp_column's order of operations):
@@ -366,34 +361,34 @@ __global__ void __launch_bounds__(kSolveThreads) k_ac_vjp_solve_staged(mpasg_mes
   if (t < ncol) {
     double prev = 0.0;
     for (int k = 0; k <= L; ++k) {
-      const double au = sb[k * kSolvePitch + t] - (k > 0 ? sg[(k - 1) * kSolvePitch + t] * prev : 0.0);
-      s1[k * kSolvePitch + t] = au;
+      const double au = sb[k * pitch + t] - (k > 0 ? sg[(k - 1) * pitch + t] * prev : 0.0);
+      s1[k * pitch + t] = au;
       prev = au;
     }
     double carry = 0.0;
     for (int k = L - 1; k >= 1; --k) {
-      const double au = s1[k * kSolvePitch + t] + carry;
-      s2[k * kSolvePitch + t] = au;
-      const double at = au * sal[k * kSolvePitch + t];
-      sb[k * kSolvePitch + t] = at;
-      carry = -at * sa[k * kSolvePitch + t];
+      const double au = s1[k * pitch + t] + carry;
+      s2[k * pitch + t] = au;
+      const double at = au * sal[k * pitch + t];
+      sb[k * pitch + t] = at;
+      carry = -at * sa[k * pitch + t];
     }
-    sb[L * kSolvePitch + t] = s1[L * kSolvePitch + t];
+    sb[L * pitch + t] = s1[L * pitch + t];
     sb[t] = s1[t] + carry;
   }
   __syncthreads();
-  for (uint32_t idx = t; idx < nw; idx += kSolveThreads) {
+  for (uint32_t idx = t; idx < nw; idx += kBlock) {
     const uint32_t col = fl1.div(idx), k = idx - col * (L + 1);
-    g.ac_x[ow0 + idx] = sb[k * kSolvePitch + col];
+    g.ac_x[ow0 + idx] = sb[k * pitch + col];
   }
-  for (uint32_t idx = t; idx < nl; idx += kSolveThreads) {
+  for (uint32_t idx = t; idx < nl; idx += kBlock) {
     const uint32_t col = fl.div(idx), k = idx - col * L;
-    const size_t q = k * kSolvePitch + col;
-    const double xk1 = sx[q + kSolvePitch];
+    const size_t q = k * pitch + col;
+    const double xk1 = sx[q + pitch];
     g.gamma_tri[o0 + idx] += -s1[q] * xk1;
     if (k >= 1) {
       const double u_k = sx[q] + sg[q] * xk1;
-      const double u_km1 = sx[q - kSolvePitch] + sg[q - kSolvePitch] * sx[q];
+      const double u_km1 = sx[q - pitch] + sg[q - pitch] * sx[q];
       const double au = s2[q];
       g.alpha_tri[o0 + idx] += au * (u_k * rcp_nr(sal[q]));
       g.a_tri[o0 + idx] += -(au * sal[q]) * u_km1;
@@ -401,7 +396,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_ac_vjp_solve_staged(mpasg_mes
   }
 }
 
-size_t solve_vjp_smem_bytes(int L) { return (size_t)(3 * (L + 1) + 4 * L) * kSolvePitch * sizeof(double); }
+size_t solve_vjp_smem_bytes(int L, int cols) {
+  return (size_t)(3 * (L + 1) + 4 * L) * (cols | 1) * sizeof(double);
+}
 
 // The tridiagonal right-hand side (acoustic_step.py:675) and rs / ts read backwards, per
 // mass level: -> tend_theta, tend_rho, cofwz, cofwt, the rs / ts cotangents (rsb, tsb), the
@@ -822,15 +819,16 @@ int mpasgi_acoustic_vjp_rev(const mpasg_mesh* m, const mpasg_config* c, mpasg_fi
   MPASG_LAUNCH_CHECK();
   // the staged solve needs more than 48 KB of dynamic shared memory: opt in once per device
   // (the first call on a device should come before any stream capture)
-  const size_t smem = solve_vjp_smem_bytes(L);
+  const int cols = columns_per_block(m->nCells, L + 1, 400, 31, 6);
+  const size_t smem = solve_vjp_smem_bytes(L, cols);
   static bool opt_in[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MPASG_E_CUDA;
   if (!opt_in[dev])
     opt_in[dev] = cudaFuncSetAttribute(k_ac_vjp_solve_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       200 * 1024) == cudaSuccess;
-  if (opt_in[dev] && smem <= 200 * 1024)
-    k_ac_vjp_solve_staged<<<nblocks(m->nCells, kSolveCols), kSolveThreads, smem, s>>>(*m, *f, *g, fl, fl1);
+                                       (int)kMaxSmem) == cudaSuccess;
+  if (opt_in[dev] && smem <= kMaxSmem)
+    k_ac_vjp_solve_staged<<<nblocks(m->nCells, cols), kBlock, smem, s>>>(*m, *f, *g, fl, fl1, cols);
   else
     k_ac_vjp_solve<<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f, *g);
   MPASG_LAUNCH_CHECK();
@@ -891,15 +889,16 @@ int mpasgi_vimp_vjp_core(const mpasg_mesh* m, const mpasg_config* c, const mpasg
   double* gc = w.c[9];
   // the staged kernel needs more than 48 KB of dynamic shared memory: opt in once per device
   // (the first call on a device should come before any stream capture)
-  const size_t smem = vimp_factor_vjp_smem_bytes(L);
+  const int cols = columns_per_block(m->nCells, L, 400, 31, 6);
+  const size_t smem = vimp_factor_vjp_smem_bytes(L, cols);
   static bool opt_in[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MPASG_E_CUDA;
   if (!opt_in[dev])
     opt_in[dev] = cudaFuncSetAttribute(k_vimp_factor_vjp_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       200 * 1024) == cudaSuccess;
-  if (opt_in[dev] && smem <= 200 * 1024)
-    k_vimp_factor_vjp_staged<<<nblocks(m->nCells, kFacCols), kFacThreads, smem, s>>>(*m, *f, *g, FastDiv(L), gb, gc);
+                                       (int)kMaxSmem) == cudaSuccess;
+  if (opt_in[dev] && smem <= kMaxSmem)
+    k_vimp_factor_vjp_staged<<<nblocks(m->nCells, cols), kBlock, smem, s>>>(*m, *f, *g, FastDiv(L), cols, gb, gc);
   else
     k_vimp_factor_vjp<<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f, *g, gb, gc);
   MPASG_LAUNCH_CHECK();

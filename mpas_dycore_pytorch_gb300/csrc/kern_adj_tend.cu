@@ -15,6 +15,9 @@
 // Smagorinsky deformation and kdiff, the del2 field of u and its del4 divergence and curl)
 // are recomputed here from the stage's inputs, with the forward's expressions.
 #include "adj_common.cuh"
+#include "advstencil.cuh"
+#include "branches.cuh"
+#include "trisk.cuh"
 
 namespace {
 
@@ -121,32 +124,34 @@ struct WdtzGrad {
   double rw, rws;
 };
 MPASG_D WdtzGrad wdtz_grad(const mpasg_mesh& m, const double* th, const double* ths, const double* rw,
-                           const double* rws, int q, int L, double coef3) {
+                           const double* rws, int q, int L, double coef3, double b) {  // times b
   WdtzGrad d = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0}, 0.0, 0.0};
   const double fm = m.fzm[q], fp = m.fzp[q];
   if (q == L - 1 && q != 1) {
-    d.th[2] = rws[q] * fm;
-    d.th[1] = rws[q] * fp;
-    d.rws = fm * th[q] + fp * th[q - 1];
+    const double r = b * rws[q];
+    d.th[2] = r * fm;
+    d.th[1] = r * fp;
+    d.rws = b * (fm * th[q] + fp * th[q - 1]);
     return d;
   }
   if (q == 1) {
-    d.th[2] = rw[q] * fm;
-    d.th[1] = rw[q] * fp;
-    d.rw = fm * th[q] + fp * th[q - 1];
+    const double r = b * rw[q];
+    d.th[2] = r * fm;
+    d.th[1] = r * fp;
+    d.rw = b * (fm * th[q] + fp * th[q - 1]);
   } else {
-    const Flux3Grad g = flux3_grad(th[q - 2], th[q - 1], th[q], th[q + 1], rw[q], coef3);
+    const Flux3Grad g = flux3_grad(th[q - 2], th[q - 1], th[q], th[q + 1], rw[q], coef3, b);
     d.th[0] = g.qm2;
     d.th[1] = g.qm1;
     d.th[2] = g.q0;
     d.th[3] = g.qp1;
     d.rw = g.ua;
   }
-  const double tse = fm * ths[q] + fp * ths[q - 1];
-  d.rw -= tse;
-  d.rws = tse;
-  d.ths[1] = (rws[q] - rw[q]) * fm;
-  d.ths[0] = (rws[q] - rw[q]) * fp;
+  d.rws = b * (fm * ths[q] + fp * ths[q - 1]);
+  d.rw -= d.rws;
+  const double r = b * (rws[q] - rw[q]);
+  d.ths[1] = r * fm;
+  d.ths[0] = r * fp;
   return d;
 }
 
@@ -155,23 +160,21 @@ struct WdwzGrad {
   double w[4];
   double rwm, rw;
 };
-MPASG_D WdwzGrad wdwz_grad(const double* w, const double* rw, int q, int L) {
+MPASG_D WdwzGrad wdwz_grad(const double* w, const double* rw, int q, int L, double b) {  // times b
   WdwzGrad d = {{0.0, 0.0, 0.0, 0.0}, 0.0, 0.0};
+  const double rw2 = rw[q] + rw[q - 1], h = 0.5 * b;
   if (q == 1 || q == L - 1) {
-    const double a = 0.25 * (w[q] + w[q - 1]), b = 0.25 * (rw[q] + rw[q - 1]);
-    d.rw = a;
-    d.rwm = a;
-    d.w[2] = b;
-    d.w[1] = b;
+    d.rw = d.rwm = (0.5 * h) * (w[q] + w[q - 1]);
+    d.w[2] = d.w[1] = (0.5 * h) * rw2;
     return d;
   }
-  const Flux3Grad g = flux3_grad(w[q - 2], w[q - 1], w[q], w[q + 1], 0.5 * (rw[q] + rw[q - 1]), 1.0);
+  // the mean of rw is rw2 / 2: the factor goes into b
+  const Flux3Grad g = flux3_grad(w[q - 2], w[q - 1], w[q], w[q + 1], rw2, 1.0, h);
   d.w[0] = g.qm2;
   d.w[1] = g.qm1;
   d.w[2] = g.q0;
   d.w[3] = g.qp1;
-  d.rw = 0.5 * g.ua;
-  d.rwm = 0.5 * g.ua;
+  d.rw = d.rwm = g.ua;
   return d;
 }
 
@@ -179,43 +182,86 @@ MPASG_D WdwzGrad wdwz_grad(const double* w, const double* rw, int q, int L) {
 // vertical fluxes of theta and w, the flux divergences' area factor, the buoyancy /
 // pressure-gradient residual (rk 1), the diabatic term, and the Euler tendencies
 // (collected for the mixing at rk 1, passed through at rk 2 and 3)
-__global__ void k_tadj_columns(mpasg_mesh m, mpasg_fields f, mpasg_fields g, FastDiv fl1, AdjTendScalars p,
-                               double* __restrict__ tt1b, double* __restrict__ tw1b, double* __restrict__ tweb,
-                               double* __restrict__ tteb) {
+// Each thread forms its own interface's partials once and the levels collect them through shared
+// memory; a block covers three interfaces more than levels (one below, two above), so none is
+// formed twice within it.  Every level evaluating its four interfaces itself took ~200
+// float64 operations a level, the pipe that bounds the kernel: 27 -> 20 us at 2562 x 26.
+constexpr int kColumnLevels = kBlock - 3;
+struct ColumnPart {
+  double th[4], w[4];  // to theta_m and w at levels q-2 .. q+1
+  double ths[2];       // to theta_m_save at q-1, q
+  double rwm;          // to rw at q-1
+  double rw, rws;      // to rw and rw_save at q
+};
+
+MPASG_D ColumnPart column_part(const mpasg_mesh& m, const mpasg_fields& f, const mpasg_fields& g, size_t oc, size_t ow,
+                               int q, int L, double coef3) {
+  ColumnPart d = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}, {0.0, 0.0}, 0.0, 0.0, 0.0};
+  if (q < 1 || q > L - 1) return d;
+  const double bt = g.tend_theta[oc + q] * m.rdzw[q] - g.tend_theta[oc + q - 1] * m.rdzw[q - 1];
+  if (!fx::is_zero(bt)) {
+    const WdtzGrad t = wdtz_grad(m, f.theta_m + oc, f.theta_m_save + oc, f.rw + ow, f.rw_save + ow, q, L, coef3, bt);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) d.th[j] = t.th[j];
+    d.ths[0] = t.ths[0];
+    d.ths[1] = t.ths[1];
+    d.rw = t.rw;
+    d.rws = t.rws;
+  }
+  const double bw = g.tend_w[ow + q] * m.rdzu[q] - (q > 1 ? g.tend_w[ow + q - 1] * m.rdzu[q - 1] : 0.0);
+  if (!fx::is_zero(bw)) {
+    const WdwzGrad t = wdwz_grad(f.w + ow, f.rw + ow, q, L, bw);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) d.w[j] = t.w[j];
+    d.rw += t.rw;
+    d.rwm = t.rwm;
+  }
+  return d;
+}
+
+__global__ void __launch_bounds__(kBlock) k_tadj_columns(mpasg_mesh m, mpasg_fields f, mpasg_fields g, FastDiv fl1,
+                                                         AdjTendScalars p, double* __restrict__ tt1b,
+                                                         double* __restrict__ tw1b, double* __restrict__ tweb,
+                                                         double* __restrict__ tteb) {
+  __shared__ double s_th[4][kBlock], s_w[4][kBlock], s_ths[kBlock], s_rwm[kBlock];
   const int L = m.nVertLevels;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (uint32_t)m.nCells * (L + 1)) return;
+  const int me = (int)threadIdx.x;
+  const long long at = (long long)blockIdx.x * kColumnLevels + me - 1;
+  const bool inside = at >= 0 && at < (long long)m.nCells * (L + 1);
+  const uint32_t i = inside ? (uint32_t)at : 0u;
   const uint32_t c = fl1.div(i);
   const int k = (int)(i - c * (L + 1));
   const size_t oc = (size_t)c * L, ow = (size_t)c * (L + 1);
+  const ColumnPart own = column_part(m, f, g, oc, ow, k, L, p.coef3);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    s_th[j][me] = own.th[j];
+    s_w[j][me] = own.w[j];
+  }
+  s_ths[me] = own.ths[0];
+  s_rwm[me] = own.rwm;
+  __syncthreads();
+  if (!inside || me < 1 || me > kColumnLevels) return;
   const double ia = m.invAreaCell[c];
-  const double* th = f.theta_m + oc;
-  const double* ths = f.theta_m_save + oc;
-  const double* rw = f.rw + ow;
-  const double* rws = f.rw_save + ow;
-  const double* w = f.w + ow;
-  auto Gtt = [&](int q) { return (q >= 0 && q < L) ? g.tend_theta[oc + q] : 0.0; };
-  auto Gtw = [&](int q) { return (q >= 1 && q <= L - 1) ? g.tend_w[ow + q] : 0.0; };
-  auto wdtzb = [&](int q) { return Gtt(q) * (q < L ? m.rdzw[q] : 0.0) - Gtt(q - 1) * (q >= 1 ? m.rdzw[q - 1] : 0.0); };
-  auto wdwzb = [&](int q) { return Gtw(q) * m.rdzu[q < L ? q : 0] * (q <= L - 1 ? 1.0 : 0.0) -
-                                   Gtw(q - 1) * (q - 1 >= 1 ? m.rdzu[q - 1] : 0.0); };
+  double gth = 0.0, gths = own.ths[1], gw = 0.0, grw = own.rw;
+  const double grws = own.rws;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {  // interface k + 2 - j holds this level in slot j
+    const int q = k + 2 - j;
+    if (q < 1 || q > L - 1) continue;
+    gth += s_th[j][me + 2 - j];
+    gw += s_w[j][me + 2 - j];
+  }
+  if (k + 1 <= L - 1) {
+    gths += s_ths[me + 1];
+    grw += s_rwm[me + 1];
+  }
   // ---- mass level k: theta
   if (k < L) {
     const size_t o = oc + k;
     const double G = g.tend_theta[o];
     g.rho_zz[o] += G * f.rt_diabatic_tend[o];
     tt1b[o] = G * ia;
-    double gth = 0.0, gths = 0.0;
-    for (int q = k - 1; q <= k + 2; ++q) {
-      if (q < 1 || q > L - 1) continue;
-      const double b = wdtzb(q);
-      if (b == 0.0) continue;
-      const WdtzGrad d = wdtz_grad(m, th, ths, rw, rws, q, L, p.coef3);
-      const int s = k - (q - 2);  // position of level k in q-2..q+1
-      gth += b * d.th[s];
-      if (k == q - 1) gths += b * d.ths[0];
-      if (k == q) gths += b * d.ths[1];
-    }
     g.theta_m[o] += gth;
     g.theta_m_save[o] += gths;
     if (p.rk_step == 1) {
@@ -224,23 +270,7 @@ __global__ void k_tadj_columns(mpasg_mesh m, mpasg_fields f, mpasg_fields g, Fas
       g.tend_theta_euler[o] += G;
     }
   }
-  // ---- w level k: rw / rw_save from the theta flux, w / rw from the w flux
-  double grw = 0.0, grws = 0.0, gw = 0.0;
-  if (k >= 1 && k <= L - 1) {
-    const double b = wdtzb(k);
-    const WdtzGrad d = wdtz_grad(m, th, ths, rw, rws, k, L, p.coef3);
-    grw += b * d.rw;
-    grws += b * d.rws;
-  }
-  for (int q = k - 1; q <= k + 2; ++q) {
-    if (q < 1 || q > L - 1) continue;
-    const double b = wdwzb(q);
-    if (b == 0.0) continue;
-    const WdwzGrad d = wdwz_grad(w, rw, q, L);
-    gw += b * d.w[k - (q - 2)];
-    if (k == q) grw += b * d.rw;
-    if (k == q - 1) grw += b * d.rwm;
-  }
+  // ---- w level k
   g.rw[ow + k] += grw;
   g.rw_save[ow + k] += grws;
   g.w[ow + k] += gw;
@@ -296,19 +326,25 @@ MPASG_D bool nonneg(double x) {
 // its flux cotangent; level k also needs level k+1's (shared memory, recomputed at the
 // block's edge).  The upwind sides of the theta and w stencils are stored as bits in sel
 // for the cell gather.
+// The theta sum runs on the integer pipes (fixdot.cuh), the w sum on the float64 pipe, as in the
+// tendencies: 28 -> 24 us at 2562 x 26.
+template <int N>
 __global__ void __launch_bounds__(kBlock) k_tadj_adv_edges(mpasg_mesh m, mpasg_fields f, mpasg_fields g,
                                                            mpasg_transpose t, FastDiv fl, AdjTendScalars p,
                                                            const double* __restrict__ tt1b,
                                                            const double* __restrict__ tw1b, double* __restrict__ fltb,
                                                            double* __restrict__ flwb, uint8_t* __restrict__ sel) {
+  extern __shared__ fx::Weight s_w[];
   __shared__ double s_pw[kBlock];
   const int L = m.nVertLevels;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = i < (uint32_t)m.nEdges * L;
-  const int me = m.maxEdges, na = m.nAdvMax;
+  const int me = m.maxEdges;
+  const uint32_t n_all = (uint32_t)m.nEdges * L, i0 = blockIdx.x * kBlock;
+  const uint32_t e0 = fl.div(i0), e1 = fl.div(min(i0 + kBlock, n_all) - 1u);
+  adv::load<N>(m, e0, e1 - e0 + 1, s_w);
   uint32_t e = 0;
-  int k = 0, nadv = 0;
-  const int32_t* cells = m.advCellsForEdge;
+  int k = 0;
   // cotangents of the edge fluxes from the two cells' sums (x = -sign * flux)
   auto edge_b = [&](const double* src, int kk, size_t pitch) {
     double s = 0.0;
@@ -320,28 +356,17 @@ __global__ void __launch_bounds__(kBlock) k_tadj_adv_edges(mpasg_mesh m, mpasg_f
     }
     return s;
   };
-  auto adv_sum = [&](const double* fld, int kk, size_t pitch, bool up) {
-    const double* cf = (up ? m.adv_coefs_p : m.adv_coefs_m) + (size_t)e * na;
-    double acc = 0.0;
-    for (int a = 0; a < nadv; ++a) {
-      const double tt = cf[a] * fld[(size_t)cells[a] * pitch + kk];
-      acc = (a == 0) ? tt : acc + tt;
-    }
-    return acc;
-  };
   auto ru_w = [&](int kk) { return m.fzm[kk] * f.ru[(size_t)e * L + kk] + m.fzp[kk] * f.ru[(size_t)e * L + kk - 1]; };
   auto w_part = [&](int kk, bool* up) {  // fweb_kk * sum_a cf_a w_a, and the flux cotangent's product
     const double rwk = ru_w(kk);
     *up = nonneg(rwk);
-    return edge_b(tw1b, kk, L + 1) * adv_sum(f.w, kk, L + 1, *up);
+    return edge_b(tw1b, kk, L + 1) * adv::sum(m, e, !*up, f.w, L + 1, kk);
   };
   double pw = 0.0;
   bool up_w = true;
   if (active) {
     e = fl.div(i);
     k = (int)(i - e * L);
-    nadv = m.nAdvCellsForEdge[e];
-    cells = m.advCellsForEdge + (size_t)e * na;
     if (k >= 1) pw = w_part(k, &up_w);
   }
   s_pw[threadIdx.x] = pw;
@@ -351,7 +376,12 @@ __global__ void __launch_bounds__(kBlock) k_tadj_adv_edges(mpasg_mesh m, mpasg_f
   const bool up_t = nonneg(rue);
   // theta
   const double fteb = edge_b(tt1b, k, L);
-  double gru = fteb * adv_sum(f.theta_m, k, L, up_t);
+  const fx::Weight* w = s_w + (e - e0) * (2 * N) + (up_t ? 0 : N);
+  double x[N], th;
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = f.theta_m[(uint32_t)w[j].row * L + k];
+  if (!fx::dot<N>(x, w, &th)) th = adv::sum(m, e, !up_t, f.theta_m, L, k);
+  double gru = fteb * th;
   fltb[i] = fteb * rue;
   // w at level k (k >= 1) and k + 1: ru_w = fzm ru_k + fzp ru_(k-1)
   if (k >= 1) {
@@ -451,19 +481,54 @@ MPASG_D WduzPart wduz_part(const mpasg_mesh& m, const mpasg_fields& f, const dou
     w.pr = b * (m.fzm[q] * ue[q] + m.fzp[q] * ue[q - 1]);
     return w;
   }
-  const Flux3Grad d = flux3_grad(ue[q - 2], ue[q - 1], ue[q], ue[q + 1], rwe, 1.0);
-  w.c[0] = b * d.qm2;
-  w.c[1] = b * d.qm1;
-  w.c[2] = b * d.q0;
-  w.c[3] = b * d.qp1;
-  w.pr = b * d.ua;
+  const Flux3Grad d = flux3_grad(ue[q - 2], ue[q - 1], ue[q], ue[q + 1], rwe, 1.0, b);
+  w.c[0] = d.qm2;
+  w.c[1] = d.qm1;
+  w.c[2] = d.q0;
+  w.c[3] = d.qp1;
+  w.pr = d.ua;
   return w;
 }
 
 // Each thread forms the parts of its own interface k once; level k collects c[3], c[2],
 // c[1], c[0] of interfaces k-1, k, k+1, k+2 from its neighbours in the block (shared
 // memory), recomputing the few that fall outside it.
-__global__ void __launch_bounds__(kBlock) k_tadj_u(mpasg_mesh m, mpasg_fields f, mpasg_fields g, mpasg_transpose t,
+// The four stencil sums run on the integer pipes (fixdot.cuh; 40 of ~85 float64 operations a
+// level, which bound the kernel): 55 -> 45 us at 2562 x 26, mean of a step's launches.
+template <int N>
+MPASG_D void load_transposed(const mpasg_mesh& m, const mpasg_transpose& t, uint32_t e0, uint32_t n, fx::Weight* tab) {
+  const int me2 = m.maxEdges2;
+  for (uint32_t q = threadIdx.x; q < n * N; q += blockDim.x) {
+    const uint32_t el = q / N, j = q - el * N, e = e0 + el;
+    const int n2 = m.nEdgesOnEdge[e];
+    fx::Weight w{0, 0, n2 > N ? fx::kBadWeight : 0u, n2 > 0 ? m.edgesOnEdge[e * me2] : (int)e};
+    if ((int)j < n2 && n2 <= N) {
+      const int jt = t.eoeTransSlot[e * me2 + j], eo = m.edgesOnEdge[e * me2 + j];
+      if (jt >= 0) w = fx::weight(m.weightsOnEdge[(size_t)eo * me2 + jt], eo);
+    }
+    tab[q] = w;
+  }
+}
+
+template <int N>
+MPASG_D double sum_transposed(const mpasg_mesh& m, const mpasg_transpose& t, const double* __restrict__ field,
+                              const fx::Weight* w, uint32_t e, uint32_t k, uint32_t L) {
+  double x[N], out;
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = field[(uint32_t)w[j].row * L + k];
+  if (!fx::dot<N>(x, w, &out)) {
+    out = 0.0;
+    const int me2 = m.maxEdges2;
+    for (int j = 0; j < m.nEdgesOnEdge[e]; ++j) {
+      const int jt = t.eoeTransSlot[e * me2 + j], eo = m.edgesOnEdge[e * me2 + j];
+      if (jt >= 0) out = fma(m.weightsOnEdge[(size_t)eo * me2 + jt], field[(size_t)eo * L + k], out);
+    }
+  }
+  return out;
+}
+
+template <int N>
+__global__ void __launch_bounds__(kBlock, 4) k_tadj_u(mpasg_mesh m, mpasg_fields f, mpasg_fields g, mpasg_transpose t,
                                                    FastDiv fl, AdjTendScalars p, const double* __restrict__ hd,
                                                    const double* __restrict__ kd, const double* __restrict__ ud,
                                                    const double* __restrict__ dsd, const double* __restrict__ dsv,
@@ -473,8 +538,13 @@ __global__ void __launch_bounds__(kBlock) k_tadj_u(mpasg_mesh m, mpasg_fields f,
                                                    double* __restrict__ pd4, const double* __restrict__ qa,
                                                    double* __restrict__ pdz, const double* __restrict__ qapv,
                                                    const double* __restrict__ pvu) {
+  extern __shared__ fx::Weight s_w[];
   __shared__ double s_c[4][kBlock];
   const int L = m.nVertLevels;
+  const uint32_t n_all = (uint32_t)m.nEdges * L, i0 = blockIdx.x * kBlock;
+  const uint32_t e0 = fl.div(i0), ne = fl.div(min(i0 + kBlock, n_all) - 1u) - e0 + 1;
+  trisk::load<N>(m, e0, ne, s_w);
+  load_transposed<N>(m, t, e0, ne, s_w + ne * N);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = i < (uint32_t)m.nEdges * L;
   uint32_t e = 0;
@@ -501,24 +571,12 @@ __global__ void __launch_bounds__(kBlock) k_tadj_u(mpasg_mesh m, mpasg_fields f,
   const double inv_dc = m.invDcEdge[e];
   // PV flux q_e = 0.5 sum_j w_j u_j (pv_e + pv_j), with its transpose over edgesOnEdge: the
   // neighbour eo's sum reads u_e and pv_e at its slot jt (cotangent of q_eo: G_eo rho_edge_eo)
-  // four sums over the stencil, combined after the loop (four multiply-adds per slot, the
-  // per-edge products from k_tadj_qa): s1 = sum w u, s2 = sum w (pv u), s3 = sum wt A,
-  // s4 = sum wt (A pv), A = G_eo rho_edge_eo
-  const int n2 = m.nEdgesOnEdge[e], me2 = m.maxEdges2;
+  // four sums over the stencil, combined after it (the per-edge products from k_tadj_qa):
+  // s1 = sum w u, s2 = sum w (pv u), s3 = sum wt A, s4 = sum wt (A pv), A = G_eo rho_edge_eo
   const double pv_self = f.pv_edge[i], u_self = ue[k];
-  double s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
-  for (int j = 0; j < n2; ++j) {
-    const int eo = m.edgesOnEdge[e * me2 + j];
-    const size_t io = (size_t)eo * L + k;
-    const double w = m.weightsOnEdge[e * me2 + j];
-    s1 = fma(w, f.u[io], s1);
-    s2 = fma(w, pvu[io], s2);
-    const int jt = t.eoeTransSlot[e * me2 + j];
-    if (jt < 0) continue;
-    const double wt = m.weightsOnEdge[(size_t)eo * me2 + jt];
-    s3 = fma(wt, qa[io], s3);
-    s4 = fma(wt, qapv[io], s4);
-  }
+  const fx::Weight *w = s_w + (e - e0) * N, *wt = w + ne * N;
+  const double s1 = trisk::sum<N>(m, f.u, w, e, k, L), s2 = trisk::sum<N>(m, pvu, w, e, k, L);
+  const double s3 = sum_transposed<N>(m, t, qa, wt, e, k, L), s4 = sum_transposed<N>(m, t, qapv, wt, e, k, L);
   const double q = 0.5 * (pv_self * s1 + s2);
   double gh = G * (q - (f.ke[i2] - f.ke[i1]) * inv_dc);
   pke[i] = G * rho_e * inv_dc;
@@ -1124,6 +1182,10 @@ int mpasgi_dyn_tend_vjp_core(const mpasg_mesh* m, const mpasg_config* c, const m
   double* dsv = w.v[0];
   double* dsvb = w.v[1];
 
+  const size_t rows = (size_t)((kBlock - 1) / L + 2);  // edges a block covers, at most
+  // the columns and the advection beside the u tendency: they write different cotangents and
+  // work arrays
+  GraphBranches branches(s);
   k_tadj_values<<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p, hd, kd, ddb, dob);
   MPASG_LAUNCH_CHECK();
   if (rk_step == 1 && p.del4) {
@@ -1134,7 +1196,20 @@ int mpasgi_dyn_tend_vjp_core(const mpasg_mesh* m, const mpasg_config* c, const m
     k_tadj_del4_vertices<<<nblocks(nvl), kBlock, 0, s>>>(*m, fl, ud, dsv);
     MPASG_LAUNCH_CHECK();
   }
-  k_tadj_columns<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, *g, fl1, p, tt1b, tw1b, tweb, tteb);
+  double* qa = w.e[11];  // a4t's, formed later
+  double* qapv = w.e[19];
+  double* pvu = w.e[20];
+  k_tadj_qa<<<nblocks(nel), kBlock, 0, s>>>((int)nel, g->tend_u, f->h_edge, f->pv_edge, f->u, qa, qapv, pvu);
+  MPASG_LAUNCH_CHECK();
+  const auto tadj_u = [&](auto kernel, int n) {
+    kernel<<<nblocks(nel), kBlock, rows * 2 * n * sizeof(fx::Weight), s>>>(
+        *m, *f, *g, *t, fl, p, hd, kd, ud, dsd, dsv, pke, phd, prwe, ppp, pkd, udb, pd4, qa, pdz, qapv, pvu);
+  };
+  if (m->maxEdges2 <= 10) tadj_u(k_tadj_u<10>, 10);
+  else tadj_u(k_tadj_u<14>, 14);
+  MPASG_LAUNCH_CHECK();
+  CHECK_RC(branches.next());
+  k_tadj_columns<<<nblocks(ncw, kColumnLevels), kBlock, 0, s>>>(*m, *f, *g, fl1, p, tt1b, tw1b, tweb, tteb);
   MPASG_LAUNCH_CHECK();
   if (rk_step == 1) {
     k_tadj_wres<<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, *g, fl, tweb);
@@ -1145,18 +1220,16 @@ int mpasgi_dyn_tend_vjp_core(const mpasg_mesh* m, const mpasg_config* c, const m
     }
   }
   uint8_t* sel = reinterpret_cast<uint8_t*>(w.e[2]);  // (E+1) x L bytes within one edge array
-  k_tadj_adv_edges<<<nblocks(nel), kBlock, 0, s>>>(*m, *f, *g, *t, fl, p, tt1b, tw1b, fltb, flwb, sel);
+  if (m->nAdvMax <= 10)
+    k_tadj_adv_edges<10><<<nblocks(nel), kBlock, rows * 10 * adv::kEntryBytes, s>>>(*m, *f, *g, *t, fl, p, tt1b, tw1b,
+                                                                                  fltb, flwb, sel);
+  else
+    k_tadj_adv_edges<14><<<nblocks(nel), kBlock, rows * 14 * adv::kEntryBytes, s>>>(*m, *f, *g, *t, fl, p, tt1b, tw1b,
+                                                                                  fltb, flwb, sel);
   MPASG_LAUNCH_CHECK();
   k_tadj_adv_cells<<<nblocks(ncw), kBlock, 0, s>>>(*m, *g, *t, fl1, FastDiv(m->nAdvMax), fltb, flwb, sel);
   MPASG_LAUNCH_CHECK();
-  double* qa = w.e[2];  // sel's bytes (read by the advection gather above) are no longer needed
-  double* qapv = w.e[19];
-  double* pvu = w.e[20];
-  k_tadj_qa<<<nblocks(nel), kBlock, 0, s>>>((int)nel, g->tend_u, f->h_edge, f->pv_edge, f->u, qa, qapv, pvu);
-  MPASG_LAUNCH_CHECK();
-  k_tadj_u<<<nblocks(nel), kBlock, 0, s>>>(*m, *f, *g, *t, fl, p, hd, kd, ud, dsd, dsv, pke, phd, prwe, ppp, pkd,
-                                          udb, pd4, qa, pdz, qapv, pvu);
-  MPASG_LAUNCH_CHECK();
+  CHECK_RC(branches.join());
   k_tadj_u_cells<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, *g, fl1, p, pke, phd, prwe, ppp, pkd, pd4, pdz, hdb, kdb,
                                                  dsdb);
   MPASG_LAUNCH_CHECK();

@@ -6,9 +6,8 @@
 // order (mpas_pytorch/dynamics/*.py, cited per kernel); slot sums run in connectivity
 // slot order, left to right, so results are deterministic and need no atomics.
 #include "common.cuh"
+#include "columns.cuh"
 #include "pow_exner.cuh"
-
-#include <algorithm>
 
 namespace {
 
@@ -44,20 +43,6 @@ __global__ void k_moist_edges(int ne, int L, FastDiv fl, int ms, int me, const i
     cqu[i] = 1.0;
   }
 }
-
-// Columns of a block in the kernels that keep whole columns in shared memory (`items`: the
-// levels or faces of one that the block's 256 threads share out).  Two full passes of the
-// threads over a block's items, so that no pass is nearly empty (33 levels, 10242 columns:
-// acoustic stage 276 us with 14 columns, 303 with 11, whose last pass fills 46 of 256 threads),
-// and at most 18: the serial sweeps take one lane a column, and more than that buys nothing.
-// A small mesh takes fewer, one pass, down to 4: float64 work is bound to its SM and the
-// sweeps of a block wait for all its levels (162 columns of 12 levels: step 666 us with 4, 674
-// with 16, 724 with 32; 642 of 55: 1013, 1159, 1319).
-inline int columns_per_block(int nCells, int items, int cells_per_column) {
-  const int least = std::max(2, std::min(4, kBlock / items));
-  return std::max(least, std::min({18, 2 * kBlock / items, nCells / cells_per_column}));
-}
-constexpr size_t kMaxSmem = 200 * 1024;
 
 // ---------------------------------------------------------------- vertical implicit coefficients
 // dynamics/vert_imp_coefs.py:188 (coefficients :343-446, Thomas factor :100-121).
@@ -208,7 +193,7 @@ MPASG_D void factor_column(const double* a, const double* b, const double* c, do
 // Coefficients and factorisation of `cols` columns in one launch, what passes between them in
 // shared memory ([level][column], odd pitch).  In place of two launches, each a few waves of
 // latency on a small mesh: a step of 162 columns x 12 levels 664 -> 640 us, 2562 x 26 1359 ->
-// 1334, 40962 x 55 25.58 -> 25.52 ms (mixed form 17.61 -> 17.56).
+// 1334, 40962 x 55 25.58 -> 25.37 ms (mixed form 17.61 -> 17.27).
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fields f, FastDiv fl, int cols,
                                                          VimpScalars s) {
@@ -1247,7 +1232,7 @@ __global__ void k_recover_w(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
   if (kMixed) f.w_f32[i] = d2f_bits(wk);
 }
 
-// part 0: cells, 1: edges, 2: w over terrain
+// part 0: cells, 1: edges, 2: w over terrain, 3: rho alone
 template <typename T>
 int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv_ns, double rk_dt, cudaStream_t s,
                    bool finish, double damp_coef, bool one_substep, int part) {
@@ -1261,6 +1246,8 @@ int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv
     if (finish && one_substep) k_recover_edges<T, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef);
     else if (finish) k_recover_edges<T, true, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef);
     else k_recover_edges<T, false, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, 0.0);
+  } else if (part == 3) {
+    k_recover_rho<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, (uint32_t)m->nCells * L);
   } else if (!m->flatTerrain) {  // slope fluxes need the new ru of k_recover_edges
     k_recover_w<T><<<nw, kBlock, 0, s>>>(*m, *f, fl1);
   }
@@ -1276,7 +1263,7 @@ static int launch_ac_columns(const mpasg_mesh* m, const mpasg_fields* f, bool mi
                              double epssm, double resm, bool keep, bool last, cudaStream_t s, bool* done) {
   const int L = m->nVertLevels, N = m->maxEdges <= 6 ? 6 : 10;
   const bool first = small_step == 1;
-  const int cols = columns_per_block(m->nCells, L + 1, 600), nb = nblocks(m->nCells, cols);
+  const int cols = columns_per_block(m->nCells, L + 1, 600, 18, 2), nb = nblocks(m->nCells, cols);
   const size_t smem = mixed ? ac_columns_mixed_smem_bytes(L, cols) : ac_columns_smem_bytes(L, cols, N, first);
   // the mixed form refuses the columns its staged solve cannot hold, on either path
   *done = smem <= kMaxSmem && !(mixed && thomas_smem_bytes(L) > kMaxSmem);
@@ -1323,7 +1310,7 @@ extern "C" int mpasg_vert_imp_coefs(const mpasg_mesh* m, const mpasg_config* c, 
   const int L = m->nVertLevels;
   const VimpScalars vs = vimp_scalars(dts, c->epssm);
   const FastDiv fl(L);
-  const int cols = columns_per_block(m->nCells, L, 400);
+  const int cols = columns_per_block(m->nCells, L, 400, 31, 6);
   const size_t smem = vimp_columns_smem_bytes(L, cols);
   const bool mixed = c->precision == MPASG_PRECISION_MIXED;
   if (smem <= kMaxSmem) {
