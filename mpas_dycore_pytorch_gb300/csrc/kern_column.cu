@@ -7,7 +7,7 @@
 // slot order, left to right, so results are deterministic and need no atomics.
 #include "common.cuh"
 #include "columns.cuh"
-#include "pow_exner.cuh"
+#include "pow_exner_fx.cuh"
 
 namespace {
 
@@ -1099,7 +1099,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
       const double rcv = kRgas / (kCp - kRgas);
       double zz = m.zz[o];
       if (sizeof(T) == sizeof(double)) {
-        double ex = mpasg_pow::pow_exner(zz * (kRgas / kP0) * (rtheta_p + rtb), rcv);
+        const double ex = mpasg_pow::pow_exner_fx(zz * (kRgas / kP0) * (rtheta_p + rtb), rcv);
         f.exner[o] = ex;
         f.pressure_p[o] = zz * kRgas * __dadd_rn(__dmul_rn(ex, rtheta_p), __dmul_rn(rtb, ex - f.exner_base[o]));
       } else {
