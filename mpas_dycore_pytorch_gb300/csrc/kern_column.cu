@@ -62,6 +62,7 @@ struct VimpScalars {
   double cg;      // 0.5 dtseps g
   double c2;      // dtseps cp R/cv
   double cm;      // mixed form: dtseps (0.5 R/cv g)
+  double cwg;     // cw g
 };
 inline VimpScalars vimp_scalars(double dts, double epssm) {
   const double rcv = kRgas / (kCp - kRgas);
@@ -71,6 +72,7 @@ inline VimpScalars vimp_scalars(double dts, double epssm) {
   p.cg = 0.5 * p.dtseps * kGravity;
   p.c2 = p.dtseps * (kCp * rcv);
   p.cm = p.dtseps * (0.5 * rcv * kGravity);
+  p.cwg = p.cw * kGravity;
   return p;
 }
 
@@ -84,7 +86,7 @@ MPASG_D VimpLevel vimp_level(const mpasg_mesh& m, const mpasg_fields& f, size_t 
   double rt = f.rtheta_p[o + k], q = f.qtot[o + k];
   const bool dry = fx::is_zero(q);  // x / (1 + q) is x itself: the division is skipped, not changed
   if (sizeof(T) == sizeof(double)) {
-    const double x = s.cw * zz * kGravity * rb;
+    const double x = (fx::is_one(zz) ? s.cwg : s.cw * zz * kGravity) * rb;
     v.cofwt = fdiv<T>((dry ? x : fdiv<T>(x, 1.0 + q)) * p, (rtb + rt) * pb);
   } else {  // constants folded into one factor
     const double x = s.cm * zz * rb;
@@ -99,31 +101,72 @@ MPASG_D VimpLevel vimp_level(const mpasg_mesh& m, const mpasg_fields& f, size_t 
 struct VimpRow {
   double a, b, c;
 };
+
+// What depends on the level alone, for a level over flat terrain (zz exactly 1 here and
+// below): the values the expressions of vimp_row round to, formed once per block.
+struct VimpFlat {
+  double rz, rz_lo, drz;  // dts (1 + epssm) / 2 rdzw at k and k-1, and their difference
+  double cofwr, cz, sum;  // cg z, c2 z rdzu, rdzw_k + rdzw_km1
+};
+MPASG_D VimpFlat vimp_flat(const mpasg_mesh& m, uint32_t k, const VimpScalars& s) {
+  VimpFlat t;
+  const double z = m.fzm[k] + m.fzp[k], rz = m.rdzw[k], rzm = m.rdzw[k - 1];
+  t.rz = s.dtseps * rz;
+  t.rz_lo = s.dtseps * rzm;
+  t.drz = t.rz - t.rz_lo;
+  t.cofwr = s.cg * z;
+  t.cz = s.c2 * z * m.rdzu[k];
+  t.sum = rz + rzm;
+  return t;
+}
+
 template <typename T>
 MPASG_D VimpRow vimp_row(const mpasg_mesh& m, const mpasg_fields& f, size_t o, size_t ow, uint32_t k,
-                         const VimpLevel& at, const VimpLevel& lo, double ct_kp1, const VimpScalars& s) {
+                         const VimpLevel& at, const VimpLevel& lo, double ct_kp1, const VimpScalars& s,
+                         const VimpFlat* flat = nullptr) {
   const double zz = m.zz[o + k], zzm = m.zz[o + k - 1];
   const double fzm = m.fzm[k], fzp = m.fzp[k];
-  const double z_i = fzm * zz + fzp * zzm;
-  const double cofwr = s.cg * z_i;
   const double p_i = fzm * f.exner[o + k] + fzp * f.exner[o + k - 1];
-  const double cofwz = s.c2 * z_i * m.rdzu[k] * f.cqw[ow + k] * p_i;
-  f.cofwr[o + k] = cofwr;
-  f.cofwz[o + k] = cofwz;
   const double ct_km1 = lo.coftz, ct_k = at.coftz;
   const double cw_k = at.cofwt, cw_km1 = lo.cofwt;
   const double rdzw_k = m.rdzw[k], rdzw_km1 = m.rdzw[k - 1];
-  const double cofrz_k = s.dtseps * rdzw_k, cofrz_km1 = s.dtseps * rdzw_km1;
   // the reference's coefficients (vert_imp_coefs.py:388-428) with their common factors taken out
   const double tm = ct_km1 * rdzw_km1, tp = ct_kp1 * rdzw_k;
   VimpRow r;
-  r.a = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
-  r.b = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
-        cofwr * (cofrz_k - cofrz_km1);
-  if (sizeof(T) == sizeof(double))
-    r.c = fma(cw_k, tp, -fma(cofwz * zz, tp, cofwr * cofrz_k));
-  else
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const bool one = flat && fx::is_one(zz) && fx::is_one(zzm);
+    VimpFlat t;
+    if (one) {
+      t = flat[k];
+    } else {
+      const double z_i = fma(fzm, zz, fzp * zzm);
+      t.rz = s.dtseps * rdzw_k;
+      t.rz_lo = s.dtseps * rdzw_km1;
+      t.drz = t.rz - t.rz_lo;
+      t.cofwr = s.cg * z_i;
+      t.cz = s.c2 * z_i * m.rdzu[k];
+      t.sum = fma(rdzw_k, zz, rdzw_km1 * zzm);
+    }
+    const double cqw = f.cqw[ow + k];
+    const double cofwz = (fx::is_one(cqw) ? t.cz : t.cz * cqw) * p_i;
+    f.cofwr[o + k] = t.cofwr;
+    f.cofwz[o + k] = cofwz;
+    const double wlo = one ? cofwz + cw_km1 : fma(cofwz, zzm, cw_km1), wk = one ? cofwz : cofwz * zz;
+    r.a = fma(t.cofwr, t.rz_lo, -(tm * wlo));
+    r.b = fma(t.cofwr, t.drz, fma(ct_k, fma(cofwz, t.sum, -fma(cw_k, rdzw_k, -(cw_km1 * rdzw_km1))), 1.0));
+    r.c = fma(cw_k, tp, -fma(wk, tp, t.cofwr * t.rz));
+  } else {
+    const double z_i = fzm * zz + fzp * zzm;
+    const double cofwr = s.cg * z_i;
+    const double cofwz = s.c2 * z_i * m.rdzu[k] * f.cqw[ow + k] * p_i;
+    f.cofwr[o + k] = cofwr;
+    f.cofwz[o + k] = cofwz;
+    const double cofrz_k = s.dtseps * rdzw_k, cofrz_km1 = s.dtseps * rdzw_km1;
+    r.a = cofwr * cofrz_km1 - tm * (cofwz * zzm + cw_km1);
+    r.b = 1.0 + ct_k * (cofwz * (rdzw_k * zz + rdzw_km1 * zzm) - (cw_k * rdzw_k - cw_km1 * rdzw_km1)) +
+          cofwr * (cofrz_k - cofrz_km1);
     r.c = tp * (cw_k - cofwz * zz) - cofwr * cofrz_k;
+  }
   return r;
 }
 
@@ -204,8 +247,11 @@ __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fie
   double* sa = s_ct + nlp;
   double* sb = sa + nlp;
   double* sc = sb + nlp;
+  VimpFlat* s_flat = reinterpret_cast<VimpFlat*>(sc + nlp);
   const uint32_t c0 = blockIdx.x * (uint32_t)cols, ncol = min((uint32_t)cols, (uint32_t)m.nCells - c0), nl = ncol * L;
   const size_t o0 = (size_t)c0 * L, ow0 = o0 + c0;
+  if (sizeof(T) == sizeof(double))
+    for (uint32_t k = 1 + threadIdx.x; k < L; k += kBlock) s_flat[k] = vimp_flat(m, k, s);
   for (uint32_t i = threadIdx.x; i < nl; i += kBlock) {
     const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
     const VimpLevel v = vimp_level<T>(m, f, o0 + col * L, k, s);
@@ -225,7 +271,7 @@ __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fie
       f.coftz[ow0 + i + col + L] = 0.0;
     } else {
       r = vimp_row<T>(m, f, o0 + col * L, ow0 + col * (L + 1), k, VimpLevel{s_cw[q], s_ct[q]},
-                      VimpLevel{s_cw[q - pitch], s_ct[q - pitch]}, k + 1 < L ? s_ct[q + pitch] : 0.0, s);
+                      VimpLevel{s_cw[q - pitch], s_ct[q - pitch]}, k + 1 < L ? s_ct[q + pitch] : 0.0, s, s_flat);
     }
     f.a_tri[o0 + i] = sa[q] = r.a;
     f.b_tri[o0 + i] = sb[q] = r.b;
@@ -245,7 +291,9 @@ __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fie
   }
 }
 
-size_t vimp_columns_smem_bytes(int L, int cols) { return (size_t)5 * L * (cols | 1) * sizeof(double); }
+size_t vimp_columns_smem_bytes(int L, int cols) {
+  return (size_t)L * (5 * (cols | 1) * sizeof(double) + sizeof(VimpFlat));
+}
 
 template <typename T>
 __global__ void k_vimp_factor(mpasg_mesh m, mpasg_fields f) {

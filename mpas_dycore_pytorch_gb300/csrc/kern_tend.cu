@@ -73,8 +73,13 @@ __global__ void k_tend_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendSca
   double hdiv = 0.0;
   for (int j = 0; j < n; ++j) {
     int e = m.edgesOnCell[c * me + j];
-    double t = m.cell_edge_sdv[c * me + j] * f.ru[(size_t)e * L + k];  // (sign * dvEdge) * ru
-    hdiv = (j == 0) ? t : hdiv + t;
+    const double ru = f.ru[(size_t)e * L + k], sdv = m.cell_edge_sdv[c * me + j];  // sign * dvEdge
+    if constexpr (sizeof(T) == sizeof(double)) {
+      hdiv = fma(sdv, ru, hdiv);
+    } else {
+      double t = sdv * ru;
+      hdiv = (j == 0) ? t : hdiv + t;
+    }
   }
   hdiv = hdiv * m.invAreaCell[c];
   f.h_divergence[i] = hdiv;
@@ -418,6 +423,9 @@ void launch_tend_u_fx(const mpasg_mesh* m, const mpasg_fields* f, const TendScal
     k_tend_u_fx<14, RAY><<<nb, kBlock, ne * (14 * sizeof(fx::Weight) + sizeof(EdgeConst)), s>>>(*m, *f, FastDiv(L), p);
 }
 
+// The del4 filter's curl and divergence of delsq_u.  In float64 the geometry is one table value a
+// slot (three operations a slot otherwise, on the pipe that bounds these kernels): 40962 x 55
+// 97 -> 43 us and 87 -> 43 us.
 template <typename T>
 __global__ void k_del4_vertex(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const int L = m.nVertLevels;
@@ -429,6 +437,12 @@ __global__ void k_del4_vertex(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const T* dc = G(dcEdge);
   const T* sg = G(edgesOnVertex_sign);
   T acc = T(0);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    for (int j = 0; j < vd; ++j)
+      acc = fma(m.vertex_edge_sdc[v * vd + j], f.delsq_u[(size_t)m.edgesOnVertex[v * vd + j] * L + k], acc);
+    f.delsq_vort[i] = iat[v] * acc;
+    return;
+  }
   for (int j = 0; j < vd; ++j) {
     int e = m.edgesOnVertex[v * vd + j];
     T es = iat[v] * dc[e] * sg[v * vd + j];
@@ -450,6 +464,12 @@ __global__ void k_del4_cell(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
   const T* dv = G(dvEdge);
   const T* sg = G(edgesOnCell_sign);
   T acc = T(0);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    for (int j = 0; j < n; ++j)
+      acc = fma(m.cell_edge_geo[c * me + j], f.delsq_u[(size_t)m.edgesOnCell[c * me + j] * L + k], acc);
+    f.delsq_div[i] = acc;
+    return;
+  }
   for (int j = 0; j < n; ++j) {
     int e = m.edgesOnCell[c * me + j];
     T es = ia[c] * dv[e] * sg[c * me + j];
@@ -462,20 +482,42 @@ __global__ void k_del4_cell(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
 // rk 1 completion of the u tendency when k_tend_u deferred it: del4 filter (if enabled),
 // then vertical mixing of u (dyn_tend.py:2730-2780; full state, interior levels, heights
 // of the edge's interfaces as the mean of its two cells), then tend_u += tend_u_euler
+// In float64 the filter's factors are formed once per block and edge: 40962 x 55 211 -> 184 us.
+struct Del4Edge {
+  double r_dc, r_dv;
+};
+
 template <typename T>
-__global__ void k_tend_u_finish(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
+__global__ void __launch_bounds__(kBlock) k_tend_u_finish(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
+  extern __shared__ Del4Edge s_d4[];
   const int L = m.nVertLevels;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (uint32_t)m.nEdges * L) return;
+  const uint32_t n_all = (uint32_t)m.nEdges * L, i0 = blockIdx.x * kBlock, e0 = fl.div(i0);
+  if (sizeof(T) == sizeof(double) && p.del4) {
+    const uint32_t ne = fl.div(min(i0 + kBlock, n_all) - 1u) - e0 + 1;
+    for (uint32_t t = threadIdx.x; t < ne; t += kBlock) {
+      const double mix = m.meshScalingDel4[e0 + t] * p.h_mom_visc4, idc = m.invDcEdge[e0 + t];
+      s_d4[t] = Del4Edge{mix * p.del4u_div * idc, mix * fmin(m.invDvEdge[e0 + t], 4.0 * idc)};
+    }
+    __syncthreads();
+  }
+  uint32_t i = i0 + threadIdx.x;
+  if (i >= n_all) return;
   uint32_t e = fl.div(i), k = i - e * L;
   const int c1 = m.cellsOnEdge[2 * e], c2 = m.cellsOnEdge[2 * e + 1];
   T teu = cv<T>(f.tend_u_euler[i]);
   if (p.del4) {
     const int v1 = m.verticesOnEdge[2 * e], v2 = m.verticesOnEdge[2 * e + 1];
-    const T inv_dc = G(invDcEdge)[e];
-    T u_mix = G(meshScalingDel4)[e] * cv<T>(p.h_mom_visc4);
-    T r_dc4 = u_mix * cv<T>(p.del4u_div) * inv_dc;
-    T r_dv4 = u_mix * vmin(G(invDvEdge)[e], T(4) * inv_dc);
+    T r_dc4, r_dv4;
+    if constexpr (sizeof(T) == sizeof(double)) {
+      const Del4Edge d = s_d4[e - e0];
+      r_dc4 = d.r_dc;
+      r_dv4 = d.r_dv;
+    } else {
+      const T inv_dc = G(invDcEdge)[e];
+      T u_mix = G(meshScalingDel4)[e] * cv<T>(p.h_mom_visc4);
+      r_dc4 = u_mix * cv<T>(p.del4u_div) * inv_dc;
+      r_dv4 = u_mix * vmin(G(invDvEdge)[e], T(4) * inv_dc);
+    }
     T u_diff4 = (cv<T>(f.delsq_div[(size_t)c2 * L + k]) - cv<T>(f.delsq_div[(size_t)c1 * L + k])) * r_dc4 -
                 (cv<T>(f.delsq_vort[(size_t)v2 * L + k]) - cv<T>(f.delsq_vort[(size_t)v1 * L + k])) * r_dv4;
     teu = teu - cv<T>(f.h_edge[i]) * u_diff4;
@@ -1145,7 +1187,8 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
       MPASG_LAUNCH_CHECK();
     }
     if (p.defer) {
-      k_tend_u_finish<T><<<nblocks(nel), kBlock, 0, s>>>(*m, *f, fl, p);
+      const size_t sd = sizeof(T) == sizeof(double) ? cellsum::max_cells(L) * sizeof(Del4Edge) : 0;
+      k_tend_u_finish<T><<<nblocks(nel), kBlock, sd, s>>>(*m, *f, fl, p);
       MPASG_LAUNCH_CHECK();
     }
   }
