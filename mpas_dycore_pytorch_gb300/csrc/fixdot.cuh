@@ -54,6 +54,12 @@ FX_HD double from_bits(uint64_t b) {
 FX_HD bool is_zero(double x) { return (bits_of(x) << 1) == 0u; }
 FX_HD bool is_one(double x) { return bits_of(x) == 0x3ff0000000000000ull; }
 FX_HD bool is_two(double x) { return bits_of(x) == 0x4000000000000000ull; }
+// x / 2
+FX_HD double half(double x) {
+  const uint64_t b = bits_of(x);
+  const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
+  return e - 2u < 2045u ? from_bits(b - ((uint64_t)1 << 52)) : 0.5 * x;  // e in [2, 2046]
+}
 FX_HD int clz64(uint64_t x) {  // x != 0
 #ifdef __CUDA_ARCH__
   return __clzll((long long)x);

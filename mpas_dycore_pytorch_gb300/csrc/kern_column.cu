@@ -330,7 +330,7 @@ MPASG_D double damped_ru_p(const mpasg_fields& f, uint32_t i, size_t i1, size_t 
 // (the second substep's: FROM_ZERO)
 template <typename T, bool DAMP, bool FROM_ZERO = false>
 __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int small_step,
-                                 double dts, double c2, double damp_coef) {
+                                 double dts, double c2, double damp_coef) {  // float64: c2 halved
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
@@ -340,10 +340,17 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
   if (small_step != 1) {
     int c1 = m.cellsOnEdge[2 * e], c2i = m.cellsOnEdge[2 * e + 1];
     size_t i1 = (size_t)c1 * L + k, i2 = (size_t)c2i * L + k;
-    T pgrad = (cv<T>(f.rtheta_pp[i2]) - cv<T>(f.rtheta_pp[i1])) * cv<T>(m.invDcEdge[e]);
+    T pgrad = cv<T>(f.rtheta_pp[i2]) - cv<T>(f.rtheta_pp[i1]);
+    if (!kDouble) pgrad = pgrad * cv<T>(m.invDcEdge[e]);
     const T z2 = cv<T>(m.zz[i2]) + cv<T>(m.zz[i1]);
     if (!is_two(z2)) pgrad = pgrad / (T(0.5) * z2);
-    pgrad = cv<T>(f.cqu_e[i]) * (T(0.5) * cv<T>(c2)) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
+    if constexpr (kDouble) {
+      const double cqu = f.cqu_e[i];
+      pgrad = pgrad * (f.exner[i1] + f.exner[i2]) * (c2 * m.invDcEdge[e]);
+      if (!fx::is_one(cqu)) pgrad = cqu * pgrad;
+    } else {
+      pgrad = cv<T>(f.cqu_e[i]) * (T(0.5) * cv<T>(c2)) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
+    }
     if (!m.flatTerrain)  // no slope: adds exact zeros
       pgrad = pgrad + T(0.5) * cv<T>(m.zxu[i]) * T(kGravity) * (cv<T>(f.rho_pp[i1]) + cv<T>(f.rho_pp[i2]));
     const double before = DAMP ? damped_ru_p<T, FROM_ZERO>(f, i, i1, i2, damp_coef) : f.ru_p[i];
@@ -405,15 +412,17 @@ MPASG_D AcLevel ac_level(const mpasg_mesh& m, const mpasg_fields& f, const fx::W
   const uint32_t L = (uint32_t)m.nVertLevels;
   const size_t g = (size_t)c * m.maxEdges;
   const int n = m.nEdgesOnCell[c];
-  double x[N], s1, s2 = 0.0;
+  const auto flux = [&](const double* __restrict__ q) {
+    double x[N], sum;
 #pragma unroll
-  for (int j = 0; j < N; ++j) x[j] = f.ru_p[(uint32_t)w[j].row * L + k];
-  for (int j = 0; j < n; ++j)
-    s2 = fma(m.cell_edge_geo[g + j], f.ke_edge[(size_t)m.edgesOnCell[g + j] * L + k], s2);
-  if (!fx::dot<N>(x, w, &s1)) {
-    s1 = 0.0;
-    for (int j = 0; j < n; ++j) s1 = fma(m.cell_edge_geo[g + j], f.ru_p[(size_t)m.edgesOnCell[g + j] * L + k], s1);
-  }
+    for (int j = 0; j < N; ++j) x[j] = q[(uint32_t)w[j].row * L + k];
+    if (!fx::dot<N>(x, w, &sum)) {
+      sum = 0.0;
+      for (int j = 0; j < n; ++j) sum = fma(m.cell_edge_geo[g + j], q[(size_t)m.edgesOnCell[g + j] * L + k], sum);
+    }
+    return sum;
+  };
+  const double s1 = flux(f.ru_p), s2 = flux(f.ke_edge);
   const size_t o = (size_t)c * L + k, ow = (size_t)c * (L + 1) + k;
   AcLevel a;
   if (FIRST) {
@@ -1218,11 +1227,12 @@ __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double
   const double rho_1 = f.rho_zz[i1], rho_2 = f.rho_zz[i2];
   const double rho2 = rho_1 + rho_2;
   // 2 ru / rho2 (the factor two is exact wherever it is applied)
-  const double u = kDouble ? fx::quotient(ru, 0.5 * rho2) : 2.0 * ru * rcp_nr1(rho2);
+  const double h = kDouble ? fx::half(rho2) : 0.0;
+  const double u = kDouble ? fx::quotient(ru, h) : 2.0 * ru * rcp_nr1(rho2);
   f.u[i] = u;
   if (!kDouble) f.u_f32[i] = d2f_bits(u);
   if (FINISH) {
-    f.h_edge[i] = kDouble ? 0.5 * rho2 : f64(T(0.5) * (cv<T>(rho_1) + cv<T>(rho_2)));
+    f.h_edge[i] = kDouble ? h : f64(T(0.5) * (cv<T>(rho_1) + cv<T>(rho_2)));
     const T u_t = cv<T>(u);
     const T dcdv = kDouble ? cv<T>(m.edge_dcdv[e]) : G(dcEdge)[e] * G(dvEdge)[e];
     fpw<T>(f.ke_edge, f.ke_edge_f32)[i] = dcdv * (u_t * u_t);
@@ -1437,15 +1447,15 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
       if (mixed && fuse.damp_before && small_step == 2)
         k_acoustic_edges<float, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
       else if (fuse.damp_before && small_step == 2)
-        k_acoustic_edges<double, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+        k_acoustic_edges<double, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, 0.5 * c2, coef);
       else if (mixed && fuse.damp_before)
         k_acoustic_edges<float, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
       else if (mixed)
         k_acoustic_edges<float, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
       else if (fuse.damp_before)
-        k_acoustic_edges<double, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+        k_acoustic_edges<double, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, 0.5 * c2, coef);
       else
-        k_acoustic_edges<double, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, c2, coef);
+        k_acoustic_edges<double, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, small_step, dts, 0.5 * c2, coef);
       MPASG_LAUNCH_CHECK();
     }
     if (part == -1) {

@@ -265,11 +265,20 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg
       ok = fx::dot<N>(x, s_k + t, &pv) && ok;
     }
 #pragma unroll
-    for (int j = 0; j < N; ++j)
-      if (j < n) {
-        kee = j == 0 ? f.ke_edge[(uint32_t)s_w[t + j].row * L + k] : kee + f.ke_edge[(uint32_t)s_w[t + j].row * L + k];
-        kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
-      }
+    for (int j = 0; j < N; ++j) {
+      x[j] = j < n ? f.ke_edge[(uint32_t)s_w[t + j].row * L + k] : 0.0;
+      if (j < n) kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
+    }
+    bool summed = false;
+    if constexpr (N <= 8) {
+      const uint32_t plus[N] = {};
+      summed = fx::sum<N>(x, plus, &kee);
+    }
+    if (!summed) {
+      kee = 0.0;
+#pragma unroll
+      for (int j = 0; j < N; ++j) kee += x[j];
+    }
     if (!ok) {
       double a, b;
       wide_cell_sums(m, f, c, k, &div, &a, &b, &pv);

@@ -115,6 +115,82 @@ __global__ void k_tend_cells_a(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendSca
   }
 }
 
+// k_tend_cells_a in float64 with the three stencil sums (mass-flux divergence, the two
+// deformations) on the integer pipes: 36 of its ~60 operations a level, of which it kept the
+// float64 pipe 87 % busy; 189 -> 152 us at 40962 x 55.
+// Block table, a cell: 6 divergence weights, then (Smagorinsky) 12 of the deformation a u - b v
+// and 12 of b u + a v.
+constexpr int kDefW = 30;
+
+template <bool CAM>
+__global__ void __launch_bounds__(kBlock, 5) k_tend_cells_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, TendScalars p) {
+  extern __shared__ fx::Weight s_w[];
+  const uint32_t L = (uint32_t)m.nVertLevels, n_all = (uint32_t)m.nCells * L;
+  const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
+  const uint32_t c0 = fl.div(i0), nc = fl.div(min(i0 + kBlock, n_all) - 1u) - c0 + 1;
+  const bool def = p.smag && p.rk_step == 1;
+  for (uint32_t t = threadIdx.x; t < nc * 6; t += kBlock) {
+    const uint32_t cl = t / 6, j = t - cl * 6, c = c0 + cl;
+    const size_t o = (size_t)c * m.maxEdges;
+    const int n = m.nEdgesOnCell[c], e = n > 0 ? m.edgesOnCell[o + ((int)j < n ? j : 0)] : 0;
+    const auto w = [&](double x) { return (int)j < n ? fx::weight(x, e) : fx::Weight{0, 0, 0u, e}; };
+    const size_t q = (int)j < n ? o + j : o;
+    fx::Weight* tab = s_w + cl * kDefW + j;
+    tab[0] = w(m.cell_edge_sdv[q]);
+    if (def) {
+      const double a = m.defc_a[q], b = m.defc_b[q];
+      tab[6] = w(a);
+      tab[12] = w(-b);
+      tab[18] = w(b);
+      tab[24] = w(a);
+    }
+  }
+  __syncthreads();
+  if (i >= n_all) return;
+  const uint32_t c = fl.div(i), k = i - c * L;
+  const fx::Weight* w = s_w + (c - c0) * kDefW;
+  const size_t o = (size_t)c * m.maxEdges;
+  const int n = m.nEdgesOnCell[c];
+  double ru[6], hdiv;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) ru[j] = f.ru[(uint32_t)w[j].row * L + k];
+  if (!fx::dot<6>(ru, w, &hdiv)) {
+    hdiv = 0.0;
+    for (int j = 0; j < n; ++j) hdiv = fma(m.cell_edge_sdv[o + j], f.ru[(size_t)m.edgesOnCell[o + j] * L + k], hdiv);
+  }
+  hdiv = hdiv * m.invAreaCell[c];
+  f.h_divergence[i] = hdiv;
+  if (p.rk_step != 1) return;
+  const size_t ow = (size_t)c * (L + 1) + k;
+  f.tend_rho[i] = -hdiv - m.rdzw[k] * (f.rw[ow + 1] - f.rw[ow]);
+  const double q = f.qtot[i];
+  f.dpdz[i] = -kGravity * (m.rho_base[i] * q + f.rr_save[i] * (1.0 + q));
+  double kd = p.visc2;  // 2d_fixed: the theta del2 coefficient everywhere
+  if (p.smag) {
+    double x[12];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      const uint32_t e = (uint32_t)w[j].row * L + k;
+      x[j] = f.u[e];
+      x[6 + j] = f.v[e];
+    }
+    double dd, dof;
+    const bool ok = fx::dot<12>(x, w + 6, &dd);
+    if (!(fx::dot<12>(x, w + 18, &dof) && ok)) {
+      dd = dof = 0.0;
+      for (int j = 0; j < n; ++j) {
+        const size_t e = (size_t)m.edgesOnCell[o + j] * L + k;
+        const double a = m.defc_a[o + j], b = m.defc_b[o + j];
+        dd = fma(-b, f.v[e], fma(a, f.u[e], dd));
+        dof = fma(a, f.v[e], fma(b, f.u[e], dof));
+      }
+    }
+    kd = fx::min_nonneg(p.c_s_len2 * sqrt(dd * dd + dof * dof), p.kdiff_cap);
+  }
+  if (CAM && (int)k >= (int)L - p.ncam) kd = cam_kdiff(kd, p, k, (int)L);
+  f.kdiff[i] = kd;
+}
+
 // Rayleigh damping of u on the top ray_n levels (dyn_tend.py:2956-2990), every RK stage:
 // tend_u - rho_edge u ((k + 1) - k0) / (ray_n timescale), k0 = L - ray_n
 template <typename T>
@@ -983,7 +1059,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_tend_w_theta(mpasg_mesh m, mpasg_
   }
   if (k < L) {
     const size_t o = oc + k;
-    double tt = fma(-ia, cellsum::f64<N>(m, c, n, s, f.flux_th_e, L, k), m.rdzw[k] * (wt_k - wt_k1));
+    double tt = fma(-ia, cellsum::fixed<N>(m, c, n, s, f.flux_th_e, L, k), m.rdzw[k] * (wt_k - wt_k1));
     const double rz = f.rho_zz[o];
     // unfused: the difference cancels strongly (as rounded by the reference)
     f.rthdynten[o] = fx::quotient(sub_rn(tt, mul_rn(f.tend_rho[o], f.theta_m[o])), rz);
@@ -1152,10 +1228,16 @@ int launch_dyn_tend(const mpasg_mesh* m, mpasg_fields* f, const TendScalars& p, 
   const long long ncw = (long long)m->nCells * (L + 1), nvl = (long long)m->nVertices * L;
   FastDiv fl(L), fl1(L + 1);
   if (rk_step == 1 || !hdiv_current) {
-    if (p.ncam > 0 && rk_step == 1)
+    const bool cam = p.ncam > 0 && rk_step == 1;
+    if (sizeof(T) == sizeof(double) && m->maxEdges <= 6) {
+      const size_t sd = cellsum::max_cells(L) * kDefW * sizeof(fx::Weight);
+      if (cam) k_tend_cells_fx<true><<<nblocks(ncl), kBlock, sd, s>>>(*m, *f, fl, p);
+      else k_tend_cells_fx<false><<<nblocks(ncl), kBlock, sd, s>>>(*m, *f, fl, p);
+    } else if (cam) {
       k_tend_cells_a<T, true><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
-    else
+    } else {
       k_tend_cells_a<T><<<nblocks(ncl), kBlock, 0, s>>>(*m, *f, fl, p);
+    }
     MPASG_LAUNCH_CHECK();
   }
   GraphBranches branches(s);  // u beside w and theta
