@@ -336,8 +336,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_edges_b_fx(mpasg_mesh m, mpa
   if (apvm) {
     const size_t c1 = (size_t)m.cellsOnEdge[2 * e], c2 = (size_t)m.cellsOnEdge[2 * e + 1];
     const ApvmEdge a = s_a[e - e0];
-    const double delta = fma(u, (f.pv_cell[c2 * L + k] - f.pv_cell[c1 * L + k]) * a.gn, vv * ((pv2 - pv1) * a.gt));
-    pve = fma(0.5, pv1 + pv2, -delta);
+    // (pv1 + pv2) / 2 - vv gt (pv2 - pv1) - u gn (pvc2 - pvc1)
+    pve = fma(pv2 - pv1, fma(-vv, a.gt, 0.5), pv1);
+    pve = fma(-(u * a.gn), f.pv_cell[c2 * L + k] - f.pv_cell[c1 * L + k], pve);
   } else {
     pve = 0.5 * (pv1 + pv2);
   }

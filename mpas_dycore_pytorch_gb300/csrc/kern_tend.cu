@@ -400,14 +400,17 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
 // N: slots a thread sums (unused slots hold zero weights); an edge with more than N
 // neighbours, and a sum the fixed-point format refuses, are summed in float64.
 
-// 12 times the vertical flux of u at interface kk; rw2 = rw1 + rw2 of the edge's two cells
+// 12 times the vertical flux of u at interface kk; rw2 = rw1 + rw2 of the edge's two cells.  The
+// second-order interfaces 1 and L-1 take the same instructions with other coefficients: as a
+// branch of their own they cost nearly every warp its operations again.
 MPASG_D double wduz12_at(const double* __restrict__ u, double rw2, int kk, int L, const double* fzm,
                          const double* fzp) {
   if (kk <= 0 || kk >= L) return 0.0;
-  if (kk == 1 || kk == L - 1) return rw2 * (6.0 * (fzm[kk] * u[kk] + fzp[kk] * u[kk - 1]));
-  const bool down = __double2hiint(rw2) < 0;
-  const double a = u[down ? kk - 1 : kk], b = u[down ? kk : kk - 1], c = u[down ? kk + 1 : kk - 2];
-  return rw2 * fma(2.0, a, fma(5.0, b, -c));
+  const bool low = kk == 1 || kk == L - 1, down = !low && __double2hiint(rw2) < 0;
+  const double a = u[down || low ? kk - 1 : kk], b = u[down || low ? kk : kk - 1];
+  const double c = low ? 0.0 : u[down ? kk + 1 : kk - 2];
+  const double f = fma(low ? fzp[kk] : 2.0, a, fma(low ? fzm[kk] : 5.0, b, -c));
+  return (low ? 6.0 * rw2 : rw2) * f;
 }
 
 // Per-edge constants of the u tendency, formed once per block and edge
@@ -967,32 +970,28 @@ __global__ void __launch_bounds__(kBlock, 6) k_adv_edges_fx(mpasg_mesh m, mpasg_
 // Vertical fluxes of the float64 form at interface kk, the upwind combination of flux3 taken
 // out (as in wduz12_at): of w (coefficient 1, times 12) and of theta (coefficient c,
 //   12 flux = rw ((7 + 3c) a + (7 - 3c) b - (1 + c) a' - (1 - c) b'),  a upwind, a' behind it)
+// (the second-order interfaces: the same instructions with other coefficients, as above)
 MPASG_D double wdwz12_at(const double* __restrict__ w, const double* __restrict__ rw, int kk, int L) {
   if (kk <= 0 || kk >= L) return 0.0;
   const double rw2 = rw[kk] + rw[kk - 1];
-  if (kk == 1 || kk == L - 1) return rw2 * (3.0 * (w[kk] + w[kk - 1]));
-  const bool down = __double2hiint(rw2) < 0;
-  const double a = w[down ? kk - 1 : kk], b = w[down ? kk : kk - 1], c = w[down ? kk + 1 : kk - 2];
-  return rw2 * fma(2.0, a, fma(5.0, b, -c));
+  const bool low = kk == 1 || kk == L - 1, down = __double2hiint(rw2) < 0;
+  const double a = w[down ? kk - 1 : kk], b = w[down ? kk : kk - 1];
+  const double c = low ? 0.0 : w[down ? kk + 1 : kk - 2];
+  return rw2 * fma(low ? 3.0 : 2.0, a, fma(low ? 3.0 : 5.0, b, -c));
 }
 
 MPASG_D double wdtz_fx_at(const double* __restrict__ th, const double* __restrict__ ths,
                           const double* __restrict__ rw, const double* __restrict__ rws, int kk, int L,
                           const double* fzm, const double* fzp, const TendScalars& p) {
   if (kk <= 0 || kk >= L) return 0.0;
-  const double fm = fzm[kk], fp = fzp[kk];
-  if (kk == L - 1 && kk != 1) return rws[kk] * (fm * th[kk] + fp * th[kk - 1]);
-  const double r = rw[kk];
-  double v;
-  if (kk == 1) {
-    v = r * (fm * th[kk] + fp * th[kk - 1]);
-  } else {
-    const bool down = __double2hiint(r) < 0;
-    const double a = th[down ? kk : kk - 1], b = th[down ? kk - 1 : kk];
-    const double a2 = th[down ? kk + 1 : kk - 2], b2 = th[down ? kk - 2 : kk + 1];
-    v = (r * kInv12) * fma(p.f3[0], a, fma(p.f3[1], b, -fma(p.f3[2], a2, p.f3[3] * b2)));
-  }
-  return fma(rws[kk] - r, fm * ths[kk] + fp * ths[kk - 1], v);
+  const double fm = fzm[kk], fp = fzp[kk], r = rw[kk], rs = rws[kk];
+  const bool top = kk == L - 1 && kk != 1, low = top || kk == 1;  // top: of theta_m by rw_save alone
+  const bool down = low || __double2hiint(r) < 0;
+  const double a = th[down ? kk : kk - 1], b = th[down ? kk - 1 : kk];
+  const double a2 = low ? 0.0 : th[down ? kk + 1 : kk - 2], b2 = low ? 0.0 : th[down ? kk - 2 : kk + 1];
+  const double v = fma(low ? fm : p.f3[0], a, fma(low ? fp : p.f3[1], b, -fma(p.f3[2], a2, p.f3[3] * b2)));
+  const double r12 = r * kInv12, dr = rs - r;
+  return fma(top ? 0.0 : dr, fma(fm, ths[kk], fp * ths[kk - 1]), (top ? rs : low ? r : r12) * v);
 }
 
 // w and theta tendencies (float64 form); index space (C, L+1).  Bound by the float64 pipe: 89
