@@ -142,15 +142,14 @@ MPASG_D CellRow cell_row(uint32_t i, uint32_t row, const FastDiv& fr, const Fast
 // factor 1 or 1/12 that goes with it
 MPASG_D double interface_value(const double* __restrict__ q, uint32_t S, double ww, uint32_t k, uint32_t L,
                                const double* fnm, const double* fnp, const double* f3, double* factor) {
-  if (k == 1 || k == L - 1) {
-    *factor = 1.0;
-    return fma(fnm[k], q[0], fnp[k] * q[-(int)S]);
-  }
-  *factor = kInv12;
-  const bool down = __double2hiint(ww) < 0;
+  // (the second-order interfaces: the same instructions with other coefficients, a branch of
+  // theirs would cost nearly every warp its operations again)
+  const bool low = k == 1 || k == L - 1, down = low || __double2hiint(ww) < 0;
   const int s = (int)S;
-  const double a = q[down ? 0 : -s], b = q[down ? -s : 0], a2 = q[down ? s : -2 * s], b2 = q[down ? -2 * s : s];
-  return fma(f3[0], a, fma(f3[1], b, -fma(f3[2], a2, f3[3] * b2)));
+  const double a = q[down ? 0 : -s], b = q[down ? -s : 0];
+  const double a2 = low ? 0.0 : q[down ? s : -2 * s], b2 = low ? 0.0 : q[down ? -2 * s : s];
+  *factor = low ? 1.0 : kInv12;
+  return fma(low ? fnm[k] : f3[0], a, fma(low ? fnp[k] : f3[1], b, -fma(f3[2], a2, f3[3] * b2)));
 }
 
 // explicit stage update: 17 float64 operations a value and one integer sum, about 33 in the
