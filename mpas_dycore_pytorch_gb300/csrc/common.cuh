@@ -211,8 +211,16 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
 // recovery with the last acoustic substep's divergence damping (step dts) before it and the
 // diagnostics' edge fields after it; part 0: cells, 1: edges, 2: w over terrain (after both);
 // rho_p and rho_zz before them, by the last substep (AcousticFusion::last) or as part 3
+// What a dynamics substep's last RK stage leaves besides, in the recovery's own passes: the sums
+// of the substeps' mean fluxes and the saves of the next substep.
+struct RecoverTail {
+  enum Sum { kNone, kFirst, kNext } sum = kNone;
+  double scale = 0.0;  // last substep: the fluxes become scale times their sum
+  bool saves = false;
+};
 int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
-                          double rk_dt, double dts, cudaStream_t s, int part);
+                          double rk_dt, double dts, cudaStream_t s, int part,
+                          const RecoverTail& tail = RecoverTail());
 
 // Number of kernels this library has launched (for launch accounting by callers).
 extern "C" long long mpasg_launch_count(void);

@@ -12,28 +12,24 @@
 
 namespace {
 
-// Elementwise work on up to ten arrays in one launch (blockIdx.y selects the array): the saves
-// and the flux sums at a substep's ends.  One launch instead of ten copies: on the small meshes
+// Copies of up to ten arrays in one launch (blockIdx.y selects the array): the saves at the start
+// of a step.  One launch instead of ten copies: on the small meshes
 // each of them cost a graph node of 1.5 to 2 us.
 struct ArrayJob {
   static constexpr int kMax = 10;
-  enum Op { kCopy, kAdd, kScale };
   const double* src[kMax];
   double* dst[kMax];
   double* dst2[kMax];     // second destination of a copy, or null
   long long n[kMax];
-  long long zero_from[kMax];  // kCopy: values from this index on are zero, in src too
-  int op[kMax];
-  double scale;
+  long long zero_from[kMax];  // values from this index on are zero, in src too
   int count = 0;
   long long longest = 0;
-  void push(Op o, double* d, const double* s, long long len, double* d2 = nullptr, long long zero = -1) {
+  void push(double* d, const double* s, long long len, double* d2 = nullptr, long long zero = -1) {
     src[count] = s;
     dst[count] = d;
     dst2[count] = d2;
     n[count] = len;
     zero_from[count] = zero < 0 ? len : zero;
-    op[count] = o;
     ++count;
     longest = len > longest ? len : longest;
   }
@@ -46,15 +42,9 @@ __global__ void k_arrays(const __grid_constant__ ArrayJob job) {
   double* dst = job.dst[a];
   double* dst2 = job.dst2[a];
   const long long zero = job.zero_from[a];
-  const int op = job.op[a];
-  const double scale = job.scale;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
     double x = src[i];
-    if (op == ArrayJob::kAdd) {
-      x = dst[i] + x;
-    } else if (op == ArrayJob::kScale) {
-      x = x * scale;
-    } else if (i >= zero) {
+    if (i >= zero) {
       x = 0.0;
       const_cast<double*>(src)[i] = 0.0;
     }
@@ -365,19 +355,17 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
 
   // ---- RK integration setup
   MARK(MPASG_STAGE_BEGIN);
-  // the time-level saves of a dynamics substep (theta_m's padding row is zeroed)
-  auto push_saves = [&](ArrayJob& job) {
-    job.push(ArrayJob::kCopy, f.ru_save, f.ru, nel);
-    job.push(ArrayJob::kCopy, f.rw_save, f.rw, ncw);
-    job.push(ArrayJob::kCopy, f.rtheta_p_save, f.rtheta_p, ncl);
-    job.push(ArrayJob::kCopy, f.rho_p_save, f.rho_p, ncl, f.rr_save);
-    job.push(ArrayJob::kCopy, f.theta_m_save, f.theta_m, ncl, nullptr, nc * L);
-  };
+  // the time-level saves of the first dynamics substep (theta_m's padding row is zeroed); the
+  // recovery leaves the later ones' (RecoverTail)
   {
     ArrayJob job;
-    push_saves(job);
-    job.push(ArrayJob::kCopy, f.rho_zz_old_split, f.rho_zz, ncl);
-    if (S > 0) job.push(ArrayJob::kCopy, f.scalars_init, f.scalars, ncs, advect && coupled ? f.scalars_a : nullptr);
+    job.push(f.ru_save, f.ru, nel);
+    job.push(f.rw_save, f.rw, ncw);
+    job.push(f.rtheta_p_save, f.rtheta_p, ncl);
+    job.push(f.rho_p_save, f.rho_p, ncl, f.rr_save);
+    job.push(f.theta_m_save, f.theta_m, ncl, nullptr, nc * L);
+    job.push(f.rho_zz_old_split, f.rho_zz, ncl);
+    if (S > 0) job.push(f.scalars_init, f.scalars, ncs, advect && coupled ? f.scalars_a : nullptr);
     CHECK_RC(run_arrays(job, s));
   }
   GraphBranches setup(s);
@@ -421,8 +409,14 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
         MARK(MPASG_STAGE_ACOUSTIC);
       }
       // with the last substep's divergence damping and the diagnostics' edge fields
+      RecoverTail tail;
+      if (rk == 3) {
+        tail.sum = sub == 1 ? RecoverTail::kFirst : RecoverTail::kNext;
+        tail.scale = sub == split ? 1.0 / (double)split : 0.0;
+        tail.saves = sub < split;
+      }
       auto recover = [&](int part) {
-        return mpasgi_recover_finish(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], dts, s, part);
+        return mpasgi_recover_finish(m, c, &f, rk, nsub[rk - 1], rk_ts[rk - 1], dts, s, part, tail);
       };
       // the cells' recovery beside the edges' and the diagnostics, which read only the edges;
       // over terrain w needs both, and so does the coupled transport
@@ -453,23 +447,9 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
       CHECK_RC(cells.join());
       MARK(MPASG_STAGE_DIAG);
     }
-    // split bookkeeping: the substeps' mass fluxes summed, the saves of the next substep
-    ArrayJob job;
-    const ArrayJob::Op op = sub == 1 ? ArrayJob::kCopy : ArrayJob::kAdd;
-    job.push(op, f.ruAvg_split, f.ruAvg, nel);
-    job.push(op, f.wwAvg_split, f.wwAvg, ncw);
-    if (sub < split) push_saves(job);
-    CHECK_RC(run_arrays(job, s));
     if (sub < split) CHECK_RC(mpasgi_theta_edge(m, &f, c->precision == MPASG_PRECISION_MIXED, s));
   }
   MARK(MPASG_STAGE_SPLIT);
-  {
-    ArrayJob job;
-    job.scale = 1.0 / (double)split;
-    job.push(ArrayJob::kScale, f.ruAvg, f.ruAvg_split, nel);
-    job.push(ArrayJob::kScale, f.wwAvg, f.wwAvg_split, ncw);
-    CHECK_RC(run_arrays(job, s));
-  }
   // coupled mode: the scalars of the last RK stage are the step's (active rows only)
   if (advect && coupled) CHECK_RC(copy(f.scalars, f.scalars_a, nc * L * S, s));
   MARK(MPASG_STAGE_SPLIT);

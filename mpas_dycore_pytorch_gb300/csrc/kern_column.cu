@@ -1113,6 +1113,14 @@ MPASG_D double pow1p_rcv_m1(double x) {
   return p * x;
 }
 
+// a mean flux and the sum of the substeps' (RecoverTail)
+MPASG_D double tail_flux(const RecoverTail& t, double* sum, double v) {
+  if (t.sum == RecoverTail::kNone) return v;
+  const double all = t.sum == RecoverTail::kNext ? *sum + v : v;
+  *sum = all;
+  return t.scale != 0.0 ? t.scale * all : v;
+}
+
 // Float64 in both forms; T selects the division (exact / Newton reciprocal) and, at
 // rk 3, the Exner function: pow in the float64 form; in the mixed form the identity
 // exner = exner_base (1 + x)^(R/cv), x = rtheta_p / rtheta_base, with the increment
@@ -1123,7 +1131,7 @@ MPASG_D double pow1p_rcv_m1(double x) {
 // thread (shared memory) -- the same expressions k_recover_w evaluates, one launch fewer.
 template <typename T, bool FLAT = false>
 __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fields f, FastDiv fl1, int rk_step,
-                                                          double inv_ns, double rk_dt, bool rho_done) {
+                                                          double inv_ns, double rk_dt, bool rho_done, RecoverTail tail) {
   __shared__ double s_rho[FLAT ? kBlock : 1];
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1151,7 +1159,14 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
       rtheta_p = f.rtheta_p_save[o] + f.rtheta_pp[o];
     double rtb = f.rtheta_base[o];
     f.rtheta_p[o] = rtheta_p;
-    f.theta_m[o] = sizeof(T) == sizeof(double) ? fx::quotient(rtheta_p + rtb, rho_zz) : (rtheta_p + rtb) * rcp_nr1(rho_zz);
+    const double theta =
+        sizeof(T) == sizeof(double) ? fx::quotient(rtheta_p + rtb, rho_zz) : (rtheta_p + rtb) * rcp_nr1(rho_zz);
+    f.theta_m[o] = theta;
+    if (tail.saves) {
+      f.rtheta_p_save[o] = rtheta_p;
+      f.theta_m_save[o] = theta;
+      f.rr_save[o] = f.rho_p_save[o] = f.rho_p[o];
+    }
     if (rk_step == 3) {
       const double rcv = kRgas / (kCp - kRgas);
       double zz = m.zz[o];
@@ -1178,9 +1193,10 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
   if (k >= 1 && k < (uint32_t)L) {
     size_t ow = (size_t)c * (L + 1) + k;
     double rws = f.rw_save[ow];
-    f.wwAvg[ow] = rws + f.wwAvg[ow] * inv_ns;
+    f.wwAvg[ow] = tail_flux(tail, f.wwAvg_split + ow, rws + f.wwAvg[ow] * inv_ns);
     double rw = rws + f.rw_p[ow];
     f.rw[ow] = rw;
+    if (tail.saves) f.rw_save[ow] = rw;
     if (sizeof(T) != sizeof(double)) f.rw_f32[ow] = d2f_bits(rw);
     size_t oc = (size_t)c * L;
     const double den = m.fzm[k] * m.zz[oc + k] + m.fzp[k] * m.zz[oc + k - 1];
@@ -1196,17 +1212,22 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
       f.w[ow] = wk;
       if (sizeof(T) != sizeof(double)) f.w_f32[ow] = d2f_bits(wk);
     }
-  } else if (FLAT) {  // bottom and top interfaces: no slope flux, w = 0
+  } else {  // bottom and top interfaces
     const size_t ow = (size_t)c * (L + 1) + k;
-    f.w[ow] = 0.0;
-    if (sizeof(T) != sizeof(double)) f.w_f32[ow] = 0.0f;
+    if (tail.sum != RecoverTail::kNone) f.wwAvg[ow] = tail_flux(tail, f.wwAvg_split + ow, f.wwAvg[ow]);
+    if (FLAT) {  // no slope flux, w = 0
+      f.w[ow] = 0.0;
+      if (sizeof(T) != sizeof(double)) f.w_f32[ow] = 0.0f;
+    }
   }
 }
 
 // FINISH: with the last acoustic substep's divergence damping before it and the diagnostics'
-// edge fields (k_diag_edges_a) after it: one pass over the edges instead of three
+// edge fields (k_diag_edges_a) after it: one pass over the edges instead of three.  Bound by the
+// float64 pipe (80 %, 11 operations an edge level; 168 us at 40962 x 55).
 template <typename T, bool FINISH, bool FROM_ZERO>
-__global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns, double damp_coef) {
+__global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns, double damp_coef,
+                                RecoverTail tail) {
   const int L = m.nVertLevels;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (uint32_t)m.nEdges * L) return;
@@ -1214,7 +1235,7 @@ __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double
   constexpr bool kDouble = sizeof(T) == sizeof(double);
   const size_t i1 = (size_t)m.cellsOnEdge[2 * e] * L + k, i2 = (size_t)m.cellsOnEdge[2 * e + 1] * L + k;
   double rus = f.ru_save[i];
-  f.ruAvg[i] = rus + f.ruAvg[i] * inv_ns;
+  f.ruAvg[i] = tail_flux(tail, f.ruAvg_split + i, rus + f.ruAvg[i] * inv_ns);
   double rup;
   if (FINISH) {
     rup = damped_ru_p<T, FROM_ZERO>(f, i, i1, i2, damp_coef);
@@ -1224,6 +1245,7 @@ __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double
   }
   double ru = rus + rup;
   f.ru[i] = ru;
+  if (tail.saves) f.ru_save[i] = ru;
   const double rho_1 = f.rho_zz[i1], rho_2 = f.rho_zz[i2];
   const double rho2 = rho_1 + rho_2;
   // 2 ru / rho2 (the factor two is exact wherever it is applied)
@@ -1293,17 +1315,17 @@ __global__ void k_recover_w(mpasg_mesh m, mpasg_fields f, FastDiv fl1) {
 // part 0: cells, 1: edges, 2: w over terrain, 3: rho alone
 template <typename T>
 int launch_recover(const mpasg_mesh* m, mpasg_fields* f, int rk_step, double inv_ns, double rk_dt, cudaStream_t s,
-                   bool finish, double damp_coef, bool one_substep, int part) {
+                   bool finish, double damp_coef, bool one_substep, int part, const RecoverTail& tail) {
   const int L = m->nVertLevels;
   const int nw = nblocks((long long)m->nCells * (L + 1)), ne = nblocks((long long)m->nEdges * L);
   const FastDiv fl(L), fl1(L + 1);
   if (part == 0) {
-    if (m->flatTerrain) k_recover_cells<T, true><<<nw, kBlock, 0, s>>>(*m, *f, fl1, rk_step, inv_ns, rk_dt, finish);
-    else k_recover_cells<T><<<nw, kBlock, 0, s>>>(*m, *f, fl1, rk_step, inv_ns, rk_dt, finish);
+    if (m->flatTerrain) k_recover_cells<T, true><<<nw, kBlock, 0, s>>>(*m, *f, fl1, rk_step, inv_ns, rk_dt, finish, tail);
+    else k_recover_cells<T><<<nw, kBlock, 0, s>>>(*m, *f, fl1, rk_step, inv_ns, rk_dt, finish, tail);
   } else if (part == 1) {
-    if (finish && one_substep) k_recover_edges<T, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef);
-    else if (finish) k_recover_edges<T, true, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef);
-    else k_recover_edges<T, false, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, 0.0);
+    if (finish && one_substep) k_recover_edges<T, true, true><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef, tail);
+    else if (finish) k_recover_edges<T, true, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, damp_coef, tail);
+    else k_recover_edges<T, false, false><<<ne, kBlock, 0, s>>>(*m, *f, fl, inv_ns, 0.0, tail);
   } else if (part == 3) {
     k_recover_rho<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, (uint32_t)m->nCells * L);
   } else if (!m->flatTerrain) {  // slope fluxes need the new ru of k_recover_edges
@@ -1549,12 +1571,12 @@ extern "C" int mpasg_smlstep_pert(const mpasg_mesh* m, const mpasg_config* c, mp
 
 namespace {
 int recover(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns, double rk_dt,
-            cudaStream_t s, bool finish, double damp_coef, int part) {
+            cudaStream_t s, bool finish, double damp_coef, int part, const RecoverTail& tail = RecoverTail()) {
   if (!m || !c || !f || ns < 1) return MPASG_E_ARG;
   const double inv_ns = 1.0 / (double)ns;
   if (c->precision == MPASG_PRECISION_MIXED)
-    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1, part);
-  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1, part);
+    return launch_recover<float>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1, part, tail);
+  return launch_recover<double>(m, f, rk_step, inv_ns, rk_dt, s, finish, damp_coef, ns == 1, part, tail);
 }
 }  // namespace
 
@@ -1567,6 +1589,6 @@ extern "C" int mpasg_recover_large_step(const mpasg_mesh* m, const mpasg_config*
 }
 
 int mpasgi_recover_finish(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, int ns,
-                          double rk_dt, double dts, cudaStream_t s, int part) {
-  return recover(m, c, f, rk_step, ns, rk_dt, s, true, c ? damping_coefficient(c, dts) : 0.0, part);
+                          double rk_dt, double dts, cudaStream_t s, int part, const RecoverTail& tail) {
+  return recover(m, c, f, rk_step, ns, rk_dt, s, true, c ? damping_coefficient(c, dts) : 0.0, part, tail);
 }
