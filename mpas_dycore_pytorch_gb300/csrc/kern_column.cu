@@ -398,10 +398,10 @@ __global__ void k_theta_edge(mpasg_mesh m, mpasg_fields f, FastDiv fl) {
 //   ts = rtheta_pp + dts (tend_theta - S2) - resm rdzw d(coftz rw_p),  P = ts + resm rtheta_pp
 //   x  = rw_p + dts tend_rw - cofwz (zz_k P_k - zz_km1 P_km1) - cofwr (R_k + R_km1)
 //        + cofwt_k P_k + cofwt_km1 P_km1
-// Bound by the float64 pipe (63 operations a level, 268 us at 40962 x 55).  S1 is formed on
-// the integer pipes (fixdot.cuh), S2 over products formed once per edge, and the first
-// substep, whose perturbations are all zero, has its own instance: 28 operations a level (145
-// us), 17 in the first substep (105 us).
+// Bound by the float64 pipe (63 operations a level, 268 us at 40962 x 55).  S1, and S2 over
+// products formed once per edge, are formed on the integer pipes (fixdot.cuh), and the first
+// substep, whose perturbations are all zero, has its own instance: 22 operations a level, 11 in
+// the first substep.
 struct AcLevel {
   double rs, ts, R, P;
 };
@@ -864,7 +864,8 @@ __global__ void __launch_bounds__(kBlock) k_ac_post(mpasg_mesh m, mpasg_fields f
 // start and leave the chip idle in the sweeps (one lane a column, ~190 clocks a level); here
 // the sweeps run beside other blocks' level work.  Step of 162 columns x 12 levels 744 -> 666
 // us, 2562 x 26 1443 -> 1353, 10242 x 33 4530 -> 4314, 40962 x 55 25.81 -> 25.49 ms; acoustic
-// stage at 40962 x 55 1505 -> 1440 us.  Bound by the float64 pipe on a large mesh, by the
+// stage at 40962 x 55 1505 -> 1440 us (1391 with S2 on the integer pipes; 215-227 us a first
+// substep, 261 a later one).  Bound by the float64 pipe on a large mesh, by the
 // chain of its phases on a small one.
 // keep: leave rs, ts and the undamped solution in ac_rs, ac_ts, ac_x (the reverse mode).
 // last: rho_p and rho_zz too, so that the recovery of u need not wait for that of the cells.
@@ -1224,7 +1225,8 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
 
 // FINISH: with the last acoustic substep's divergence damping before it and the diagnostics'
 // edge fields (k_diag_edges_a) after it: one pass over the edges instead of three.  Bound by the
-// float64 pipe (80 %, 11 operations an edge level; 168 us at 40962 x 55).
+// float64 pipe (80 %, 11 operations an edge level; 168 us at 40962 x 55, 233 with the saves and
+// flux sums of a substep's end).
 template <typename T, bool FINISH, bool FROM_ZERO>
 __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns, double damp_coef,
                                 RecoverTail tail) {

@@ -182,9 +182,9 @@ __global__ void __launch_bounds__(kBlock) k_diag_vertices_fx(mpasg_mesh m, mpasg
 }
 
 // k_diag_cells in float64 took 52 operations a level (217 us at 40962 x 55), most of them the
-// per-slot products of the vertex blend.  The area factors are taken out of the sums, the
-// divergence and the PV sum run on the integer pipes (fixdot.cuh), the kinetic energies on
-// the float64 pipe: 17 operations a level.
+// per-slot products of the vertex blend.  The area factors are taken out of the sums; all but
+// the vertices' kinetic energy run on the integer pipes (fixdot.cuh): 11 operations a level,
+// 97-118 us.
 // Block tables: per cell N divergence weights sign dvEdge (row: edge), then N kite weights
 // (row: vertex), then the kite areas as float64.
 template <int N>
@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg
   if (apvm) f.pv_cell[i] = pv * ia;
 }
 
-// k_diag_edges_b in float64 (165 us, mean of a step's launches): the APVM factors are formed
-// once per block and edge, the tangential wind (rk 3 and preparation) on the integer pipes;
+// k_diag_edges_b in float64 (165 us at 40962 x 55, mean of a step's launches; 113 here, 203 with
+// the tangential wind): the APVM factors are formed once per block and edge, the tangential wind (rk 3 and preparation) on the integer pipes;
 // pv_edge * u, which the next u tendency reads, is left in ke_edge.
 struct ApvmEdge {
   double gt, gn;  // apvm_dt / dv, apvm_dt / dc

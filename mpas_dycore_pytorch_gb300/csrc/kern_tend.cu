@@ -11,9 +11,9 @@
 //   k_tend_w_theta   w and theta flux divergence, vertical fluxes, buoyancy,
 //                    diabatic term                                                :10386, :10679
 //
-// Every kernel is a template on the stencil arithmetic type T (common.cuh): double for
-// the float64 form, whose slot sums follow the reference's order (first slot assigned,
-// then left to right); float for the mixed form, which reads the float32 copies of the
+// Kernels are templates on the stencil arithmetic type T (common.cuh), double for the float64
+// form, or have a float64 version of their own (_fx, k_mix_edges_* and k_mix_cells), whose
+// stencil sums run in fixed point on the integer pipes; float for the mixed form, which reads the float32 copies of the
 // geometry and of u, w, rw, pv_edge (fp<T> / G) and float64 fields through cv<T>.
 #include <cmath>
 
@@ -388,10 +388,11 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
 // The PV flux sums of k_tend_u on the integer pipes (fixdot.cuh): sum_j w_j u_j and
 // sum_j w_j (pv u)_j over the TRiSK stencil were 20 of the ~44 float64 operations an edge level
 // issued on the pipe that bounded the kernel (82 % active, 14 % of the issue slots used).
-// 40962 x 55, a later RK stage: 628 us in float64, 359 us here (both sums on the integer
-// side; one of them in float64: 382 us), the first stage 970 -> 489 us.  48 registers (5 blocks
-// an SM): 346 us in a tuning loop against 593 us at 80 registers, 362 at 64 and 361 at 40, the
-// latency of 22 warps an SM being what held the 80-register build.
+// 40962 x 55, a later RK stage: 628 us in float64, 378 us here with the first acoustic edge
+// update (one of the sums in float64: 23 us more), the first stage 970 -> 434 us.  48 registers
+// (5 blocks an SM): 346 us in a tuning loop against 593 us at 80 registers, 362 at 64 and 361 at
+// 40, the latency of 22 warps an SM being what held the 80-register build.  The float64 pipe
+// is now 66 % busy with ~21 operations an edge level, the issue slots 39 %.
 // The block converts the weights of the 5-7 edges it covers once, into shared memory
 // (with the neighbour rows), so a term costs its thread one 16-byte broadcast and one gather.
 // The upwind combination of flux3 with coefficient 1 is a three-point formula,
@@ -996,8 +997,8 @@ MPASG_D double wdtz_fx_at(const double* __restrict__ th, const double* __restric
 
 // w and theta tendencies (float64 form); index space (C, L+1).  Bound by the float64 pipe: 89
 // operations a level before (369 us at 40962 x 55), about 40 with the upwind vertical fluxes,
-// the perturbation flux on the edges (k_adv_edges_fx, 216 -> 243 us for it), the w divergence
-// on the integer pipes and the quotient of fastdiv64.cuh (220 us).
+// the perturbation flux on the edges (k_adv_edges_fx, 216 -> 243 us for it), both divergences
+// on the integer pipes and the quotient of fastdiv64.cuh (161 us, the first stage 184).
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_tend_w_theta(mpasg_mesh m, mpasg_fields f, FastDiv fl1, TendScalars p) {
   extern __shared__ cellsum::Slot s_c[];
