@@ -61,7 +61,7 @@ WORKLOADS = {
 # DRAM bytes (read + write) per call and cell-level of a float64 stage, from an ncu capture
 # of the tendency stage on the level-5 mesh (10242 cells x 41 levels), scaled to the
 # workload by its cell-levels
-TRAFFIC_B_PER_CELL_LEVEL = {"dyn_tend": 542.7}
+TRAFFIC_B_PER_CELL_LEVEL = {"dyn_tend": 661.0}
 # executed float64 flops (2 per FMA) per call and cell-level of a float64 stage, averaged
 # over a large step's calls, from an ncu count on the same level-5 x 41 case
 FP64_FLOP_PER_CELL_LEVEL = {"dyn_tend": 264.0}
