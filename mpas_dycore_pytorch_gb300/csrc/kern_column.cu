@@ -237,17 +237,21 @@ MPASG_D void factor_column(const double* a, const double* b, const double* c, do
 // shared memory ([level][column], odd pitch).  In place of two launches, each a few waves of
 // latency on a small mesh: a step of 162 columns x 12 levels 664 -> 640 us, 2562 x 26 1359 ->
 // 1334, 40962 x 55 25.58 -> 25.37 ms (mixed form 17.61 -> 17.27).
-template <typename T>
+// SHARED: the levels' cofwt and coftz wait for their neighbours in shared memory too; without it
+// the neighbours are read back from memory and an SM holds five blocks of 27 columns of 55
+// levels instead of three: 255 -> 228 us at 40962 x 55 (step 21.67 -> 21.55 ms).  Where five fit
+// all the same, memory only adds latency (step at 2562 x 26 1025 -> 1053 us).
+template <typename T, bool SHARED>
 __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fields f, FastDiv fl, int cols,
                                                          VimpScalars s) {
   extern __shared__ double s_col[];
   const uint32_t L = (uint32_t)m.nVertLevels, pitch = (uint32_t)cols | 1u, nlp = L * pitch;
-  double* s_cw = s_col;  // L x pitch each
-  double* s_ct = s_cw + nlp;
-  double* sa = s_ct + nlp;
+  double* sa = s_col;  // L x pitch each
   double* sb = sa + nlp;
   double* sc = sb + nlp;
-  VimpFlat* s_flat = reinterpret_cast<VimpFlat*>(sc + nlp);
+  double* s_cw = sc + nlp;  // SHARED
+  double* s_ct = s_cw + nlp;
+  VimpFlat* s_flat = reinterpret_cast<VimpFlat*>(SHARED ? s_ct + nlp : s_cw);
   const uint32_t c0 = blockIdx.x * (uint32_t)cols, ncol = min((uint32_t)cols, (uint32_t)m.nCells - c0), nl = ncol * L;
   const size_t o0 = (size_t)c0 * L, ow0 = o0 + c0;
   if (sizeof(T) == sizeof(double))
@@ -256,8 +260,10 @@ __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fie
     const uint32_t col = fl.div(i), k = i - col * L, q = k * pitch + col;
     const VimpLevel v = vimp_level<T>(m, f, o0 + col * L, k, s);
     if (c0 + col == 0) f.cofrz[k] = s.dtseps * m.rdzw[k];
-    s_cw[q] = v.cofwt;
-    s_ct[q] = v.coftz;
+    if (SHARED) {
+      s_cw[q] = v.cofwt;
+      s_ct[q] = v.coftz;
+    }
     f.cofwt[o0 + i] = v.cofwt;
     f.coftz[ow0 + i + col] = v.coftz;
   }
@@ -270,8 +276,11 @@ __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fie
       f.cofwz[o0 + i] = 0.0;
       f.coftz[ow0 + i + col + L] = 0.0;
     } else {
-      r = vimp_row<T>(m, f, o0 + col * L, ow0 + col * (L + 1), k, VimpLevel{s_cw[q], s_ct[q]},
-                      VimpLevel{s_cw[q - pitch], s_ct[q - pitch]}, k + 1 < L ? s_ct[q + pitch] : 0.0, s, s_flat);
+      const double* cw = SHARED ? s_cw + q : f.cofwt + o0 + i;
+      const double* ct = SHARED ? s_ct + q : f.coftz + ow0 + i + col;
+      const int below = SHARED ? -(int)pitch : -1;
+      r = vimp_row<T>(m, f, o0 + col * L, ow0 + col * (L + 1), k, VimpLevel{cw[0], ct[0]},
+                      VimpLevel{cw[below], ct[below]}, k + 1 < L ? ct[-below] : 0.0, s, s_flat);
     }
     f.a_tri[o0 + i] = sa[q] = r.a;
     f.b_tri[o0 + i] = sb[q] = r.b;
@@ -291,8 +300,8 @@ __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fie
   }
 }
 
-size_t vimp_columns_smem_bytes(int L, int cols) {
-  return (size_t)L * (5 * (cols | 1) * sizeof(double) + sizeof(VimpFlat));
+size_t vimp_columns_smem_bytes(int L, int cols, bool shared) {
+  return (size_t)L * ((shared ? 5 : 3) * (cols | 1) * sizeof(double) + sizeof(VimpFlat));
 }
 
 template <typename T>
@@ -1393,21 +1402,21 @@ extern "C" int mpasg_vert_imp_coefs(const mpasg_mesh* m, const mpasg_config* c, 
   const VimpScalars vs = vimp_scalars(dts, c->epssm);
   const FastDiv fl(L);
   const int cols = columns_per_block(m->nCells, L, 400, 31, 6);
-  const size_t smem = vimp_columns_smem_bytes(L, cols);
+  // all five arrays in shared memory as long as an SM still holds five blocks of them
+  const bool shared = vimp_columns_smem_bytes(L, cols, true) <= 44 * 1024;
+  const size_t smem = vimp_columns_smem_bytes(L, cols, shared);
   const bool mixed = c->precision == MPASG_PRECISION_MIXED;
   if (smem <= kMaxSmem) {
-    if (smem > 48 * 1024) {
-      const int b = (int)kMaxSmem;
-      const cudaError_t rc =
-          mixed ? cudaFuncSetAttribute(k_vimp_columns<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b)
-                : cudaFuncSetAttribute(k_vimp_columns<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-      if (rc != cudaSuccess) return MPASG_E_CUDA;
-    }
-    const int nb = nblocks(m->nCells, cols);
-    if (mixed) k_vimp_columns<float><<<nb, kBlock, smem, s>>>(*m, *f, fl, cols, vs);
-    else k_vimp_columns<double><<<nb, kBlock, smem, s>>>(*m, *f, fl, cols, vs);
-    MPASG_LAUNCH_CHECK();
-    return MPASG_OK;
+    const auto run = [&](auto kernel) -> int {
+      if (smem > 48 * 1024 &&
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess)
+        return MPASG_E_CUDA;
+      kernel<<<nblocks(m->nCells, cols), kBlock, smem, s>>>(*m, *f, fl, cols, vs);
+      MPASG_LAUNCH_CHECK();
+      return MPASG_OK;
+    };
+    if (mixed) return shared ? run(k_vimp_columns<float, true>) : run(k_vimp_columns<float, false>);
+    return shared ? run(k_vimp_columns<double, true>) : run(k_vimp_columns<double, false>);
   }
   const int nb = nblocks((long long)m->nCells * L), nf = nblocks(m->nCells, 64);
   if (mixed) k_vimp_coefs<float><<<nb, kBlock, 0, s>>>(*m, *f, fl, vs);

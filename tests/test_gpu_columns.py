@@ -76,3 +76,25 @@ def test_captured_step_with_branches(options, terrain):
     got = model.export()
     for k, v in want.items():
         assert torch.equal(got[k], v), k
+
+
+def test_implicit_coefficients_of_high_columns():
+    """Blocks whose columns leave no room for the level coefficients in shared memory (2562
+    columns of 300 levels) against blocks that hold them (the same columns on 162 cells)."""
+    need_gpu()
+    big, _ = _model(300, level=4)
+    small, _ = _model(300, level=2)
+    big.call("mpasg_moist_coefficients")
+    nc = small.dmesh.nCells
+    columns = ("exner", "exner_base", "rtheta_base", "rtheta_p", "qtot", "theta_m", "cqw")
+    for k in columns:
+        small.state.f[k][:nc].copy_(big.state.f[k][:nc])
+    small.dmesh._keep["rho_base"][:nc].copy_(big.dmesh._keep["rho_base"][:nc])
+    assert torch.equal(small.dmesh._keep["zz"][:nc], big.dmesh._keep["zz"][:nc])
+    for model in (big, small):
+        model.call("mpasg_vert_imp_coefs", C.c_double(DT / 6.0))
+    for k in ("cofrz",):
+        assert torch.equal(small.state.f[k].flatten()[:300], big.state.f[k].flatten()[:300])
+    for k in ("cofwr", "cofwz", "cofwt", "coftz", "a_tri", "b_tri", "c_tri", "alpha_tri", "gamma_tri"):
+        assert torch.equal(small.state.f[k][:nc], big.state.f[k][:nc]), k
+        assert torch.isfinite(small.state.f[k][:nc]).all(), k
