@@ -15,6 +15,7 @@
 class GraphBranches {
  public:
   explicit GraphBranches(cudaStream_t s) : s_(s) { on_ = current(base_) && !base_.empty(); }
+  bool active() const { return on_; }
   int next() { return on_ && !(collect() && set(base_)) ? MPASG_E_CUDA : MPASG_OK; }
   int join() {
     if (!on_) return MPASG_OK;

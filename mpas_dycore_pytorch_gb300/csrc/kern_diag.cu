@@ -2,6 +2,7 @@
 // cell-centre wind reconstruction (dynamics/vector_reconstruction.py:311) and the
 // cold-start coupled diagnostics (dynamics/init_coupled_diagnostics.py:147).
 #include "common.cuh"
+#include "branches.cuh"
 #include "trisk.cuh"
 #include "pow_exner.cuh"
 
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kBlock) k_diag_vertices_fx(mpasg_mesh m, mpasg
 // 97-118 us.
 // Block tables: per cell N divergence weights sign dvEdge (row: edge), then N kite weights
 // (row: vertex), then the kite areas as float64.
-template <int N>
+template <int N, bool KITES>
 MPASG_D void load_cell_tables(const mpasg_mesh& m, uint32_t c0, uint32_t n, fx::Weight* edge, fx::Weight* kite,
                               double* area) {
   for (uint32_t t = threadIdx.x; t < n * N; t += blockDim.x) {
@@ -199,7 +200,7 @@ MPASG_D void load_cell_tables(const mpasg_mesh& m, uint32_t c0, uint32_t n, fx::
     double a = 0.0;
     if ((int)j < nc && nc <= N) {
       we = fx::weight(m.cell_edge_sdv[o + j], m.edgesOnCell[o + j]);
-      const int v = m.verticesOnCell[o + j], kk = m.kiteForCell[o + j];
+      const int v = KITES ? m.verticesOnCell[o + j] : m.nVertices, kk = KITES ? m.kiteForCell[o + j] : -1;
       if (v < m.nVertices && kk >= 0) {
         a = m.kiteAreasOnVertex[(size_t)v * m.vertexDegree + kk];
         wk = fx::weight(a, v);
@@ -237,7 +238,9 @@ MPASG_D double wide_divergence(const mpasg_mesh& m, const double* flux, uint32_t
   return d;
 }
 
-template <int N>
+// PART 1: the divergences, which read the edges only; PART 2: the kinetic energy and the PV,
+// which read the vertices too; PART 3: both.
+template <int N, int PART>
 __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, int apvm,
                                                           int hdiv) {
   extern __shared__ fx::Weight s_w[];
@@ -246,46 +249,50 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg
   const uint32_t c0 = fl.div(i0), nc = fl.div(min(i0 + kBlock, n_all) - 1u) - c0 + 1;
   fx::Weight* s_k = s_w + nc * N;
   double* s_a = reinterpret_cast<double*>(s_k + nc * N);
-  load_cell_tables<N>(m, c0, nc, s_w, s_k, s_a);
+  load_cell_tables<N, (PART & 2) != 0>(m, c0, nc, s_w, s_k, s_a);
   __syncthreads();
   if (i >= n_all) return;
   const uint32_t c = fl.div(i), k = i - c * L, t = (c - c0) * N;
   const int n = m.nEdgesOnCell[c];
-  double div, kee = 0.0, kev = 0.0, pv = 0.0;
+  double div = 0.0, kee = 0.0, kev = 0.0, pv = 0.0;
   if (n > N) {
-    wide_cell_sums(m, f, c, k, &div, &kee, &kev, &pv);
+    if (PART == 1) div = wide_divergence(m, f.u, c, k);
+    else wide_cell_sums(m, f, c, k, &div, &kee, &kev, &pv);
   } else {
     double x[N];
 #pragma unroll
-    for (int j = 0; j < N; ++j) x[j] = f.u[(uint32_t)s_w[t + j].row * L + k];
-    bool ok = fx::dot<N>(x, s_w + t, &div);
-    if (apvm) {
+    for (int j = 0; j < N; ++j) x[j] = PART & 1 ? f.u[(uint32_t)s_w[t + j].row * L + k] : 0.0;
+    bool ok = PART & 1 ? fx::dot<N>(x, s_w + t, &div) : true;
+    if ((PART & 2) && apvm) {
 #pragma unroll
       for (int j = 0; j < N; ++j) x[j] = f.pv_vertex[(uint32_t)s_k[t + j].row * L + k];
       ok = fx::dot<N>(x, s_k + t, &pv) && ok;
     }
+    if (PART & 2) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      x[j] = j < n ? f.ke_edge[(uint32_t)s_w[t + j].row * L + k] : 0.0;
-      if (j < n) kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
-    }
-    bool summed = false;
-    if constexpr (N <= 8) {
-      const uint32_t plus[N] = {};
-      summed = fx::sum<N>(x, plus, &kee);
-    }
-    if (!summed) {
-      kee = 0.0;
+      for (int j = 0; j < N; ++j) {
+        x[j] = j < n ? f.ke_edge[(uint32_t)s_w[t + j].row * L + k] : 0.0;
+        if (j < n) kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
+      }
+      bool summed = false;
+      if constexpr (N <= 8) {
+        const uint32_t plus[N] = {};
+        summed = fx::sum<N>(x, plus, &kee);
+      }
+      if (!summed) {
+        kee = 0.0;
 #pragma unroll
-      for (int j = 0; j < N; ++j) kee += x[j];
+        for (int j = 0; j < N; ++j) kee += x[j];
+      }
     }
     if (!ok) {
       double a, b;
-      wide_cell_sums(m, f, c, k, &div, &a, &b, &pv);
+      if (PART == 1) div = wide_divergence(m, f.u, c, k);
+      else wide_cell_sums(m, f, c, k, &div, &a, &b, &pv);
     }
   }
   const double ia = m.invAreaCell[c];
-  if (hdiv) {  // divergence of ru, for the next stage's tendencies
+  if ((PART & 1) && hdiv) {  // divergence of ru, for the next stage's tendencies
     double x[N], hd;
     bool ok = n <= N;
     if (ok) {
@@ -296,7 +303,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg
     if (!ok) hd = wide_divergence(m, f.ru, c, k);
     f.h_divergence[i] = hd * ia;
   }
-  f.divergence[i] = div * ia;
+  if (PART & 1) f.divergence[i] = div * ia;
+  if (!(PART & 2)) return;
   // 0.25 (0.625 sum_j ke_edge + 0.375 sum_j kite ke_vertex) / area
   f.ke[i] = ia * fma(0.625 * 0.25, kee, (0.375 * 0.25) * kev);
   if (apvm) f.pv_cell[i] = pv * ia;
@@ -357,13 +365,29 @@ int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_field
     MPASG_LAUNCH_CHECK();
   }
   const int nv = nblocks((long long)m->nVertices * L);
+  const size_t slot = 2 * sizeof(fx::Weight) + sizeof(double);
+  const auto cells = [&](auto narrow, auto wide) -> int {
+    if (m->maxEdges <= 6) narrow<<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
+    else wide<<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
+    MPASG_LAUNCH_CHECK();
+    return MPASG_OK;
+  };
+  // a captured step of a small mesh (at most a block of cells an SM): the divergences beside the
+  // vertices (step of 162 x 12 455 -> 447 us, 642 x 26 581 -> 573, 642 x 55 787 -> 786; from
+  // 2562 x 26 on the launch costs what the overlap gives)
+  GraphBranches branches(s);
+  const bool split = branches.active() && nc <= 152;
+  if (split) {
+    int rc = cells(k_diag_cells_fx<6, 1>, k_diag_cells_fx<10, 1>);
+    if (rc == MPASG_OK) rc = branches.next();
+    if (rc != MPASG_OK) return rc;
+  }
   if (m->vertexDegree == 3) k_diag_vertices_fx<<<nv, kBlock, rows * 3 * sizeof(fx::Weight), s>>>(*m, *f, fl);
   else k_diag_vertices<double, false><<<nv, kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
-  const size_t slot = 2 * sizeof(fx::Weight) + sizeof(double);
-  if (m->maxEdges <= 6) k_diag_cells_fx<6><<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
-  else k_diag_cells_fx<10><<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
-  MPASG_LAUNCH_CHECK();
+  const int rc = split ? cells(k_diag_cells_fx<6, 2>, k_diag_cells_fx<10, 2>)
+                       : cells(k_diag_cells_fx<6, 3>, k_diag_cells_fx<10, 3>);
+  if (rc != MPASG_OK) return rc;
   const double adt = c->apvm_upwinding * c->dt;
   const size_t se = rows * sizeof(ApvmEdge);
   if (rk_step != 3)
@@ -373,7 +397,7 @@ int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_field
   else
     k_diag_edges_b_fx<14, true><<<ne, kBlock, se + rows * 14 * sizeof(fx::Weight), s>>>(*m, *f, fl, adt, apvm);
   MPASG_LAUNCH_CHECK();
-  return MPASG_OK;
+  return branches.join();
 }
 
 // mpas_reconstruct_2d: RBF reconstruction of the cell-centre wind
