@@ -357,11 +357,19 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
       const double cqu = f.cqu_e[i];
       pgrad = pgrad * (f.exner[i1] + f.exner[i2]) * (c2 * m.invDcEdge[e]);
       if (!fx::is_one(cqu)) pgrad = cqu * pgrad;
+      if (!m.flatTerrain)  // no slope: adds an exact zero
+        pgrad = pgrad + 0.5 * m.zxu[i] * kGravity * (f.rho_pp[i1] + f.rho_pp[i2]);
     } else {
-      pgrad = cv<T>(f.cqu_e[i]) * (T(0.5) * cv<T>(c2)) * (cv<T>(f.exner[i1]) + cv<T>(f.exner[i2])) * pgrad;
+      // the product is rounded once, with the slope term where there is one, on every route:
+      // float32 stencils carry a last bit of it to the seventh digit of a step
+      const float a = cv<float>(f.cqu_e[i]) * (0.5f * cv<float>(c2)) * (cv<float>(f.exner[i1]) + cv<float>(f.exner[i2]));
+      if (m.flatTerrain) {
+        pgrad = __fmul_rn(a, pgrad);
+      } else {
+        const float slope = 0.5f * cv<float>(m.zxu[i]) * float(kGravity);
+        pgrad = __fmaf_rn(a, pgrad, __fmul_rn(slope, cv<float>(f.rho_pp[i1]) + cv<float>(f.rho_pp[i2])));
+      }
     }
-    if (!m.flatTerrain)  // no slope: adds exact zeros
-      pgrad = pgrad + T(0.5) * cv<T>(m.zxu[i]) * T(kGravity) * (cv<T>(f.rho_pp[i1]) + cv<T>(f.rho_pp[i2]));
     const double before = DAMP ? damped_ru_p<T, FROM_ZERO>(f, i, i1, i2, damp_coef) : f.ru_p[i];
     if constexpr (kDouble) rup = fma(dts, f.tend_u[i] - pgrad, before);
     else rup = before + f64(cv<T>(dts) * (cv<T>(f.tend_u[i]) - pgrad));
