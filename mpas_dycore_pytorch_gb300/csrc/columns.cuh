@@ -19,4 +19,3 @@ inline int columns_per_block(int nCells, int items, int cells_per_column, int mo
   const int least = std::max(2, std::min(4, kBlock / items));
   return std::max(least, std::min({most, passes * kBlock / items, nCells / cells_per_column}));
 }
-constexpr size_t kMaxSmem = 200 * 1024;  // dynamic shared memory those kernels opt in to

@@ -162,6 +162,16 @@ inline int nblocks(long long n, int block = kBlock) {
   return (int)(b < 1 ? 1 : b);
 }
 
+// Dynamic shared memory beyond the 48 KB a kernel has without asking, up to kMaxSmem (set on the
+// function, not on a stream: works in a capture).  False where a launch with it would fail.
+constexpr size_t kMaxSmem = 200 * 1024;
+template <typename K>
+inline bool allow_smem(K* kernel, size_t bytes) {
+  if (bytes <= 48 * 1024) return true;
+  return bytes <= kMaxSmem && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)kMaxSmem) == cudaSuccess;
+}
+
 // ---------------------------------------------------------------- internal entry points
 // The mixed form's stencils read float32 copies of u, pv_edge, w and rw.  The step driver
 // keeps them current (pack once at step start; recover and diagnostics rewrite them), so

@@ -1368,9 +1368,7 @@ static int launch_ac_columns(const mpasg_mesh* m, const mpasg_fields* f, bool mi
   *done = smem <= kMaxSmem && !(mixed && thomas_smem_bytes(L) > kMaxSmem);
   if (!*done) return MPASG_OK;
   const auto run = [&](auto kernel, auto... args) -> int {
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess)
-      return MPASG_E_CUDA;
+    if (!allow_smem(kernel, smem)) return MPASG_E_CUDA;
     kernel<<<nb, kBlock, smem, s>>>(*m, *f, FastDiv(L), FastDiv(L + 1), cols, keep, last, args...);
     MPASG_LAUNCH_CHECK();
     return MPASG_OK;
@@ -1416,9 +1414,7 @@ extern "C" int mpasg_vert_imp_coefs(const mpasg_mesh* m, const mpasg_config* c, 
   const bool mixed = c->precision == MPASG_PRECISION_MIXED;
   if (smem <= kMaxSmem) {
     const auto run = [&](auto kernel) -> int {
-      if (smem > 48 * 1024 &&
-          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) != cudaSuccess)
-        return MPASG_E_CUDA;
+      if (!allow_smem(kernel, smem)) return MPASG_E_CUDA;
       kernel<<<nblocks(m->nCells, cols), kBlock, smem, s>>>(*m, *f, fl, cols, vs);
       MPASG_LAUNCH_CHECK();
       return MPASG_OK;

@@ -366,9 +366,13 @@ int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_field
   }
   const int nv = nblocks((long long)m->nVertices * L);
   const size_t slot = 2 * sizeof(fx::Weight) + sizeof(double);
+  // (one or two levels: a block covers many rows, up to 101 KB of tables)
   const auto cells = [&](auto narrow, auto wide) -> int {
-    if (m->maxEdges <= 6) narrow<<<nc, kBlock, rows * 6 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
-    else wide<<<nc, kBlock, rows * 10 * slot, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
+    const bool six = m->maxEdges <= 6;
+    const auto kernel = six ? narrow : wide;
+    const size_t smem = rows * (six ? 6 : 10) * slot;
+    if (!allow_smem(kernel, smem)) return MPASG_E_CUDA;
+    kernel<<<nc, kBlock, smem, s>>>(*m, *f, fl, apvm, fuse.hdiv ? 1 : 0);
     MPASG_LAUNCH_CHECK();
     return MPASG_OK;
   };
@@ -385,18 +389,23 @@ int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_field
   if (m->vertexDegree == 3) k_diag_vertices_fx<<<nv, kBlock, rows * 3 * sizeof(fx::Weight), s>>>(*m, *f, fl);
   else k_diag_vertices<double, false><<<nv, kBlock, 0, s>>>(*m, *f, fl);
   MPASG_LAUNCH_CHECK();
-  const int rc = split ? cells(k_diag_cells_fx<6, 2>, k_diag_cells_fx<10, 2>)
-                       : cells(k_diag_cells_fx<6, 3>, k_diag_cells_fx<10, 3>);
-  if (rc != MPASG_OK) return rc;
+  if (const int rc = split ? cells(k_diag_cells_fx<6, 2>, k_diag_cells_fx<10, 2>)
+                           : cells(k_diag_cells_fx<6, 3>, k_diag_cells_fx<10, 3>);
+      rc != MPASG_OK)
+    return rc;
   const double adt = c->apvm_upwinding * c->dt;
   const size_t se = rows * sizeof(ApvmEdge);
-  if (rk_step != 3)
-    k_diag_edges_b_fx<1, false><<<ne, kBlock, se, s>>>(*m, *f, fl, adt, apvm);
-  else if (m->maxEdges2 <= 10)
-    k_diag_edges_b_fx<10, true><<<ne, kBlock, se + rows * 10 * sizeof(fx::Weight), s>>>(*m, *f, fl, adt, apvm);
-  else
-    k_diag_edges_b_fx<14, true><<<ne, kBlock, se + rows * 14 * sizeof(fx::Weight), s>>>(*m, *f, fl, adt, apvm);
-  MPASG_LAUNCH_CHECK();
+  const auto edges = [&](auto kernel, size_t smem) -> int {
+    if (!allow_smem(kernel, smem)) return MPASG_E_CUDA;
+    kernel<<<ne, kBlock, smem, s>>>(*m, *f, fl, adt, apvm);
+    MPASG_LAUNCH_CHECK();
+    return MPASG_OK;
+  };
+  if (const int rc = rk_step != 3           ? edges(k_diag_edges_b_fx<1, false>, se)
+                     : m->maxEdges2 <= 10 ? edges(k_diag_edges_b_fx<10, true>, se + rows * 10 * sizeof(fx::Weight))
+                                          : edges(k_diag_edges_b_fx<14, true>, se + rows * 14 * sizeof(fx::Weight));
+      rc != MPASG_OK)
+    return rc;
   return branches.join();
 }
 

@@ -113,15 +113,15 @@ template <bool MONO>
 int launch_edge_flux_fx(const mpasg_mesh* m, int S, double dt, const double* uh, const double* q, const double* s_old,
                         double* out, double* out2, cudaStream_t s) {
   const uint32_t half = ((uint32_t)m->nVertLevels * S + 1) / 2, n = (uint32_t)m->nEdges * half;
+  // (rows of few values: a block covers many edges, up to 115 KB of them at one value and 14 slots)
   const size_t smem = (size_t)((kBlock - 1) / half + 2) * adv::kEntryBytes;
-  if (m->nAdvMax <= 10)
-    k_edge_flux_fx<10, MONO><<<nblocks(n), kBlock, smem * 10, s>>>(*m, FastDiv(half), FastDiv(S), n, half, dt, uh, q,
-                                                                   s_old, out, out2);
-  else
-    k_edge_flux_fx<14, MONO><<<nblocks(n), kBlock, smem * 14, s>>>(*m, FastDiv(half), FastDiv(S), n, half, dt, uh, q,
-                                                                   s_old, out, out2);
-  MPASG_LAUNCH_CHECK();
-  return MPASG_OK;
+  const auto run = [&](auto kernel, int slots) -> int {
+    if (!allow_smem(kernel, smem * slots)) return MPASG_E_CUDA;
+    kernel<<<nblocks(n), kBlock, smem * slots, s>>>(*m, FastDiv(half), FastDiv(S), n, half, dt, uh, q, s_old, out, out2);
+    MPASG_LAUNCH_CHECK();
+    return MPASG_OK;
+  };
+  return m->nAdvMax <= 10 ? run(k_edge_flux_fx<10, MONO>, 10) : run(k_edge_flux_fx<14, MONO>, 14);
 }
 
 // the thread's place in a (cell, level, scalar) row
