@@ -38,13 +38,14 @@ MPASG_D double wide(const mpasg_mesh& m, uint32_t c, const double* __restrict__ 
 }
 
 // on the float64 pipe
-template <int N>
+// (Index: the type of an index into f; size_t where rows times pitch may pass 2^32)
+template <int N, typename Index = uint32_t>
 MPASG_D double f64(const mpasg_mesh& m, uint32_t c, int n, const Slot* s, const double* __restrict__ f,
                    uint32_t pitch, uint32_t k) {
   if (n > N) return wide(m, c, f, pitch, k);
   double x[N];
 #pragma unroll
-  for (int j = 0; j < N; ++j) x[j] = j < n ? f[s[j].row * pitch + k] : 0.0;
+  for (int j = 0; j < N; ++j) x[j] = j < n ? f[(Index)s[j].row * pitch + k] : 0.0;
   double acc = flip(x[0], s[0].sgn);
 #pragma unroll
   for (int j = 1; j < N; ++j)
@@ -53,7 +54,7 @@ MPASG_D double f64(const mpasg_mesh& m, uint32_t c, int n, const Slot* s, const 
 }
 
 // on the integer pipes
-template <int N>
+template <int N, typename Index = uint32_t>
 MPASG_D double fixed(const mpasg_mesh& m, uint32_t c, int n, const Slot* s, const double* __restrict__ f,
                      uint32_t pitch, uint32_t k) {
   if (n > N) return wide(m, c, f, pitch, k);
@@ -61,7 +62,7 @@ MPASG_D double fixed(const mpasg_mesh& m, uint32_t c, int n, const Slot* s, cons
   uint32_t sgn[N];
 #pragma unroll
   for (int j = 0; j < N; ++j) {
-    x[j] = j < n ? f[s[j].row * pitch + k] : 0.0;
+    x[j] = j < n ? f[(Index)s[j].row * pitch + k] : 0.0;
     sgn[j] = s[j].sgn;
   }
   return fx::sum<N>(x, sgn, &out) ? out : wide(m, c, f, pitch, k);

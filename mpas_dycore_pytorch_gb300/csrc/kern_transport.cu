@@ -2,6 +2,7 @@
 // composition :861, Pattern-C edge values dynamics/pattern_c.py:234-305) and the monotone
 // flux-corrected final stage (dynamics/advance_scalars_mono.py:3332, tile :1476, neighbour
 // bounds autodiff/soft_limiter.py:72).  Scalar fields are (C+1, L, S), edge fluxes (E+1, L, S).
+#include <algorithm>
 #include <mutex>
 
 #include "advstencil.cuh"
@@ -47,6 +48,28 @@ __global__ void k_pattern_c(mpasg_mesh m, FastDiv fl, int S, const double* __res
 // values and a scalar costs no strided pass; the horizontal sums run on the integer pipes
 // (fixdot.cuh), comparisons, minima and clamps on the integer side too (each would take a
 // float64 slot).
+// A launch numbers its (row, value) threads in 32 bits and divides by FastDiv, which holds below
+// 2^31: rows that reach it are taken in several launches, each from its own first row, and
+// indices into the fields are 64 bits wide (monotone stage at 40962 x 55 x 3 1404 -> 1413 us,
+// explicit at 2562 x 37 x 8 84.0 -> 84.2, the first rows' 64-bit offset rather than the gathers'
+// width).  (A build may lower the limit to test the split.)
+#ifndef MPASG_MAX_THREADS
+#define MPASG_MAX_THREADS (0x7fffffffu - kBlock)
+#endif
+constexpr uint32_t kMaxThreads = MPASG_MAX_THREADS;
+
+// calls launch(first row, rows) over n rows of `width` threads each
+template <typename Launch>
+int launch_rows(int n, uint32_t width, Launch launch) {
+  const int most = (int)std::min<uint32_t>((uint32_t)n, std::max(1u, kMaxThreads / width));
+  for (int first = 0; first < n; first += most) {
+    launch((uint32_t)first, (uint32_t)std::min(most, n - first));
+    MPASG_LAUNCH_CHECK();
+    if (most > n - first) break;  // (first + most may pass the last int)
+  }
+  return MPASG_OK;
+}
+
 struct TransportScalars {
   double dt, w_old, w_new, f3[4];  // f3: 7 + 3 c, 7 - 3 c, 1 + c, 1 - c of the upwind flux3
 };
@@ -80,8 +103,8 @@ MPASG_D void store_edge_flux(const mpasg_mesh& m, uint32_t e, uint32_t row, uint
 }
 
 template <int N, bool MONO>
-__global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t n_all,
-                                                         uint32_t half, double dt, const double* __restrict__ uh,
+__global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t first,
+                                                         uint32_t n_all, double dt, const double* __restrict__ uh,
                                                          const double* __restrict__ q,
                                                          const double* __restrict__ s_old, double* __restrict__ out,
                                                          double* __restrict__ out2) {
@@ -89,11 +112,11 @@ __global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDi
   const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
   const uint32_t e0 = fh.div(i0), e1 = fh.div(min(i0 + kBlock, n_all) - 1u);
-  adv::load<N>(m, e0, e1 - e0 + 1, s_w);
+  adv::load<N>(m, first + e0, e1 - e0 + 1, s_w);
   __syncthreads();
   if (i >= n_all) return;
-  const uint32_t e = fh.div(i), a = i - e * half, b = a + half;
-  const fx::Weight* w = s_w + (e - e0) * (2 * N);
+  const uint32_t er = fh.div(i), e = first + er, a = i - er * fh.d, b = a + fh.d;
+  const fx::Weight* w = s_w + (er - e0) * (2 * N);
   double x[N], acc;
   const double ua = uh[(size_t)e * L + fs.div(a)], dvdt = MONO ? m.dvEdge[e] * dt : 0.0;
   const bool back = __double2hiint(ua) < 0;
@@ -112,28 +135,32 @@ __global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDi
 template <bool MONO>
 int launch_edge_flux_fx(const mpasg_mesh* m, int S, double dt, const double* uh, const double* q, const double* s_old,
                         double* out, double* out2, cudaStream_t s) {
-  const uint32_t half = ((uint32_t)m->nVertLevels * S + 1) / 2, n = (uint32_t)m->nEdges * half;
+  const uint32_t half = ((uint32_t)m->nVertLevels * S + 1) / 2;
   // (rows of few values: a block covers many edges, up to 115 KB of them at one value and 14 slots)
   const size_t smem = (size_t)((kBlock - 1) / half + 2) * adv::kEntryBytes;
   const auto run = [&](auto kernel, int slots) -> int {
     if (!allow_smem(kernel, smem * slots)) return MPASG_E_CUDA;
-    kernel<<<nblocks(n), kBlock, smem * slots, s>>>(*m, FastDiv(half), FastDiv(S), n, half, dt, uh, q, s_old, out, out2);
-    MPASG_LAUNCH_CHECK();
-    return MPASG_OK;
+    return launch_rows(m->nEdges, half, [&](uint32_t first, uint32_t n) {
+      kernel<<<nblocks((long long)n * half), kBlock, smem * slots, s>>>(*m, FastDiv(half), FastDiv(S), first, n * half,
+                                                                        dt, uh, q, s_old, out, out2);
+    });
   };
   return m->nAdvMax <= 10 ? run(k_edge_flux_fx<10, MONO>, 10) : run(k_edge_flux_fx<14, MONO>, 14);
 }
 
-// the thread's place in a (cell, level, scalar) row
+// the place of a launch's thread i in a (cell, level, scalar) row; at: its index in the fields
 struct CellRow {
   uint32_t c, r, k, s;
+  size_t at;
 };
-MPASG_D CellRow cell_row(uint32_t i, uint32_t row, const FastDiv& fr, const FastDiv& fs) {
+MPASG_D CellRow cell_row(uint32_t i, uint32_t first, const FastDiv& fr, const FastDiv& fs) {
   CellRow t;
-  t.c = fr.div(i);
-  t.r = i - t.c * row;
+  const uint32_t cr = fr.div(i);
+  t.c = first + cr;
+  t.r = i - cr * fr.d;
   t.k = fs.div(t.r);
   t.s = t.r - t.k * fs.d;
+  t.at = (size_t)first * fr.d + i;
   return t;
 }
 
@@ -156,17 +183,18 @@ MPASG_D double interface_value(const double* __restrict__ q, uint32_t S, double 
 // per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage)
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
-                                                              TransportScalars p, const double* __restrict__ s_old,
+                                                              uint32_t first, uint32_t n_all, TransportScalars p,
+                                                              const double* __restrict__ s_old,
                                                               const double* __restrict__ s_new,
                                                               double* __restrict__ s_out) {
   extern __shared__ cellsum::Slot s_c[];
   __shared__ double s_wd[kBlock];
-  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S, n_all = (uint32_t)m.nCells * row;
+  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
-  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
+  const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   const bool active = i < n_all;
-  CellRow t{c0, 0, 0, 0};
+  CellRow t{c0, 0, 0, 0, 0};
   auto flux_at = [&](uint32_t k) {  // at the interface below level k of this thread's column
     if (k == 0 || k >= L) return 0.0;
     const double ww = f.wwAvg[(size_t)t.c * (L + 1) + k];
@@ -176,20 +204,20 @@ __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, m
   };
   double lo = 0.0;
   if (active) {
-    t = cell_row(i, row, fr, fs);
+    t = cell_row(i, first, fr, fs);
     lo = flux_at(t.k);
   }
   s_wd[threadIdx.x] = lo;
   __syncthreads();
   if (!active) return;
   const double hi = t.k + 1 >= L ? 0.0 : threadIdx.x + S < kBlock ? s_wd[threadIdx.x + S] : flux_at(t.k + 1);
-  const double div = cellsum::fixed<N>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
+  const double div = cellsum::fixed<N, size_t>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
   const size_t ic = (size_t)t.c * L + t.k;
   const double tend = fma(m.rdnw[t.k], lo - hi, -(div * m.invAreaCell[t.c]));
   const double rho_old = f.rho_zz_old_split[ic];
   double rho = f.rho_zz[ic];
   if (p.w_old != 0.0) rho = p.w_old * rho_old + p.w_new * rho;
-  s_out[i] = fx::quotient(fma(p.dt, tend, s_old[i] * rho_old), rho);
+  s_out[t.at] = fx::quotient(fma(p.dt, tend, s_old[t.at] * rho_old), rho);
 }
 
 // monotone stage: density at its end
@@ -211,13 +239,14 @@ __global__ void k_mono_density_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, doub
 // (735 -> 273 us at 40962 x 55 x 3, and 40 us for the density).
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
-                                                            TransportScalars p, const double* __restrict__ so,
+                                                            uint32_t first, uint32_t n_all, TransportScalars p,
+                                                            const double* __restrict__ so,
                                                             const double* __restrict__ sn) {
   __shared__ double s_wm[kBlock], s_fu[kBlock];
-  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S, n_all = (uint32_t)m.nCells * row;
+  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
   const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   const bool active = i < n_all;
-  CellRow t{0, 0, 0, 0};
+  CellRow t{0, 0, 0, 0, 0};
   auto fluxes = [&](uint32_t k, double* wm, double* fu) {
     *wm = *fu = 0.0;
     if (k == 0 || k >= L) return;
@@ -230,7 +259,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
   };
   double wm_lo = 0.0, fu_lo = 0.0;
   if (active) {
-    t = cell_row(i, row, fr, fs);
+    t = cell_row(i, first, fr, fs);
     fluxes(t.k, &wm_lo, &fu_lo);
   }
   s_wm[threadIdx.x] = wm_lo;
@@ -248,15 +277,16 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
   }
   if (t.k >= 1) f.wflux[((size_t)t.c * (L + 1) + t.k) * S + t.s] = wm_lo;
   // bounds over the column's neighbours and the adjacent cells
-  const double here = so[i];
+  const size_t at = t.at;
+  const double here = so[at];
   int64_t kmax = fx::order_key(here), kmin = kmax;
   auto bound = [&](double x) {
     const int64_t q = fx::order_key(x);
     kmax = q > kmax ? q : kmax;
     kmin = q < kmin ? q : kmin;
   };
-  if (t.k >= 1) bound(so[i - S]);
-  if (t.k + 1 < L) bound(so[i + S]);
+  if (t.k >= 1) bound(so[at - S]);
+  if (t.k + 1 < L) bound(so[at + S]);
   const size_t oc = (size_t)t.c * m.maxEdges;
   const int n = m.nEdgesOnCell[t.c];
 #pragma unroll
@@ -277,39 +307,40 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
       smax = fmax(smax, x);
       smin = fmin(smin, x);
     };
-    if (t.k >= 1) wide(so[i - S]);
-    if (t.k + 1 < L) wide(so[i + S]);
+    if (t.k >= 1) wide(so[at - S]);
+    if (t.k + 1 < L) wide(so[at + S]);
     for (int j = 0; j < n; ++j) {
       const int nb = m.cellsOnCell[oc + j];
       if (nb < m.nCells) wide(so[(size_t)nb * row + t.r]);
     }
   }
   const double rd = m.rdnw[t.k];
-  f.rows[i] = fma(rd, fu_lo - fu_hi, here * f.rho_zz_old_split[(size_t)t.c * L + t.k]);
+  f.rows[at] = fma(rd, fu_lo - fu_hi, here * f.rho_zz_old_split[(size_t)t.c * L + t.k]);
   // in and out fluxes of the correction through the level's two interfaces
-  f.scale_in[i] = rd * (fx::positive(wm_lo) + fx::positive(-wm_hi));
-  f.scale_out[i] = -rd * (fx::positive(wm_hi) + fx::positive(-wm_lo));
-  f.s_max[i] = smax;
-  f.s_min[i] = smin;
+  f.scale_in[at] = rd * (fx::positive(wm_lo) + fx::positive(-wm_hi));
+  f.scale_out[at] = -rd * (fx::positive(wm_hi) + fx::positive(-wm_lo));
+  f.s_max[at] = smax;
+  f.s_min[at] = smin;
 }
 
 // per value: horizontal upwind update and scale sums, then the limiter factors.  Three integer
 // sums and 13 float64 operations a value, about 65 with the comparisons and divisions of the
 // per-cell loop (913 -> 256 us at 40962 x 55 x 3).
 template <int N>
-__global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs) {
+__global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
+                                                            uint32_t first, uint32_t n_all) {
   extern __shared__ cellsum::Slot s_c[];
-  const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d, n_all = (uint32_t)m.nCells * row;
+  const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
-  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
+  const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   __syncthreads();
   if (i >= n_all) return;
-  const CellRow t = cell_row(i, row, fr, fs);
+  const CellRow t = cell_row(i, first, fr, fs);
   const int n = m.nEdgesOnCell[t.c];
   const cellsum::Slot* s = s_c + (t.c - c0) * N;
   const double ia = m.invAreaCell[t.c], rint = f.rho_int[(size_t)t.c * L + t.k];
-  const double up = cellsum::fixed<N>(m, t.c, n, s, f.flux_up, row, t.r);
+  const double up = cellsum::fixed<N, size_t>(m, t.c, n, s, f.flux_up, row, t.r);
   double out = 0.0, in = 0.0;
   bool ok = n <= N;
   if (ok) {
@@ -331,47 +362,51 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpa
       in = in + mz(-sf);
     }
   }
-  const double rows = fma(-ia, up, f.rows[i]), eps = 1.0e-20;
-  const double sin_ = fma(ia, in, f.scale_in[i]) + eps, sout = fma(ia, out, -f.scale_out[i]) + eps;
-  f.rows[i] = rows;
-  f.scale_in[i] = fx::clamp01(fx::quotient(fma(f.s_max[i], rint, -rows), sin_));
-  f.scale_out[i] = fx::clamp01(fx::quotient(fma(-f.s_min[i], rint, rows), sout));
+  const size_t at = t.at;
+  const double rows = fma(-ia, up, f.rows[at]), eps = 1.0e-20;
+  const double sin_ = fma(ia, in, f.scale_in[at]) + eps, sout = fma(ia, out, -f.scale_out[at]) + eps;
+  f.rows[at] = rows;
+  f.scale_in[at] = fx::clamp01(fx::quotient(fma(f.s_max[at], rint, -rows), sin_));
+  f.scale_out[at] = fx::clamp01(fx::quotient(fma(-f.s_min[at], rint, rows), sout));
 }
 
 // per (edge, value): limited horizontal flux (stored in hflux)
-__global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint32_t n_all) {
+__global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint32_t first, uint32_t n_all) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_all) return;
-  const uint32_t e = fr.div(i), r = i - e * fr.d;
-  const double ft = f.flux_tmp[i];
+  const uint32_t er = fr.div(i), e = first + er, r = i - er * fr.d;
+  const size_t at = (size_t)first * fr.d + i;
+  const double ft = f.flux_tmp[at];
   const uint32_t back = __double2hiint(ft) < 0 ? 1u : 0u;
   const size_t from = (size_t)m.cellsOnEdge[2 * e + back] * fr.d + r;
   const size_t to = (size_t)m.cellsOnEdge[2 * e + 1 - back] * fr.d + r;
-  f.hflux[i] = ft * fx::min_nonneg(f.scale_out[from], f.scale_in[to]);
+  f.hflux[at] = ft * fx::min_nonneg(f.scale_out[from], f.scale_in[to]);
 }
 
 // per value: limited horizontal and vertical fluxes, positivity
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_c_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
+                                                            uint32_t first, uint32_t n_all,
                                                             double* __restrict__ s_out) {
   extern __shared__ cellsum::Slot s_c[];
-  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S, n_all = (uint32_t)m.nCells * row;
+  const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
-  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
+  const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   __syncthreads();
   if (i >= n_all) return;
-  const CellRow t = cell_row(i, row, fr, fs);
+  const CellRow t = cell_row(i, first, fr, fs);
+  const size_t at = t.at;
   const double* wf = f.wflux + ((size_t)t.c * (L + 1) + t.k) * S + t.s;
-  auto limited = [&](double wm, uint32_t below, uint32_t above) {  // an upward flux leaves `below`
+  auto limited = [&](double wm, size_t below, size_t above) {  // an upward flux leaves `below`
     const bool down = __double2hiint(wm) < 0;
     return wm * fx::min_nonneg(f.scale_out[down ? above : below], f.scale_in[down ? below : above]);
   };
-  const double lo = t.k >= 1 ? limited(wf[0], i - S, i) : 0.0;
-  const double hi = t.k + 1 < L ? limited(wf[S], i, i + S) : 0.0;
-  const double h = cellsum::fixed<N>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
-  const double rows = fma(m.rdnw[t.k], lo - hi, fma(-m.invAreaCell[t.c], h, f.rows[i]));
-  s_out[i] = fx::positive(fx::quotient(rows, f.rho_int[(size_t)t.c * L + t.k]));
+  const double lo = t.k >= 1 ? limited(wf[0], at - S, at) : 0.0;
+  const double hi = t.k + 1 < L ? limited(wf[S], at, at + S) : 0.0;
+  const double h = cellsum::fixed<N, size_t>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
+  const double rows = fma(m.rdnw[t.k], lo - hi, fma(-m.invAreaCell[t.c], h, f.rows[at]));
+  s_out[at] = fx::positive(fx::quotient(rows, f.rho_int[(size_t)t.c * L + t.k]));
 }
 
 template <typename T>
@@ -699,34 +734,39 @@ int launch_scalars_fx(const mpasg_mesh* m, const mpasg_fields& g, const Transpor
   const int rc = launch_edge_flux_fx<false>(m, S, 0.0, g.ruAvg, g.scalars_a, nullptr, g.hflux, nullptr, s);
   if (rc != MPASG_OK) return rc;
   const size_t smem = cellsum::max_cells(row) * N * sizeof(cellsum::Slot);
-  k_scalars_update_fx<N><<<nblocks((long long)m->nCells * row), kBlock, smem, s>>>(
-      *m, g, FastDiv(row), FastDiv(S), p, g.scalars_init, g.scalars_a, g.scalars_b);
-  MPASG_LAUNCH_CHECK();
-  return MPASG_OK;
+  return launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
+    k_scalars_update_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(
+        *m, g, FastDiv(row), FastDiv(S), first, n * row, p, g.scalars_init, g.scalars_a, g.scalars_b);
+  });
 }
 
 template <int N>
 int launch_scalars_mono_fx(const mpasg_mesh* m, const mpasg_fields* f, const TransportScalars& p, int S,
                            cudaStream_t s) {
   const int L = m->nVertLevels, row = L * S;
-  const int nb = nblocks((long long)m->nCells * row);
-  const uint32_t ne = (uint32_t)m->nEdges * row;
   const FastDiv fr(row), fs(S);
   const size_t smem = cellsum::max_cells(row) * N * sizeof(cellsum::Slot);
-  const int rc = launch_edge_flux_fx<true>(m, S, p.dt, f->ruAvg, f->scalars_a, f->scalars_init, f->flux_up,
-                                           f->flux_tmp, s);
+  int rc = launch_edge_flux_fx<true>(m, S, p.dt, f->ruAvg, f->scalars_a, f->scalars_init, f->flux_up, f->flux_tmp, s);
   if (rc != MPASG_OK) return rc;
   k_mono_density_fx<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), p.dt);
   MPASG_LAUNCH_CHECK();
-  k_mono_cells_a_fx<N><<<nb, kBlock, 0, s>>>(*m, *f, fr, fs, p, f->scalars_init, f->scalars_a);
-  MPASG_LAUNCH_CHECK();
-  k_mono_cells_b_fx<N><<<nb, kBlock, smem, s>>>(*m, *f, fr, fs);
-  MPASG_LAUNCH_CHECK();
-  k_mono_edges_b_fx<<<nblocks(ne), kBlock, 0, s>>>(*m, *f, fr, ne);
-  MPASG_LAUNCH_CHECK();
-  k_mono_cells_c_fx<N><<<nb, kBlock, smem, s>>>(*m, *f, fr, fs, f->scalars_b);
-  MPASG_LAUNCH_CHECK();
-  return MPASG_OK;
+  rc = launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
+    k_mono_cells_a_fx<N><<<nblocks((long long)n * row), kBlock, 0, s>>>(*m, *f, fr, fs, first, n * row, p,
+                                                                        f->scalars_init, f->scalars_a);
+  });
+  if (rc != MPASG_OK) return rc;
+  rc = launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
+    k_mono_cells_b_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, *f, fr, fs, first, n * row);
+  });
+  if (rc != MPASG_OK) return rc;
+  rc = launch_rows(m->nEdges, row, [&](uint32_t first, uint32_t n) {
+    k_mono_edges_b_fx<<<nblocks((long long)n * row), kBlock, 0, s>>>(*m, *f, fr, first, n * row);
+  });
+  if (rc != MPASG_OK) return rc;
+  return launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
+    k_mono_cells_c_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, *f, fr, fs, first, n * row,
+                                                                           f->scalars_b);
+  });
 }
 
 // One explicit RK transport stage with the edge values (mixed form) or fluxes in `hflux` (f->hflux
