@@ -271,8 +271,13 @@ int mpasg_prepare_derived(const mpasg_mesh *m, const mpasg_config *c, mpasg_fiel
 int mpasg_step(const mpasg_mesh *m, const mpasg_config *c, mpasg_fields *f, void *stream);
 /* The same step, recording events[i] (cudaEvent_t, timing enabled) at every stage
  * boundary and stage_kinds[i] = the MPASG_STAGE_* that ended there (i < n_events).
- * Works under stream capture (records external event nodes). Returns the number of
- * boundaries (>= 0) or a negative status. */
+ * Works under stream capture (records external event nodes). The stages run one after the
+ * other, so that the intervals are theirs alone; mpasg_step under capture runs independent
+ * ones side by side and takes less time than their sum. What a kernel of one stage does for
+ * another counts where it runs: the first acoustic edge update and, over flat terrain, the
+ * small-step w tendency in the tendencies, divergence damping in the acoustic substeps and
+ * the recovery, the saves and flux sums of a dynamics substep in the recovery. Returns the
+ * number of boundaries (>= 0) or a negative status. */
 int mpasg_step_timed(const mpasg_mesh *m, const mpasg_config *c, mpasg_fields *f,
                      void *const *events, int32_t *stage_kinds, int n_events, void *stream);
 /* Autotuner: times the tile shapes of the tuned kernels on the current state (the u

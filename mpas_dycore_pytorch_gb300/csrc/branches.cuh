@@ -14,7 +14,10 @@
 
 class GraphBranches {
  public:
-  explicit GraphBranches(cudaStream_t s) : s_(s) { on_ = current(base_) && !base_.empty(); }
+  // wanted = false: the launches keep the order they are issued in
+  explicit GraphBranches(cudaStream_t s, bool wanted = true) : s_(s) {
+    on_ = wanted && current(base_) && !base_.empty();
+  }
   bool active() const { return on_; }
   int next() { return on_ && !(collect() && set(base_)) ? MPASG_E_CUDA : MPASG_OK; }
   int join() {

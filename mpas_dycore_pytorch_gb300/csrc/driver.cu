@@ -353,6 +353,10 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
   mpasg_fields fa = f;
   fa.ke_edge = f.delsq_u;
 
+  // stages run beside each other in a captured step, but not where their boundaries are recorded:
+  // an interval between two of them is then one stage's own time
+  const bool overlap = rec == nullptr;
+
   // ---- RK integration setup
   MARK(MPASG_STAGE_BEGIN);
   // the time-level saves of the first dynamics substep (theta_m's padding row is zeroed); the
@@ -368,7 +372,7 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
     if (S > 0) job.push(f.scalars_init, f.scalars, ncs, advect && coupled ? f.scalars_a : nullptr);
     CHECK_RC(run_arrays(job, s));
   }
-  GraphBranches setup(s);
+  GraphBranches setup(s, overlap);
   if (c->precision == MPASG_PRECISION_MIXED) CHECK_RC(mpasgi_pack_f32(m, &f, s));
   else CHECK_RC(mpasgi_pvu(m, &f, s));
   // edge mean of theta_m_save and its reciprocal sum
@@ -382,7 +386,7 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
   for (int sub = 1; sub <= split; ++sub) {
     for (int rk = 1; rk <= 3; ++rk) {
       const double dts = rk_sub[rk - 1];
-      GraphBranches branches(s);  // the implicit coefficients beside the tendencies
+      GraphBranches branches(s, overlap);  // the implicit coefficients beside the tendencies
       if (rk == 1 || (rk == 2 && c->time_integration_order == 3)) {
         CHECK_RC(mpasg_vert_imp_coefs(m, c, &f, dts, stream));
         MARK(MPASG_STAGE_VIMP);
@@ -420,12 +424,12 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
       };
       // the cells' recovery beside the edges' and the diagnostics, which read only the edges;
       // over terrain w needs both, and so does the coupled transport
-      GraphBranches cells(s);
+      GraphBranches cells(s, overlap);
       CHECK_RC(recover(0));
       CHECK_RC(cells.next());
       CHECK_RC(recover(1));
       if (!m->flatTerrain || (coupled && advect)) CHECK_RC(cells.join());
-      GraphBranches terrain(s);
+      GraphBranches terrain(s, overlap);
       CHECK_RC(recover(2));
       MARK(MPASG_STAGE_RECOVER);
       if (!(coupled && advect)) CHECK_RC(terrain.next());
@@ -453,7 +457,7 @@ int step_impl(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* fin, cud
   // coupled mode: the scalars of the last RK stage are the step's (active rows only)
   if (advect && coupled) CHECK_RC(copy(f.scalars, f.scalars_a, nc * L * S, s));
   MARK(MPASG_STAGE_SPLIT);
-  GraphBranches last(s);  // the reconstructed wind beside the transport
+  GraphBranches last(s, overlap);  // the reconstructed wind beside the transport
   CHECK_RC(mpasgi_reconstruct(m, c, &f, s, true));
   MARK(MPASG_STAGE_RECONSTRUCT);
   if (part == 0) return MPASG_OK;
