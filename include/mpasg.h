@@ -150,8 +150,9 @@ typedef struct mpasg_config {
   int32_t horiz_mixing_smagorinsky; /* 1: 2d_smagorinsky */
   int32_t num_scalars, moist_start, moist_end;
   int32_t precision;                /* MPASG_PRECISION_FLOAT64 or MPASG_PRECISION_MIXED */
-  int32_t tile_tend_u;              /* levels per thread of the u tendency: 1 (0), 2 or 4
-                                       (autotuned; tiles agree to one FMA rounding) */
+  int32_t tile_tend_u;              /* mixed form: levels per thread of the u tendency, 1 (0), 2
+                                       or 4 (autotuned; tiles agree to one FMA rounding); the
+                                       float64 form has one tile and ignores it */
   /* mixing options of the large-step tendencies (dyn_tend.py:3367-3456, 2730-2780,
    * 4612-4650, 5064-5100): 2d_fixed del2 coefficient (kdiff everywhere), vertical mixing
    * of u and w / of theta (full state; 0 = off), CAM-style top-level damping (0 = off) */
@@ -189,7 +190,7 @@ typedef struct mpasg_fields {
   double *vorticity;                                                /* (V+1, L) */
   double *scalars;                                                  /* (C+1, L, S) */
   /* RK-step saves and split bookkeeping */
-  double *ru_save, *ruAvg_split;                                    /* (E+1, L) */
+  double *ru_save, *ruAvg_split;   /* (E+1, L)  *_split: sums of the substeps' mean fluxes */
   double *rw_save, *wwAvg_split;                                    /* (C+1, L+1) */
   double *rtheta_p_save, *rho_p_save, *theta_m_save, *rr_save, *rho_zz_old_split; /* (C+1, L) */
   double *scalars_init, *scalars_a, *scalars_b;                     /* (C+1, L, S) */
@@ -210,20 +211,27 @@ typedef struct mpasg_fields {
   double *ru_p;                                                     /* (E+1, L) */
   double *rw_p;                                                     /* (C+1, L+1) */
   double *rho_pp, *rtheta_pp, *rtheta_pp_old;                       /* (C+1, L) */
-  /* diagnostics scratch */
+  /* diagnostics scratch.  ke_edge, float64 form: the edge kinetic-energy weights inside the
+   * diagnostics, pv_edge u after them (read by the next tendencies of a step; mpasg_dyn_tend
+   * forms its own), ru_p times the edge theta after mpasg_acoustic_step.  A step keeps that
+   * theta flux in delsq_u, whose del2 of u is used up when tend_u is complete, and leaves
+   * delsq_w and delsq_theta unwritten without del4. */
   double *ke_edge;                                                  /* (E+1, L) */
   double *ke_vertex, *pv_vertex;                                    /* (V+1, L) */
   double *pv_cell;                                                  /* (C+1, L) */
   /* transport scratch */
-  double *hflux;        /* (E+1, L, S)  edge high-order values / limited fluxes */
-  double *flux_up, *flux_tmp;   /* (E+1, L, S) */
+  double *hflux;        /* (E+1, L, S)  explicit stage: ruAvg times the edge high-order value
+                           (mixed form: the value alone); monotone stage: limited fluxes */
+  double *flux_up, *flux_tmp;   /* (E+1, L, S)  monotone stage: upwind flux, high order minus it */
   double *s_max, *s_min, *scale_in, *scale_out, *rows;  /* (C+1, L, S) */
   double *wflux;        /* (C+1, L+1, S)  limiter vertical fluxes */
   double *rho_int;      /* (C+1, L) */
-  /* edge-side horizontal advective fluxes of w and theta_m (one value per edge) */
+  /* edge-side horizontal advective fluxes of w and theta_m (one value per edge; float64 form,
+   * later RK stages: with the perturbation flux dvEdge (ru_save - ru) theta_save) */
   double *flux_w_e, *flux_th_e;                                     /* (E+1, L) */
-  /* acoustic-step column scratch: rs / ts right-hand sides, tridiagonal rhs -> solution,
-   * and the b / c diagonals of the implicit system */
+  /* acoustic-step column scratch: rs / ts right-hand sides, tridiagonal rhs -> solution
+   * (left by mpasg_acoustic_step, not by a step), and the b / c diagonals of the implicit
+   * system */
   double *ac_rs, *ac_ts;                                            /* (C+1, L) */
   double *ac_x;                                                     /* (C+1, L+1) */
   double *b_tri, *c_tri;                                            /* (C+1, L) */

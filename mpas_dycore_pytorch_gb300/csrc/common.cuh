@@ -189,6 +189,9 @@ struct TendFusion {
   bool hdiv_current = false;  // h_divergence already holds ru's divergence (later RK stages)
   bool v_current = false;     // v is the TRiSK sum of u (left by the last RK stage's diagnostics)
 };
+// copies_current, float64 form: ke_edge holds pv_edge u, that is, mpasgi_pvu or the diagnostics
+// were the last to write it (the acoustic substeps between them take another ke_edge), and
+// theta_edge_save is that of theta_m_save
 int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f, int rk_step, cudaStream_t s,
                     bool copies_current, const TendFusion& fuse = TendFusion());
 struct DiagFusion {

@@ -11,9 +11,11 @@
 //
 // Accuracy.  A value is 60 bits wide after alignment (53 significant), a weight 60 bits;
 // of their product the low x low partial is dropped (a balanced split, so it is centred).
-// The error of a sum of n terms is below (n + 1) 2^-55 of its largest term, about an eighth
-// of what n rounded multiply-adds may lose; sums whose terms are exact and cancel exactly
-// give zero.  Sums the format cannot hold (a non-finite or subnormal-range value, a total
+// A sum of n terms loses below (n + 1) 2^-55 of its largest term before it is rounded (2^-54.9
+// the worst of 10 and 14 terms spread over 16 binades), and the one rounding adds at most 2^-53
+// of the result.  Against a chain of n multiply-adds, which rounds n times, that is 0.4 to 0.65
+// of its root mean square error and a third to a half of its worst.  Sums whose terms are
+// exact and cancel exactly give zero.  Sums the format cannot hold (a non-finite or subnormal-range value, a total
 // near the ends of the exponent range) are reported to the caller, which evaluates them in
 // float64; values that are all zero sum to +0.
 #pragma once
