@@ -386,9 +386,10 @@ __global__ void k_acoustic_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, int s
 // ---------------------------------------------------------------- acoustic substep, columns
 // dynamics/acoustic_step.py:456 (cell flux sums), :675 (RHS), :772 (Thomas solve,
 // implicit Rayleigh damping, post-solve rho_pp / rtheta_pp); Thomas sweeps from
-// autodiff/tridiagonal_solve.py:56-63.  Three kernels: k_ac_prep (every level in
-// parallel: flux sums, rs / ts, tridiagonal right-hand side), k_ac_thomas (one thread
-// per column: forward elimination and back substitution only) and k_ac_post (every
+// autodiff/tridiagonal_solve.py:56-63.  One launch (k_ac_columns, k_ac_columns_mixed), or in
+// float64 three, for the forward mode and for columns too high for shared memory: k_ac_prep
+// (every level in parallel: flux sums, rs / ts, tridiagonal right-hand side), k_ac_thomas (one
+// thread per column: forward elimination and back substitution only) and k_ac_post (every
 // level in parallel: Rayleigh damping, ww accumulation, rho_pp / rtheta_pp update).
 
 // edge mean of theta_m_save, 0.5 (theta_2 + theta_1), the value the acoustic right-hand
@@ -631,8 +632,8 @@ MPASG_D AcLevelF ac_level_mixed(const mpasg_mesh& m, const mpasg_fields& f, int 
   a.drs = dts * cv<float>(f.tend_rho[o]) + rs - cv<float>(f.cofrz[k]) * resm * (rwp_k1 - rwp_k);
   a.dts = dts * cv<float>(f.tend_theta[o]) + ts -
           resm * m.rdzw_f32[k] * (cv<float>(f.coftz[ow + 1]) * rwp_k1 - cv<float>(f.coftz[ow]) * rwp_k);
-  if (rs64) *rs64 = rho_in + f64(a.drs);
-  if (ts64) *ts64 = rt_in + f64(a.dts);
+  *rs64 = rho_in + f64(a.drs);
+  *ts64 = rt_in + f64(a.dts);
   return a;
 }
 
@@ -648,45 +649,6 @@ MPASG_D float ac_rhs_mixed(const mpasg_mesh& m, const mpasg_fields& f, size_t o,
              ((zz_k * ts_k - zz_km1 * ts_km1) + resm * (zz_k * lv.rt_in - zz_km1 * lo.rt_in)) -
          cv<float>(f.cofwr[o + k]) * ((rs_k + rs_km1) + resm * (lv.rho_in + lo.rho_in)) +
          cw_k * (ts_k + resm * lv.rt_in) + cw_km1 * (ts_km1 + resm * lo.rt_in);
-}
-
-__global__ void __launch_bounds__(kBlock) k_ac_prep_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl1,
-                                                          int small_step, float dts, float epssm, float resm) {
-  __shared__ AcLevelF s_lv[kBlock];
-  const int L = m.nVertLevels;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i < (uint32_t)m.nCells * (L + 1);
-  const bool first = (small_step == 1);
-  uint32_t c = 0, k = 0;
-  AcLevelF lv{0.0f, 0.0f, 0.0f, 0.0f};
-  double rs64 = 0.0, ts64 = 0.0;
-  if (active) {
-    c = fl1.div(i);
-    k = i - c * (L + 1);
-    if (k < (uint32_t)L) lv = ac_level_mixed(m, f, c, k, first, dts, resm, &rs64, &ts64);
-  }
-  s_lv[threadIdx.x] = lv;
-  __syncthreads();
-  if (!active) return;
-  const size_t o = (size_t)c * L;
-  const size_t ow = (size_t)c * (L + 1);
-  if (k < (uint32_t)L) {
-    f.ac_rs[o + k] = rs64;
-    f.ac_ts[o + k] = ts64;
-    f.rtheta_pp_old[o + k] = first ? 0.0 : f.rtheta_pp[o + k];
-  }
-  const double rwp_k = first ? 0.0 : f.rw_p[ow + k];
-  if (k == 0 || k == (uint32_t)L) {  // boundary values pass through the solve unchanged
-    f.ac_x[ow + k] = rwp_k;
-    if (first) f.wwAvg[ow + k] = 0.0;
-    return;
-  }
-  const AcLevelF lo = (threadIdx.x >= 1) ? s_lv[threadIdx.x - 1]
-                                         : ac_level_mixed(m, f, c, k - 1, first, dts, resm, nullptr, nullptr);
-  const double ww_in = first ? 0.0 : f.wwAvg[ow + k];
-  f.wwAvg[ow + k] = ww_in + f64(0.5f * (1.0f - epssm) * cv<float>(rwp_k));
-  const float inc = ac_rhs_mixed(m, f, o, ow, k, lv, lo, dts, resm);
-  f.ac_x[ow + k] = rwp_k + f64(inc);
 }
 
 // Rayleigh damping of the solution (float64); levels without damping pass through
@@ -711,33 +673,6 @@ MPASG_D double ac_level_out_mixed(const mpasg_mesh& m, const mpasg_fields& f, si
   f.rho_pp[o] = rho;
   f.rtheta_pp[o] = ts - f64(m.rdzw_f32[k] * (cv<float>(f.coftz[ow + 1]) * x1 - cv<float>(f.coftz[ow]) * x0));
   return rho;
-}
-
-__global__ void __launch_bounds__(kBlock) k_ac_post_mixed(mpasg_mesh m, mpasg_fields f, FastDiv fl1, double dts,
-                                                          float epssm) {
-  __shared__ double s_xr[kBlock];
-  const int L = m.nVertLevels;
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = i < (uint32_t)m.nCells * (L + 1);
-  uint32_t c = 0, k = 0;
-  size_t o = 0, ow = 0;
-  double xr = 0.0;
-  if (active) {
-    c = fl1.div(i);
-    k = i - c * (L + 1);
-    o = (size_t)c * L;
-    ow = (size_t)c * (L + 1);
-    xr = ac_damped_mixed(m, f, o, ow, k, L, f.ac_x[ow + k], dts);
-  }
-  s_xr[threadIdx.x] = xr;
-  __syncthreads();
-  if (!active) return;
-  f.rw_p[ow + k] = xr;
-  if (k >= 1 && k < (uint32_t)L) f.wwAvg[ow + k] = f.wwAvg[ow + k] + f64(0.5f * (1.0f + epssm) * cv<float>(xr));
-  if (k == (uint32_t)L) return;
-  const double xr1 = (threadIdx.x + 1 < blockDim.x) ? s_xr[threadIdx.x + 1]
-                                                    : ac_damped_mixed(m, f, o, ow, k + 1, L, f.ac_x[ow + k + 1], dts);
-  ac_level_out_mixed(m, f, o + k, ow + k, k, f.ac_rs[o + k], f.ac_ts[o + k], xr, xr1);
 }
 
 // The same sweeps with the columns staged through shared memory: one warp solves 32
@@ -777,43 +712,6 @@ __global__ void __launch_bounds__(kThomasThreads) k_ac_thomas_staged(mpasg_mesh 
   }
   __syncthreads();
   if (t < ncol) thomas_column(sx + t, sa + t, sal + t, sg + t, L, kThomasPitch);
-  __syncthreads();
-  double* gxo = f.ac_x + (size_t)c0 * (L + 1);
-  for (uint32_t idx = t; idx < nw; idx += kThomasThreads) {
-    uint32_t col = fl1.div(idx), k = idx - col * (L + 1);
-    gxo[idx] = sx[k * kThomasPitch + col];
-  }
-}
-
-// Mixed form (still float64): u_k = alpha_k x_k + m_k u_(k-1) with m_k = -alpha_k a_k
-// precomputed by the factorisation, so the serial dependence is one FMA per level
-// (alpha_k x_k does not depend on the chain and issues ahead).
-__global__ void __launch_bounds__(kThomasThreads) k_ac_thomas_staged_mixed(mpasg_mesh m, mpasg_fields f,
-                                                                           FastDiv fl, FastDiv fl1) {
-  extern __shared__ double s_col[];
-  const int L = m.nVertLevels;
-  double* sx = s_col;
-  double* sm = sx + (size_t)(L + 1) * kThomasPitch;
-  double* sal = sm + (size_t)L * kThomasPitch;
-  double* sg = sal + (size_t)L * kThomasPitch;
-  const int c0 = blockIdx.x * kThomasCols;
-  const int ncol = min(kThomasCols, m.nCells - c0);
-  const int t = threadIdx.x;
-  const uint32_t nw = (uint32_t)ncol * (L + 1), nl = (uint32_t)ncol * L;
-  const double* gx = f.ac_x + (size_t)c0 * (L + 1);
-  const size_t o0 = (size_t)c0 * L;
-  for (uint32_t idx = t; idx < nw; idx += kThomasThreads) {
-    uint32_t col = fl1.div(idx), k = idx - col * (L + 1);
-    sx[k * kThomasPitch + col] = gx[idx];
-  }
-  for (uint32_t idx = t; idx < nl; idx += kThomasThreads) {
-    uint32_t col = fl.div(idx), k = idx - col * L;
-    sm[k * kThomasPitch + col] = f.tri_m[o0 + idx];
-    sal[k * kThomasPitch + col] = f.alpha_tri[o0 + idx];
-    sg[k * kThomasPitch + col] = f.gamma_tri[o0 + idx];
-  }
-  __syncthreads();
-  if (t < ncol) thomas_column<true>(sx + t, sm + t, sal + t, sg + t, L, kThomasPitch);
   __syncthreads();
   double* gxo = f.ac_x + (size_t)c0 * (L + 1);
   for (uint32_t idx = t; idx < nw; idx += kThomasThreads) {
@@ -1364,7 +1262,7 @@ static int launch_ac_columns(const mpasg_mesh* m, const mpasg_fields* f, bool mi
   const bool first = small_step == 1;
   const int cols = columns_per_block(m->nCells, L + 1, 600, 18, 2), nb = nblocks(m->nCells, cols);
   const size_t smem = mixed ? ac_columns_mixed_smem_bytes(L, cols) : ac_columns_smem_bytes(L, cols, N, first);
-  // the mixed form refuses the columns its staged solve cannot hold, on either path
+  // (the mixed form takes up to 193 levels, 32 columns of its solve's four arrays)
   *done = smem <= kMaxSmem && !(mixed && thomas_smem_bytes(L) > kMaxSmem);
   if (!*done) return MPASG_OK;
   const auto run = [&](auto kernel, auto... args) -> int {
@@ -1500,43 +1398,19 @@ int mpasgi_acoustic_parts(const mpasg_mesh* m, const mpasg_config* c, mpasg_fiel
       const int rc = launch_ac_columns(m, f, mixed, small_step, dts, c->epssm, resm, !fuse.scratch, fuse.last, s, &done);
       if (rc != MPASG_OK || done) return rc;
     }
-    if (mixed) {
-      k_ac_prep_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), small_step, (float)dts,
-                                                      (float)c->epssm, (float)resm);
-      MPASG_LAUNCH_CHECK();
-    } else {
-      const int rc = launch_ac_prep(m, f, small_step, dts, c->epssm, resm, s);
-      if (rc != MPASG_OK) return rc;
-    }
-    if (part == 0) return MPASG_OK;
+    if (mixed) return MPASG_E_ARG;  // its columns in one launch only
+    const int rc = launch_ac_prep(m, f, small_step, dts, c->epssm, resm, s);
+    if (rc != MPASG_OK || part == 0) return rc;
   }
-  // the staged solve needs more than 48 KB of dynamic shared memory: opt in once per
-  // device (the first call on a device should come before any stream capture)
   const size_t smem = thomas_smem_bytes(L);
-  static bool smem_opt_in[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MPASG_E_CUDA;
-  if (!smem_opt_in[dev])
-    smem_opt_in[dev] =
-        cudaFuncSetAttribute(k_ac_thomas_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
-            cudaSuccess &&
-        cudaFuncSetAttribute(k_ac_thomas_staged_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
-            cudaSuccess;
-  if (smem_opt_in[dev] && smem <= 200 * 1024 && mixed)
-    k_ac_thomas_staged_mixed<<<nblocks(m->nCells, kThomasCols), kThomasThreads, smem, s>>>(*m, *f, FastDiv(L),
-                                                                                        FastDiv(L + 1));
-  else if (smem_opt_in[dev] && smem <= 200 * 1024)
-    k_ac_thomas_staged<<<nblocks(m->nCells, kThomasCols), kThomasThreads, smem, s>>>(*m, *f, FastDiv(L),
-                                                                                  FastDiv(L + 1));
-  else if (mixed)
-    return MPASG_E_ARG;  // the mixed sweep needs the staged kernel (L <= 200)
-  else
+  if (smem <= kMaxSmem) {
+    if (!allow_smem(k_ac_thomas_staged, smem)) return MPASG_E_CUDA;
+    k_ac_thomas_staged<<<nblocks(m->nCells, kThomasCols), kThomasThreads, smem, s>>>(*m, *f, FastDiv(L), FastDiv(L + 1));
+  } else {
     k_ac_thomas<<<nblocks(m->nCells, 64), 64, 0, s>>>(*m, *f);
+  }
   MPASG_LAUNCH_CHECK();
-  if (mixed)
-    k_ac_post_mixed<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, (float)c->epssm);
-  else
-    k_ac_post<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, 0.5 * (1.0 + c->epssm));
+  k_ac_post<<<nblocks(ncw), kBlock, 0, s>>>(*m, *f, FastDiv(L + 1), dts, 0.5 * (1.0 + c->epssm));
   MPASG_LAUNCH_CHECK();
   if (fuse.last) {
     k_recover_rho<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, (uint32_t)m->nCells * L);
