@@ -1400,8 +1400,9 @@ int mpasgi_dyn_tend(const mpasg_mesh* m, const mpasg_config* c, mpasg_fields* f,
 
 // Autotuner: times the u-tendency kernel with 1, 2 and 4 levels per thread on the current
 // state (rk-2 form, 3 launches each after one warm-up) and keeps the fastest in
-// c->tile_tend_u.  (The float64 form has one tile: its three candidates are the same kernel.)  Host-synchronising: call it outside stream capture.  The kernels only
-// write their outputs (tend_u, ...) and the ke_edge scratch, so the state is unchanged.
+// c->tile_tend_u.  The float64 form has one tile: it is timed once and kept, its time reported
+// for all three.  Host-synchronising: call it outside stream capture.  The kernels only write
+// their outputs (tend_u, ...) and the ke_edge scratch, so the state is unchanged.
 extern "C" int mpasg_autotune(const mpasg_mesh* m, mpasg_config* c, mpasg_fields* f, float* times_ms,
                               void* stream) {
   if (!m || !c || !f) return MPASG_E_ARG;
@@ -1428,6 +1429,10 @@ extern "C" int mpasg_autotune(const mpasg_mesh* m, mpasg_config* c, mpasg_fields
   int best_tile = 1;
   int rc = MPASG_OK;
   for (int t = 0; t < 3 && rc == MPASG_OK; ++t) {
+    if (!mixed && t > 0) {
+      if (times_ms) times_ms[t] = times_ms[0];
+      continue;
+    }
     const int vt = tiles[t];
     const int nchunk = (L + vt - 1) / vt;
     const long long nth = (long long)m->nEdges * nchunk;

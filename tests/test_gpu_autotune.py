@@ -60,3 +60,11 @@ def test_autotune_picks_a_candidate():
     res = m.autotune()
     assert res["tend_u_levels_per_thread"] in (1, 2, 4)
     assert all(t > 0 for t in res["tend_u_ms"].values())
+
+
+def test_autotuner_of_the_float64_form():
+    """One tile, timed once."""
+    need_gpu()
+    res = _model("float64", 4).autotune()
+    assert res["tend_u_levels_per_thread"] == 1
+    assert len(set(res["tend_u_ms"].values())) == 1
