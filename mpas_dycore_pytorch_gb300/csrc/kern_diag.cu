@@ -354,6 +354,14 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_edges_b_fx(mpasg_mesh m, mpa
   f.ke_edge[i] = pve * u;
 }
 
+int sm_count() {  // of the current device; 0 where it cannot be told
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+    return n;
+  cudaGetLastError();
+  return 0;
+}
+
 int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_fields* f, int rk_step, cudaStream_t s,
                    const DiagFusion& fuse) {
   const int apvm = c->apvm_upwinding > 0.0 ? 1 : 0;
@@ -377,10 +385,11 @@ int launch_diag_fx(const mpasg_mesh* m, const mpasg_config* c, const mpasg_field
     return MPASG_OK;
   };
   // a captured step of a small mesh (at most a block of cells an SM): the divergences beside the
-  // vertices (step of 162 x 12 455 -> 447 us, 642 x 26 581 -> 573, 642 x 55 787 -> 786; from
-  // 2562 x 26 on the launch costs what the overlap gives)
+  // vertices (step of 162 x 12 475 -> 469 us, 642 x 26 589 -> 584, 642 x 55, 138 blocks of
+  // cells, 798 -> 794; 2562 x 26 within the 0.8 % two builds differ by; 40962 x 55 22.72 ->
+  // 22.89 ms)
   GraphBranches branches(s);
-  const bool split = branches.active() && nc <= 152;
+  const bool split = branches.active() && nc <= sm_count();
   if (split) {
     int rc = cells(k_diag_cells_fx<6, 1>, k_diag_cells_fx<10, 1>);
     if (rc == MPASG_OK) rc = branches.next();
