@@ -239,8 +239,8 @@ MPASG_D void factor_column(const double* a, const double* b, const double* c, do
 // 1334, 40962 x 55 25.58 -> 25.37 ms (mixed form 17.61 -> 17.27).
 // SHARED: the levels' cofwt and coftz wait for their neighbours in shared memory too; without it
 // the neighbours are read back from memory and an SM holds five blocks of 27 columns of 55
-// levels instead of three: 255 -> 228 us at 40962 x 55 (step 21.67 -> 21.55 ms).  Where five fit
-// all the same, memory only adds latency (step at 2562 x 26 1025 -> 1053 us).
+// levels instead of three: 255 -> 228 us at 40962 x 55 (step 22.82 -> 22.72 ms).  Where five fit
+// all the same, memory only adds latency (step at 2562 x 26 1071 -> 1096 us).
 template <typename T, bool SHARED>
 __global__ void __launch_bounds__(kBlock) k_vimp_columns(mpasg_mesh m, mpasg_fields f, FastDiv fl, int cols,
                                                          VimpScalars s) {

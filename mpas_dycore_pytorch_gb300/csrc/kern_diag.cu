@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_diag_cells_fx(mpasg_mesh m, mpasg
 #pragma unroll
       for (int j = 0; j < N; ++j) {
         x[j] = j < n ? f.ke_edge[(uint32_t)s_w[t + j].row * L + k] : 0.0;
-        if (j < n) kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
+        // (a corner without a kite has a zero weight and names another vertex, which may hold NaN)
+        if (s_k[t + j].e != 0u) kev = fma(s_a[t + j], f.ke_vertex[(uint32_t)s_k[t + j].row * L + k], kev);
       }
       bool summed = false;
       if constexpr (N <= 8) {
