@@ -49,10 +49,10 @@ __global__ void k_pattern_c(mpasg_mesh m, FastDiv fl, int S, const double* __res
 // (fixdot.cuh), comparisons, minima and clamps on the integer side too (each would take a
 // float64 slot).
 // A launch numbers its (row, value) threads in 32 bits and divides by FastDiv, which holds below
-// 2^31: rows that reach it are taken in several launches, each from its own first row, and
-// indices into the fields are 64 bits wide (monotone stage at 40962 x 55 x 3 1404 -> 1413 us,
-// explicit at 2562 x 37 x 8 84.0 -> 84.2, the first rows' 64-bit offset rather than the gathers'
-// width).  (A build may lower the limit to test the split.)
+// 2^31: rows that reach it are taken in several launches.  A launch gets its first row and, for
+// the fields its threads index by their own number, pointers to that row (a 64-bit index in the
+// thread instead cost the monotone stage at 40962 x 55 x 3 0.6 %); gathers by row are 64 bits
+// wide.  (A build may lower the limit to test the split.)
 #ifndef MPASG_MAX_THREADS
 #define MPASG_MAX_THREADS (0x7fffffffu - kBlock)
 #endif
@@ -148,10 +148,9 @@ int launch_edge_flux_fx(const mpasg_mesh* m, int S, double dt, const double* uh,
   return m->nAdvMax <= 10 ? run(k_edge_flux_fx<10, MONO>, 10) : run(k_edge_flux_fx<14, MONO>, 14);
 }
 
-// the place of a launch's thread i in a (cell, level, scalar) row; at: its index in the fields
+// the place of a launch's thread i in a (cell, level, scalar) row
 struct CellRow {
   uint32_t c, r, k, s;
-  size_t at;
 };
 MPASG_D CellRow cell_row(uint32_t i, uint32_t first, const FastDiv& fr, const FastDiv& fs) {
   CellRow t;
@@ -160,7 +159,6 @@ MPASG_D CellRow cell_row(uint32_t i, uint32_t first, const FastDiv& fr, const Fa
   t.r = i - cr * fr.d;
   t.k = fs.div(t.r);
   t.s = t.r - t.k * fs.d;
-  t.at = (size_t)first * fr.d + i;
   return t;
 }
 
@@ -179,6 +177,7 @@ MPASG_D double interface_value(const double* __restrict__ q, uint32_t S, double 
   return fma(low ? fnm[k] : f3[0], a, fma(low ? fnp[k] : f3[1], b, -fma(f3[2], a2, f3[3] * b2)));
 }
 
+// (s_old, s_out: from the launch's first row; s_new: all rows)
 // explicit stage update: 17 float64 operations a value and one integer sum, about 33 in the
 // per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage)
 template <int N>
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, m
   const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   const bool active = i < n_all;
-  CellRow t{c0, 0, 0, 0, 0};
+  CellRow t{c0, 0, 0, 0};
   auto flux_at = [&](uint32_t k) {  // at the interface below level k of this thread's column
     if (k == 0 || k >= L) return 0.0;
     const double ww = f.wwAvg[(size_t)t.c * (L + 1) + k];
@@ -217,7 +216,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, m
   const double rho_old = f.rho_zz_old_split[ic];
   double rho = f.rho_zz[ic];
   if (p.w_old != 0.0) rho = p.w_old * rho_old + p.w_new * rho;
-  s_out[t.at] = fx::quotient(fma(p.dt, tend, s_old[t.at] * rho_old), rho);
+  s_out[i] = fx::quotient(fma(p.dt, tend, s_old[i] * rho_old), rho);
 }
 
 // monotone stage: density at its end
@@ -241,12 +240,13 @@ template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
                                                             uint32_t first, uint32_t n_all, TransportScalars p,
                                                             const double* __restrict__ so,
+                                                            const double* __restrict__ so_own,
                                                             const double* __restrict__ sn) {
   __shared__ double s_wm[kBlock], s_fu[kBlock];
   const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
   const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   const bool active = i < n_all;
-  CellRow t{0, 0, 0, 0, 0};
+  CellRow t{0, 0, 0, 0};
   auto fluxes = [&](uint32_t k, double* wm, double* fu) {
     *wm = *fu = 0.0;
     if (k == 0 || k >= L) return;
@@ -277,16 +277,15 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
   }
   if (t.k >= 1) f.wflux[((size_t)t.c * (L + 1) + t.k) * S + t.s] = wm_lo;
   // bounds over the column's neighbours and the adjacent cells
-  const size_t at = t.at;
-  const double here = so[at];
+  const double here = so_own[i];
   int64_t kmax = fx::order_key(here), kmin = kmax;
   auto bound = [&](double x) {
     const int64_t q = fx::order_key(x);
     kmax = q > kmax ? q : kmax;
     kmin = q < kmin ? q : kmin;
   };
-  if (t.k >= 1) bound(so[at - S]);
-  if (t.k + 1 < L) bound(so[at + S]);
+  if (t.k >= 1) bound(so_own[i - S]);
+  if (t.k + 1 < L) bound(so_own[i + S]);
   const size_t oc = (size_t)t.c * m.maxEdges;
   const int n = m.nEdgesOnCell[t.c];
 #pragma unroll
@@ -307,20 +306,20 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
       smax = fmax(smax, x);
       smin = fmin(smin, x);
     };
-    if (t.k >= 1) wide(so[at - S]);
-    if (t.k + 1 < L) wide(so[at + S]);
+    if (t.k >= 1) wide(so_own[i - S]);
+    if (t.k + 1 < L) wide(so_own[i + S]);
     for (int j = 0; j < n; ++j) {
       const int nb = m.cellsOnCell[oc + j];
       if (nb < m.nCells) wide(so[(size_t)nb * row + t.r]);
     }
   }
   const double rd = m.rdnw[t.k];
-  f.rows[at] = fma(rd, fu_lo - fu_hi, here * f.rho_zz_old_split[(size_t)t.c * L + t.k]);
+  f.rows[i] = fma(rd, fu_lo - fu_hi, here * f.rho_zz_old_split[(size_t)t.c * L + t.k]);
   // in and out fluxes of the correction through the level's two interfaces
-  f.scale_in[at] = rd * (fx::positive(wm_lo) + fx::positive(-wm_hi));
-  f.scale_out[at] = -rd * (fx::positive(wm_hi) + fx::positive(-wm_lo));
-  f.s_max[at] = smax;
-  f.s_min[at] = smin;
+  f.scale_in[i] = rd * (fx::positive(wm_lo) + fx::positive(-wm_hi));
+  f.scale_out[i] = -rd * (fx::positive(wm_hi) + fx::positive(-wm_lo));
+  f.s_max[i] = smax;
+  f.s_min[i] = smin;
 }
 
 // per value: horizontal upwind update and scale sums, then the limiter factors.  Three integer
@@ -362,12 +361,11 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpa
       in = in + mz(-sf);
     }
   }
-  const size_t at = t.at;
-  const double rows = fma(-ia, up, f.rows[at]), eps = 1.0e-20;
-  const double sin_ = fma(ia, in, f.scale_in[at]) + eps, sout = fma(ia, out, -f.scale_out[at]) + eps;
-  f.rows[at] = rows;
-  f.scale_in[at] = fx::clamp01(fx::quotient(fma(f.s_max[at], rint, -rows), sin_));
-  f.scale_out[at] = fx::clamp01(fx::quotient(fma(-f.s_min[at], rint, rows), sout));
+  const double rows = fma(-ia, up, f.rows[i]), eps = 1.0e-20;
+  const double sin_ = fma(ia, in, f.scale_in[i]) + eps, sout = fma(ia, out, -f.scale_out[i]) + eps;
+  f.rows[i] = rows;
+  f.scale_in[i] = fx::clamp01(fx::quotient(fma(f.s_max[i], rint, -rows), sin_));
+  f.scale_out[i] = fx::clamp01(fx::quotient(fma(-f.s_min[i], rint, rows), sout));
 }
 
 // per (edge, value): limited horizontal flux (stored in hflux)
@@ -375,12 +373,11 @@ __global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_all) return;
   const uint32_t er = fr.div(i), e = first + er, r = i - er * fr.d;
-  const size_t at = (size_t)first * fr.d + i;
-  const double ft = f.flux_tmp[at];
+  const double ft = f.flux_tmp[i];
   const uint32_t back = __double2hiint(ft) < 0 ? 1u : 0u;
   const size_t from = (size_t)m.cellsOnEdge[2 * e + back] * fr.d + r;
   const size_t to = (size_t)m.cellsOnEdge[2 * e + 1 - back] * fr.d + r;
-  f.hflux[at] = ft * fx::min_nonneg(f.scale_out[from], f.scale_in[to]);
+  f.hflux[i] = ft * fx::min_nonneg(f.scale_out[from], f.scale_in[to]);
 }
 
 // per value: limited horizontal and vertical fluxes, positivity
@@ -396,17 +393,16 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_c_fx(mpasg_mesh m, mpa
   __syncthreads();
   if (i >= n_all) return;
   const CellRow t = cell_row(i, first, fr, fs);
-  const size_t at = t.at;
   const double* wf = f.wflux + ((size_t)t.c * (L + 1) + t.k) * S + t.s;
-  auto limited = [&](double wm, size_t below, size_t above) {  // an upward flux leaves `below`
+  auto limited = [&](double wm, uint32_t below, uint32_t above) {  // an upward flux leaves `below`
     const bool down = __double2hiint(wm) < 0;
     return wm * fx::min_nonneg(f.scale_out[down ? above : below], f.scale_in[down ? below : above]);
   };
-  const double lo = t.k >= 1 ? limited(wf[0], at - S, at) : 0.0;
-  const double hi = t.k + 1 < L ? limited(wf[S], at, at + S) : 0.0;
+  const double lo = t.k >= 1 ? limited(wf[0], i - S, i) : 0.0;
+  const double hi = t.k + 1 < L ? limited(wf[S], i, i + S) : 0.0;
   const double h = cellsum::fixed<N, size_t>(m, t.c, m.nEdgesOnCell[t.c], s_c + (t.c - c0) * N, f.hflux, row, t.r);
-  const double rows = fma(m.rdnw[t.k], lo - hi, fma(-m.invAreaCell[t.c], h, f.rows[at]));
-  s_out[at] = fx::positive(fx::quotient(rows, f.rho_int[(size_t)t.c * L + t.k]));
+  const double rows = fma(m.rdnw[t.k], lo - hi, fma(-m.invAreaCell[t.c], h, f.rows[i]));
+  s_out[i] = fx::positive(fx::quotient(rows, f.rho_int[(size_t)t.c * L + t.k]));
 }
 
 template <typename T>
@@ -736,7 +732,8 @@ int launch_scalars_fx(const mpasg_mesh* m, const mpasg_fields& g, const Transpor
   const size_t smem = cellsum::max_cells(row) * N * sizeof(cellsum::Slot);
   return launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
     k_scalars_update_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(
-        *m, g, FastDiv(row), FastDiv(S), first, n * row, p, g.scalars_init, g.scalars_a, g.scalars_b);
+        *m, g, FastDiv(row), FastDiv(S), first, n * row, p, g.scalars_init + (size_t)first * row, g.scalars_a,
+        g.scalars_b + (size_t)first * row);
   });
 }
 
@@ -750,22 +747,38 @@ int launch_scalars_mono_fx(const mpasg_mesh* m, const mpasg_fields* f, const Tra
   if (rc != MPASG_OK) return rc;
   k_mono_density_fx<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), p.dt);
   MPASG_LAUNCH_CHECK();
+  // the fields a launch's threads index by their own number, from its first row
+  const auto own_cells = [&](size_t at) {
+    mpasg_fields g = *f;
+    g.rows += at;
+    g.scale_in += at;
+    g.scale_out += at;
+    g.s_max += at;
+    g.s_min += at;
+    return g;
+  };
   rc = launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
-    k_mono_cells_a_fx<N><<<nblocks((long long)n * row), kBlock, 0, s>>>(*m, *f, fr, fs, first, n * row, p,
-                                                                        f->scalars_init, f->scalars_a);
+    const size_t at = (size_t)first * row;
+    k_mono_cells_a_fx<N><<<nblocks((long long)n * row), kBlock, 0, s>>>(
+        *m, own_cells(at), fr, fs, first, n * row, p, f->scalars_init, f->scalars_init + at, f->scalars_a);
   });
   if (rc != MPASG_OK) return rc;
   rc = launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
-    k_mono_cells_b_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, *f, fr, fs, first, n * row);
+    k_mono_cells_b_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, own_cells((size_t)first * row), fr, fs,
+                                                                           first, n * row);
   });
   if (rc != MPASG_OK) return rc;
   rc = launch_rows(m->nEdges, row, [&](uint32_t first, uint32_t n) {
-    k_mono_edges_b_fx<<<nblocks((long long)n * row), kBlock, 0, s>>>(*m, *f, fr, first, n * row);
+    mpasg_fields g = *f;
+    g.flux_tmp += (size_t)first * row;
+    g.hflux += (size_t)first * row;
+    k_mono_edges_b_fx<<<nblocks((long long)n * row), kBlock, 0, s>>>(*m, g, fr, first, n * row);
   });
   if (rc != MPASG_OK) return rc;
   return launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
-    k_mono_cells_c_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, *f, fr, fs, first, n * row,
-                                                                           f->scalars_b);
+    const size_t at = (size_t)first * row;
+    k_mono_cells_c_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, own_cells(at), fr, fs, first, n * row,
+                                                                           f->scalars_b + at);
   });
 }
 
