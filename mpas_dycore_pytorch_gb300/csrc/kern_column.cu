@@ -1140,8 +1140,8 @@ __global__ void __launch_bounds__(kBlock) k_recover_cells(mpasg_mesh m, mpasg_fi
 
 // FINISH: with the last acoustic substep's divergence damping before it and the diagnostics'
 // edge fields (k_diag_edges_a) after it: one pass over the edges instead of three.  Bound by the
-// float64 pipe (80 %, 11 operations an edge level; 168 us at 40962 x 55, 233 with the saves and
-// flux sums of a substep's end).
+// float64 pipe (73-75 % of the time at 10242 x 41): 13 operations an edge level, 18 with the saves
+// and flux sums of a substep's end, 168 and 233 us at 40962 x 55.
 template <typename T, bool FINISH, bool FROM_ZERO>
 __global__ void k_recover_edges(mpasg_mesh m, mpasg_fields f, FastDiv fl, double inv_ns, double damp_coef,
                                 RecoverTail tail) {

@@ -391,8 +391,9 @@ __global__ void __launch_bounds__(kBlock) k_tend_u_chunk(mpasg_mesh m, mpasg_fie
 // 40962 x 55, a later RK stage: 628 us in float64, 378 us here with the first acoustic edge
 // update (one of the sums in float64: 23 us more), the first stage 970 -> 434 us.  48 registers
 // (5 blocks an SM): 346 us in a tuning loop against 593 us at 80 registers, 362 at 64 and 361 at
-// 40, the latency of 22 warps an SM being what held the 80-register build.  The float64 pipe
-// is now 66 % busy with ~21 operations an edge level, the issue slots 39 %.
+// 40, the latency of 22 warps an SM being what held the 80-register build; at 48 it spills 216
+// bytes of stores and 204 of loads a thread (14 slots: 492 and 504).  The float64 pipe
+// is now 74 % busy with ~21 operations an edge level, the issue slots 32 % (10242 x 41).
 // The block converts the weights of the 5-7 edges it covers once, into shared memory
 // (with the neighbour rows), so a term costs its thread one 16-byte broadcast and one gather.
 // The upwind combination of flux3 with coefficient 1 is a three-point formula,
@@ -657,7 +658,7 @@ MPASG_D double theta_vmix(const mpasg_mesh& m, const mpasg_fields& f, uint32_t c
 //   k_mix_cells    their divergences: 2 delsq_w, delsq_theta                  (del4 on only)
 //   k_mix_edges_b  the del2 fluxes with the eddy viscosity, minus the del4 fluxes, in place
 //   k_mix_cells    their divergences: tend_w_euler, tend_theta_euler
-// 11 + 8 float64 operations an edge level and 14 a cell level instead of 193 a cell level; the
+// 8 + 12 float64 operations an edge level and 8 a cell level and pass instead of 193 a cell level; the
 // four kernels take 1.16 ms a step at 40962 x 55, the two cell kernels before them 2.44 ms.
 struct MixEdge {
   double dvdc;      // dvEdge / dcEdge

@@ -177,9 +177,9 @@ MPASG_D double interface_value(const double* __restrict__ q, uint32_t S, double 
   return fma(low ? fnm[k] : f3[0], a, fma(low ? fnp[k] : f3[1], b, -fma(f3[2], a2, f3[3] * b2)));
 }
 
-// (s_old, s_out: from the launch's first row; s_new: all rows)
-// explicit stage update: 17 float64 operations a value and one integer sum, about 33 in the
-// per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage)
+// explicit stage update: 20 float64 operations a value and one integer sum, about 33 in the
+// per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage).  s_old and s_out start
+// at the launch's first row, s_new at row 0.
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
                                                               uint32_t first, uint32_t n_all, TransportScalars p,
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
 }
 
 // per value: horizontal upwind update and scale sums, then the limiter factors.  Three integer
-// sums and 13 float64 operations a value, about 65 with the comparisons and divisions of the
+// sums and 17 float64 operations a value, about 65 with the comparisons and divisions of the
 // per-cell loop (913 -> 256 us at 40962 x 55 x 3).
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
