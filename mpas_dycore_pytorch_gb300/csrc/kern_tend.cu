@@ -52,9 +52,11 @@ MPASG_D double cam_kdiff(double kd, const TendScalars& p, uint32_t k, int L) {
 // (k_acoustic_edges with small_step 1)
 template <typename T>
 MPASG_D void complete_tend_u(const mpasg_fields& f, size_t i, T tu, const TendScalars& p) {
-  f.tend_u[i] = f64(tu);
+  const double stored = f64(tu);
+  f.tend_u[i] = stored;
   if (p.first_dts > 0.0) {
-    const double rup = f64(cv<T>(p.first_dts) * tu);
+    // of the stored value: a float32 beyond the normal range does not come back from it as it was
+    const double rup = f64(cv<T>(p.first_dts) * cv<T>(stored));
     f.ru_p[i] = rup;
     f.ruAvg[i] = rup;
     if (sizeof(T) == sizeof(double)) p.first_flux[i] = rup * f.theta_edge_save[i];

@@ -8,6 +8,7 @@ import ctypes as C
 import hashlib
 
 import pytest
+import torch
 
 from gpu_helpers import need_gpu
 
@@ -132,3 +133,24 @@ def test_acoustic_stage(case):
     assert model.check_finite() == 0
     digests.append(_digest(model.export()))
     assert digests == STAGES[case].split()
+
+
+# a step from rest whose u tendencies lie about the smallest normal float32 (those below it are
+# kept as zero, and so the substeps take them)
+TINY_STEP = "5f47b54a917551f9"
+
+
+def test_tendencies_about_the_smallest_normal():
+    need_gpu()
+    model = _model(0.0, False, config_horiz_mixing="2d_fixed")  # (without mixing: its coefficients are zero)
+    f = model.state.f
+    for k in ("u", "v", "ru", "w", "rw", "rho_p", "rtheta_p", "divergence", "vorticity", "ke", "pv_edge"):
+        f[k].zero_()
+    base = (f["rtheta_base"][:-1] / f["theta_m"][:-1])  # rho_zz of the base state for this theta
+    f["rho_zz"][:-1].copy_(base)
+    n = f["pressure_p"].numel()
+    k = torch.arange(n, dtype=torch.float64, device="cuda") % 41
+    f["pressure_p"].copy_((2.0 ** (-110.0 + k % 7) * (1.0 + k)).view_as(f["pressure_p"]))
+    model.step()
+    assert 0.0 < f["ru"].abs().max().item() < 1e-20
+    assert _digest(model.export()) == TINY_STEP

@@ -32,17 +32,22 @@ def _model(nlev, tracers, level=2):
     return model
 
 
-@pytest.mark.parametrize("limit", [1, 3000])  # one row a launch; a few, the last launch shorter
-@pytest.mark.parametrize("nlev,tracers", [(4, 1), (13, 3), (26, 8)])
-def test_several_launches(tmp_path, limit, nlev, tracers):
+@pytest.fixture(scope="module", params=[1, 3000])  # one row a launch; a few, the last launch shorter
+def few(request, tmp_path_factory):
+    """The transport's entry points, built with that many threads a launch."""
     need_gpu()
     from mpas_dycore_pytorch_gb300 import build
-    stub, so = tmp_path / "count.cu", tmp_path / "libtransport.so"
+    d = tmp_path_factory.mktemp("transport")
+    stub, so = d / "count.cu", d / "libtransport.so"
     stub.write_text("void mpasg_count_launch() {}\n")
-    flags = build._flags((f"-DMPASG_MAX_THREADS={limit}",))
+    flags = build._flags((f"-DMPASG_MAX_THREADS={request.param}",))
     subprocess.run([build.nvcc_path(), *flags, "-shared", "-o", str(so), str(build.CSRC / "kern_transport.cu"),
                     str(stub)], check=True)
-    few = C.CDLL(str(so))
+    return C.CDLL(str(so))
+
+
+@pytest.mark.parametrize("nlev,tracers", [(4, 1), (13, 3), (26, 8)])
+def test_several_launches(few, nlev, tracers):
     model = _model(nlev, tracers)
     model.step()
     f = model.state.f
