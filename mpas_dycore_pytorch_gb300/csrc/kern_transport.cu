@@ -49,10 +49,10 @@ __global__ void k_pattern_c(mpasg_mesh m, FastDiv fl, int S, const double* __res
 // (fixdot.cuh), comparisons, minima and clamps on the integer side too (each would take a
 // float64 slot).
 // A launch numbers its (row, value) threads in 32 bits and divides by FastDiv, which holds below
-// 2^31: rows that reach it are taken in several launches.  A launch gets its first row and, for
-// the fields its threads index by their own number, pointers to that row (a 64-bit index in the
-// thread instead cost the monotone stage at 40962 x 55 x 3 0.6 %); gathers by row are 64 bits
-// wide.  (A build may lower the limit to test the split.)
+// 2^31: rows that reach it are taken in several launches, each of which gets what it indexes by
+// its rows as pointers to its first one (cells_from, edges_from; offsets added in the thread cost
+// the explicit stage at 10242 x 41 x 3 2 %).  Gathers over all rows are 64 bits wide.  (A build may
+// lower the limit to test the split.)
 #ifndef MPASG_MAX_THREADS
 #define MPASG_MAX_THREADS (0x7fffffffu - kBlock)
 #endif
@@ -68,6 +68,43 @@ int launch_rows(int n, uint32_t width, Launch launch) {
     if (most > n - first) break;  // (first + most may pass the last int)
   }
   return MPASG_OK;
+}
+
+// the mesh and the fields the cells' kernels index by cell, from a cell on
+mpasg_mesh cells_from(const mpasg_mesh& m, size_t first) {
+  mpasg_mesh g = m;
+  g.nEdgesOnCell += first;
+  g.edgesOnCell += first * m.maxEdges;
+  g.edgesOnCell_sign += first * m.maxEdges;
+  g.cellsOnCell += first * m.maxEdges;
+  g.invAreaCell += first;
+  return g;
+}
+mpasg_fields cells_from(const mpasg_mesh& m, const mpasg_fields& f, int S, size_t first) {
+  const size_t L = m.nVertLevels, row = first * L * S;
+  mpasg_fields g = f;
+  g.wwAvg += first * (L + 1);
+  g.rho_zz += first * L;
+  g.rho_zz_old_split += first * L;
+  g.rho_int += first * L;
+  g.wflux += first * (L + 1) * S;
+  g.rows += row;
+  g.scale_in += row;
+  g.scale_out += row;
+  g.s_max += row;
+  g.s_min += row;
+  return g;
+}
+// the mesh the edges' kernels index by edge, from an edge on
+mpasg_mesh edges_from(const mpasg_mesh& m, size_t first) {
+  mpasg_mesh g = m;
+  g.nAdvCellsForEdge += first;
+  g.advCellsForEdge += first * m.nAdvMax;
+  g.adv_coefs_p += first * m.nAdvMax;
+  g.adv_coefs_m += first * m.nAdvMax;
+  g.dvEdge += first;
+  g.cellsOnEdge += 2 * first;
+  return g;
 }
 
 struct TransportScalars {
@@ -103,8 +140,8 @@ MPASG_D void store_edge_flux(const mpasg_mesh& m, uint32_t e, uint32_t row, uint
 }
 
 template <int N, bool MONO>
-__global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t first,
-                                                         uint32_t n_all, double dt, const double* __restrict__ uh,
+__global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDiv fh, FastDiv fs, uint32_t n_all,
+                                                         uint32_t half, double dt, const double* __restrict__ uh,
                                                          const double* __restrict__ q,
                                                          const double* __restrict__ s_old, double* __restrict__ out,
                                                          double* __restrict__ out2) {
@@ -112,11 +149,11 @@ __global__ void __launch_bounds__(kBlock, 5) k_edge_flux_fx(mpasg_mesh m, FastDi
   const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
   const uint32_t e0 = fh.div(i0), e1 = fh.div(min(i0 + kBlock, n_all) - 1u);
-  adv::load<N>(m, first + e0, e1 - e0 + 1, s_w);
+  adv::load<N>(m, e0, e1 - e0 + 1, s_w);
   __syncthreads();
   if (i >= n_all) return;
-  const uint32_t er = fh.div(i), e = first + er, a = i - er * fh.d, b = a + fh.d;
-  const fx::Weight* w = s_w + (er - e0) * (2 * N);
+  const uint32_t e = fh.div(i), a = i - e * half, b = a + half;
+  const fx::Weight* w = s_w + (e - e0) * (2 * N);
   double x[N], acc;
   const double ua = uh[(size_t)e * L + fs.div(a)], dvdt = MONO ? m.dvEdge[e] * dt : 0.0;
   const bool back = __double2hiint(ua) < 0;
@@ -141,22 +178,23 @@ int launch_edge_flux_fx(const mpasg_mesh* m, int S, double dt, const double* uh,
   const auto run = [&](auto kernel, int slots) -> int {
     if (!allow_smem(kernel, smem * slots)) return MPASG_E_CUDA;
     return launch_rows(m->nEdges, half, [&](uint32_t first, uint32_t n) {
-      kernel<<<nblocks((long long)n * half), kBlock, smem * slots, s>>>(*m, FastDiv(half), FastDiv(S), first, n * half,
-                                                                        dt, uh, q, s_old, out, out2);
+      const size_t L = m->nVertLevels, at = first * L * S;
+      kernel<<<nblocks((long long)n * half), kBlock, smem * slots, s>>>(edges_from(*m, first), FastDiv(half), FastDiv(S),
+                                                                        n * half, half, dt, uh + first * L, q, s_old,
+                                                                        out + at, out2 ? out2 + at : nullptr);
     });
   };
   return m->nAdvMax <= 10 ? run(k_edge_flux_fx<10, MONO>, 10) : run(k_edge_flux_fx<14, MONO>, 14);
 }
 
-// the place of a launch's thread i in a (cell, level, scalar) row
+// the thread's place in a (cell, level, scalar) row
 struct CellRow {
   uint32_t c, r, k, s;
 };
-MPASG_D CellRow cell_row(uint32_t i, uint32_t first, const FastDiv& fr, const FastDiv& fs) {
+MPASG_D CellRow cell_row(uint32_t i, uint32_t row, const FastDiv& fr, const FastDiv& fs) {
   CellRow t;
-  const uint32_t cr = fr.div(i);
-  t.c = first + cr;
-  t.r = i - cr * fr.d;
+  t.c = fr.div(i);
+  t.r = i - t.c * row;
   t.k = fs.div(t.r);
   t.s = t.r - t.k * fs.d;
   return t;
@@ -178,11 +216,10 @@ MPASG_D double interface_value(const double* __restrict__ q, uint32_t S, double 
 }
 
 // explicit stage update: 20 float64 operations a value and one integer sum, about 33 in the
-// per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage).  s_old and s_out start
-// at the launch's first row, s_new at row 0.
+// per-cell loop over the scalars (40962 x 55 x 3: 380 -> 283 us a stage)
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
-                                                              uint32_t first, uint32_t n_all, TransportScalars p,
+                                                              uint32_t n_all, TransportScalars p,
                                                               const double* __restrict__ s_old,
                                                               const double* __restrict__ s_new,
                                                               double* __restrict__ s_out) {
@@ -190,7 +227,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, m
   __shared__ double s_wd[kBlock];
   const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
-  const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
+  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   const bool active = i < n_all;
   CellRow t{c0, 0, 0, 0};
@@ -203,7 +240,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_scalars_update_fx(mpasg_mesh m, m
   };
   double lo = 0.0;
   if (active) {
-    t = cell_row(i, first, fr, fs);
+    t = cell_row(i, row, fr, fs);
     lo = flux_at(t.k);
   }
   s_wd[threadIdx.x] = lo;
@@ -238,9 +275,9 @@ __global__ void k_mono_density_fx(mpasg_mesh m, mpasg_fields f, FastDiv fl, doub
 // (735 -> 273 us at 40962 x 55 x 3, and 40 us for the density).
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
-                                                            uint32_t first, uint32_t n_all, TransportScalars p,
+                                                            uint32_t n_all, TransportScalars p,
+                                                            const double* __restrict__ so_all,
                                                             const double* __restrict__ so,
-                                                            const double* __restrict__ so_own,
                                                             const double* __restrict__ sn) {
   __shared__ double s_wm[kBlock], s_fu[kBlock];
   const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
@@ -259,7 +296,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
   };
   double wm_lo = 0.0, fu_lo = 0.0;
   if (active) {
-    t = cell_row(i, first, fr, fs);
+    t = cell_row(i, row, fr, fs);
     fluxes(t.k, &wm_lo, &fu_lo);
   }
   s_wm[threadIdx.x] = wm_lo;
@@ -277,27 +314,27 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
   }
   if (t.k >= 1) f.wflux[((size_t)t.c * (L + 1) + t.k) * S + t.s] = wm_lo;
   // bounds over the column's neighbours and the adjacent cells
-  const double here = so_own[i];
+  const double here = so[i];
   int64_t kmax = fx::order_key(here), kmin = kmax;
   auto bound = [&](double x) {
     const int64_t q = fx::order_key(x);
     kmax = q > kmax ? q : kmax;
     kmin = q < kmin ? q : kmin;
   };
-  if (t.k >= 1) bound(so_own[i - S]);
-  if (t.k + 1 < L) bound(so_own[i + S]);
+  if (t.k >= 1) bound(so[i - S]);
+  if (t.k + 1 < L) bound(so[i + S]);
   const size_t oc = (size_t)t.c * m.maxEdges;
   const int n = m.nEdgesOnCell[t.c];
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     if (j < n) {
       const int nb = m.cellsOnCell[oc + j];
-      if (nb < m.nCells) bound(so[(size_t)nb * row + t.r]);
+      if (nb < m.nCells) bound(so_all[(size_t)nb * row + t.r]);
     }
   }
   for (int j = N; j < n; ++j) {
     const int nb = m.cellsOnCell[oc + j];
-    if (nb < m.nCells) bound(so[(size_t)nb * row + t.r]);
+    if (nb < m.nCells) bound(so_all[(size_t)nb * row + t.r]);
   }
   double smax = fx::from_order_key(kmax), smin = fx::from_order_key(kmin);
   if (!(fx::is_finite(smax) && fx::is_finite(smin))) {  // a NaN among them: left out, as fmax / fmin do
@@ -306,11 +343,11 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
       smax = fmax(smax, x);
       smin = fmin(smin, x);
     };
-    if (t.k >= 1) wide(so_own[i - S]);
-    if (t.k + 1 < L) wide(so_own[i + S]);
+    if (t.k >= 1) wide(so[i - S]);
+    if (t.k + 1 < L) wide(so[i + S]);
     for (int j = 0; j < n; ++j) {
       const int nb = m.cellsOnCell[oc + j];
-      if (nb < m.nCells) wide(so[(size_t)nb * row + t.r]);
+      if (nb < m.nCells) wide(so_all[(size_t)nb * row + t.r]);
     }
   }
   const double rd = m.rdnw[t.k];
@@ -327,15 +364,15 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_a_fx(mpasg_mesh m, mpa
 // per-cell loop (913 -> 256 us at 40962 x 55 x 3).
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
-                                                            uint32_t first, uint32_t n_all) {
+                                                            uint32_t n_all) {
   extern __shared__ cellsum::Slot s_c[];
   const uint32_t L = (uint32_t)m.nVertLevels, row = L * fs.d;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
-  const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
+  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   __syncthreads();
   if (i >= n_all) return;
-  const CellRow t = cell_row(i, first, fr, fs);
+  const CellRow t = cell_row(i, row, fr, fs);
   const int n = m.nEdgesOnCell[t.c];
   const cellsum::Slot* s = s_c + (t.c - c0) * N;
   const double ia = m.invAreaCell[t.c], rint = f.rho_int[(size_t)t.c * L + t.k];
@@ -369,10 +406,10 @@ __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_b_fx(mpasg_mesh m, mpa
 }
 
 // per (edge, value): limited horizontal flux (stored in hflux)
-__global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint32_t first, uint32_t n_all) {
+__global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint32_t n_all) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_all) return;
-  const uint32_t er = fr.div(i), e = first + er, r = i - er * fr.d;
+  const uint32_t e = fr.div(i), r = i - e * fr.d;
   const double ft = f.flux_tmp[i];
   const uint32_t back = __double2hiint(ft) < 0 ? 1u : 0u;
   const size_t from = (size_t)m.cellsOnEdge[2 * e + back] * fr.d + r;
@@ -383,16 +420,15 @@ __global__ void k_mono_edges_b_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, uint
 // per value: limited horizontal and vertical fluxes, positivity
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_mono_cells_c_fx(mpasg_mesh m, mpasg_fields f, FastDiv fr, FastDiv fs,
-                                                            uint32_t first, uint32_t n_all,
-                                                            double* __restrict__ s_out) {
+                                                            uint32_t n_all, double* __restrict__ s_out) {
   extern __shared__ cellsum::Slot s_c[];
   const uint32_t L = (uint32_t)m.nVertLevels, S = fs.d, row = L * S;
   const uint32_t i0 = blockIdx.x * kBlock, i = i0 + threadIdx.x;
-  const uint32_t c0 = first + fr.div(i0), c1 = first + fr.div(min(i0 + kBlock, n_all) - 1u);
+  const uint32_t c0 = fr.div(i0), c1 = fr.div(min(i0 + kBlock, n_all) - 1u);
   cellsum::load<N>(m, c0, c1 - c0 + 1, s_c);
   __syncthreads();
   if (i >= n_all) return;
-  const CellRow t = cell_row(i, first, fr, fs);
+  const CellRow t = cell_row(i, row, fr, fs);
   const double* wf = f.wflux + ((size_t)t.c * (L + 1) + t.k) * S + t.s;
   auto limited = [&](double wm, uint32_t below, uint32_t above) {  // an upward flux leaves `below`
     const bool down = __double2hiint(wm) < 0;
@@ -731,9 +767,10 @@ int launch_scalars_fx(const mpasg_mesh* m, const mpasg_fields& g, const Transpor
   if (rc != MPASG_OK) return rc;
   const size_t smem = cellsum::max_cells(row) * N * sizeof(cellsum::Slot);
   return launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
+    const size_t at = (size_t)first * row;
     k_scalars_update_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(
-        *m, g, FastDiv(row), FastDiv(S), first, n * row, p, g.scalars_init + (size_t)first * row, g.scalars_a,
-        g.scalars_b + (size_t)first * row);
+        cells_from(*m, first), cells_from(*m, g, S, first), FastDiv(row), FastDiv(S), n * row, p, g.scalars_init + at,
+        g.scalars_a + at, g.scalars_b + at);
   });
 }
 
@@ -747,38 +784,28 @@ int launch_scalars_mono_fx(const mpasg_mesh* m, const mpasg_fields* f, const Tra
   if (rc != MPASG_OK) return rc;
   k_mono_density_fx<<<nblocks((long long)m->nCells * L), kBlock, 0, s>>>(*m, *f, FastDiv(L), p.dt);
   MPASG_LAUNCH_CHECK();
-  // the fields a launch's threads index by their own number, from its first row
-  const auto own_cells = [&](size_t at) {
-    mpasg_fields g = *f;
-    g.rows += at;
-    g.scale_in += at;
-    g.scale_out += at;
-    g.s_max += at;
-    g.s_min += at;
-    return g;
-  };
   rc = launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
     const size_t at = (size_t)first * row;
     k_mono_cells_a_fx<N><<<nblocks((long long)n * row), kBlock, 0, s>>>(
-        *m, own_cells(at), fr, fs, first, n * row, p, f->scalars_init, f->scalars_init + at, f->scalars_a);
+        cells_from(*m, first), cells_from(*m, *f, S, first), fr, fs, n * row, p, f->scalars_init, f->scalars_init + at,
+        f->scalars_a + at);
   });
   if (rc != MPASG_OK) return rc;
   rc = launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
-    k_mono_cells_b_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, own_cells((size_t)first * row), fr, fs,
-                                                                           first, n * row);
+    k_mono_cells_b_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(
+        cells_from(*m, first), cells_from(*m, *f, S, first), fr, fs, n * row);
   });
   if (rc != MPASG_OK) return rc;
   rc = launch_rows(m->nEdges, row, [&](uint32_t first, uint32_t n) {
     mpasg_fields g = *f;
     g.flux_tmp += (size_t)first * row;
     g.hflux += (size_t)first * row;
-    k_mono_edges_b_fx<<<nblocks((long long)n * row), kBlock, 0, s>>>(*m, g, fr, first, n * row);
+    k_mono_edges_b_fx<<<nblocks((long long)n * row), kBlock, 0, s>>>(edges_from(*m, first), g, fr, n * row);
   });
   if (rc != MPASG_OK) return rc;
   return launch_rows(m->nCells, row, [&](uint32_t first, uint32_t n) {
-    const size_t at = (size_t)first * row;
-    k_mono_cells_c_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(*m, own_cells(at), fr, fs, first, n * row,
-                                                                           f->scalars_b + at);
+    k_mono_cells_c_fx<N><<<nblocks((long long)n * row), kBlock, smem, s>>>(
+        cells_from(*m, first), cells_from(*m, *f, S, first), fr, fs, n * row, f->scalars_b + (size_t)first * row);
   });
 }
 
